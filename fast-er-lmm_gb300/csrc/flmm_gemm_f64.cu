@@ -2,6 +2,7 @@
 // (fasterlmm/io.py:257-265) and the eigenbasis rotations (fasterlmm/core.py:518, :629).  GB300's FP64 pipe is the
 // bound here, so a 64 x 64 register-blocked tile with 16-deep shared-memory stages is enough to keep it busy.
 #include "flmm_common.cuh"
+#include "flmm_oz64.cuh"
 
 using namespace flmm;
 
@@ -82,6 +83,54 @@ extern "C" int flmm_gemm_nt_f64(const double* A, int64_t lda, const double* B, i
     dim3 grid(ceil_div(Nr, BN), ceil_div(Mr, BM));
     k_gemm_f64<true, true><<<grid, NT, 0, as_stream(stream)>>>(A, lda, B, ldb, C, ldc, Mr, Nr, K, alpha, 0.0);
     return check_launch("k_gemm_f64<nt>");
+}
+
+namespace {
+
+// Rows of one operand digitised at a time: digit planes of at most 256 MB (16 bytes per element).
+int oz_block(int rows, int unit, int K) {
+    const size_t fit = (size_t(256) << 20) / (16 * static_cast<size_t>(K)) / unit * unit;
+    if (fit < static_cast<size_t>(unit)) return unit;
+    return fit < static_cast<size_t>(rows) ? static_cast<int>(fit) : rows;
+}
+
+}  // namespace
+
+extern "C" int flmm_gemm_nt_f64_tc_workspace_bytes(int Mr, int Nr, int K, size_t* bytes) {
+    FLMM_REQUIRE(bytes && Mr >= 0 && Nr >= 0 && K > 0, "flmm_gemm_nt_f64_tc_workspace_bytes: bad arguments");
+    *bytes = oz_operand_bytes(oz_block(Mr, kOzRowsA, K), K, 1, kOzRowsA) +
+             oz_operand_bytes(oz_block(Nr, kOzRowsB, K), K, 1, kOzRowsB) + 1024;
+    return FLMM_OK;
+}
+
+extern "C" int flmm_gemm_nt_f64_tc(const double* A, int64_t lda, const double* B, int64_t ldb, const double* D,
+                                   int64_t ldd, double* C, int64_t ldc, int Mr, int Nr, int K, void* work,
+                                   size_t work_bytes, void* stream) {
+    FLMM_REQUIRE(A && B && C && work && Mr >= 0 && Nr >= 0 && K > 0 && lda >= K && ldb >= K && ldc >= Nr &&
+                     (!D || ldd >= Nr),
+                 "flmm_gemm_nt_f64_tc: bad arguments");
+    size_t need = 0;
+    flmm_gemm_nt_f64_tc_workspace_bytes(Mr, Nr, K, &need);
+    if (work_bytes < need)
+        return fail(FLMM_ERR_WORKSPACE, "flmm_gemm_nt_f64_tc: need %zu bytes, got %zu", need, work_bytes);
+    if (Mr == 0 || Nr == 0) return FLMM_OK;
+    cudaStream_t st = as_stream(stream);
+    const int ra = oz_block(Mr, kOzRowsA, K), rb = oz_block(Nr, kOzRowsB, K);
+    char* wa = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(work) + 1023) / 1024 * 1024);
+    char* wb = wa + oz_operand_bytes(ra, K, 1, kOzRowsA);
+    for (int j0 = 0; j0 < Nr; j0 += rb) {
+        const OzOperand b = oz_carve(wb, Nr - j0 < rb ? Nr - j0 : rb, K, 1, kOzRowsB);
+        int rc = oz_digits(b, 0, B + j0 * ldb, ldb, false, st);
+        if (rc) return rc;
+        for (int i0 = 0; i0 < Mr; i0 += ra) {
+            const OzOperand a = oz_carve(wa, Mr - i0 < ra ? Mr - i0 : ra, K, 1, kOzRowsA);
+            if ((rc = oz_digits(a, 0, A + i0 * lda, lda, false, st))) return rc;
+            const OzProduct p{A + i0 * lda, lda, 0, B + j0 * ldb, ldb, 0, false, C + i0 * ldc + j0, ldc, 0,
+                              D ? D + i0 * ldd + j0 : nullptr, ldd};
+            if ((rc = oz_gemm(a, b, p, st))) return rc;
+        }
+    }
+    return FLMM_OK;
 }
 
 extern "C" int flmm_gram_f64(const double* Zt, int64_t ldzt, int M, int N, double beta, double* Gc, int64_t ldg,

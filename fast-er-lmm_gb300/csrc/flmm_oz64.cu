@@ -1,0 +1,536 @@
+// FP64 products on the FP16 tensor cores.
+//
+// GB300's FP64 pipe gives ~1.1 TFLOP/s, its FP16 tensor cores ~1,900, so a product C = A B^T of FP64 matrices is faster
+// as several exact FP16 products.  Method: the error-free splitting of Ozaki, Ogita, Oishi and Rump (Numer. Algorithms
+// 59, 2012) on tensor cores as in Mukunoki, Ozaki, Ogita and Imamura (ISC 2020), with the level sums kept as integers.
+// Every row is rounded once to 55 bits below its leading bit and written as eight balanced digits,
+//     x = 2^(e - 6) (d_0 + d_1 2^-7 + ... + d_7 2^-49),  -64 <= d_t <= 64,
+// e the binary exponent of the row's largest |x|.  Digits are exact in FP16; products of two digits are integers of at
+// most 12 bits.  Plane pairs (i, j) of equal level l = i + j share one FP32 accumulator in tensor memory; levels 0..7
+// are kept (36 pairs).  A level holds at most eight pairs, so its sum over a chunk of 512 terms is at most
+// 8 * 512 * 2^12 = 2^24 in magnitude: every accumulation is exact.  The epilogue converts the level sums to integers
+// and adds them into two 64-bit integers per output (levels 0..3 and 4..7), exactly, over all chunks, and rounds once:
+//     C = 2^(e_a + e_b - 61) (2^28 hi + lo).
+// What is lost is the rounding to 55 bits and the levels from 8 on (weight 2^-56 against the row maxima).  For rows
+// whose largest entry is a few times their rms this is several times smaller than the rounding of an FP64 sum of K
+// terms (~0.4 * 2^-53 * K times the rms product; measured against exact sums in tests/test_gpu_oz64.py).  The loss
+// grows with max/rms of both rows, so every tile of rows carries its largest ratio; a tile pair whose product of
+// ratios exceeds quality_limit(K), and any row that is not finite or whose exponent is out of range, is left to
+// k_marked_f64, which forms those tiles on the FP64 pipe as before.
+//
+// Kernel: persistent, one CTA per SM; tiles of 128 A rows x 64 B rows, 8 levels x 64 columns = all of tensor memory.
+// Warp 0 issues the TMA loads (a stage is 32 deep: 8 x 8 KB + 8 x 4 KB = 96 KB, two stages), warp 1 the 72 MMAs of a
+// stage (M = 128, N = 64, K = 16); A's plane stays in the tensor core's collector while the pairs that share it are
+// issued, because operand reads (6 KB per 32-cycle MMA) would otherwise exceed shared memory's 128 B per cycle.  Warps
+// 2..17 drain the levels; tensor memory is handed back before the outputs are rounded and stored, so only the drain
+// itself (8 x 64 columns per 512 terms) interrupts the MMAs.
+#include <cuda.h>
+#include <math.h>
+
+#include <cstring>
+#include <mutex>
+
+#include "flmm_oz64.cuh"
+#include "flmm_tc.cuh"
+
+using namespace flmm;
+using namespace flmm::tc;
+
+namespace {
+
+constexpr int kLevels = 8;
+constexpr int kChunk = 512;  // terms of one exact accumulation
+constexpr int kBK = 32;      // depth of one stage (64-byte rows, 64-byte swizzle)
+constexpr int kATile = kOzRowsA * kBK * 2;
+constexpr int kBTile = kOzRowsB * kBK * 2;
+constexpr int kStageBytes = kOzPlanes * (kATile + kBTile);
+constexpr int kStages = 2;
+constexpr uint32_t kSBO = 8u * kBK * 2u;
+constexpr uint32_t kSwizzle64 = 4u;
+constexpr int kTmemCols = kLevels * kOzRowsB;
+constexpr int kEpiWarps = 16;
+constexpr int kThreads = 64 + 32 * kEpiWarps;
+constexpr int kEpiCols = kOzRowsB / (kEpiWarps / 4);  // output columns per epilogue thread
+constexpr int kSmemBytes = kStages * kStageBytes + 256 + 1024;
+constexpr int kMaxExp = 450;  // |e| beyond this: the scale 2^(e_a + e_b - 61) could leave FP64's range
+static_assert(kTmemCols == 512 && kSmemBytes <= 227 * 1024 && kEpiCols == 16, "budgets");
+
+// Largest product of two tiles' max/rms ratios that the digits take.  The dropped levels and the rounding leave
+// ~8e-16 sqrt(K / 1000) r_a r_b (in units of the rms product), an FP64 sum ~4.5e-14 K / 1000: equal at 57 sqrt(K / 1000).
+__host__ __device__ inline float quality_limit(int K) { return 1.8f * sqrtf(static_cast<float>(K)); }
+
+struct OzMaps {
+    CUtensorMap a, b;
+};
+
+struct OzArgs {
+    int Ma, Nb, K, batches;
+    int tiles_i, tiles_m;
+    const int* ea;
+    const int* eb;
+    const float* qa;
+    const float* qb;
+    float limit[2];  // per batch
+    double* C;
+    int64_t ldc, c_stride;
+    const double* D;
+    int64_t ldd;
+    int* err;
+};
+
+// ---- digits ---------------------------------------------------------------------------------------------------
+
+// One warp per row.  Pass 1: the row's largest |x| as its bit pattern (integer maximum); pass 2: the 55-bit integer
+// of every element, its digits by integer shifts, packed two elements to a word (1536 + d is exact in FP16 with unit
+// spacing, so subtracting 1536 leaves the digit).  16 bytes written per 8 read: bandwidth-bound.
+template <bool SQ>
+__global__ void __launch_bounds__(256)
+k_digits64(const double* __restrict__ X, int64_t ldx, int rows, int K, __half* __restrict__ planes, int64_t ldp,
+           int64_t plane_stride, int* __restrict__ expo, float* __restrict__ qual, int tile_rows) {
+    const int lane = threadIdx.x & 31;
+    const int64_t j = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5;
+    if (j >= rows) return;
+    const double* x = X + j * ldx;
+    unsigned long long mb = 0;
+    for (int n = lane; n < K; n += 32) {
+        double v = x[n];
+        if (SQ) v = mul_rn(v, v);
+        const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(v)) & 0x7fffffffffffffffull;
+        mb = b > mb ? b : mb;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long b = __shfl_xor_sync(0xffffffffu, mb, o);
+        mb = b > mb ? b : mb;
+    }
+    const int e = mb == 0 ? 0 : static_cast<int>(mb >> 52) - 1022;  // max = f 2^e, f in [0.5, 1)
+    const bool bad = e > kMaxExp || e < -kMaxExp;                   // includes infinities, NaN and denormals
+    const double up = __longlong_as_double(static_cast<long long>(1023 + 55 - (bad ? 0 : e)) << 52);
+    __half* out = planes + j * ldp;
+    float ss = 0.0f;
+    for (int n = 2 * lane; n < K; n += 64) {
+        long long v[2] = {0, 0};
+        if (!bad) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (n + h >= K) continue;
+                double y = x[n + h];
+                if (SQ) y = mul_rn(y, y);
+                v[h] = __double2ll_rn(y * up);
+                const float t = static_cast<float>(static_cast<int>(v[h] >> 32)) * 0x1p-23f;
+                ss = fmaf(t, t, ss);
+            }
+        }
+#pragma unroll
+        for (int t = kOzPlanes - 1; t >= 0; --t) {
+            int d[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (t > 0) {
+                    d[h] = static_cast<int>((static_cast<unsigned>(v[h]) + 64u) & 127u) - 64;
+                    v[h] = (v[h] - d[h]) >> 7;
+                } else {
+                    d[h] = static_cast<int>(v[h]);
+                }
+            }
+            const unsigned word = (static_cast<unsigned>(0x6600 + d[1]) << 16) | static_cast<unsigned>(0x6600 + d[0]);
+            const __half2 p = __hsub2(*reinterpret_cast<const __half2*>(&word), __half2half2(__ushort_as_half(0x6600)));
+            *reinterpret_cast<__half2*>(out + t * plane_stride + n) = p;
+        }
+    }
+    ss = warp_sum(ss);
+    if (lane == 0) {
+        expo[j] = bad ? 0 : e;
+        const float top = mb == 0 ? 1.0f : static_cast<float>(__longlong_as_double((mb & 0xfffffffffffffull) | (1022ull << 52)));
+        const float q = bad ? INFINITY : (mb == 0 ? 1.0f : fmaxf(1.0f, top * sqrtf(static_cast<float>(K) / ss)));
+        atomicMax(reinterpret_cast<int*>(qual) + j / tile_rows, __float_as_int(q));
+    }
+}
+
+__global__ void k_zero_f32(float* __restrict__ x, int n) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) x[i] = 0.0f;
+}
+
+// ---- the product ------------------------------------------------------------------------------------------------
+
+// Tile t of the schedule: groups of at most kGroup A blocks, inside a group the A block fastest, so that the ~152
+// tiles in flight share few A and B blocks in L2.
+constexpr int kGroup = 12;
+
+struct Tile {
+    int b, ti, tm;
+};
+
+__device__ __forceinline__ Tile tile_at(int t, int tiles_i, int tiles_m) {
+    const int per = tiles_i * tiles_m;
+    Tile r;
+    r.b = t / per;
+    int rem = t - r.b * per;
+    const int g = rem / (kGroup * tiles_m);
+    rem -= g * kGroup * tiles_m;
+    const int gi = min(kGroup, tiles_i - g * kGroup);
+    r.tm = rem / gi;
+    r.ti = g * kGroup + rem - r.tm * gi;
+    return r;
+}
+
+__device__ __forceinline__ bool tile_good(const OzArgs& a, const Tile& t) {
+    // (an infinite quality makes the product infinite: qualities are at least 1, or 0 for tiles past the rows)
+    return a.qa[t.b * a.tiles_i + t.ti] * a.qb[t.b * a.tiles_m + t.tm] <= a.limit[t.b];
+}
+
+// MMA whose A operand is read into the collector (fill), taken from it (use), or taken for the last time.
+enum class Collect { kFill, kUse, kLast, kNone };
+
+template <Collect C>
+__device__ __forceinline__ void mma_collect(uint32_t d, uint64_t ad, uint64_t bd, uint32_t idesc, uint32_t acc) {
+    if constexpr (C == Collect::kFill)
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                     "tcgen05.mma.cta_group::1.kind::f16.collector::a::fill [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
+                     "l"(ad), "l"(bd), "r"(idesc), "r"(acc)
+                     : "memory");
+    else if constexpr (C == Collect::kUse)
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                     "tcgen05.mma.cta_group::1.kind::f16.collector::a::use [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
+                     "l"(ad), "l"(bd), "r"(idesc), "r"(acc)
+                     : "memory");
+    else if constexpr (C == Collect::kLast)
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                     "tcgen05.mma.cta_group::1.kind::f16.collector::a::lastuse [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
+                     "l"(ad), "l"(bd), "r"(idesc), "r"(acc)
+                     : "memory");
+    else
+        mma_f16(d, ad, bd, idesc, acc);
+}
+
+template <int I, int J>
+__device__ __forceinline__ void mma_pair(uint32_t tmem, uint32_t sbase, int kk, bool first, uint32_t idesc) {
+    constexpr int kLastJ = kLevels - 1 - I;
+    constexpr Collect c = kLastJ == 0 ? Collect::kNone
+                          : J == 0    ? Collect::kFill
+                          : J == kLastJ ? Collect::kLast
+                                        : Collect::kUse;
+    const uint64_t ad = smem_desc(sbase + I * kATile, kSBO, kSwizzle64) + 2u * kk;
+    const uint64_t bd = smem_desc(sbase + kOzPlanes * kATile + J * kBTile, kSBO, kSwizzle64) + 2u * kk;
+    mma_collect<c>(tmem + static_cast<uint32_t>((I + J) * kOzRowsB), ad, bd, idesc, (first && I == 0) ? 0u : 1u);
+    if constexpr (J < kLastJ) mma_pair<I, J + 1>(tmem, sbase, kk, first, idesc);
+    else if constexpr (I < kOzPlanes - 1) mma_pair<I + 1, 0>(tmem, sbase, kk, first, idesc);
+}
+
+__global__ void __launch_bounds__(kThreads, 1) k_oz64(const __grid_constant__ OzMaps maps, const OzArgs args) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStages * kStageBytes);
+    uint64_t* full = bars;                  // [kStages]
+    uint64_t* empty = bars + kStages;       // [kStages]
+    uint64_t* acc_full = empty + kStages;   // chunk accumulated (MMA -> epilogue)
+    uint64_t* acc_empty = acc_full + 1;     // chunk drained (epilogue -> MMA)
+    uint64_t* final_bar = acc_empty + 1;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(final_bar + 1);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n_tiles = args.batches * args.tiles_i * args.tiles_m;
+    const int n_kb = (args.K + kBK - 1) / kBK;
+    constexpr int kChunkKb = kChunk / kBK;
+    constexpr uint32_t idesc = idesc_f16_f32(kOzRowsA, kOzRowsB);
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kStages; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        mbar_init(acc_full, 1);
+        mbar_init(acc_empty, kEpiWarps);
+        mbar_init(final_bar, 1);
+        fence_barrier_init();
+    }
+    if (warp == 0 && lane == 0) {
+        tma_prefetch_desc(&maps.a);
+        tma_prefetch_desc(&maps.b);
+    }
+    if (warp == 1) {
+        tmem_alloc(tmem_slot, kTmemCols);
+        tmem_relinquish();
+    }
+    fence_before_sync();
+    __syncthreads();
+    fence_after_sync();
+    const uint32_t tmem_base = *tmem_slot;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            int stage = 0;
+            uint32_t phase = 0;
+            bool armed[kStages] = {};
+            uint32_t armed_phase[kStages] = {};
+            bool ok = true;
+            for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
+                const Tile tl = tile_at(t, args.tiles_i, args.tiles_m);
+                if (!tile_good(args, tl)) continue;
+                const int ya = tl.b * args.Ma + tl.ti * kOzRowsA, yb = tl.b * args.Nb + tl.tm * kOzRowsB;
+                for (int kb = 0; kb < n_kb; ++kb) {
+                    if (!mbar_wait(&empty[stage], phase ^ 1u, args.err, 21)) { ok = false; break; }
+                    mbar_arrive_expect_tx(&full[stage], kStageBytes);
+                    armed[stage] = true;
+                    armed_phase[stage] = phase;
+                    uint8_t* base = smem + stage * kStageBytes;
+                    const int x = kb * kBK;
+#pragma unroll
+                    for (int p = 0; p < kOzPlanes; ++p) {
+                        tma_load_2d(base + p * kATile, &maps.a, x, p * args.batches * args.Ma + ya, &full[stage]);
+                        tma_load_2d(base + kOzPlanes * kATile + p * kBTile, &maps.b, x,
+                                    p * args.batches * args.Nb + yb, &full[stage]);
+                    }
+                    if (++stage == kStages) { stage = 0; phase ^= 1u; }
+                }
+            }
+            for (int s = 0; s < kStages; ++s)
+                if (armed[s]) mbar_drain(&full[s], armed_phase[s]);
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            int stage = 0;
+            uint32_t phase = 0, tphase = 0;
+            bool ok = true;
+            for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
+                if (!tile_good(args, tile_at(t, args.tiles_i, args.tiles_m))) continue;
+                for (int kb = 0; kb < n_kb && ok; ++kb) {
+                    const bool first = kb % kChunkKb == 0;
+                    if (first) {
+                        if (!mbar_wait(acc_empty, tphase ^ 1u, args.err, 22)) { ok = false; break; }
+                        fence_after_sync();
+                    }
+                    if (!mbar_wait(&full[stage], phase, args.err, 23)) { ok = false; break; }
+                    fence_after_sync();
+                    const uint32_t sbase = smem_u32(smem + stage * kStageBytes);
+#pragma unroll 1
+                    for (int kk = 0; kk < kBK / 16; ++kk)
+                        mma_pair<0, 0>(tmem_base, sbase, kk, first && kk == 0, idesc);
+                    mma_commit(&empty[stage]);
+                    if (++stage == kStages) { stage = 0; phase ^= 1u; }
+                    if ((kb + 1) % kChunkKb == 0 || kb + 1 == n_kb) {
+                        mma_commit(acc_full);
+                        tphase ^= 1u;
+                    }
+                }
+            }
+            mma_commit(final_bar);
+            mbar_drain(final_bar, 0);
+        }
+    } else {
+        // warp w reads TMEM lanes 32 (w % 4) .. +31 (thread = one A row) and columns 16 ((w - 2) / 4) .. +15 of every
+        // level
+        const int q = warp & 3;
+        const int c0 = ((warp - 2) >> 2) * kEpiCols;
+        const uint32_t tl0 = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(c0);
+        uint32_t tphase = 0;
+        bool ok = true;
+        for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
+            const Tile tl = tile_at(t, args.tiles_i, args.tiles_m);
+            if (!tile_good(args, tl)) continue;
+            long long hi[kEpiCols], lo[kEpiCols];
+#pragma unroll
+            for (int c = 0; c < kEpiCols; ++c) hi[c] = lo[c] = 0;
+            for (int kb = 0; kb < n_kb; kb += kChunkKb) {
+                if (!mbar_wait(acc_full, tphase, args.err, 24)) { ok = false; break; }
+                fence_after_sync();
+                float v[kEpiCols];
+#pragma unroll
+                for (int l = 0; l < kLevels / 2; ++l) {
+                    tmem_ld16_wait(tl0 + static_cast<uint32_t>(l * kOzRowsB), v);
+#pragma unroll
+                    for (int c = 0; c < kEpiCols; ++c)
+                        hi[c] += static_cast<long long>(__float2int_rn(v[c])) * (1 << (7 * (kLevels / 2 - 1 - l)));
+                }
+#pragma unroll
+                for (int l = kLevels / 2; l < kLevels; ++l) {
+                    tmem_ld16_wait(tl0 + static_cast<uint32_t>(l * kOzRowsB), v);
+#pragma unroll
+                    for (int c = 0; c < kEpiCols; ++c)
+                        lo[c] += static_cast<long long>(__float2int_rn(v[c])) * (1 << (7 * (kLevels - 1 - l)));
+                }
+                fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(acc_empty);
+                tphase ^= 1u;
+            }
+            if (!ok) break;
+            const int i = tl.ti * kOzRowsA + q * 32 + lane;
+            if (i < args.Ma) {
+                const int ea = args.ea[tl.b * args.Ma + i];
+                const int m0 = tl.tm * kOzRowsB + c0;
+                const int* eb = args.eb + tl.b * args.Nb + m0;
+                double* out = args.C + tl.b * args.c_stride + static_cast<int64_t>(i) * args.ldc + m0;
+                const double* d = args.D ? args.D + static_cast<int64_t>(i) * args.ldd + m0 : nullptr;
+#pragma unroll
+                for (int c = 0; c < kEpiCols; ++c) {
+                    if (m0 + c < args.Nb) {
+                        const double s = __longlong_as_double(static_cast<long long>(1023 + ea + eb[c] - 61) << 52);
+                        const double v = fma(static_cast<double>(hi[c]), 0x1p28, static_cast<double>(lo[c])) * s;
+                        out[c] = d ? d[c] - v : v;
+                    }
+                }
+            }
+        }
+    }
+
+    fence_before_sync();
+    __syncthreads();
+    if (warp == 1) {
+        fence_after_sync();
+        tmem_dealloc(tmem_base, kTmemCols);
+    }
+}
+
+// ---- tiles left to the FP64 pipe ----------------------------------------------------------------------------------
+
+constexpr int kST = 64, kSK = 16, kSThreads = 256;
+
+// The 64 x 64 tiles of C whose digit tiles are not good, in FP64 (one block per tile; the others leave at once).
+__global__ void __launch_bounds__(kSThreads)
+k_marked_f64(const OzArgs args, const double* __restrict__ Xa, int64_t lda, int64_t xa_stride,
+             const double* __restrict__ Xb, int64_t ldb, int64_t xb_stride, int square_b1) {
+    const int b = blockIdx.z;
+    const int i0 = blockIdx.y * kST, j0 = blockIdx.x * kST;
+    if (tile_good(args, Tile{b, i0 / kOzRowsA, j0 / kOzRowsB})) return;
+    __shared__ double As[kSK][kST + 1];
+    __shared__ double Bs[kSK][kST + 1];
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const bool sq = square_b1 && b == 1;
+    const double* A = Xa + b * xa_stride;
+    const double* B = Xb + b * xb_stride;
+    double acc[4][4] = {};
+    for (int k0 = 0; k0 < args.K; k0 += kSK) {
+#pragma unroll
+        for (int l = 0; l < (kST * kSK) / kSThreads; ++l) {
+            const int t = tid + l * kSThreads, r = t / kSK, k = t % kSK;
+            const bool kin = k0 + k < args.K;
+            As[k][r] = (kin && i0 + r < args.Ma) ? A[static_cast<int64_t>(i0 + r) * lda + k0 + k] : 0.0;
+            const double v = (kin && j0 + r < args.Nb) ? B[static_cast<int64_t>(j0 + r) * ldb + k0 + k] : 0.0;
+            Bs[k][r] = sq ? mul_rn(v, v) : v;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kSK; ++k) {
+            double a[4], v[4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) a[r] = As[k][ty + 16 * r];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) v[c] = Bs[k][tx + 16 * c];
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) acc[r][c] = fma(a[r], v[c], acc[r][c]);
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const int i = i0 + ty + 16 * r;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const int j = j0 + tx + 16 * c;
+            if (i < args.Ma && j < args.Nb) {
+                double* o = args.C + b * args.c_stride + static_cast<int64_t>(i) * args.ldc + j;
+                *o = args.D ? args.D[static_cast<int64_t>(i) * args.ldd + j] - acc[r][c] : acc[r][c];
+            }
+        }
+    }
+}
+
+size_t align_up(size_t n) { return (n + 1023) / 1024 * 1024; }
+
+}  // namespace
+
+namespace flmm {
+
+size_t oz_operand_bytes(int rows, int K, int batches, int tile_rows) {
+    const size_t ldp = (static_cast<size_t>(K) + 7) / 8 * 8, n = static_cast<size_t>(rows) * batches;
+    const size_t tiles = static_cast<size_t>((rows + tile_rows - 1) / tile_rows) * batches;
+    return align_up(sizeof(__half) * kOzPlanes * n * ldp) + align_up(sizeof(int) * n) + align_up(sizeof(float) * tiles);
+}
+
+OzOperand oz_carve(void* base, int rows, int K, int batches, int tile_rows) {
+    OzOperand op;
+    op.ldp = (static_cast<int64_t>(K) + 7) / 8 * 8;
+    op.rows = rows;
+    op.K = K;
+    op.batches = batches;
+    op.tile_rows = tile_rows;
+    const size_t n = static_cast<size_t>(rows) * batches;
+    char* p = static_cast<char*>(base);
+    op.planes = reinterpret_cast<__half*>(p);
+    p += align_up(sizeof(__half) * kOzPlanes * n * op.ldp);
+    op.expo = reinterpret_cast<int*>(p);
+    p += align_up(sizeof(int) * n);
+    op.qual = reinterpret_cast<float*>(p);
+    return op;
+}
+
+int oz_digits(const OzOperand& op, int b, const double* X, int64_t ldx, bool square, cudaStream_t st) {
+    if (op.rows == 0) return FLMM_OK;
+    const int64_t off = static_cast<int64_t>(b) * op.rows;
+    const int64_t plane_stride = static_cast<int64_t>(op.batches) * op.rows * op.ldp;
+    float* qual = op.qual + static_cast<int64_t>(b) * op.tiles();
+    k_zero_f32<<<ceil_div(op.tiles(), 256), 256, 0, st>>>(qual, op.tiles());
+    int rc = check_launch("k_zero_f32");
+    if (rc) return rc;
+    auto* k = square ? k_digits64<true> : k_digits64<false>;
+    k<<<ceil_div(static_cast<int64_t>(op.rows) * 32, 256), 256, 0, st>>>(
+        X, ldx, op.rows, op.K, op.planes + off * op.ldp, op.ldp, plane_stride, op.expo + off, qual, op.tile_rows);
+    return check_launch("k_digits64");
+}
+
+int oz_gemm(const OzOperand& A, const OzOperand& B, const OzProduct& p, cudaStream_t st) {
+    if (A.rows == 0 || B.rows == 0) return FLMM_OK;
+    if (A.batches > 2 || A.batches != B.batches || A.K != B.K) return fail(FLMM_ERR_ARG, "oz_gemm: operands differ");
+    const int64_t ra = static_cast<int64_t>(A.rows) * A.batches * kOzPlanes;
+    const int64_t rb = static_cast<int64_t>(B.rows) * B.batches * kOzPlanes;
+    if (ra > 0x7fffffffLL || rb > 0x7fffffffLL) return fail(FLMM_ERR_ARG, "oz_gemm: too many rows for a TMA map");
+    OzMaps maps;
+    std::memset(&maps, 0, sizeof(maps));
+    int rc;
+    if ((rc = tc::make_map_f16(&maps.a, A.planes, static_cast<int>(ra), A.K, A.ldp, kBK, kOzRowsA))) return rc;
+    if ((rc = tc::make_map_f16(&maps.b, B.planes, static_cast<int>(rb), B.K, B.ldp, kBK, kOzRowsB))) return rc;
+    static std::once_flag once;
+    static cudaError_t attr_rc = cudaSuccess;
+    std::call_once(once, [] {
+        attr_rc = cudaFuncSetAttribute(k_oz64, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+    });
+    if (attr_rc != cudaSuccess) return fail(FLMM_ERR_CUDA, "k_oz64: %s", cudaGetErrorString(attr_rc));
+    int dev = 0, sm = 0;
+    FLMM_CUDA(cudaGetDevice(&dev));
+    FLMM_CUDA(cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev));
+    OzArgs a{};
+    a.err = device_err_flag(dev);
+    if (!a.err) return fail(FLMM_ERR_CUDA, "oz_gemm: cannot allocate the device error flag");
+    a.Ma = A.rows;
+    a.Nb = B.rows;
+    a.K = A.K;
+    a.batches = A.batches;
+    a.tiles_i = A.tiles();
+    a.tiles_m = B.tiles();
+    a.ea = A.expo;
+    a.eb = B.expo;
+    a.qa = A.qual;
+    a.qb = B.qual;
+    a.limit[0] = quality_limit(A.K);
+    // a sum of products of non-negative numbers grows with its length, and with it an FP64 sum's own rounding
+    a.limit[1] = p.square_b1 ? 4.0f * a.limit[0] : a.limit[0];
+    a.C = p.C;
+    a.ldc = p.ldc;
+    a.c_stride = p.c_stride;
+    a.D = p.D;
+    a.ldd = p.ldd;
+    const int64_t tiles = static_cast<int64_t>(a.batches) * a.tiles_i * a.tiles_m;
+    k_oz64<<<static_cast<int>(tiles < sm ? tiles : sm), kThreads, kSmemBytes, st>>>(maps, a);
+    if ((rc = check_launch("k_oz64"))) return rc;
+    const dim3 grid(ceil_div(B.rows, kST), ceil_div(A.rows, kST), a.batches);
+    k_marked_f64<<<grid, kSThreads, 0, st>>>(a, p.Xa, p.lda, p.xa_stride, p.Xb, p.ldb, p.xb_stride, p.square_b1);
+    return check_launch("k_marked_f64");
+}
+
+bool oz_worth(int64_t Mr, int64_t Nr, int64_t K) { return K >= 32 && Mr * Nr * K >= 20000000; }
+
+}  // namespace flmm

@@ -1,10 +1,13 @@
-// Plain FP64 form of the compat Wald scan (fasterlmm/core.py:601-671), fused: the two per-chromosome products
-// sWy = (w o UY)^T US and sWs = w^T (US o US) share one tile loop, and the epilogue (beta, var_beta, F, SE, SFVE,
-// the per-column genome max) runs on the accumulators in registers.  Nothing of size (P, Mc) is written except
-// the real columns' detail.
+// Plain FP64 form of the compat Wald scan (fasterlmm/core.py:601-671): the two per-chromosome products
+// sWy = (w o UY)^T US and sWs = w^T (US o US), then beta, var_beta, F, SE, SFVE and the per-column genome max.
+// The products are FP64 sums of Neff terms per test and bound by the FP64 pipe (1.08 TFLOP/s measured of ~1.25), so
+// where they are large they run on the tensor cores from exact digit planes (flmm_oz64.cu) in blocks of columns and
+// variants whose sums an epilogue kernel reads back (16 bytes per test); 1,100 columns x 4,096 variants x 995 with its
+// rotation: 23.9 -> 1.83 ms.  Small products stay in the fused FP64 tile kernel, which needs one launch.
 #include <math.h>
 
 #include "flmm_common.cuh"
+#include "flmm_oz64.cuh"
 
 using namespace flmm;
 
@@ -129,9 +132,140 @@ k_wald_f64(const double* __restrict__ W, const double* __restrict__ A1, const do
     }
 }
 
-size_t wald_ws(int P, int Neff) {
-    return sizeof(double) * (2 * static_cast<size_t>(P) * Neff + static_cast<size_t>(P)) + 512;
+// beta, F, SE and SFVE of one test from its two sums (fasterlmm/core.py:651-655, in the reference's operation order)
+struct Test {
+    double F, b, var_b, q, denom;
+};
+
+__device__ __forceinline__ Test wald_test(double swy, double sws, double rwr, double var_df) {
+    Test t;
+    t.denom = fmax(sws, kPosFloor);
+    t.b = swy / t.denom;
+    t.q = mul_rn(swy, swy);
+    const double rss = fmax(add_rn(rwr, -(t.q / t.denom)), kPosFloor);
+    t.var_b = (rss / var_df) / t.denom;
+    t.F = mul_rn(t.b, t.b) / t.var_b;
+    return t;
 }
+
+// Epilogue over the sums of a (Pc, Mc) block, G[0] = sWy and G[1] = sWs (pitch ldg, batch stride g_stride): a block
+// takes 32 columns x kFinM variants in tiles of 64, transposed through shared memory so that the reads run along the
+// variants and the detail stores along the columns.  Real columns get the full epilogue.  A permutation column needs its
+// largest F only, and F grows with q / denom, so its tests are ranked by cross-multiplication (three FP64 operations
+// instead of four divisions; GB300's FP64 pipe is the bound here) and one F is formed per thread; sums outside
+// 1e-100 .. 1e100, and NaN, take the full formula.
+constexpr int kFinP = 32, kFinTile = 64, kFinM = 256;
+
+__global__ void __launch_bounds__(256)
+k_wald_finish(const double* __restrict__ G, int64_t ldg, int64_t g_stride, const double* __restrict__ rWr,
+              double var_df, int P, int n_real, int Mc, const int64_t* __restrict__ rows, double* __restrict__ f,
+              double* __restrict__ beta, double* __restrict__ se, double* __restrict__ sfve, int64_t ldo,
+              double* __restrict__ max_F) {
+    __shared__ double sy[kFinP][kFinTile + 1];
+    __shared__ double ss[kFinP][kFinTile + 1];
+    __shared__ double red[8][kFinP];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int p0 = blockIdx.y * kFinP, p = p0 + lane;
+    const bool p_ok = p < P, real = p < n_real;
+    const double rwr = p_ok ? rWr[p] : 1.0;
+    double best = -INFINITY, bq = -1.0, bden = 1.0, bsy = 0.0;
+    bool any_nan = false;
+    const int m_end = min(Mc, (static_cast<int>(blockIdx.x) + 1) * kFinM);
+    for (int m0 = blockIdx.x * kFinM; m0 < m_end; m0 += kFinTile) {
+        __syncthreads();
+#pragma unroll
+        for (int l = 0; l < kFinP * kFinTile / 256; ++l) {
+            const int t = tid + l * 256, r = t / kFinTile, c = t % kFinTile;
+            if (p0 + r < P && m0 + c < m_end) {
+                const int64_t o = static_cast<int64_t>(p0 + r) * ldg + m0 + c;
+                sy[r][c] = G[o];
+                ss[r][c] = G[g_stride + o];
+            }
+        }
+        __syncthreads();
+        if (!p_ok) continue;
+        for (int c = warp; c < kFinTile && m0 + c < m_end; c += 8) {
+            const double swy = sy[lane][c], den = fmax(ss[lane][c], kPosFloor), q = mul_rn(swy, swy);
+            if (!real && q < 1e100 && den < 1e100 && den > 1e-100) {
+                if (q * bden > bq * den) {
+                    bq = q;
+                    bden = den;
+                    bsy = swy;
+                }
+                continue;
+            }
+            const Test t = wald_test(swy, ss[lane][c], rwr, var_df);
+            best = fmax(best, t.F);
+            any_nan |= isnan(t.F);
+            if (real) {
+                const int64_t o = rows[m0 + c] * ldo + p;
+                f[o] = t.F;
+                beta[o] = t.b;
+                se[o] = sqrt(t.var_b);
+                sfve[o] = sqrt(fmax(t.q / mul_rn(t.denom, rwr), 0.0));
+            }
+        }
+    }
+    if (bq >= 0.0) {
+        const double F = wald_test(bsy, bden, rwr, var_df).F;
+        best = fmax(best, F);
+        any_nan |= isnan(F);
+    }
+    red[warp][lane] = any_nan ? NAN : best;
+    __syncthreads();
+    if (warp == 0 && p_ok) {
+        double v = -INFINITY;
+        bool nan = false;
+        for (int r = 0; r < 8; ++r) {
+            nan |= isnan(red[r][lane]);
+            v = fmax(v, red[r][lane]);
+        }
+        if (nan) v = NAN;
+        if (v >= 0.0 || isnan(v)) atomic_max_nonneg(max_F + p, v);
+    }
+}
+
+// The scan runs over blocks of at most kBlockP columns x kBlockM variants, fewer where their digit planes (32 bytes
+// per element of a column or variant) would pass kPlaneBytes: the workspace does not grow with P or Mc.
+constexpr int kBlockP = 2048, kBlockM = 4096;
+constexpr size_t kPlaneBytes = size_t(256) << 20;
+
+int block_rows(int most, int unit, int K) {
+    const size_t fit = kPlaneBytes / (32 * static_cast<size_t>(K)) / unit * unit;
+    return static_cast<int>(fit < static_cast<size_t>(unit) ? unit : fit < static_cast<size_t>(most) ? fit : most);
+}
+
+struct WaldWs {
+    int pc, mc;                // columns and variants of a block
+    double *rWr, *A1, *W, *G;  // A1 and W adjacent (pc, Neff) matrices; G (2, pc, mc)
+    char *cols, *vars;         // digit operands of [A1 | W] and [US | US^2]
+    size_t bytes;
+};
+
+WaldWs carve_wald(void* base, int P, int Neff) {
+    WaldWs w{};
+    w.pc = block_rows(kBlockP, kOzRowsA, Neff);
+    if (P < w.pc) w.pc = P > 0 ? P : 1;
+    w.mc = block_rows(kBlockM, kOzRowsB, Neff);
+    size_t off = 0;
+    const uintptr_t b = reinterpret_cast<uintptr_t>(base);
+    const uintptr_t b0 = (b + 1023) / 1024 * 1024;
+    auto take = [&](size_t n) {
+        const uintptr_t p = b0 + off;
+        off += (n + 1023) / 1024 * 1024;
+        return p;
+    };
+    w.rWr = reinterpret_cast<double*>(take(sizeof(double) * w.pc));
+    w.A1 = reinterpret_cast<double*>(take(2 * sizeof(double) * static_cast<size_t>(w.pc) * Neff));
+    w.W = w.A1 + static_cast<size_t>(w.pc) * Neff;
+    w.G = reinterpret_cast<double*>(take(2 * sizeof(double) * static_cast<size_t>(w.pc) * w.mc));
+    w.cols = reinterpret_cast<char*>(take(oz_operand_bytes(w.pc, Neff, 2, kOzRowsA)));
+    w.vars = reinterpret_cast<char*>(take(oz_operand_bytes(w.mc, Neff, 2, kOzRowsB)));
+    w.bytes = off + 1024;
+    return w;
+}
+
+size_t wald_ws(int P, int Neff) { return carve_wald(nullptr, P, Neff).bytes; }
 
 }  // namespace
 
@@ -159,20 +293,48 @@ __global__ void k_spectrum_pad(const double* __restrict__ s, int k, int n0, doub
     if (i < k + n0) out[i] = i < k ? s[i] : 0.0;
 }
 
+// Column blocks outside, variant blocks inside.  A block's two products run on the tensor cores from digit planes
+// (flmm_oz64.cu) where they are large enough, else in the fused FP64 tile kernel.
 int wald_impl(const double* s, int Neff, const double* UYt, int64_t ldu, const double* log_delta, int P, int n_real,
               const double* USt, int64_t ldus, int Mc, const int64_t* rows, double* f, double* beta, double* se,
               double* sfve, int64_t ldo, double* max_F, double var_df, void* work, cudaStream_t st) {
-    double* W = static_cast<double*>(work);
-    double* A1 = W + static_cast<size_t>(P) * Neff;
-    double* rWr = A1 + static_cast<size_t>(P) * Neff;
-    k_wald_prep<<<ceil_div(static_cast<int64_t>(P) * 32, 256), 256, 0, st>>>(s, Neff, UYt, ldu, log_delta, P, W, A1,
-                                                                             rWr);
-    int rc = check_launch("k_wald_prep");
-    if (rc) return rc;
-    dim3 grid(ceil_div(Mc, TM), ceil_div(P, TP));
-    k_wald_f64<<<grid, NT, 0, st>>>(W, A1, rWr, Neff, var_df, P, n_real, USt, ldus, Mc, rows, f, beta, se, sfve, ldo,
-                                    max_F);
-    return check_launch("k_wald_f64");
+    const WaldWs w = carve_wald(work, P, Neff);
+    int rc;
+    for (int p0 = 0; p0 < P; p0 += w.pc) {
+        const int pc = P - p0 < w.pc ? P - p0 : w.pc;
+        const int nr = n_real > p0 ? (n_real - p0 < pc ? n_real - p0 : pc) : 0;
+        double* W = w.A1 + static_cast<size_t>(pc) * Neff;
+        k_wald_prep<<<ceil_div(static_cast<int64_t>(pc) * 32, 256), 256, 0, st>>>(s, Neff, UYt + p0 * ldu, ldu,
+                                                                                 log_delta + p0, pc, W, w.A1, w.rWr);
+        if ((rc = check_launch("k_wald_prep"))) return rc;
+        auto out = [&](double* x) { return x ? x + p0 : x; };
+        const bool tensor = oz_worth(pc, Mc < w.mc ? Mc : w.mc, Neff);
+        if (!tensor) {
+            const dim3 grid(ceil_div(Mc, TM), ceil_div(pc, TP));
+            k_wald_f64<<<grid, NT, 0, st>>>(W, w.A1, w.rWr, Neff, var_df, pc, nr, USt, ldus, Mc, rows, out(f), out(beta),
+                                            out(se), out(sfve), ldo, max_F + p0);
+            if ((rc = check_launch("k_wald_f64"))) return rc;
+            continue;
+        }
+        const OzOperand cols = oz_carve(w.cols, pc, Neff, 2, kOzRowsA);
+        if ((rc = oz_digits(cols, 0, w.A1, Neff, false, st))) return rc;
+        if ((rc = oz_digits(cols, 1, W, Neff, false, st))) return rc;
+        for (int m0 = 0; m0 < Mc; m0 += w.mc) {
+            const int mc = Mc - m0 < w.mc ? Mc - m0 : w.mc;
+            const double* US = USt + m0 * ldus;
+            const OzOperand vars = oz_carve(w.vars, mc, Neff, 2, kOzRowsB);
+            if ((rc = oz_digits(vars, 0, US, ldus, false, st))) return rc;
+            if ((rc = oz_digits(vars, 1, US, ldus, true, st))) return rc;
+            const int64_t gs = static_cast<int64_t>(pc) * mc;
+            const OzProduct prod{w.A1, Neff, static_cast<int64_t>(pc) * Neff, US, ldus, 0, true, w.G, mc, gs, nullptr, 0};
+            if ((rc = oz_gemm(cols, vars, prod, st))) return rc;
+            const dim3 grid(ceil_div(mc, kFinM), ceil_div(pc, kFinP));
+            k_wald_finish<<<grid, 256, 0, st>>>(w.G, mc, gs, w.rWr, var_df, pc, nr, mc, rows ? rows + m0 : rows, out(f),
+                                                out(beta), out(se), out(sfve), ldo, max_F + p0);
+            if ((rc = check_launch("k_wald_finish"))) return rc;
+        }
+    }
+    return FLMM_OK;
 }
 
 size_t lowrank_cat_doubles(int k, int N, int P, int Mc) {

@@ -49,6 +49,8 @@ SIGNATURES: dict[str, list] = {
     "flmm_compat_spectrum_f32": [_p, _i, _i, _p, _p],
     "flmm_regress_out": [_p, _i64, _i, _i, _p, _i, _p, _p, _i64, _p],
     "flmm_gemm_nt_f64": [_p, _i64, _p, _i64, _p, _i64, _i, _i, _i, _d, _p],
+    "flmm_gemm_nt_f64_tc_workspace_bytes": [_i, _i, _i, _psz],
+    "flmm_gemm_nt_f64_tc": [_p, _i64, _p, _i64, _p, _i64, _p, _i64, _i, _i, _i, _p, _sz, _p],
     "flmm_delta_grid_nodes": [_d, _d, _i, _p, _p],
     "flmm_fit_delta_f64_workspace_bytes": [_i, _i, _psz],
     "flmm_fit_delta_f64": [_p, _i, _p, _i64, _i, _i, _d, _d, _i, _p, _p, _p, _sz, _p],

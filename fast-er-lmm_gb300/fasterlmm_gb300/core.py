@@ -282,6 +282,32 @@ def rotate_rows(At: Tensor, Ut: Tensor) -> Tensor:
     return out
 
 
+# Products of at least this many multiply-adds run on the tensor cores: below it the digit planes, the product and the
+# check of its tiles (three launches and a pass over 16 bytes per element) cost as much as the FP64 pipe's sum.
+TENSOR_MACS = 20_000_000
+
+
+def rotate_variants(At: Tensor, Ut: Tensor, minus_from: Tensor | None = None) -> Tensor:
+    """rotate_rows for tested variants, (rows, N) x (Neff, N)^T, or minus_from - that; on the tensor cores to FP64
+    accuracy where the product is large.  The null model's operands keep rotate_rows: the golden section stops at the
+    rounding noise of the loss, so another rounding of UY moves log delta by ~1e-7."""
+    rows, N = At.shape
+    Neff = Ut.shape[0]
+    if rows * Neff * N < TENSOR_MACS:
+        out = rotate_rows(At, Ut)
+        if minus_from is not None:
+            res = minus_from.clone()
+            _lib.call("flmm_axpy_f64", res.numel(), -1.0, _ptr(out), _ptr(res), _stream(At.device))
+            return res
+        return out
+    out = torch.empty((rows, Neff), dtype=F64, device=At.device)
+    w, wb = _work.get(At.device, _lib.query_bytes("flmm_gemm_nt_f64_tc_workspace_bytes", rows, Neff, N))
+    _lib.call("flmm_gemm_nt_f64_tc", _ptr(At), At.stride(0), _ptr(Ut), Ut.stride(0), _ptr(minus_from),
+              0 if minus_from is None else minus_from.stride(0), _ptr(out), Neff, rows, Neff, N, w, wb,
+              _stream(At.device))
+    return out
+
+
 def fastlmm_compat_rotate(K: Tensor, X: Tensor, Y: Tensor) -> CompatSpectrum:
     """Drop-in for core.fastlmm_compat_rotate (fasterlmm/core.py:487-519)."""
     dev = _cuda_device(K)
@@ -363,7 +389,7 @@ def snp_wald_scan_compat(spec: CompatSpectrum, log_delta: Tensor, S: Tensor, *, 
     n_real = P if n_real is None else min(n_real, P)
     St = _rows_major(_f64(S, dev, contiguous=False))
     M = St.shape[0]
-    USt = rotate_rows(basis.regress_out(St), Ut)
+    USt = rotate_variants(basis.regress_out(St), Ut)
     out, max_F = _alloc_outputs(M, n_real, P, dev)
     rows = torch.arange(M, dtype=torch.int64, device=dev)
     ld = _f64(log_delta, dev)
@@ -456,7 +482,7 @@ def scan_t(Zt: Tensor, X: Tensor, Yt: Tensor, chrom: np.ndarray, *, n_real: int,
         UYt = rotate_rows(Yrt, Ut)
         ld, _ = fit_delta_t(s, UYt, n_grid=n_grid, log_delta_min=log_delta_min, log_delta_max=log_delta_max,
                             refine=refine)
-        USt = rotate_rows(basis.regress_out(_take_rows(Zt, blk)), Ut)
+        USt = rotate_variants(basis.regress_out(_take_rows(Zt, blk)), Ut)
         wald_t(s, UYt, ld, USt, n_real, blk[0], out, max_F)
         log_deltas[c if c is not None else 0] = ld
         if on_chrom is not None:

@@ -20,7 +20,7 @@ from torch import Tensor
 
 from . import _lib
 from .core import (F64, ScanResult, _alloc_outputs, _chrom_blocks, _cuda_device, _f64, _ptr, _rows_major, _stream,
-                   _take_rows, _to_device, _work, gram_t, kinship_from_gram, rotate_rows, transpose)
+                   _take_rows, _to_device, _work, gram_t, kinship_from_gram, rotate_rows, rotate_variants, transpose)
 
 JITTER = 1e-6  # eigendecompose's diagonal jitter (fasterlmm/core.py:89)
 
@@ -240,7 +240,7 @@ def scan_t(Zt: Tensor, X: Tensor, Yt: Tensor, chrom: np.ndarray, *, n_real: int,
             K = kinship_from_gram(Gtot, grams.get(c), M_kin - int((kin_chrom == c).sum()))
         s, Ut, Xrt, Yrt = rotate_t(K, X, Yt)
         ld, _ = fit_delta_t(s, Xrt, Yrt)
-        Srt = rotate_rows(_take_rows(Zt, blk).contiguous(), Ut)
+        Srt = rotate_variants(_take_rows(Zt, blk).contiguous(), Ut)
         wald_t(s, Xrt, Yrt, ld, Srt, n_real, blk[0], out, max_F)
         log_deltas[c if c is not None else 0] = ld
         if on_chrom is not None:

@@ -20,7 +20,8 @@ from torch import Tensor
 
 from . import _lib
 from .core import (F64, CovariateBasis, ScanResult, _alloc_outputs, _BasisView, _cuda_device, _f64, _ptr,
-                   _rows_major, _stream, _to_device, _work, gram_t, kinship_from_gram, rotate_rows, transpose)
+                   _rows_major, _stream, _to_device, _work, gram_t, kinship_from_gram, rotate_rows, rotate_variants,
+                   transpose)
 
 
 @dataclass
@@ -170,7 +171,9 @@ def wald_t(s: Tensor, Ut: Tensor, UYt: Tensor, UUYt: Tensor, Neff: int, log_delt
     dev = s.device
     k, N = Ut.shape
     P = UYt.shape[0]
-    USt, UUSt = rotate_t(St, Ut, basis)
+    Sr = basis.regress_out(St)
+    USt = rotate_variants(Sr, Ut)
+    UUSt = rotate_variants(USt, transpose(Ut), minus_from=Sr)
     Mc = USt.shape[0]
     w, wb = _work.get(dev, _lib.query_bytes("flmm_wald_lowrank_f64_workspace_bytes", k, N, P, Mc))
     _lib.call("flmm_wald_lowrank_f64", _ptr(s), k, _ptr(UYt), UYt.stride(0), _ptr(UUYt), UUYt.stride(0), N, int(Neff),

@@ -149,6 +149,12 @@ int flmm_regress_out(const double* A, int64_t lda, int rows, int N, const double
 int flmm_gemm_nt_f64(const double* A, int64_t lda, const double* B, int64_t ldb, double* C, int64_t ldc, int Mr,
                      int Nr, int K, double alpha, void* stream);
 
+/* The same product on the FP16 tensor cores from exact digit planes, to FP64 accuracy (rows that the digits cannot hold
+ * are formed on the FP64 pipe): C = A B^T, or C = D - A B^T where D (Mr, Nr) is not NULL (D may be C). */
+int flmm_gemm_nt_f64_tc_workspace_bytes(int Mr, int Nr, int K, size_t* bytes);
+int flmm_gemm_nt_f64_tc(const double* A, int64_t lda, const double* B, int64_t ldb, const double* D, int64_t ldd,
+                        double* C, int64_t ldc, int Mr, int Nr, int K, void* work, size_t work_bytes, void* stream);
+
 /* ---- null-model delta fit (fasterlmm/core.py:525-595) --------------------------------------------------------- */
 
 /* Grid node values exactly as torch.linspace(lo, hi, n_grid) in FP64. */

@@ -1,0 +1,143 @@
+"""
+FP64 products on the tensor cores (csrc/flmm_oz64.cu) against exact sums and against the FP64-pipe kernel.
+
+The digit planes must lose no more than an FP64 sum does: over sampled outputs the rms error against exact sums (exact
+products by Dekker's splitting, exact addition by math.fsum) is at most that of flmm_gemm_nt_f64.  Rows that digits
+cannot hold (not finite, exponents out of range, one entry far above the rest) take the FP64 pipe, bit for bit.
+"""
+from __future__ import annotations
+
+import math
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _products(A, B, D=None):
+    from fasterlmm_gb300 import _lib, build
+    from fasterlmm_gb300.core import _ptr, _stream, _work
+    build()
+    Mr, K = A.shape
+    Nr = B.shape[0]
+    dev = A.device
+    tc = torch.full((Mr, Nr), 7.0, dtype=torch.float64, device=dev)
+    ref = torch.empty((Mr, Nr), dtype=torch.float64, device=dev)
+    w, wb = _work.get(dev, _lib.query_bytes("flmm_gemm_nt_f64_tc_workspace_bytes", Mr, Nr, K))
+    _lib.call("flmm_gemm_nt_f64_tc", _ptr(A), A.stride(0), _ptr(B), B.stride(0), _ptr(D), 0 if D is None else Nr,
+              _ptr(tc), Nr, Mr, Nr, K, w, wb, _stream(dev))
+    _lib.call("flmm_gemm_nt_f64", _ptr(A), A.stride(0), _ptr(B), B.stride(0), _ptr(ref), Nr, Mr, Nr, K, 1.0, _stream(dev))
+    _lib.call("flmm_context_check", _lib.context(dev.index), _stream(dev))
+    return tc, ref
+
+
+def _exact(a, b):
+    """Correctly rounded sum of a[k] b[k]."""
+    split = lambda x: (lambda c: (c - (c - x), x - (c - (c - x))))(134217729.0 * x)
+    (ah, al), (bh, bl) = split(a), split(b)
+    p = a * b
+    e = ((ah * bh - p) + ah * bl + al * bh) + al * bl
+    return math.fsum(np.concatenate([p, e]))
+
+
+def _rms(x):
+    return float(np.sqrt(np.mean(np.square(x))))
+
+
+@pytest.mark.parametrize("Mr,Nr,K", [(1, 1, 32), (127, 63, 33), (128, 64, 512), (129, 65, 513), (257, 200, 1000),
+                                     (300, 130, 1537), (40, 70, 5003)])
+@pytest.mark.parametrize("kind", ["normal", "positive"])
+def test_no_less_exact_than_fp64(Mr, Nr, K, kind):
+    g = torch.Generator(device="cuda").manual_seed(Mr * 7 + K)
+    A = torch.randn(Mr, K, generator=g, device="cuda", dtype=torch.float64)
+    B = torch.randn(Nr, K, generator=g, device="cuda", dtype=torch.float64) * 3.0
+    if kind == "positive":  # weights and squares, rows of different sizes
+        A = 1.0 / (A.abs() + 0.3) * torch.logspace(-20, 20, Mr, device="cuda", dtype=torch.float64)[:, None]
+        B = B * B
+    tc, ref = _products(A, B)
+    a, b, tc, ref = (t.cpu().numpy() for t in (A, B, tc, ref))
+    rng = np.random.default_rng(0)
+    at = {(0, 0), (Mr - 1, Nr - 1)} | {(int(rng.integers(Mr)), int(rng.integers(Nr))) for _ in range(300)}
+    scale = lambda i, j: np.linalg.norm(a[i]) * np.linalg.norm(b[j])
+    ex = {ij: _exact(a[ij[0]], b[ij[1]]) for ij in at}
+    err = lambda c: _rms([(c[ij] - ex[ij]) / scale(*ij) for ij in at])
+    assert err(tc) <= max(err(ref), 2.0 ** -53)
+
+
+def test_difference_form():
+    g = torch.Generator(device="cuda").manual_seed(5)
+    A, B = (torch.randn(n, 300, generator=g, device="cuda", dtype=torch.float64) for n in (150, 90))
+    D = torch.randn(150, 90, generator=g, device="cuda", dtype=torch.float64)
+    tc, _ = _products(A, B)
+    dif, _ = _products(A, B, D)
+    assert torch.equal(dif, D - tc)
+
+
+def test_rows_that_digits_cannot_hold():
+    """Only the tiles of such rows change path, and there the bits are the FP64 pipe's."""
+    g = torch.Generator(device="cuda").manual_seed(6)
+    Mr, Nr, K = 400, 200, 600
+    A = torch.randn(Mr, K, generator=g, device="cuda", dtype=torch.float64)
+    B = torch.randn(Nr, K, generator=g, device="cuda", dtype=torch.float64)
+    A[130, 7] = float("nan")
+    A[131, 8] = float("inf")
+    A[140] *= 1e200
+    A[150, 3] = 1e9      # one entry far above the rest of its row
+    A[160] = 0.0
+    B[70] *= 1e-200
+    tc, ref = _products(A, B)
+    bad = torch.zeros(Mr, Nr, dtype=torch.bool, device="cuda")
+    bad[128:256] = True
+    bad[:, 64:128] = True
+    assert torch.equal(torch.isnan(tc), torch.isnan(ref))
+    same = (tc == ref) | (torch.isnan(tc) & torch.isnan(ref))
+    assert bool(same[bad].all())
+    torch.testing.assert_close(tc[~bad], ref[~bad], rtol=0, atol=1e-11)
+    assert not same[~bad].all()  # the other tiles ran on the tensor cores
+
+
+@pytest.mark.parametrize("P,Mc,Neff,n_real", [(40, 300, 130, 40), (129, 1000, 700, 1), (2049, 300, 100, 2049),
+                                              (100, 4097, 150, 33), (64, 4160, 257, 1)])
+def test_wald_blocks(P, Mc, Neff, n_real):
+    """flmm_wald_f64 over its blocks of columns and variants, on either path, against the formulas in FP64."""
+    from fasterlmm_gb300 import build, core
+    build()
+    g = torch.Generator(device="cuda").manual_seed(P + Mc)
+    dev = torch.device("cuda", torch.cuda.current_device())
+    rn = lambda *s: torch.randn(*s, generator=g, device=dev, dtype=torch.float64)
+    s, UY, US = rn(Neff).abs() + 0.05, rn(P, Neff), rn(Mc, Neff)
+    ld = rn(P)
+    US[5] = 0.0
+    out, max_F = core._alloc_outputs(Mc, n_real, P, dev)
+    rows = torch.randperm(Mc, generator=g, device=dev)
+    core.wald_t(s, UY, ld, US, n_real, rows, out, max_F)
+    w = 1.0 / (s[None, :] + ld.exp()[:, None])
+    num, den, rwr = (w * UY) @ US.T, (w @ (US * US).T).clamp(min=1e-300), (w * UY * UY).sum(1)
+    var = (rwr[:, None] - num * num / den).clamp(min=1e-300) / (Neff - 1) / den
+    F = (num / den) ** 2 / var
+    close = lambda x, y: torch.testing.assert_close(x, y, rtol=1e-9, atol=1e-12)
+    close(max_F, F.max(1).values)
+    r = slice(0, n_real)
+    close(out["f"][rows], F[r].T)
+    close(out["beta"][rows], (num / den)[r].T)
+    close(out["se"][rows], var[r].sqrt().T)
+    close(out["sfve"][rows], (num * num / (den * rwr[:, None]))[r].sqrt().T)
+
+
+def test_wald_keeps_nan():
+    from fasterlmm_gb300 import build, core
+    build()
+    g = torch.Generator(device="cuda").manual_seed(3)
+    dev = torch.device("cuda", torch.cuda.current_device())
+    rn = lambda *s: torch.randn(*s, generator=g, device=dev, dtype=torch.float64)
+    P, Mc, Neff = 200, 600, 300
+    UY = rn(P, Neff)
+    UY[3, 5] = UY[150, 2] = float("nan")
+    out, max_F = core._alloc_outputs(Mc, 10, P, dev)
+    core.wald_t(rn(Neff).abs(), UY, rn(P), rn(Mc, Neff), 10, torch.arange(Mc, device=dev), out, max_F)
+    nan = torch.zeros(P, dtype=torch.bool, device=dev)
+    nan[3] = nan[150] = True
+    assert torch.equal(torch.isnan(max_F), nan)
+    assert torch.equal(torch.isnan(out["f"]).any(0), nan[:10])
