@@ -14,6 +14,7 @@
 #include <math.h>
 
 #include "flmm_common.cuh"
+#include "flmm_oz64.cuh"
 
 using namespace flmm;
 
@@ -318,12 +319,14 @@ __global__ void k_gls_golden(const double* __restrict__ s, int N, const double* 
 // ---- Wald ------------------------------------------------------------------------------------------------------
 
 // Null fit of column p at its log delta (fasterlmm/core.py:328-341): A_p, L_p (identity when the Cholesky fails),
-// beta_x = A^-1 u, r = y~ - X~ beta_x, rWr = sum w r^2, and the left operands of the scan
-// Lv[p] = (w o r, w o x~_0 .. w o x~_{C-1}, w), each of N entries.
+// beta_x = A^-1 u, r = y~ - X~ beta_x, rWr = sum w r^2, and the left operands of the scan, rows of N entries: w o r at
+// Rv, w at Wv (column pitch rv_stride), and C rows at Qv (column pitch qv_stride): w o x~_c, or with `solved` the rows
+// of L^-1 X~^T W, whose products with a variant are the terms of B^T A^-1 B as squares.
 __global__ void k_gls_wald_prep(const double* __restrict__ s, int N, const double* __restrict__ Xrt, int64_t ldx,
                                 int C, const double* __restrict__ Yrt, int64_t ldy, int P,
-                                const double* __restrict__ ld, double* __restrict__ Lv, double* __restrict__ Lp,
-                                double* __restrict__ rWr) {
+                                const double* __restrict__ ld, int solved, double* __restrict__ Rv,
+                                double* __restrict__ Wv, int64_t rv_stride, double* __restrict__ Qv, int64_t qv_stride,
+                                double* __restrict__ Lp, double* __restrict__ rWr) {
     extern __shared__ double sm[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t p = static_cast<int64_t>(blockIdx.x) * kEvalWarps + warp;
@@ -343,11 +346,16 @@ __global__ void k_gls_wald_prep(const double* __restrict__ s, int N, const doubl
         if (!chol_lower(A, C)) set_identity(A, C);
         forward_solve(A, C, z);
         back_solve(A, C, z);  // z = beta_x
-        double* L = Lp + p * C * C;
-        for (int i = 0; i < C * C; ++i) L[i] = A[i];
+        if (solved) {
+            for (int i = 0; i < C; ++i) Gs[i] = 1.0 / A[i * C + i];
+        } else {
+            double* L = Lp + p * C * C;
+            for (int i = 0; i < C * C; ++i) L[i] = A[i];
+        }
     }
     __syncwarp();
-    double* lv = Lv + p * static_cast<int64_t>(C + 2) * N;
+    double* rv = Rv + p * rv_stride;
+    double* wv = Wv + p * rv_stride;
     double acc = 0.0;
     for (int n = lane; n < N; n += 32) {
         const double w = 1.0 / (s[n] + delta);
@@ -356,9 +364,17 @@ __global__ void k_gls_wald_prep(const double* __restrict__ s, int N, const doubl
         const double r = add_rn(y[n], -fit);
         const double wr = mul_rn(w, r);
         acc += mul_rn(wr, r);
-        lv[n] = wr;
-        for (int c = 0; c < C; ++c) lv[static_cast<int64_t>(1 + c) * N + n] = mul_rn(w, Xrt[c * ldx + n]);
-        lv[static_cast<int64_t>(C + 1) * N + n] = w;
+        rv[n] = wr;
+        double* col = Qv + p * qv_stride + n;  // this sample's entries of the C rows, N apart
+        for (int c = 0; c < C; ++c) {
+            double v = mul_rn(w, Xrt[c * ldx + n]);
+            if (solved) {
+                for (int k = 0; k < c; ++k) v = fma(-A[c * C + k], col[static_cast<int64_t>(k) * N], v);
+                v = mul_rn(v, Gs[c]);
+            }
+            col[static_cast<int64_t>(c) * N] = v;
+        }
+        wv[n] = w;
     }
     acc = warp_sum(acc);
     if (lane == 0) rWr[p] = acc;
@@ -484,11 +500,54 @@ GridWs carve_grid(void* base, int N, int C, int P, int G) {
     return w;
 }
 
-constexpr int kWaldChunk = 4096;  // columns prepared per pass of the Wald scan
+constexpr int kWaldChunk = 4096;  // columns prepared per pass of the FP64 tile kernel
+
+// Blocks of the tensor-core path: (C + 2) operand rows per column, kBlockRows rows and kBlockM variants at most, fewer
+// where their digit planes (16 bytes per element) would pass kPlaneBytes.
+constexpr int kBlockRows = 6144, kBlockM = 4096;
+constexpr size_t kPlaneBytes = size_t(256) << 20;
+
+struct WaldWs {
+    int pc, mc;             // columns and variants of a block
+    double *RW, *Q, *rWr;   // w o r and w (2, pc, N), L^-1 X~^T W (pc, C, N)
+    double *G, *Gq;         // sums: num and sWs (2, pc, mc), the quadratic form's terms (pc, C, mc)
+    char *rw_op, *q_op, *s_op;
+    size_t bytes;
+};
+
+WaldWs carve_wald(void* base, int N, int C, int P) {
+    WaldWs w{};
+    const size_t fit = kPlaneBytes / (16 * static_cast<size_t>(N));
+    const size_t rows = fit < static_cast<size_t>(kBlockRows) ? fit : kBlockRows;
+    w.pc = static_cast<int>(rows / (C + 2));
+    w.pc = w.pc < 1 ? 1 : (P < w.pc ? (P > 0 ? P : 1) : w.pc);
+    w.mc = static_cast<int>(fit / 2 < static_cast<size_t>(kBlockM) ? fit / 2 / kOzRowsB * kOzRowsB : kBlockM);
+    w.mc = w.mc < kOzRowsB ? kOzRowsB : w.mc;
+    size_t off = 0;
+    const uintptr_t b0 = (reinterpret_cast<uintptr_t>(base) + 1023) / 1024 * 1024;
+    auto take = [&](size_t n) {
+        const uintptr_t p = b0 + off;
+        off += (n + 1023) / 1024 * 1024;
+        return p;
+    };
+    const size_t n = N, pc = w.pc, mc = w.mc;
+    w.rWr = reinterpret_cast<double*>(take(sizeof(double) * pc));
+    w.RW = reinterpret_cast<double*>(take(2 * sizeof(double) * pc * n));
+    w.Q = reinterpret_cast<double*>(take(sizeof(double) * pc * C * n));
+    w.G = reinterpret_cast<double*>(take(2 * sizeof(double) * pc * mc));
+    w.Gq = reinterpret_cast<double*>(take(sizeof(double) * pc * C * mc));
+    w.rw_op = reinterpret_cast<char*>(take(oz_operand_bytes(w.pc, N, 2, kOzRowsA)));
+    w.q_op = reinterpret_cast<char*>(take(oz_operand_bytes(w.pc * C, N, 1, kOzRowsA)));
+    w.s_op = reinterpret_cast<char*>(take(oz_operand_bytes(w.mc, N, 2, kOzRowsB)));
+    w.bytes = off + 1024;
+    return w;
+}
 
 size_t wald_ws(int N, int C, int P) {
     const size_t pc = static_cast<size_t>(P < kWaldChunk ? P : kWaldChunk);
-    return sizeof(double) * (pc * (C + 2) * N + pc * C * C + pc) + 1024;
+    const size_t tiles = sizeof(double) * (pc * (C + 2) * N + pc * C * C + pc) + 1024;
+    const size_t tensor = carve_wald(nullptr, N, C, P).bytes;
+    return tiles > tensor ? tiles : tensor;
 }
 
 __global__ void k_shift_diagonal(double* __restrict__ A, int N, int64_t lda, double v) {
@@ -613,6 +672,44 @@ extern "C" int flmm_wald_gls_f64(const double* s, int N, const double* Xrt, int6
     const size_t smem_prep = eval_smem_bytes(C);
     if (smem_prep > 48 * 1024)
         FLMM_CUDA(cudaFuncSetAttribute(k_gls_wald_prep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_prep));
+    // Large scans: the products (w o r)^T s, w^T (s o s) and (L^-1 X~^T W) s on the tensor cores from digit planes.  The
+    // tile kernel reads two shared-memory operands per FP64 multiply-add and reached 0.87 TFLOP/s (660 columns x 4,000
+    // variants x 800 samples, C = 5: 33.9 ms).
+    const WaldWs w = carve_wald(work, N, C, P);
+    if (oz_worth(static_cast<int64_t>(w.pc) * (C + 2), M < w.mc ? M : w.mc, N)) {
+        for (int p0 = 0; p0 < P; p0 += w.pc) {
+            const int pc = P - p0 < w.pc ? P - p0 : w.pc;
+            const int nr = n_real > p0 ? (n_real - p0 < pc ? n_real - p0 : pc) : 0;
+            const int64_t half = static_cast<int64_t>(pc) * N, gs = static_cast<int64_t>(pc) * (M < w.mc ? M : w.mc);
+            k_gls_wald_prep<<<ceil_div(pc, kEvalWarps), 32 * kEvalWarps, smem_prep, st>>>(
+                s, N, Xrt, ldx, C, Yrt + static_cast<int64_t>(p0) * ldy, ldy, pc, log_delta + p0, 1, w.RW, w.RW + half, N,
+                w.Q, static_cast<int64_t>(C) * N, nullptr, w.rWr);
+            if ((rc = check_launch("k_gls_wald_prep"))) return rc;
+            const OzOperand rw = oz_carve(w.rw_op, pc, N, 2, kOzRowsA), qo = oz_carve(w.q_op, pc * C, N, 1, kOzRowsA);
+            if ((rc = oz_digits(rw, 0, w.RW, N, false, st))) return rc;
+            if ((rc = oz_digits(rw, 1, w.RW + half, N, false, st))) return rc;
+            if ((rc = oz_digits(qo, 0, w.Q, N, false, st))) return rc;
+            auto out = [&](double* x) { return nr > 0 ? x + p0 : nullptr; };
+            for (int m0 = 0; m0 < M; m0 += w.mc) {
+                const int mc = M - m0 < w.mc ? M - m0 : w.mc;
+                const double* S = Srt + m0 * lds;
+                const OzOperand so = oz_carve(w.s_op, mc, N, 2, kOzRowsB);
+                if ((rc = oz_digits(so, 0, S, lds, false, st))) return rc;
+                if ((rc = oz_digits(so, 1, S, lds, true, st))) return rc;
+                const OzProduct g{w.RW, N, half, S, lds, {false, true}, false, w.G, mc, gs, nullptr, 0};
+                // (the terms enter as squares subtracted from sWs: an error small against the row norms is enough, and
+                // the rotated intercept's row is one entry)
+                const OzProduct gq{w.Q, N, 0, S, lds, {false, false}, true, w.Gq, mc, 0, nullptr, 0};
+                if ((rc = oz_gemm(rw, so, g, st))) return rc;
+                if ((rc = oz_gemm(qo, so, gq, st))) return rc;
+                if ((rc = wald_finish(w.G, w.G + gs, w.Gq, C, mc, w.rWr, static_cast<double>(N - C - 1), pc, nr, mc,
+                                      nr > 0 ? rows + m0 : nullptr, out(f), out(beta), out(se), out(sfve), ldo,
+                                      max_F + p0, st)))
+                    return rc;
+            }
+        }
+        return FLMM_OK;
+    }
     const size_t smem_wald = sizeof(double) * (static_cast<size_t>(WP) * (C + 2) * WK + WM * WK);
     for (int q0 = 0; q0 < P; q0 += kWaldChunk) {
         const int pc = (P - q0 < kWaldChunk) ? P - q0 : kWaldChunk;
@@ -620,7 +717,9 @@ extern "C" int flmm_wald_gls_f64(const double* s, int N, const double* Xrt, int6
         double* Lp = Lv + static_cast<size_t>(pc) * (C + 2) * N;
         double* rWr = Lp + static_cast<size_t>(pc) * C * C;
         k_gls_wald_prep<<<ceil_div(pc, kEvalWarps), 32 * kEvalWarps, smem_prep, st>>>(
-            s, N, Xrt, ldx, C, Yrt + static_cast<int64_t>(q0) * ldy, ldy, pc, log_delta + q0, Lv, Lp, rWr);
+            s, N, Xrt, ldx, C, Yrt + static_cast<int64_t>(q0) * ldy, ldy, pc, log_delta + q0, 0, Lv,
+            Lv + static_cast<int64_t>(C + 1) * N, static_cast<int64_t>(C + 2) * N, Lv + N,
+            static_cast<int64_t>(C + 2) * N, Lp, rWr);
         if ((rc = check_launch("k_gls_wald_prep"))) return rc;
         const int nr = n_real - q0 > 0 ? (n_real - q0 < pc ? n_real - q0 : pc) : 0;
         dim3 grid(ceil_div(M, WM), ceil_div(pc, WP));

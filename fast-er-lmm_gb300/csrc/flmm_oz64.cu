@@ -19,12 +19,14 @@
 // k_marked_f64, which forms those tiles on the FP64 pipe as before.
 //
 // Kernel: persistent, one CTA per SM; tiles of 128 A rows x 64 B rows, 8 levels x 64 columns = all of tensor memory.
-// Warp 0 issues the TMA loads (a stage is 32 deep: 8 x 8 KB + 8 x 4 KB = 96 KB, two stages), warp 1 the 72 MMAs of a
-// stage (M = 128, N = 64, K = 16); A's plane stays in the tensor core's collector while the pairs that share it are
-// issued, because operand reads (6 KB per 32-cycle MMA) would otherwise exceed shared memory's 128 B per cycle.  Warps
-// 2..17 drain the levels; tensor memory is handed back before the outputs are rounded and stored, so only the drain
-// itself (8 x 64 columns per 512 terms) interrupts the MMAs.
+// Warp 0 issues the TMA loads: a stage is 16 deep, 8 x 4 KB + 8 x 2 KB = 48 KB in four boxes of 128-byte rows that hold
+// four planes each, four stages.  Warp 1 issues the 36 MMAs of a stage (M = 128, N = 64, K = 16), warps 2..17 drain the
+// levels; tensor memory is handed back before the outputs are rounded and stored, so only the drain itself (8 x 64
+// columns per 512 terms, 4,300 cycles) interrupts the MMAs.  Shared memory is the bound: an MMA reads 6 KB of operands
+// in at least 48 cycles (32 of tensor work), and with the copies' writes it takes 73; waits for loads and for the
+// epilogue are 7 % (cycle counts around the waits, 1,100 x 4,096 x 995 twice, 743 us).
 #include <cuda.h>
+#include <float.h>
 #include <math.h>
 
 #include <cstring>
@@ -40,13 +42,13 @@ namespace {
 
 constexpr int kLevels = 8;
 constexpr int kChunk = 512;  // terms of one exact accumulation
-constexpr int kBK = 32;      // depth of one stage (64-byte rows, 64-byte swizzle)
-constexpr int kATile = kOzRowsA * kBK * 2;
-constexpr int kBTile = kOzRowsB * kBK * 2;
-constexpr int kStageBytes = kOzPlanes * (kATile + kBTile);
-constexpr int kStages = 2;
-constexpr uint32_t kSBO = 8u * kBK * 2u;
-constexpr uint32_t kSwizzle64 = 4u;
+constexpr int kBK = 16;      // depth of one stage: a row's eight planes of 16 elements are 256 bytes, two 128-byte boxes
+constexpr int kRowElems = kOzPlanes * kBK;            // elements of a row in one stage
+constexpr int kABox = kOzRowsA * 128, kBBox = kOzRowsB * 128;
+constexpr int kStageBytes = 2 * (kABox + kBBox);
+constexpr int kStages = 4;
+constexpr uint32_t kSBO = 1024;     // bytes between 8-row groups
+constexpr uint32_t kSwizzle128 = 2u;
 constexpr int kTmemCols = kLevels * kOzRowsB;
 constexpr int kEpiWarps = 16;
 constexpr int kThreads = 64 + 32 * kEpiWarps;
@@ -55,9 +57,10 @@ constexpr int kSmemBytes = kStages * kStageBytes + 256 + 1024;
 constexpr int kMaxExp = 450;  // |e| beyond this: the scale 2^(e_a + e_b - 61) could leave FP64's range
 static_assert(kTmemCols == 512 && kSmemBytes <= 227 * 1024 && kEpiCols == 16, "budgets");
 
-// Largest product of two tiles' max/rms ratios that the digits take.  The dropped levels and the rounding leave
-// ~8e-16 sqrt(K / 1000) r_a r_b (in units of the rms product), an FP64 sum ~4.5e-14 K / 1000: equal at 57 sqrt(K / 1000).
-__host__ __device__ inline float quality_limit(int K) { return 1.8f * sqrtf(static_cast<float>(K)); }
+// Largest product of two tiles' max/rms ratios that the digits take.  Measured on a scan's operands at K = 1,000 (rms
+// against exact sums, relative to the row norms): ratios 10 x 5 leave 1.1e-17 where the FP64 sum leaves 3.9e-17, so the
+// two meet near a product of 150, and both errors scale so that the line goes with sqrt(K).
+__host__ __device__ inline float quality_limit(int K) { return 4.0f * sqrtf(static_cast<float>(K)); }
 
 struct OzMaps {
     CUtensorMap a, b;
@@ -86,7 +89,7 @@ struct OzArgs {
 template <bool SQ>
 __global__ void __launch_bounds__(256)
 k_digits64(const double* __restrict__ X, int64_t ldx, int rows, int K, __half* __restrict__ planes, int64_t ldp,
-           int64_t plane_stride, int* __restrict__ expo, float* __restrict__ qual, int tile_rows) {
+           int* __restrict__ expo, float* __restrict__ qual, int tile_rows) {
     const int lane = threadIdx.x & 31;
     const int64_t j = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5;
     if (j >= rows) return;
@@ -108,7 +111,7 @@ k_digits64(const double* __restrict__ X, int64_t ldx, int rows, int K, __half* _
     const double up = __longlong_as_double(static_cast<long long>(1023 + 55 - (bad ? 0 : e)) << 52);
     __half* out = planes + j * ldp;
     float ss = 0.0f;
-    for (int n = 2 * lane; n < K; n += 64) {
+    for (int n = 2 * lane; n < (K + kBK - 1) / kBK * kBK; n += 64) {
         long long v[2] = {0, 0};
         if (!bad) {
 #pragma unroll
@@ -135,7 +138,7 @@ k_digits64(const double* __restrict__ X, int64_t ldx, int rows, int K, __half* _
             }
             const unsigned word = (static_cast<unsigned>(0x6600 + d[1]) << 16) | static_cast<unsigned>(0x6600 + d[0]);
             const __half2 p = __hsub2(*reinterpret_cast<const __half2*>(&word), __half2half2(__ushort_as_half(0x6600)));
-            *reinterpret_cast<__half2*>(out + t * plane_stride + n) = p;
+            *reinterpret_cast<__half2*>(out + (n / kBK) * kRowElems + t * kBK + n % kBK) = p;
         }
     }
     ss = warp_sum(ss);
@@ -180,42 +183,20 @@ __device__ __forceinline__ bool tile_good(const OzArgs& a, const Tile& t) {
     return a.qa[t.b * a.tiles_i + t.ti] * a.qb[t.b * a.tiles_m + t.tm] <= a.limit[t.b];
 }
 
-// MMA whose A operand is read into the collector (fill), taken from it (use), or taken for the last time.
-enum class Collect { kFill, kUse, kLast, kNone };
-
-template <Collect C>
-__device__ __forceinline__ void mma_collect(uint32_t d, uint64_t ad, uint64_t bd, uint32_t idesc, uint32_t acc) {
-    if constexpr (C == Collect::kFill)
-        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                     "tcgen05.mma.cta_group::1.kind::f16.collector::a::fill [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
-                     "l"(ad), "l"(bd), "r"(idesc), "r"(acc)
-                     : "memory");
-    else if constexpr (C == Collect::kUse)
-        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                     "tcgen05.mma.cta_group::1.kind::f16.collector::a::use [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
-                     "l"(ad), "l"(bd), "r"(idesc), "r"(acc)
-                     : "memory");
-    else if constexpr (C == Collect::kLast)
-        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                     "tcgen05.mma.cta_group::1.kind::f16.collector::a::lastuse [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
-                     "l"(ad), "l"(bd), "r"(idesc), "r"(acc)
-                     : "memory");
-    else
-        mma_f16(d, ad, bd, idesc, acc);
+// Descriptors differ in their low words only (the tile's address in 16-byte units): plane t lies in box t / 4, 32 bytes
+// further along its rows per plane.
+__device__ __forceinline__ uint64_t plane_desc(uint32_t lo, uint32_t hi) {
+    return (static_cast<uint64_t>(hi) << 32) | lo;
 }
 
 template <int I, int J>
-__device__ __forceinline__ void mma_pair(uint32_t tmem, uint32_t sbase, int kk, bool first, uint32_t idesc) {
-    constexpr int kLastJ = kLevels - 1 - I;
-    constexpr Collect c = kLastJ == 0 ? Collect::kNone
-                          : J == 0    ? Collect::kFill
-                          : J == kLastJ ? Collect::kLast
-                                        : Collect::kUse;
-    const uint64_t ad = smem_desc(sbase + I * kATile, kSBO, kSwizzle64) + 2u * kk;
-    const uint64_t bd = smem_desc(sbase + kOzPlanes * kATile + J * kBTile, kSBO, kSwizzle64) + 2u * kk;
-    mma_collect<c>(tmem + static_cast<uint32_t>((I + J) * kOzRowsB), ad, bd, idesc, (first && I == 0) ? 0u : 1u);
-    if constexpr (J < kLastJ) mma_pair<I, J + 1>(tmem, sbase, kk, first, idesc);
-    else if constexpr (I < kOzPlanes - 1) mma_pair<I + 1, 0>(tmem, sbase, kk, first, idesc);
+__device__ __forceinline__ void mma_pair(uint32_t tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t acc0,
+                                         uint32_t idesc) {
+    mma_f16(tmem + static_cast<uint32_t>((I + J) * kOzRowsB),
+            plane_desc(a_lo + (I / 4) * (kABox / 16) + 2 * (I % 4), hi),
+            plane_desc(b_lo + (J / 4) * (kBBox / 16) + 2 * (J % 4), hi), idesc, I == 0 ? acc0 : 1u);
+    if constexpr (J < kLevels - 1 - I) mma_pair<I, J + 1>(tmem, a_lo, b_lo, hi, acc0, idesc);
+    else if constexpr (I < kOzPlanes - 1) mma_pair<I + 1, 0>(tmem, a_lo, b_lo, hi, acc0, idesc);
 }
 
 __global__ void __launch_bounds__(kThreads, 1) k_oz64(const __grid_constant__ OzMaps maps, const OzArgs args) {
@@ -275,12 +256,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz64(const __grid_constant__ Oz
                     armed[stage] = true;
                     armed_phase[stage] = phase;
                     uint8_t* base = smem + stage * kStageBytes;
-                    const int x = kb * kBK;
+                    const int x = kb * kRowElems;
 #pragma unroll
-                    for (int p = 0; p < kOzPlanes; ++p) {
-                        tma_load_2d(base + p * kATile, &maps.a, x, p * args.batches * args.Ma + ya, &full[stage]);
-                        tma_load_2d(base + kOzPlanes * kATile + p * kBTile, &maps.b, x,
-                                    p * args.batches * args.Nb + yb, &full[stage]);
+                    for (int h = 0; h < 2; ++h) {
+                        tma_load_2d(base + h * kABox, &maps.a, x + h * (kRowElems / 2), ya, &full[stage]);
+                        tma_load_2d(base + 2 * kABox + h * kBBox, &maps.b, x + h * (kRowElems / 2), yb, &full[stage]);
                     }
                     if (++stage == kStages) { stage = 0; phase ^= 1u; }
                 }
@@ -303,10 +283,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz64(const __grid_constant__ Oz
                     }
                     if (!mbar_wait(&full[stage], phase, args.err, 23)) { ok = false; break; }
                     fence_after_sync();
-                    const uint32_t sbase = smem_u32(smem + stage * kStageBytes);
-#pragma unroll 1
-                    for (int kk = 0; kk < kBK / 16; ++kk)
-                        mma_pair<0, 0>(tmem_base, sbase, kk, first && kk == 0, idesc);
+                    const uint64_t d0 = smem_desc(smem_u32(smem + stage * kStageBytes), kSBO, kSwizzle128);
+                    const uint32_t lo = static_cast<uint32_t>(d0);
+                    mma_pair<0, 0>(tmem_base, lo, lo + 2 * (kABox / 16), static_cast<uint32_t>(d0 >> 32), first ? 0u : 1u,
+                                   idesc);
                     mma_commit(&empty[stage]);
                     if (++stage == kStages) { stage = 0; phase ^= 1u; }
                     if ((kb + 1) % kChunkKb == 0 || kb + 1 == n_kb) {
@@ -390,16 +370,15 @@ constexpr int kST = 64, kSK = 16, kSThreads = 256;
 // The 64 x 64 tiles of C whose digit tiles are not good, in FP64 (one block per tile; the others leave at once).
 __global__ void __launch_bounds__(kSThreads)
 k_marked_f64(const OzArgs args, const double* __restrict__ Xa, int64_t lda, int64_t xa_stride,
-             const double* __restrict__ Xb, int64_t ldb, int64_t xb_stride, int square_b1) {
+             const double* __restrict__ Xb, int64_t ldb, int square0, int square1) {
     const int b = blockIdx.z;
     const int i0 = blockIdx.y * kST, j0 = blockIdx.x * kST;
     if (tile_good(args, Tile{b, i0 / kOzRowsA, j0 / kOzRowsB})) return;
     __shared__ double As[kSK][kST + 1];
     __shared__ double Bs[kSK][kST + 1];
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const bool sq = square_b1 && b == 1;
+    const bool sq = (b == 0 ? square0 : square1) != 0;
     const double* A = Xa + b * xa_stride;
-    const double* B = Xb + b * xb_stride;
     double acc[4][4] = {};
     for (int k0 = 0; k0 < args.K; k0 += kSK) {
 #pragma unroll
@@ -407,7 +386,7 @@ k_marked_f64(const OzArgs args, const double* __restrict__ Xa, int64_t lda, int6
             const int t = tid + l * kSThreads, r = t / kSK, k = t % kSK;
             const bool kin = k0 + k < args.K;
             As[k][r] = (kin && i0 + r < args.Ma) ? A[static_cast<int64_t>(i0 + r) * lda + k0 + k] : 0.0;
-            const double v = (kin && j0 + r < args.Nb) ? B[static_cast<int64_t>(j0 + r) * ldb + k0 + k] : 0.0;
+            const double v = (kin && j0 + r < args.Nb) ? Xb[static_cast<int64_t>(j0 + r) * ldb + k0 + k] : 0.0;
             Bs[k][r] = sq ? mul_rn(v, v) : v;
         }
         __syncthreads();
@@ -446,14 +425,14 @@ size_t align_up(size_t n) { return (n + 1023) / 1024 * 1024; }
 namespace flmm {
 
 size_t oz_operand_bytes(int rows, int K, int batches, int tile_rows) {
-    const size_t ldp = (static_cast<size_t>(K) + 7) / 8 * 8, n = static_cast<size_t>(rows) * batches;
+    const size_t ldp = (static_cast<size_t>(K) + kBK - 1) / kBK * kRowElems, n = static_cast<size_t>(rows) * batches;
     const size_t tiles = static_cast<size_t>((rows + tile_rows - 1) / tile_rows) * batches;
-    return align_up(sizeof(__half) * kOzPlanes * n * ldp) + align_up(sizeof(int) * n) + align_up(sizeof(float) * tiles);
+    return align_up(sizeof(__half) * n * ldp) + align_up(sizeof(int) * n) + align_up(sizeof(float) * tiles);
 }
 
 OzOperand oz_carve(void* base, int rows, int K, int batches, int tile_rows) {
     OzOperand op;
-    op.ldp = (static_cast<int64_t>(K) + 7) / 8 * 8;
+    op.ldp = (static_cast<int64_t>(K) + kBK - 1) / kBK * kRowElems;
     op.rows = rows;
     op.K = K;
     op.batches = batches;
@@ -461,7 +440,7 @@ OzOperand oz_carve(void* base, int rows, int K, int batches, int tile_rows) {
     const size_t n = static_cast<size_t>(rows) * batches;
     char* p = static_cast<char*>(base);
     op.planes = reinterpret_cast<__half*>(p);
-    p += align_up(sizeof(__half) * kOzPlanes * n * op.ldp);
+    p += align_up(sizeof(__half) * n * op.ldp);
     op.expo = reinterpret_cast<int*>(p);
     p += align_up(sizeof(int) * n);
     op.qual = reinterpret_cast<float*>(p);
@@ -471,28 +450,28 @@ OzOperand oz_carve(void* base, int rows, int K, int batches, int tile_rows) {
 int oz_digits(const OzOperand& op, int b, const double* X, int64_t ldx, bool square, cudaStream_t st) {
     if (op.rows == 0) return FLMM_OK;
     const int64_t off = static_cast<int64_t>(b) * op.rows;
-    const int64_t plane_stride = static_cast<int64_t>(op.batches) * op.rows * op.ldp;
     float* qual = op.qual + static_cast<int64_t>(b) * op.tiles();
     k_zero_f32<<<ceil_div(op.tiles(), 256), 256, 0, st>>>(qual, op.tiles());
     int rc = check_launch("k_zero_f32");
     if (rc) return rc;
     auto* k = square ? k_digits64<true> : k_digits64<false>;
     k<<<ceil_div(static_cast<int64_t>(op.rows) * 32, 256), 256, 0, st>>>(
-        X, ldx, op.rows, op.K, op.planes + off * op.ldp, op.ldp, plane_stride, op.expo + off, qual, op.tile_rows);
+        X, ldx, op.rows, op.K, op.planes + off * op.ldp, op.ldp, op.expo + off, qual, op.tile_rows);
     return check_launch("k_digits64");
 }
 
 int oz_gemm(const OzOperand& A, const OzOperand& B, const OzProduct& p, cudaStream_t st) {
     if (A.rows == 0 || B.rows == 0) return FLMM_OK;
-    if (A.batches > 2 || A.batches != B.batches || A.K != B.K) return fail(FLMM_ERR_ARG, "oz_gemm: operands differ");
-    const int64_t ra = static_cast<int64_t>(A.rows) * A.batches * kOzPlanes;
-    const int64_t rb = static_cast<int64_t>(B.rows) * B.batches * kOzPlanes;
-    if (ra > 0x7fffffffLL || rb > 0x7fffffffLL) return fail(FLMM_ERR_ARG, "oz_gemm: too many rows for a TMA map");
+    if (A.batches > 2 || B.batches > 2 || A.K != B.K) return fail(FLMM_ERR_ARG, "oz_gemm: operands differ");
+    const int64_t ra = static_cast<int64_t>(A.rows) * A.batches, rb = static_cast<int64_t>(B.rows) * B.batches;
+    if (ra > 0x7fffffffLL || rb > 0x7fffffffLL || A.ldp > 0x7fffffffLL)
+        return fail(FLMM_ERR_ARG, "oz_gemm: too large for a TMA map");
     OzMaps maps;
     std::memset(&maps, 0, sizeof(maps));
     int rc;
-    if ((rc = tc::make_map_f16(&maps.a, A.planes, static_cast<int>(ra), A.K, A.ldp, kBK, kOzRowsA))) return rc;
-    if ((rc = tc::make_map_f16(&maps.b, B.planes, static_cast<int>(rb), B.K, B.ldp, kBK, kOzRowsB))) return rc;
+    const int w = static_cast<int>(A.ldp);
+    if ((rc = tc::make_map_f16(&maps.a, A.planes, static_cast<int>(ra), w, A.ldp, kRowElems / 2, kOzRowsA))) return rc;
+    if ((rc = tc::make_map_f16(&maps.b, B.planes, static_cast<int>(rb), w, B.ldp, kRowElems / 2, kOzRowsB))) return rc;
     static std::once_flag once;
     static cudaError_t attr_rc = cudaSuccess;
     std::call_once(once, [] {
@@ -508,16 +487,16 @@ int oz_gemm(const OzOperand& A, const OzOperand& B, const OzProduct& p, cudaStre
     a.Ma = A.rows;
     a.Nb = B.rows;
     a.K = A.K;
-    a.batches = A.batches;
+    a.batches = A.batches < B.batches ? A.batches : B.batches;
     a.tiles_i = A.tiles();
     a.tiles_m = B.tiles();
     a.ea = A.expo;
     a.eb = B.expo;
     a.qa = A.qual;
     a.qb = B.qual;
-    a.limit[0] = quality_limit(A.K);
     // a sum of products of non-negative numbers grows with its length, and with it an FP64 sum's own rounding
-    a.limit[1] = p.square_b1 ? 4.0f * a.limit[0] : a.limit[0];
+    for (int b = 0; b < 2; ++b)
+        a.limit[b] = p.any_ratio ? FLT_MAX : quality_limit(A.K) * (p.square[b] ? 4.0f : 1.0f);
     a.C = p.C;
     a.ldc = p.ldc;
     a.c_stride = p.c_stride;
@@ -527,7 +506,7 @@ int oz_gemm(const OzOperand& A, const OzOperand& B, const OzProduct& p, cudaStre
     k_oz64<<<static_cast<int>(tiles < sm ? tiles : sm), kThreads, kSmemBytes, st>>>(maps, a);
     if ((rc = check_launch("k_oz64"))) return rc;
     const dim3 grid(ceil_div(B.rows, kST), ceil_div(A.rows, kST), a.batches);
-    k_marked_f64<<<grid, kSThreads, 0, st>>>(a, p.Xa, p.lda, p.xa_stride, p.Xb, p.ldb, p.xb_stride, p.square_b1);
+    k_marked_f64<<<grid, kSThreads, 0, st>>>(a, p.Xa, p.lda, p.xa_stride, p.Xb, p.ldb, p.square[0], p.square[1]);
     return check_launch("k_marked_f64");
 }
 

@@ -12,9 +12,11 @@ constexpr int kOzPlanes = 8;      // 7-bit digit planes per operand (55 bits bel
 constexpr int kOzRowsA = 128;     // A rows per tile
 constexpr int kOzRowsB = 64;      // B rows per tile
 
-// One operand: `batches` stacked matrices of (rows, K) as digit planes, row exponents and tile qualities.
+// One operand: `batches` stacked matrices of (rows, K) as digit planes, row exponents and tile qualities.  A row keeps
+// the eight digits of every 16 elements together, [k / 16][plane][k % 16], so that a stage of the product reads 256
+// contiguous bytes of it (zeros from K to the next multiple of 16).
 struct OzOperand {
-    __half* planes;   // [plane][batch][row][ldp]
+    __half* planes;   // [batch][row][ldp]
     int* expo;        // [batch][row]
     float* qual;      // [batch][tile]: largest max|x| / rms(x) of a tile's rows, infinity where digits cannot hold a row
     int64_t ldp;
@@ -29,20 +31,31 @@ OzOperand oz_carve(void* base, int rows, int K, int batches, int tile_rows);
 int oz_digits(const OzOperand& op, int b, const double* X, int64_t ldx, bool square, cudaStream_t st);
 
 // C[b] (rows of A, rows of B; pitch ldc, batch stride c_stride) = A[b] B[b]^T, or D - A B^T where D is given (pitch
-// ldd).  Xa, Xb: the FP64 matrices the digits were taken from (batch strides xa_stride, xb_stride; batch 1 of Xb is
-// the squares of Xb itself where square_b1 is set), read where a tile's digits are not good enough.
+// ldd).  Xa, Xb: the FP64 matrices the digits were taken from (Xa with a batch stride; Xb shared by the batches, its
+// elements squared in batch b where square[b] is set), read where a tile's digits are not good enough.  any_ratio: take
+// every finite row whatever its max/rms (for sums whose error only has to be small against the product of the row norms).
+// Operands may hold more batches than the product takes; it takes the smaller count, from batch 0.
 struct OzProduct {
     const double* Xa;
     int64_t lda, xa_stride;
     const double* Xb;
-    int64_t ldb, xb_stride;
-    bool square_b1;
+    int64_t ldb;
+    bool square[2];
+    bool any_ratio;
     double* C;
     int64_t ldc, c_stride;
     const double* D;
     int64_t ldd;
 };
 int oz_gemm(const OzOperand& A, const OzOperand& B, const OzProduct& p, cudaStream_t st);
+
+// The Wald epilogue over the sums of P columns x Mc variants (flmm_wald_f64.cu), pitch ldg: a column's sWy in its row of
+// Gy, sWs in its row of Gs, and in the GLS form the nq terms whose squares add to B^T A^-1 B in nq rows of Gq (nq = 0 in
+// the compat form).  F, beta, SE, SFVE of the first n_real columns into rows `rows` of the outputs, column maxima into
+// max_F.
+int wald_finish(const double* Gy, const double* Gs, const double* Gq, int nq, int64_t ldg, const double* rWr, double var_df, int P,
+                int n_real, int Mc, const int64_t* rows, double* f, double* beta, double* se, double* sfve, int64_t ldo,
+                double* max_F, cudaStream_t st);
 
 // Products below this many multiply-adds stay on the FP64 pipe.
 bool oz_worth(int64_t Mr, int64_t Nr, int64_t K);

@@ -148,17 +148,19 @@ __device__ __forceinline__ Test wald_test(double swy, double sws, double rwr, do
     return t;
 }
 
-// Epilogue over the sums of a (Pc, Mc) block, G[0] = sWy and G[1] = sWs (pitch ldg, batch stride g_stride): a block
-// takes 32 columns x kFinM variants in tiles of 64, transposed through shared memory so that the reads run along the
+// Epilogue over the sums of a block of columns and variants (layout: flmm_oz64.cuh): a thread block takes 32 columns x
+// kFinM variants in tiles of 64, transposed through shared memory so that the reads run along the
 // variants and the detail stores along the columns.  Real columns get the full epilogue.  A permutation column needs its
 // largest F only, and F grows with q / denom, so its tests are ranked by cross-multiplication (three FP64 operations
 // instead of four divisions; GB300's FP64 pipe is the bound here) and one F is formed per thread; sums outside
 // 1e-100 .. 1e100, and NaN, take the full formula.
 constexpr int kFinP = 32, kFinTile = 64, kFinM = 256;
 
+template <bool GLS>
 __global__ void __launch_bounds__(256)
-k_wald_finish(const double* __restrict__ G, int64_t ldg, int64_t g_stride, const double* __restrict__ rWr,
-              double var_df, int P, int n_real, int Mc, const int64_t* __restrict__ rows, double* __restrict__ f,
+k_wald_finish(const double* __restrict__ Gy, const double* __restrict__ Gs, const double* __restrict__ Gq, int nq,
+              int64_t ldg,
+              const double* __restrict__ rWr, double var_df, int P, int n_real, int Mc, const int64_t* __restrict__ rows, double* __restrict__ f,
               double* __restrict__ beta, double* __restrict__ se, double* __restrict__ sfve, int64_t ldo,
               double* __restrict__ max_F) {
     __shared__ double sy[kFinP][kFinTile + 1];
@@ -178,8 +180,15 @@ k_wald_finish(const double* __restrict__ G, int64_t ldg, int64_t g_stride, const
             const int t = tid + l * 256, r = t / kFinTile, c = t % kFinTile;
             if (p0 + r < P && m0 + c < m_end) {
                 const int64_t o = static_cast<int64_t>(p0 + r) * ldg + m0 + c;
-                sy[r][c] = G[o];
-                ss[r][c] = G[g_stride + o];
+                sy[r][c] = Gy[o];
+                double w = Gs[o];
+                if (GLS) {
+                    const double* g = Gq + static_cast<int64_t>(p0 + r) * nq * ldg + m0 + c;
+                    double quad = 0.0;
+                    for (int k = 0; k < nq; ++k) quad = fma(g[k * ldg], g[k * ldg], quad);
+                    w = add_rn(w, -quad);
+                }
+                ss[r][c] = w;
             }
         }
         __syncthreads();
@@ -269,6 +278,15 @@ size_t wald_ws(int P, int Neff) { return carve_wald(nullptr, P, Neff).bytes; }
 
 }  // namespace
 
+int flmm::wald_finish(const double* Gy, const double* Gs, const double* Gq, int nq, int64_t ldg, const double* rWr,
+                      double var_df, int P, int n_real, int Mc, const int64_t* rows, double* f, double* beta, double* se,
+                      double* sfve, int64_t ldo, double* max_F, cudaStream_t st) {
+    const dim3 grid(ceil_div(Mc, kFinM), ceil_div(P, kFinP));
+    auto* k = nq > 0 ? k_wald_finish<true> : k_wald_finish<false>;
+    k<<<grid, 256, 0, st>>>(Gy, Gs, Gq, nq, ldg, rWr, var_df, P, n_real, Mc, rows, f, beta, se, sfve, ldo, max_F);
+    return check_launch("k_wald_finish");
+}
+
 extern "C" int flmm_wald_f64_workspace_bytes(int P, int Neff, size_t* bytes) {
     FLMM_REQUIRE(bytes && P >= 0 && Neff > 0, "flmm_wald_f64_workspace_bytes: bad arguments");
     *bytes = wald_ws(P, Neff);
@@ -326,12 +344,12 @@ int wald_impl(const double* s, int Neff, const double* UYt, int64_t ldu, const d
             if ((rc = oz_digits(vars, 0, US, ldus, false, st))) return rc;
             if ((rc = oz_digits(vars, 1, US, ldus, true, st))) return rc;
             const int64_t gs = static_cast<int64_t>(pc) * mc;
-            const OzProduct prod{w.A1, Neff, static_cast<int64_t>(pc) * Neff, US, ldus, 0, true, w.G, mc, gs, nullptr, 0};
+            const OzProduct prod{w.A1, Neff, static_cast<int64_t>(pc) * Neff, US, ldus, {false, true}, false, w.G, mc,
+                                 gs, nullptr, 0};
             if ((rc = oz_gemm(cols, vars, prod, st))) return rc;
-            const dim3 grid(ceil_div(mc, kFinM), ceil_div(pc, kFinP));
-            k_wald_finish<<<grid, 256, 0, st>>>(w.G, mc, gs, w.rWr, var_df, pc, nr, mc, rows ? rows + m0 : rows, out(f),
-                                                out(beta), out(se), out(sfve), ldo, max_F + p0);
-            if ((rc = check_launch("k_wald_finish"))) return rc;
+            if ((rc = wald_finish(w.G, w.G + gs, nullptr, 0, mc, w.rWr, var_df, pc, nr, mc, rows ? rows + m0 : rows, out(f),
+                                  out(beta), out(se), out(sfve), ldo, max_F + p0, st)))
+                return rc;
         }
     }
     return FLMM_OK;

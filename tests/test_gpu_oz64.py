@@ -141,3 +141,33 @@ def test_wald_keeps_nan():
     nan[3] = nan[150] = True
     assert torch.equal(torch.isnan(max_F), nan)
     assert torch.equal(torch.isnan(out["f"]).any(0), nan[:10])
+
+
+@pytest.mark.parametrize("P,Mc,N,C,n_real", [(3, 40, 50, 1, 3), (70, 300, 333, 5, 70), (130, 257, 500, 12, 1),
+                                             (900, 4100, 120, 5, 17), (40, 600, 400, 30, 40)])
+def test_gls_wald_blocks(P, Mc, N, C, n_real):
+    """flmm_wald_gls_f64 over its blocks, on either path, against the formulas in FP64."""
+    from fasterlmm_gb300 import build, core, gls
+    build()
+    g = torch.Generator(device="cuda").manual_seed(P + Mc + C)
+    dev = torch.device("cuda", torch.cuda.current_device())
+    rn = lambda *s: torch.randn(*s, generator=g, device=dev, dtype=torch.float64)
+    s, X, Y, S, ld = rn(N).abs() + 0.05, rn(C, N), rn(P, N), rn(Mc, N), rn(P)
+    out, max_F = core._alloc_outputs(Mc, n_real, P, dev)
+    rows = torch.randperm(Mc, generator=g, device=dev)
+    gls.wald_t(s, X, Y, ld, S, n_real, rows, out, max_F)
+    w = 1.0 / (s[None, :] + ld.exp()[:, None])
+    L = torch.linalg.cholesky(torch.einsum("pn,cn,dn->pcd", w, X, X))
+    u = torch.einsum("pn,cn,pn->pc", w, X, Y)
+    r = Y - torch.cholesky_solve(u[:, :, None], L)[:, :, 0] @ X
+    z = torch.linalg.solve_triangular(L, torch.einsum("pn,cn,mn->pcm", w, X, S), upper=False)
+    num, den, rwr = (w * r) @ S.T, (w @ (S * S).T) - (z * z).sum(1), (w * r * r).sum(1)
+    var = (rwr[:, None] - num * num / den) / (N - C - 1) / den
+    F = (num / den) ** 2 / var
+    close = lambda x, y: torch.testing.assert_close(x, y, rtol=1e-9, atol=1e-12)
+    close(max_F, F.max(1).values)
+    q = slice(0, n_real)
+    close(out["f"][rows], F[q].T)
+    close(out["beta"][rows], (num / den)[q].T)
+    close(out["se"][rows], var[q].sqrt().T)
+    close(out["sfve"][rows], (num * num / (den * rwr[:, None]))[q].sqrt().T)
