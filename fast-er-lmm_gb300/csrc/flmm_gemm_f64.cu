@@ -120,11 +120,11 @@ extern "C" int flmm_gemm_nt_f64_tc(const double* A, int64_t lda, const double* B
     char* wb = wa + oz_operand_bytes(ra, K, 1, kOzRowsA);
     for (int j0 = 0; j0 < Nr; j0 += rb) {
         const OzOperand b = oz_carve(wb, Nr - j0 < rb ? Nr - j0 : rb, K, 1, kOzRowsB);
-        int rc = oz_digits(b, 0, B + j0 * ldb, ldb, false, st);
+        int rc = oz_digits(b, 0, B + j0 * ldb, ldb, false, nullptr, 0, st);
         if (rc) return rc;
         for (int i0 = 0; i0 < Mr; i0 += ra) {
             const OzOperand a = oz_carve(wa, Mr - i0 < ra ? Mr - i0 : ra, K, 1, kOzRowsA);
-            if ((rc = oz_digits(a, 0, A + i0 * lda, lda, false, st))) return rc;
+            if ((rc = oz_digits(a, 0, A + i0 * lda, lda, false, nullptr, 0, st))) return rc;
             const OzProduct p{A + i0 * lda, lda, 0, B + j0 * ldb, ldb, {false, false}, false, C + i0 * ldc + j0, ldc, 0,
                               D ? D + i0 * ldd + j0 : nullptr, ldd};
             if ((rc = oz_gemm(a, b, p, st))) return rc;

@@ -512,6 +512,7 @@ struct WaldWs {
     double *RW, *Q, *rWr;   // w o r and w (2, pc, N), L^-1 X~^T W (pc, C, N)
     double *G, *Gq;         // sums: num and sWs (2, pc, mc), the quadratic form's terms (pc, C, mc)
     char *rw_op, *q_op, *s_op;
+    int* bal;               // balancing exponents, N
     size_t bytes;
 };
 
@@ -539,6 +540,7 @@ WaldWs carve_wald(void* base, int N, int C, int P) {
     w.rw_op = reinterpret_cast<char*>(take(oz_operand_bytes(w.pc, N, 2, kOzRowsA)));
     w.q_op = reinterpret_cast<char*>(take(oz_operand_bytes(w.pc * C, N, 1, kOzRowsA)));
     w.s_op = reinterpret_cast<char*>(take(oz_operand_bytes(w.mc, N, 2, kOzRowsB)));
+    w.bal = reinterpret_cast<int*>(take(sizeof(int) * n));
     w.bytes = off + 1024;
     return w;
 }
@@ -677,6 +679,9 @@ extern "C" int flmm_wald_gls_f64(const double* s, int N, const double* Xrt, int6
     // variants x 800 samples, C = 5: 33.9 ms).
     const WaldWs w = carve_wald(work, N, C, P);
     if (oz_worth(static_cast<int64_t>(w.pc) * (C + 2), M < w.mc ? M : w.mc, N)) {
+        // (the rotated intercept is one entry, where every centred variant is ~0 and w largest: balanced, it no longer
+        // sets its rows' resolution)
+        if ((rc = oz_balance(Srt, lds, M, N, w.bal, st))) return rc;
         for (int p0 = 0; p0 < P; p0 += w.pc) {
             const int pc = P - p0 < w.pc ? P - p0 : w.pc;
             const int nr = n_real > p0 ? (n_real - p0 < pc ? n_real - p0 : pc) : 0;
@@ -686,19 +691,18 @@ extern "C" int flmm_wald_gls_f64(const double* s, int N, const double* Xrt, int6
                 w.Q, static_cast<int64_t>(C) * N, nullptr, w.rWr);
             if ((rc = check_launch("k_gls_wald_prep"))) return rc;
             const OzOperand rw = oz_carve(w.rw_op, pc, N, 2, kOzRowsA), qo = oz_carve(w.q_op, pc * C, N, 1, kOzRowsA);
-            if ((rc = oz_digits(rw, 0, w.RW, N, false, st))) return rc;
-            if ((rc = oz_digits(rw, 1, w.RW + half, N, false, st))) return rc;
-            if ((rc = oz_digits(qo, 0, w.Q, N, false, st))) return rc;
+            if ((rc = oz_digits(rw, 0, w.RW, N, false, w.bal, 1, st))) return rc;
+            if ((rc = oz_digits(rw, 1, w.RW + half, N, false, w.bal, 2, st))) return rc;
+            if ((rc = oz_digits(qo, 0, w.Q, N, false, w.bal, 1, st))) return rc;
             auto out = [&](double* x) { return nr > 0 ? x + p0 : nullptr; };
             for (int m0 = 0; m0 < M; m0 += w.mc) {
                 const int mc = M - m0 < w.mc ? M - m0 : w.mc;
                 const double* S = Srt + m0 * lds;
                 const OzOperand so = oz_carve(w.s_op, mc, N, 2, kOzRowsB);
-                if ((rc = oz_digits(so, 0, S, lds, false, st))) return rc;
-                if ((rc = oz_digits(so, 1, S, lds, true, st))) return rc;
+                if ((rc = oz_digits(so, 0, S, lds, false, w.bal, -1, st))) return rc;
+                if ((rc = oz_digits(so, 1, S, lds, true, w.bal, -2, st))) return rc;
                 const OzProduct g{w.RW, N, half, S, lds, {false, true}, false, w.G, mc, gs, nullptr, 0};
-                // (the terms enter as squares subtracted from sWs: an error small against the row norms is enough, and
-                // the rotated intercept's row is one entry)
+                // what is left of the intercept's row is rounding of either input: any ratio will do
                 const OzProduct gq{w.Q, N, 0, S, lds, {false, false}, true, w.Gq, mc, 0, nullptr, 0};
                 if ((rc = oz_gemm(rw, so, g, st))) return rc;
                 if ((rc = oz_gemm(qo, so, gq, st))) return rc;

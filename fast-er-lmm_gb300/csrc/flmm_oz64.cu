@@ -14,7 +14,7 @@
 // What is lost is the rounding to 55 bits and the levels from 8 on (weight 2^-56 against the row maxima).  For rows
 // whose largest entry is a few times their rms this is several times smaller than the rounding of an FP64 sum of K
 // terms (~0.4 * 2^-53 * K times the rms product; measured against exact sums in tests/test_gpu_oz64.py).  The loss
-// grows with max/rms of both rows, so every tile of rows carries its largest ratio; a tile pair whose product of
+// grows with max/rms of both rows (after balancing, oz_balance), so every tile of rows carries its largest ratio; a tile pair whose product of
 // ratios exceeds quality_limit(K), and any row that is not finite or whose exponent is out of range, is left to
 // k_marked_f64, which forms those tiles on the FP64 pipe as before.
 //
@@ -83,22 +83,46 @@ struct OzArgs {
 
 // ---- digits ---------------------------------------------------------------------------------------------------
 
-// One warp per row.  Pass 1: the row's largest |x| as its bit pattern (integer maximum); pass 2: the 55-bit integer
-// of every element, its digits by integer shifts, packed two elements to a word (1536 + d is exact in FP16 with unit
-// spacing, so subtracting 1536 leaves the digit).  16 bytes written per 8 read: bandwidth-bound.
+constexpr int kMaxBalance = 150;  // |e_k| used at most
+
+// bal[k] = largest high word of |X[., k]| (k_balance), then its exponent (k_balance_exp).  A block reads 32 columns of a
+// range of rows.
+__global__ void __launch_bounds__(256)
+k_balance(const double* __restrict__ X, int64_t ldx, int rows, int K, int* __restrict__ bal) {
+    const int k = blockIdx.x * 32 + (threadIdx.x & 31);
+    if (k >= K) return;
+    int m = 0;
+    for (int64_t r = blockIdx.y * 8 + (threadIdx.x >> 5); r < rows; r += gridDim.y * 8)
+        m = max(m, __double2hiint(X[r * ldx + k]) & 0x7fffffff);
+    atomicMax(bal + k, m);
+}
+
+__global__ void k_balance_exp(int* __restrict__ bal, int K) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < K) bal[k] = max(-kMaxBalance, min(kMaxBalance, (bal[k] >> 20) - 1023));
+}
+
+// One warp per row.  Pass 1: the row's largest |x 2^c| (c = times bal_k) as its bit pattern (integer maximum); pass 2: the
+// 55-bit integer of every element, its digits by integer shifts, packed two elements to a word (1536 + d is exact in FP16
+// with unit spacing, so subtracting 1536 leaves the digit).  16 bytes written per 8 read: bandwidth-bound.
 template <bool SQ>
 __global__ void __launch_bounds__(256)
-k_digits64(const double* __restrict__ X, int64_t ldx, int rows, int K, __half* __restrict__ planes, int64_t ldp,
-           int* __restrict__ expo, float* __restrict__ qual, int tile_rows) {
+k_digits64(const double* __restrict__ X, int64_t ldx, int rows, int K, const int* __restrict__ bal, int times,
+           __half* __restrict__ planes, int64_t ldp, int* __restrict__ expo, float* __restrict__ qual, int tile_rows) {
     const int lane = threadIdx.x & 31;
     const int64_t j = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5;
     if (j >= rows) return;
     const double* x = X + j * ldx;
+    constexpr unsigned long long kInf = 0x7ff0000000000000ull;
     unsigned long long mb = 0;
     for (int n = lane; n < K; n += 32) {
         double v = x[n];
         if (SQ) v = mul_rn(v, v);
-        const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(v)) & 0x7fffffffffffffffull;
+        unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(v)) & 0x7fffffffffffffffull;
+        const int eb = static_cast<int>(b >> 52) + (bal ? times * bal[n] : 0);  // biased exponent of x 2^c
+        if (b >= kInf || eb >= 0x7ff) b = kInf;
+        else if (eb > 0 && b >> 52) b = (b & 0xfffffffffffffull) | (static_cast<unsigned long long>(eb) << 52);
+        else b = b != 0;  // denormal: below every usable exponent, above zero
         mb = b > mb ? b : mb;
     }
 #pragma unroll
@@ -108,7 +132,6 @@ k_digits64(const double* __restrict__ X, int64_t ldx, int rows, int K, __half* _
     }
     const int e = mb == 0 ? 0 : static_cast<int>(mb >> 52) - 1022;  // max = f 2^e, f in [0.5, 1)
     const bool bad = e > kMaxExp || e < -kMaxExp;                   // includes infinities, NaN and denormals
-    const double up = __longlong_as_double(static_cast<long long>(1023 + 55 - (bad ? 0 : e)) << 52);
     __half* out = planes + j * ldp;
     float ss = 0.0f;
     for (int n = 2 * lane; n < (K + kBK - 1) / kBK * kBK; n += 64) {
@@ -119,7 +142,8 @@ k_digits64(const double* __restrict__ X, int64_t ldx, int rows, int K, __half* _
                 if (n + h >= K) continue;
                 double y = x[n + h];
                 if (SQ) y = mul_rn(y, y);
-                v[h] = __double2ll_rn(y * up);
+                const int up = 1023 + 55 - e + (bal ? times * bal[n + h] : 0);
+                v[h] = __double2ll_rn(y * __longlong_as_double(static_cast<long long>(up) << 52));
                 const float t = static_cast<float>(static_cast<int>(v[h] >> 32)) * 0x1p-23f;
                 ss = fmaf(t, t, ss);
             }
@@ -447,7 +471,18 @@ OzOperand oz_carve(void* base, int rows, int K, int batches, int tile_rows) {
     return op;
 }
 
-int oz_digits(const OzOperand& op, int b, const double* X, int64_t ldx, bool square, cudaStream_t st) {
+int oz_balance(const double* X, int64_t ldx, int rows, int K, int* bal, cudaStream_t st) {
+    FLMM_CUDA(cudaMemsetAsync(bal, 0, sizeof(int) * K, st));
+    const int by = (rows + 63) / 64;
+    k_balance<<<dim3(ceil_div(K, 32), by < 1 ? 1 : (by < 64 ? by : 64)), 256, 0, st>>>(X, ldx, rows, K, bal);
+    int rc = check_launch("k_balance");
+    if (rc) return rc;
+    k_balance_exp<<<ceil_div(K, 256), 256, 0, st>>>(bal, K);
+    return check_launch("k_balance_exp");
+}
+
+int oz_digits(const OzOperand& op, int b, const double* X, int64_t ldx, bool square, const int* bal, int times,
+              cudaStream_t st) {
     if (op.rows == 0) return FLMM_OK;
     const int64_t off = static_cast<int64_t>(b) * op.rows;
     float* qual = op.qual + static_cast<int64_t>(b) * op.tiles();
@@ -456,7 +491,7 @@ int oz_digits(const OzOperand& op, int b, const double* X, int64_t ldx, bool squ
     if (rc) return rc;
     auto* k = square ? k_digits64<true> : k_digits64<false>;
     k<<<ceil_div(static_cast<int64_t>(op.rows) * 32, 256), 256, 0, st>>>(
-        X, ldx, op.rows, op.K, op.planes + off * op.ldp, op.ldp, op.expo + off, qual, op.tile_rows);
+        X, ldx, op.rows, op.K, bal, times, op.planes + off * op.ldp, op.ldp, op.expo + off, qual, op.tile_rows);
     return check_launch("k_digits64");
 }
 

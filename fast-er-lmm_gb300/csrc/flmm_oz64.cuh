@@ -27,8 +27,14 @@ struct OzOperand {
 size_t oz_operand_bytes(int rows, int K, int batches, int tile_rows);
 OzOperand oz_carve(void* base, int rows, int K, int batches, int tile_rows);
 
-// Digits of batch `b` of `op` from the rows of X (pitch ldx), or of their squares.
-int oz_digits(const OzOperand& op, int b, const double* X, int64_t ldx, bool square, cudaStream_t st);
+// Balancing exponents of a product's reduction: e_k of the largest |X[., k]| over the rows of X (pitch ldx), K ints.  A
+// product's operands may be digitised as A 2^e_k and B 2^-e_k (both squared where B is): the digits then resolve each
+// term against the largest term that the variants leave possible at k, not against an entry of A that meets zeros.
+int oz_balance(const double* X, int64_t ldx, int rows, int K, int* bal, cudaStream_t st);
+
+// Digits of batch `b` of `op` from the rows of X (pitch ldx), or of their squares, times 2^(times bal_k).
+int oz_digits(const OzOperand& op, int b, const double* X, int64_t ldx, bool square, const int* bal, int times,
+              cudaStream_t st);
 
 // C[b] (rows of A, rows of B; pitch ldc, batch stride c_stride) = A[b] B[b]^T, or D - A B^T where D is given (pitch
 // ldd).  Xa, Xb: the FP64 matrices the digits were taken from (Xa with a batch stride; Xb shared by the batches, its

@@ -171,3 +171,22 @@ def test_gls_wald_blocks(P, Mc, N, C, n_real):
     close(out["beta"][rows], (num / den)[q].T)
     close(out["se"][rows], var[q].sqrt().T)
     close(out["sfve"][rows], (num * num / (den * rwr[:, None]))[q].sqrt().T)
+
+
+def test_weights_that_meet_zeros():
+    """A direction whose weight is 2e4 times the others' and where every variant is 0 (the rotated intercept at a small
+    delta) must not cost the other directions their digits: SE, which is a sum of w s^2, keeps FP64's exactness."""
+    from fasterlmm_gb300 import build, core
+    build()
+    g = torch.Generator(device="cuda").manual_seed(9)
+    dev = torch.device("cuda", torch.cuda.current_device())
+    rn = lambda *s: torch.randn(*s, generator=g, device=dev, dtype=torch.float64)
+    P, Mc, Neff = 130, 700, 400
+    s, UY, US, ld = rn(Neff).abs() + 1.0, rn(P, Neff), rn(Mc, Neff), torch.full((P,), -10.0, device=dev, dtype=torch.float64)
+    s[0], UY[:, 0], US[:, 0] = 0.0, 0.0, 0.0
+    out, max_F = core._alloc_outputs(Mc, P, P, dev)
+    core.wald_t(s, UY, ld, US, P, torch.arange(Mc, device=dev), out, max_F)
+    w = 1.0 / (s[None, :] + ld.exp()[:, None])
+    num, den, rwr = (w * UY) @ US.T, w @ (US * US).T, (w * UY * UY).sum(1)
+    se = ((rwr[:, None] - num * num / den) / (Neff - 1) / den).sqrt()
+    torch.testing.assert_close(out["se"], se.T, rtol=1e-14, atol=0)
