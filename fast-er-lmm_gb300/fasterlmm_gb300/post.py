@@ -50,15 +50,15 @@ def perm_threshold_p(perm_max_F: Tensor, df2: int, q: float = 0.05) -> Tensor:
 CHI2_1_MEDIAN = 0.45493642311957283  # scipy.stats.chi2.ppf(0.5, 1)
 
 
-def _nan_median_cols(x: Tensor) -> tuple[Tensor, Tensor]:
-    """numpy.median over the non-NaN entries of each column (mean of the two middle values for even counts)."""
+def _nan_middle_rows(x: Tensor) -> tuple[Tensor, Tensor]:
+    """The two middle order statistics (2, B) of each column's non-NaN entries (equal rows for odd counts, NaN for
+    columns without any), and the counts (B,)."""
     valid = ~torch.isnan(x)
     n = valid.sum(dim=0)
     srt = torch.sort(torch.where(valid, x, torch.full_like(x, float("inf"))), dim=0).values
-    lo = ((n - 1).clamp(min=0) // 2).unsqueeze(0)
-    hi = (n // 2).clamp(max=x.shape[0] - 1).unsqueeze(0)
-    med = 0.5 * (srt.gather(0, lo) + srt.gather(0, hi)).squeeze(0)
-    return torch.where(n > 0, med, torch.full_like(med, float("nan"))), n
+    at = torch.stack([(n - 1).clamp(min=0) // 2, (n // 2).clamp(max=x.shape[0] - 1)])
+    mid = srt.gather(0, at)
+    return torch.where(n > 0, mid, torch.full_like(mid, float("nan"))), n
 
 
 def lambda_gc(F: Tensor, df2: int) -> tuple[Tensor, Tensor]:
@@ -69,10 +69,11 @@ def lambda_gc(F: Tensor, df2: int) -> tuple[Tensor, Tensor]:
     """
     dev = _cuda_device(F)
     Fd = _f64(F, dev)
-    chisq = torch.empty_like(Fd)
-    _lib.call("flmm_chisq1_from_f", _ptr(Fd), Fd.numel(), int(df2), _ptr(chisq), _stream(dev))
-    med, n = _nan_median_cols(chisq.reshape(Fd.shape[0], -1))
-    lam = med / CHI2_1_MEDIAN
+    # the quantile grows with F (and is NaN where F is), so the median's two order statistics are those of F
+    mid, n = _nan_middle_rows(Fd.reshape(Fd.shape[0], -1))
+    chisq = torch.empty_like(mid)
+    _lib.call("flmm_chisq1_from_f", _ptr(mid), mid.numel(), int(df2), _ptr(chisq), _stream(dev))
+    lam = 0.5 * (chisq[0] + chisq[1]) / CHI2_1_MEDIAN
     if isinstance(F, Tensor) and not F.is_cuda:
         return lam.to(F.device), n.to(F.device)
     return lam, n
