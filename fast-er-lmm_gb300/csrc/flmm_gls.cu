@@ -125,30 +125,33 @@ __device__ double warp_gram(const double* __restrict__ s, int N, const double* _
     return warp_sum(sl);
 }
 
+// -2 log L from the augmented Gram Gs and sum log(s + delta), by one thread; A is scratch (C * C) and z (C).
+__device__ double gram_loss(const double* Gs, double sum_log, int N, int C, bool reml, double* A, double* z) {
+    const int K = C + 1;
+    for (int i = 0; i < C; ++i) {
+        for (int j = 0; j <= i; ++j) A[i * C + j] = Gs[i * K + j];
+        z[i] = Gs[C * K + i];
+    }
+    const bool ok = chol_lower(A, C);
+    if (!ok) set_identity(A, C);
+    double logdet = 0.0;
+    for (int i = 0; i < C; ++i) logdet += log(A[i * C + i]);
+    logdet = 2.0 * logdet;
+    forward_solve(A, C, z);
+    double uAu = 0.0;
+    for (int i = 0; i < C; ++i) uAu += z[i] * z[i];
+    return ok ? gls_loss(Gs[C * K + C], uAu, sum_log, logdet, N, C, reml) : INFINITY;
+}
+
 // One column's -2 log L at its own delta (fasterlmm/core.py:190-224), by one warp; A is per-warp scratch (C * C)
-// and z (C).  The result is valid in lane 0.
+// and z (C).
 __device__ double warp_pheno_loss(const double* __restrict__ s, int N, const double* __restrict__ Xrt, int64_t ldx,
                                   int C, const double* __restrict__ y, double ld, bool reml, double* Gs, double* A,
                                   double* z) {
     const int lane = threadIdx.x & 31;
     const double sum_log = warp_gram(s, N, Xrt, ldx, C, y, exp(ld), Gs);
     double loss = 0.0;
-    if (lane == 0) {
-        const int K = C + 1;
-        for (int i = 0; i < C; ++i) {
-            for (int j = 0; j <= i; ++j) A[i * C + j] = Gs[i * K + j];
-            z[i] = Gs[C * K + i];
-        }
-        const bool ok = chol_lower(A, C);
-        if (!ok) set_identity(A, C);
-        double logdet = 0.0;
-        for (int i = 0; i < C; ++i) logdet += log(A[i * C + i]);
-        logdet = 2.0 * logdet;
-        forward_solve(A, C, z);
-        double uAu = 0.0;
-        for (int i = 0; i < C; ++i) uAu += z[i] * z[i];
-        loss = ok ? gls_loss(Gs[C * K + C], uAu, sum_log, logdet, N, C, reml) : INFINITY;
-    }
+    if (lane == 0) loss = gram_loss(Gs, sum_log, N, C, reml, A, z);
     __syncwarp();
     return __shfl_sync(0xffffffffu, loss, 0);
 }
@@ -310,10 +313,111 @@ __global__ void k_gls_golden(const double* __restrict__ s, int N, const double* 
         a = cond ? a : c;
         c = add_rn(a, mul_rn(inv_phi2, add_rn(b, -a)));
         d = add_rn(a, mul_rn(inv_phi, add_rn(b, -a)));
+        if (it == 49) break;  // the last bracket is not compared again
         fc = warp_pheno_loss(s, N, Xrt, ldx, C, y, c, rm, Gs, A, z);
         fd = warp_pheno_loss(s, N, Xrt, ldx, C, y, d, rm, Gs, A, z);
     }
     if ((threadIdx.x & 31) == 0) log_delta[p] = fmin(fmax(mul_rn(0.5, add_rn(a, b)), lo), hi);
+}
+
+// The same search with one block per column: both evaluations of a step share the block, whose threads form the weights
+// (one division per eigenvalue; a warp of k_gls_golden forms them again for every eight products of its Gram) and
+// logarithms into shared memory, and whose warps then add the Gram's products four at a time, each sum in the order of
+// k_gls_golden's lanes and butterfly, so every loss keeps its bits.  60 columns x 300 samples, C = 5, with the grid:
+// 7.5 -> 2.3 ms.  Beyond ~6,000 samples the weights no longer fit in shared memory and k_gls_golden runs.
+constexpr int kBlockThreads = 256;
+constexpr int kBlockPairs = 4;
+
+size_t golden_block_smem(int N, int C) {
+    return sizeof(double) * (4 * static_cast<size_t>(N) +
+                             2 * (static_cast<size_t>(C + 1) * (C + 1) + static_cast<size_t>(C) * C + (C + 1)));
+}
+
+__global__ void __launch_bounds__(kBlockThreads)
+k_gls_golden_block(const double* __restrict__ s, int N, const double* __restrict__ Xrt, int64_t ldx, int C,
+                   const double* __restrict__ Yrt, int64_t ldy, const double* __restrict__ grid, int G,
+                   const int32_t* __restrict__ idx, int reml, double lo, double hi, double* __restrict__ log_delta) {
+    extern __shared__ double sm[];
+    __shared__ double delta_s[2], log_s[2], loss_s[2];
+    const int64_t p = blockIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int K = C + 1, pairs = K * (K + 1) / 2;
+    double* w = sm;           // [2][N]
+    double* lg = w + 2 * N;   // [2][N]
+    double* mats = lg + 2 * N;
+    const int per = K * K + C * C + K;
+    const double* y = Yrt + p * ldy;
+    const int i = idx[p];
+    const bool lead = tid == 0 || tid == 32;  // carry the search, one evaluation each
+    const int my_e = tid >> 5;
+    double a = grid[max(i - 1, 0)], b = grid[min(i + 1, G - 1)];
+    const double inv_phi = 2.0 / (1.0 + sqrt(5.0));
+    const double inv_phi2 = mul_rn(inv_phi, inv_phi);
+    auto narrow = [&] {
+        const double c = add_rn(a, mul_rn(inv_phi2, add_rn(b, -a))), d = add_rn(a, mul_rn(inv_phi, add_rn(b, -a)));
+        const bool cond = loss_s[0] < loss_s[1];
+        b = cond ? d : b;
+        a = cond ? a : c;
+    };
+    const int groups = (pairs + kBlockPairs - 1) / kBlockPairs;  // of products; one more sum per evaluation is the log's
+    for (int it = 0; it < 50; ++it) {
+        if (lead) {
+            if (it > 0) narrow();
+            delta_s[my_e] = exp(add_rn(a, mul_rn(my_e ? inv_phi : inv_phi2, add_rn(b, -a))));
+        }
+        __syncthreads();
+        for (int t = tid; t < 2 * N; t += kBlockThreads) {
+            const double sd = s[t < N ? t : t - N] + delta_s[t >= N];
+            w[t] = 1.0 / sd;
+            lg[t] = log(sd);
+        }
+        __syncthreads();
+        for (int g = warp; g < 2 * (groups + 1); g += kBlockThreads / 32) {
+            const int e = g > groups, q = g - e * (groups + 1);
+            const double* we = w + e * N;
+            if (q == groups) {
+                double sl = 0.0;
+                for (int n = lane; n < N; n += 32) sl += lg[e * N + n];
+                sl = warp_sum(sl);
+                if (lane == 0) log_s[e] = sl;
+                continue;
+            }
+            const double *ai[kBlockPairs], *aj[kBlockPairs];
+            int at[kBlockPairs];
+#pragma unroll
+            for (int k = 0; k < kBlockPairs; ++k) {
+                const int r = min(q * kBlockPairs + k, pairs - 1);
+                int pi = static_cast<int>((sqrtf(8.0f * r + 1.0f) - 1.0f) * 0.5f);
+                if (pi * (pi + 1) / 2 > r) --pi;
+                if ((pi + 1) * (pi + 2) / 2 <= r) ++pi;
+                const int pj = r - pi * (pi + 1) / 2;
+                at[k] = pi * K + pj;
+                ai[k] = pi < C ? Xrt + pi * ldx : y;
+                aj[k] = pj < C ? Xrt + pj * ldx : y;
+            }
+            double acc[kBlockPairs] = {};
+            for (int n = lane; n < N; n += 32) {
+                const double wn = we[n];
+#pragma unroll
+                for (int k = 0; k < kBlockPairs; ++k) acc[k] += mul_rn(mul_rn(wn, ai[k][n]), aj[k][n]);
+            }
+#pragma unroll
+            for (int k = 0; k < kBlockPairs; ++k) {
+                const double v = warp_sum(acc[k]);
+                if (lane == 0 && q * kBlockPairs + k < pairs) mats[e * per + at[k]] = v;
+            }
+        }
+        __syncthreads();
+        if (lead) {
+            double* Gs = mats + my_e * per;
+            loss_s[my_e] = gram_loss(Gs, log_s[my_e], N, C, reml != 0, Gs + K * K, Gs + K * K + C * C);
+        }
+        __syncthreads();
+    }
+    if (tid == 0) {
+        narrow();
+        log_delta[p] = fmin(fmax(mul_rn(0.5, add_rn(a, b)), lo), hi);
+    }
 }
 
 // ---- Wald ------------------------------------------------------------------------------------------------------
@@ -639,6 +743,14 @@ extern "C" int flmm_fit_delta_gls_f64(const double* s, int N, const double* Xrt,
     if ((rc = check_launch("k_gls_grid_loss"))) return rc;
     k_gls_argmin<<<ceil_div(P, 256), 256, 0, st>>>(ws.loss, n_grid, P, grid_idx);
     if ((rc = check_launch("k_gls_argmin"))) return rc;
+    const size_t block_smem = golden_block_smem(N, C);
+    if (refine && block_smem <= 200 * 1024) {
+        if (block_smem > 48 * 1024)
+            FLMM_CUDA(cudaFuncSetAttribute(k_gls_golden_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)block_smem));
+        k_gls_golden_block<<<P, kBlockThreads, block_smem, st>>>(s, N, Xrt, ldx, C, Yrt, ldy, ws.grid, n_grid, grid_idx,
+                                                                 reml, lo, hi, log_delta);
+        return check_launch("k_gls_golden_block");
+    }
     const size_t smem = eval_smem_bytes(C);
     if (smem > 48 * 1024)
         FLMM_CUDA(cudaFuncSetAttribute(k_gls_golden, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

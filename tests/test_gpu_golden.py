@@ -1,0 +1,77 @@
+"""
+The golden-section delta fits with one block per column, at the edges of their chunks of eigenvalues and of the column
+counts, against the same search in torch FP64: the losses at the two answers agree to their own rounding (sums of ~n
+terms of order 1..10: n 2^-53 relative).
+"""
+from __future__ import annotations
+
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+LO, HI, G = -10.0, 10.0, 64
+
+
+def _golden(loss, P, dev):
+    grid = torch.linspace(LO, HI, G, dtype=torch.float64, device=dev)
+    i = torch.stack([loss(x.expand(P)) for x in grid]).argmin(0)
+    a, b = grid[(i - 1).clamp(min=0)], grid[(i + 1).clamp(max=G - 1)]
+    phi = 2.0 / (1.0 + math.sqrt(5.0))
+    for _ in range(50):
+        c, d = a + phi * phi * (b - a), a + phi * (b - a)
+        left = loss(c) < loss(d)
+        b, a = torch.where(left, d, b), torch.where(left, a, c)
+    return (0.5 * (a + b)).clamp(LO, HI), i
+
+
+def _inputs(n, P, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    dev = torch.device("cuda", torch.cuda.current_device())
+    rn = lambda *s: torch.randn(*s, generator=g, device=dev, dtype=torch.float64)
+    s = rn(n).abs() * 2
+    h2 = torch.rand(P, generator=g, device=dev, dtype=torch.float64)[:, None]
+    return s, rn(P, n) * (h2 * s[None, :] + (1 - h2)).sqrt(), rn
+
+
+@pytest.mark.parametrize("n,P", [(5, 1), (31, 3), (1023, 2), (1024, 5), (1025, 2), (2049, 3), (200, 700)])
+def test_compat_fit(n, P):
+    from fasterlmm_gb300 import build, core
+    build()
+    s, UY, _ = _inputs(n, P, n + P)
+    ld, idx = core.fit_delta_t(s, UY)
+
+    def loss(x):
+        sd = s[None, :] + x.exp()[:, None]
+        return n * (math.log(2 * math.pi) + torch.log((UY * UY / sd).sum(1) / n) + 1.0) + torch.log(sd).sum(1)
+
+    want, i = _golden(loss, P, s.device)
+    assert torch.equal(idx.long(), i)
+    torch.testing.assert_close(loss(ld), loss(want), rtol=n * 2.0 ** -53, atol=1e-11)
+    coarse, _ = core.fit_delta_t(s, UY, refine=False)
+    assert torch.equal(coarse, torch.linspace(LO, HI, G, dtype=torch.float64, device=s.device)[i])
+
+
+@pytest.mark.parametrize("n,C,P", [(40, 1, 1), (257, 5, 9), (1025, 3, 2), (120, 30, 3)])
+@pytest.mark.parametrize("reml", [False, True])
+def test_gls_fit(n, C, P, reml):
+    from fasterlmm_gb300 import build, gls
+    build()
+    s, Y, rn = _inputs(n, P, n + C)
+    X = rn(C, n)
+    ld, idx = gls.fit_delta_t(s, X, Y, reml=reml)
+
+    def loss(x):
+        sd = s[None, :] + x.exp()[:, None]
+        w = 1.0 / sd
+        L = torch.linalg.cholesky(torch.einsum("pn,cn,dn->pcd", w, X, X))
+        z = torch.linalg.solve_triangular(L, torch.einsum("pn,cn,pn->pc", w, X, Y)[:, :, None], upper=False)[:, :, 0]
+        rwr = (w * Y * Y).sum(1) - (z * z).sum(1)
+        m = n - C if reml else n
+        out = m * (math.log(2 * math.pi) + torch.log(rwr / m) + 1.0) + torch.log(sd).sum(1)
+        return out + 2 * torch.log(torch.diagonal(L, dim1=1, dim2=2)).sum(1) if reml else out
+
+    want, i = _golden(loss, P, s.device)
+    assert torch.equal(idx.long(), i)
+    torch.testing.assert_close(loss(ld), loss(want), rtol=4 * n * 2.0 ** -53, atol=1e-10)
