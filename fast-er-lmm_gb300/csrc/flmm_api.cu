@@ -11,6 +11,8 @@
 #include <new>
 
 #include <mutex>
+#include <system_error>
+#include <thread>
 
 #include "flmm_common.cuh"
 
@@ -33,6 +35,7 @@ struct flmm_context {
     cusolverDnHandle_t wsolver[kEighWorkers] = {};
     cudaEvent_t fork = nullptr;
     cudaEvent_t join[kEighWorkers] = {};
+    std::mutex workers_mu;  // one caller at a time on the worker handles
     cusolverDnParams_t params = nullptr;
 };
 
@@ -227,6 +230,75 @@ extern "C" int flmm_eigh(flmm_context* ctx, double* A, int N, double* evals, voi
                                            evals, dwork, lwork, info);
     if (st != CUSOLVER_STATUS_SUCCESS) return solver_fail(st, "cusolverDnDsyevd");
     return check_cuda("cusolverDnDsyevd");
+}
+
+extern "C" int flmm_eigh_many_workspace_bytes(flmm_context* ctx, const int* sizes, int count, size_t* bytes) {
+    FLMM_REQUIRE(ctx && sizes && bytes && count > 0, "flmm_eigh_many_workspace_bytes: bad arguments");
+    size_t most = 0;
+    for (int b = 0; b < count; ++b) {
+        size_t one = 0;
+        int rc = flmm_eigh_workspace_bytes(ctx, sizes[b], &one);
+        if (rc) return rc;
+        most = one > most ? one : most;
+    }
+    *bytes = align_up(most, 256) * static_cast<size_t>(count < kEighWorkers ? count : kEighWorkers);
+    return FLMM_OK;
+}
+
+// One syevd leaves most of the GPU idle at these sizes (10 of N = 600: 190 ms one after another) and its host side waits
+// for its device side, so each worker stream is fed by a thread of its own.
+extern "C" int flmm_eigh_many(flmm_context* ctx, double* const* A, const int* sizes, int count, double* const* evals,
+                              void* work, size_t work_bytes, void* stream) {
+    FLMM_REQUIRE(ctx && A && sizes && evals && work && count > 0, "flmm_eigh_many: bad arguments");
+    for (int b = 0; b < count; ++b) FLMM_REQUIRE(A[b] && evals[b] && sizes[b] > 0, "flmm_eigh_many: bad matrix %d", b);
+    size_t need = 0;
+    int rc = flmm_eigh_many_workspace_bytes(ctx, sizes, count, &need);
+    if (rc) return rc;
+    if (work_bytes < need) return fail(FLMM_ERR_WORKSPACE, "flmm_eigh_many: need %zu bytes, got %zu", need, work_bytes);
+    if (count == 1) return flmm_eigh(ctx, A[0], sizes[0], evals[0], work, work_bytes, stream);
+    const int slots = count < kEighWorkers ? count : kEighWorkers;
+    const size_t slice = need / slots;
+    size_t one[kEighWorkers] = {};
+    int status[kEighWorkers] = {};
+    std::lock_guard<std::mutex> lock(ctx->workers_mu);
+    cudaStream_t st = as_stream(stream);
+    FLMM_CUDA(cudaEventRecord(ctx->fork, st));
+    for (int w = 0; w < slots; ++w) {
+        FLMM_CUDA(cudaStreamWaitEvent(ctx->workers[w], ctx->fork, 0));
+        cusolverDnSetStream(ctx->wsolver[w], ctx->workers[w]);
+    }
+    auto run = [&](int w) {
+        if (cudaSetDevice(ctx->device) != cudaSuccess) { status[w] = -1; return; }
+        char* base = static_cast<char*>(work) + slice * static_cast<size_t>(w);
+        for (int b = w; b < count && status[w] == 0; b += slots) {
+            const int N = sizes[b];
+            if (flmm_eigh_workspace_bytes(ctx, N, &one[w])) { status[w] = -1; return; }
+            status[w] = static_cast<int>(cusolverDnDsyevd(
+                ctx->wsolver[w], CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER, N, A[b], N, evals[b],
+                reinterpret_cast<double*>(base), static_cast<int>((one[w] - 256) / sizeof(double)),
+                reinterpret_cast<int*>(base + one[w] - 256)));
+        }
+    };
+    std::thread threads[kEighWorkers];
+    for (int w = 0; w < slots; ++w) {
+        try {
+            threads[w] = std::thread(run, w);
+        } catch (const std::system_error&) {
+            run(w);  // no thread to be had: in turn
+        }
+    }
+    for (int w = 0; w < slots; ++w)
+        if (threads[w].joinable()) threads[w].join();
+    cudaError_t joined = cudaSuccess;
+    for (int w = 0; w < slots; ++w) {
+        cudaError_t e = cudaEventRecord(ctx->join[w], ctx->workers[w]);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(st, ctx->join[w], 0);
+        if (e != cudaSuccess) joined = e;
+    }
+    for (int w = 0; w < slots; ++w)
+        if (status[w] != 0) return solver_fail(static_cast<cusolverStatus_t>(status[w]), "cusolverDnDsyevd (worker)");
+    if (joined != cudaSuccess) return fail(FLMM_ERR_CUDA, "flmm_eigh_many: %s", cudaGetErrorString(joined));
+    return check_cuda("flmm_eigh_many");
 }
 
 // ---- batched eigendecomposition: all LOCO kinships of a scan at once --------------------------------------------

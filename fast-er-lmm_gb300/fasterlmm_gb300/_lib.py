@@ -37,6 +37,8 @@ SIGNATURES: dict[str, list] = {
     "flmm_project_kinship": [_p, _i64, _p, _i, _i, _p, _i64, _p, _sz, _p],
     "flmm_eigh_workspace_bytes": [_p, _i, _psz],
     "flmm_eigh": [_p, _p, _i, _p, _p, _sz, _p],
+    "flmm_eigh_many_workspace_bytes": [_p, C.POINTER(C.c_int), _i, _psz],
+    "flmm_eigh_many": [_p, C.POINTER(_p), C.POINTER(C.c_int), _i, C.POINTER(_p), _p, _sz, _p],
     "flmm_eigh_batched_workspace_bytes": [_p, _i, _i, _i, _psz],
     "flmm_eigh_batched": [_p, _p, _i, _i, _p, _i, _i, _p, _sz, _p],
     "flmm_eigh_batched_f32_workspace_bytes": [_p, _i, _i, _psz],

@@ -244,6 +244,39 @@ def eigh_batched(A: Tensor, mode: int = 1, slot: int = -1, evals: Tensor | None 
     return evals
 
 
+# Matrices decomposed side by side are held at once, up to this many bytes of them (at least one).
+EIGH_MANY_BYTES = 2 << 30
+
+
+def eigh_groups(sizes: list[int]) -> list[range]:
+    """Consecutive index ranges of matrices of the given sizes, each within EIGH_MANY_BYTES."""
+    groups, a, held = [], 0, 0
+    for i, n in enumerate(sizes):
+        if i > a and held + 8 * n * n > EIGH_MANY_BYTES:
+            groups.append(range(a, i))
+            a, held = i, 0
+        held += 8 * n * n
+    if sizes:
+        groups.append(range(a, len(sizes)))
+    return groups
+
+
+def eigh_many(mats: list[Tensor]) -> list[Tensor]:
+    """In-place FP64 eigendecompositions of contiguous square matrices, side by side: eigenvector rows overwrite each;
+    returns their ascending eigenvalues."""
+    if not mats:
+        return []
+    dev = mats[0].device
+    ctx = _lib.context(dev.index)
+    n = len(mats)
+    evals = [torch.empty(m.shape[0], dtype=F64, device=dev) for m in mats]
+    sizes = (C.c_int * n)(*(m.shape[0] for m in mats))
+    w, wb = _work.get(dev, _lib.query_bytes("flmm_eigh_many_workspace_bytes", ctx, sizes, n))
+    _lib.call("flmm_eigh_many", ctx, (C.c_void_p * n)(*(m.data_ptr() for m in mats)), sizes, n,
+              (C.c_void_p * n)(*(e.data_ptr() for e in evals)), w, wb, _stream(dev))
+    return evals
+
+
 def compat_spectrum(evals: Tensor, D: int) -> Tensor:
     N = evals.shape[0]
     s = torch.empty(N - D, dtype=F64, device=evals.device)
@@ -471,22 +504,30 @@ def scan_t(Zt: Tensor, X: Tensor, Yt: Tensor, chrom: np.ndarray, *, n_real: int,
         Gtot = gram_t(kin_Zt)
         units = [(None, (torch.arange(M, device=dev), slice(0, M)))]
     M_kin = kin_Zt.shape[0]
-    for k_idx, (c, blk) in enumerate(units):
-        if c is None:
-            K = kinship_from_gram(Gtot, None, M_kin)
-        else:
-            Gc = grams.get(c)
-            m_c = int((kin_chrom == c).sum())
-            K = kinship_from_gram(Gtot, Gc, M_kin - m_c)
-        s, Ut = compat_eigh(K, basis)
-        UYt = rotate_rows(Yrt, Ut)
-        ld, _ = fit_delta_t(s, UYt, n_grid=n_grid, log_delta_min=log_delta_min, log_delta_max=log_delta_max,
-                            refine=refine)
-        USt = rotate_variants(basis.regress_out(_take_rows(Zt, blk)), Ut)
-        wald_t(s, UYt, ld, USt, n_real, blk[0], out, max_F)
-        log_deltas[c if c is not None else 0] = ld
-        if on_chrom is not None:
-            on_chrom(k_idx + 1, len(units))
+    D = X.shape[1]
+    if N <= D:
+        raise ValueError(f"need more samples than covariate columns (N={N}, D={D})")
+    for group in eigh_groups([N] * len(units)):
+        projected = []
+        for k_idx in group:
+            c = units[k_idx][0]
+            if c is None:
+                K = kinship_from_gram(Gtot, None, M_kin)
+            else:
+                K = kinship_from_gram(Gtot, grams.get(c), M_kin - int((kin_chrom == c).sum()))
+            projected.append(project_kinship(K, basis, K.new_empty(N, N)))
+        evals = eigh_many(projected)
+        for k_idx, Kp, ev in zip(group, projected, evals):
+            c, blk = units[k_idx]
+            s, Ut = compat_spectrum(ev, D), Kp[D:]
+            UYt = rotate_rows(Yrt, Ut)
+            ld, _ = fit_delta_t(s, UYt, n_grid=n_grid, log_delta_min=log_delta_min, log_delta_max=log_delta_max,
+                                refine=refine)
+            USt = rotate_variants(basis.regress_out(_take_rows(Zt, blk)), Ut)
+            wald_t(s, UYt, ld, USt, n_real, blk[0], out, max_F)
+            log_deltas[c if c is not None else 0] = ld
+            if on_chrom is not None:
+                on_chrom(k_idx + 1, len(units))
     return ScanResult(max_F=max_F, log_delta=log_deltas, **out)
 
 

@@ -20,8 +20,8 @@ from torch import Tensor
 
 from . import _lib
 from .core import (F64, CovariateBasis, ScanResult, _alloc_outputs, _BasisView, _cuda_device, _f64, _ptr,
-                   _rows_major, _stream, _to_device, _work, gram_t, kinship_from_gram, rotate_rows, rotate_variants,
-                   transpose)
+                   _rows_major, _stream, _to_device, _work, eigh_groups, eigh_many, gram_t, kinship_from_gram, rotate_rows,
+                   rotate_variants, transpose)
 
 
 @dataclass
@@ -63,24 +63,43 @@ def _eigh_rows(A: Tensor) -> tuple[Tensor, Tensor]:
     return evals, V
 
 
+def _basis_of(evals: Tensor, V: Tensor, Gr: Tensor, sv_floor: float) -> tuple[Tensor, Tensor]:
+    """(s, Ut) from the decomposed Gram of the regressed factor rows Gr (k_in, N), or of their kinship if k_in >= N."""
+    k_in, N = Gr.shape
+    if k_in >= N:
+        keep = torch.nonzero(evals.clamp(min=0.0) > (sv_floor * sv_floor) / k_in).flatten()
+        return evals[keep].clamp(min=0.0).contiguous(), V[keep].contiguous()
+    sv = evals.clamp(min=0.0).sqrt()
+    keep = torch.nonzero(sv > sv_floor).flatten()
+    sv = sv[keep]
+    Vk = (V[keep] / sv[:, None]).contiguous()
+    return (sv * sv / k_in).contiguous(), rotate_rows(Vk, transpose(Gr))  # U_eff^T = (V / sv)^T G_^T
+
+
 def basis_t(Gt: Tensor, basis: CovariateBasis, sv_floor: float = 1e-10) -> tuple[Tensor, Tensor]:
     """Device basis from the factor rows Gt (k_in, N): (s (k,), Ut (k, N))."""
     k_in, N = Gt.shape
     Gr = basis.regress_out(Gt)
-    if k_in < N:
-        evals, V = _eigh_rows(rotate_rows(Gr, Gr))          # eigh of G_^T G_ (k_in, k_in)
-        sv = evals.clamp(min=0.0).sqrt()
-        keep = torch.nonzero(sv > sv_floor).flatten()
-        sv = sv[keep]
-        Vk = (V[keep] / sv[:, None]).contiguous()
-        Ut = rotate_rows(Vk, transpose(Gr))                # U_eff^T = (V / sv)^T G_^T
-        s = sv * sv / k_in
-    else:
-        evals, U = _eigh_rows(kinship_from_gram(gram_t(Gr), None, k_in))
-        keep = torch.nonzero(evals.clamp(min=0.0) > (sv_floor * sv_floor) / k_in).flatten()
-        s = evals[keep].clamp(min=0.0)
-        Ut = U[keep].contiguous()
-    return s.contiguous(), Ut
+    evals, V = _eigh_rows(rotate_rows(Gr, Gr) if k_in < N else kinship_from_gram(gram_t(Gr), None, k_in))
+    return _basis_of(evals, V, Gr, sv_floor)
+
+
+def loco_bases(Gt: Tensor, keeps: list[Tensor], basis: CovariateBasis, sv_floor: float = 1e-10):
+    """basis_t(Gt[keep], basis) for every row selection, one at a time.  The rows are regressed once, their Gram is formed
+    once and each selection's is a part of it; the decompositions run side by side, as many as eigh_groups holds."""
+    N = Gt.shape[1]
+    Gr = basis.regress_out(Gt)
+    gram = rotate_rows(Gr, Gr) if any(k.numel() < N for k in keeps) else None
+    for group in eigh_groups([min(k.numel(), N) for k in keeps]):
+        mats = []
+        for i in group:
+            k = keeps[i]
+            if k.numel() < N:
+                mats.append(gram.index_select(0, k).index_select(1, k))
+            else:
+                mats.append(kinship_from_gram(gram_t(Gr.index_select(0, k)), None, k.numel()))
+        for i, V, evals in zip(group, mats, eigh_many(mats)):
+            yield _basis_of(evals, V, Gr.index_select(0, keeps[i]), sv_floor)
 
 
 def rotate_t(Yt: Tensor, Ut: Tensor, basis: CovariateBasis) -> tuple[Tensor, Tensor]:
@@ -233,9 +252,8 @@ def _loco_scan_core(chroms: list, block_source, M: int, G: Tensor, g_chrom: np.n
     out, max_F = _alloc_outputs(M, n_real, P, dev, zero=True)  # a block reader need not cover every variant
     g_chrom = np.asarray(g_chrom)
     log_deltas = {}
-    for k_idx, c in enumerate(chroms):
-        keep = torch.from_numpy(np.flatnonzero(g_chrom != c)).to(dev)
-        s, Ut = basis_t(Gt.index_select(0, keep), basis)
+    keeps = [torch.from_numpy(np.flatnonzero(g_chrom != c)).to(dev) for c in chroms]
+    for k_idx, (c, (s, Ut)) in enumerate(zip(chroms, loco_bases(Gt, keeps, basis))):
         UYt, UUYt = rotate_t(Yt, Ut, basis)
         ld, _ = fit_delta_t(s, UYt, UUYt, N - D)
         log_deltas[c] = ld

@@ -100,6 +100,12 @@ int flmm_project_kinship(const double* K, int64_t ldk, const double* Qx, int N, 
 int flmm_eigh_workspace_bytes(flmm_context* ctx, int N, size_t* bytes);
 int flmm_eigh(flmm_context* ctx, double* A, int N, double* evals, void* work, size_t work_bytes, void* stream);
 
+/* flmm_eigh of `count` independent matrices of any sizes, side by side on the context's worker streams, forked from and
+ * joined back into `stream`; A, sizes and evals are host arrays.  Each result is flmm_eigh's. */
+int flmm_eigh_many_workspace_bytes(flmm_context* ctx, const int* sizes, int count, size_t* bytes);
+int flmm_eigh_many(flmm_context* ctx, double* const* A, const int* sizes, int count, double* const* evals, void* work,
+                   size_t work_bytes, void* stream);
+
 /* The same for `batch` independent matrices A (batch, N, N) contiguous, evals (batch, N): every LOCO kinship of a
  * scan at once.  mode 1 = cusolverDnXsyevBatched on the context's main solver handle (slot = -1) or on worker handle
  * `slot` (0..7, so that batches on different streams never share a handle); mode 2 = syevd calls run side by side on
