@@ -18,7 +18,7 @@
 //    per step, so 24 steps narrow the bracket as 48 halvings would).
 // 3. k_tridiag_invit: each eigenvector of T by inverse iteration in FP64 (LDL^T of T - lambda I with a pivot floor,
 //    three solves from a fixed pseudo-random start, the first fused with the factorisation), one thread each.
-// 4. k_cluster_orth: eigenvalues closer than kClusterTol * ||T|| form a cluster; one warp orthonormalises its
+// 4. k_cluster_orth: eigenvalues closer than kClusterTol * ||T|| form a cluster; one block orthonormalises its
 //    vectors (modified Gram-Schmidt in FP64).  Each vector of a cluster has converged into the cluster's invariant
 //    subspace from its own start, so the result is an orthonormal basis of that subspace.
 // 5. k_wy_factors + k_backtransform: the reflectors in blocks of kWy as I - V T V^T (forward, columnwise), applied to
@@ -524,47 +524,69 @@ k_tridiag_invit(const float* __restrict__ d_all, const float* __restrict__ e_all
     for (int i = 0; i < N; ++i) Zb[static_cast<int64_t>(i) * N + j] = static_cast<float>(sc * X[static_cast<int64_t>(i) * N]);
 }
 
-// grid (ceil(N / 4), batch), 128 threads: a warp per eigenvalue index j; the warp of each cluster's first eigenvalue
-// orthonormalises the cluster's columns of Z (modified Gram-Schmidt, lanes over the rows, FP64 sums)
-__global__ void __launch_bounds__(128)
-k_cluster_orth(const float* __restrict__ evals, const float* __restrict__ tnorm_all, int N, float* __restrict__ Z) {
-    const int b = blockIdx.y;
-    const int j = blockIdx.x * 4 + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (j >= N) return;
-    const float* lam = evals + static_cast<int64_t>(b) * N;
-    const double tol = kClusterTol * static_cast<double>(tnorm_all[b]);
-    if (j > 0 && static_cast<double>(lam[j]) - static_cast<double>(lam[j - 1]) < tol) return;
-    int jend = j + 1;
-    while (jend < N && static_cast<double>(lam[jend]) - static_cast<double>(lam[jend - 1]) < tol) ++jend;
-    if (jend - j < 2) return;
-    float* Zb = Z + static_cast<int64_t>(b) * N * N;
-    for (int m = j; m < jend; ++m) {
-        for (int q = j; q < m; ++q) {
+// grid (ceil(N / kOrthCols), batch): a block orthonormalises the clusters whose first eigenvalue is among its kOrthCols
+// (modified Gram-Schmidt on the columns of Z, lanes over the rows, FP64 sums).  Once column q is final it is taken out of
+// every later column of the cluster, a warp per column: each column sees the same subtractions in the same order as it
+// would one column after another.  (One warp did all pairs of a cluster in turn: 35 of the 43 ms of a batch of marker
+// Grams whose padding repeats one eigenvalue ~100 times.)
+constexpr int kOrthThreads = 512, kOrthCols = 16;
+
+__device__ void orth_cluster(float* __restrict__ Zb, int N, int j, int jend, float* pivot) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int q = j; q < jend; ++q) {
+        if (warp == 0) {
+            double nrm = 0.0;
+            for (int i = lane; i < N; i += 32) {
+                const double v = static_cast<double>(Zb[static_cast<int64_t>(i) * N + q]);
+                nrm = fma(v, v, nrm);
+            }
+            nrm = warp_sum(nrm);
+            const double sc = nrm > 0.0 ? 1.0 / sqrt(nrm) : 0.0;
+            for (int i = lane; i < N; i += 32) {
+                float* zq = Zb + static_cast<int64_t>(i) * N + q;
+                const float v = static_cast<float>(sc * static_cast<double>(*zq));
+                *zq = v;
+                pivot[i] = v;
+            }
+        }
+        __syncthreads();
+        for (int m = q + 1 + warp; m < jend; m += kOrthThreads / 32) {
             double pr = 0.0;
+#pragma unroll 4
             for (int i = lane; i < N; i += 32)
-                pr = fma(static_cast<double>(Zb[static_cast<int64_t>(i) * N + q]),
-                         static_cast<double>(Zb[static_cast<int64_t>(i) * N + m]), pr);
+                pr = fma(static_cast<double>(pivot[i]), static_cast<double>(Zb[static_cast<int64_t>(i) * N + m]), pr);
             pr = warp_sum(pr);
+#pragma unroll 4
             for (int i = lane; i < N; i += 32) {
                 float* zm = Zb + static_cast<int64_t>(i) * N + m;
-                *zm = static_cast<float>(static_cast<double>(*zm) - pr * static_cast<double>(Zb[static_cast<int64_t>(i) * N + q]));
+                *zm = static_cast<float>(static_cast<double>(*zm) - pr * static_cast<double>(pivot[i]));
             }
-            __syncwarp();
         }
-        double nrm = 0.0;
-        for (int i = lane; i < N; i += 32) {
-            const double v = static_cast<double>(Zb[static_cast<int64_t>(i) * N + m]);
-            nrm = fma(v, v, nrm);
-        }
-        nrm = warp_sum(nrm);
-        const double sc = nrm > 0.0 ? 1.0 / sqrt(nrm) : 0.0;
-        for (int i = lane; i < N; i += 32) {
-            float* zm = Zb + static_cast<int64_t>(i) * N + m;
-            *zm = static_cast<float>(sc * static_cast<double>(*zm));
-        }
-        __syncwarp();
+        __syncthreads();
     }
+}
+
+__global__ void __launch_bounds__(kOrthThreads)
+k_cluster_orth(const float* __restrict__ evals, const float* __restrict__ tnorm_all, int N, float* __restrict__ Z) {
+    extern __shared__ float pivot[];  // one column
+    __shared__ int end_s[kOrthCols];  // end of the cluster that starts at each of the block's columns, 0 if none does
+    const int b = blockIdx.y, j0 = blockIdx.x * kOrthCols;
+    if (threadIdx.x < kOrthCols) {
+        const int j = j0 + threadIdx.x;
+        const float* lam = evals + static_cast<int64_t>(b) * N;
+        const double tol = kClusterTol * static_cast<double>(tnorm_all[b]);
+        auto close = [&](int i) { return static_cast<double>(lam[i]) - static_cast<double>(lam[i - 1]) < tol; };
+        int e = 0;
+        if (j < N && !(j > 0 && close(j))) {
+            e = j + 1;
+            while (e < N && close(e)) ++e;
+            if (e - j < 2) e = 0;
+        }
+        end_s[threadIdx.x] = e;
+    }
+    __syncthreads();
+    for (int c = 0; c < kOrthCols; ++c)
+        if (end_s[c]) orth_cluster(Z + static_cast<int64_t>(b) * N * N, N, j0 + c, end_s[c], pivot);
 }
 
 // ---- back-transformation: U = Q Z with Q = H_0 ... H_{N-3} in WY blocks ---------------------------------------
@@ -776,7 +798,7 @@ int eigh_own_f32(float* A, int N, int batch, float* evals, void* work, cudaStrea
     // 3. eigenvectors of T
     k_tridiag_invit<<<dim3(ceil_div(N, 128), batch), 128, 0, st>>>(d, e, evals, tn, N, S, Z);
     if ((rc = check_launch("k_tridiag_invit"))) return rc;
-    k_cluster_orth<<<dim3(ceil_div(N, 4), batch), 128, 0, st>>>(evals, tn, N, Z);
+    k_cluster_orth<<<dim3(ceil_div(N, kOrthCols), batch), kOrthThreads, sizeof(float) * N, st>>>(evals, tn, N, Z);
     if ((rc = check_launch("k_cluster_orth"))) return rc;
     // 4. back-transformation into A
     const int n_refl = N > 2 ? N - 2 : 0;
