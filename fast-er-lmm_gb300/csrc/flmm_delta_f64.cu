@@ -56,14 +56,18 @@ __global__ void k_grid_weights(const double* __restrict__ s, int Neff, const dou
     }
 }
 
-// Grid loss and first argmin over g for a tile of 64 columns; g is walked in tiles of 64.  yWy[g, p] =
-// sum_n Wg[g, n] UY[p, n]^2 is the (G x Neff) x (Neff x P) product of fasterlmm/core.py:537.
-constexpr int TG = 64, TP = 64, TK = 16, NT = 256;
+// Grid loss and first argmin over g for a tile of 16 RP columns; g is walked in tiles of 64.  yWy[g, p] =
+// sum_n Wg[g, n] UY[p, n]^2 is the (G x Neff) x (Neff x P) product of fasterlmm/core.py:537, one chain of multiply-adds
+// over n per (g, p) whatever the tile.  The FP64 pipe is the bound, so tiles of 16 columns (RP = 1) are as good as tiles
+// of 64 and give four times the blocks: 2,100 columns are 33 blocks of 64 on 152 SMs.
+constexpr int TG = 64, TK = 16, NT = 256;
 
+template <int RP>
 __global__ void __launch_bounds__(NT)
 k_grid_argmin(const double* __restrict__ Wg, const double* __restrict__ sum_log, const double* __restrict__ grid,
               const double* __restrict__ UYt, int64_t ldu, int Neff, int P, int G, OffRank off,
               int32_t* __restrict__ idx_out) {
+    constexpr int TP = 16 * RP;
     __shared__ double Ws[TK][TG + 1];
     __shared__ double Us[TK][TP + 1];
     __shared__ double red_v[16][TP];
@@ -73,7 +77,7 @@ k_grid_argmin(const double* __restrict__ Wg, const double* __restrict__ sum_log,
     double best = INFINITY;
     int best_g = 0;
     for (int g0 = 0; g0 < G; g0 += TG) {
-        double acc[4][4] = {};
+        double acc[4][RP] = {};
         for (int k0 = 0; k0 < Neff; k0 += TK) {
 #pragma unroll
             for (int l = 0; l < (TG * TK) / NT; ++l) {
@@ -91,21 +95,21 @@ k_grid_argmin(const double* __restrict__ Wg, const double* __restrict__ sum_log,
             __syncthreads();
 #pragma unroll
             for (int k = 0; k < TK; ++k) {
-                double a[4], b[4];
+                double a[4], b[RP];
 #pragma unroll
                 for (int r = 0; r < 4; ++r) a[r] = Ws[k][ty + 16 * r];
 #pragma unroll
-                for (int c = 0; c < 4; ++c) b[c] = Us[k][tx + 16 * c];
+                for (int c = 0; c < RP; ++c) b[c] = Us[k][tx + 16 * c];
 #pragma unroll
                 for (int r = 0; r < 4; ++r)
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) acc[r][c] = fma(a[r], b[c], acc[r][c]);
+                    for (int c = 0; c < RP; ++c) acc[r][c] = fma(a[r], b[c], acc[r][c]);
             }
             __syncthreads();
         }
         // this thread's nodes are g0 + ty + 16 r, ascending in r: keep the first minimum per column
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
+        for (int c = 0; c < RP; ++c) {
             double bv = INFINITY;
             int bi = G;
             const int pc = p0 + tx + 16 * c;
@@ -241,7 +245,10 @@ int fit_delta_impl(const double* s, int Neff, const double* UYt, int64_t ldu, in
     if (rc) return rc;
     k_grid_weights<<<n_grid, 256, 0, st>>>(s, Neff, grid, Wg, sum_log);
     if ((rc = check_launch("k_grid_weights"))) return rc;
-    k_grid_argmin<<<ceil_div(P, TP), NT, 0, st>>>(Wg, sum_log, grid, UYt, ldu, Neff, P, n_grid, off, grid_idx);
+    if (P >= 64 * 152)
+        k_grid_argmin<4><<<ceil_div(P, 64), NT, 0, st>>>(Wg, sum_log, grid, UYt, ldu, Neff, P, n_grid, off, grid_idx);
+    else
+        k_grid_argmin<1><<<ceil_div(P, 16), NT, 0, st>>>(Wg, sum_log, grid, UYt, ldu, Neff, P, n_grid, off, grid_idx);
     if ((rc = check_launch("k_grid_argmin"))) return rc;
     if (refine) {
         k_golden<<<P, kBlockThreads, 0, st>>>(s, Neff, UYt, ldu, grid, n_grid, grid_idx, lo, hi, off, log_delta);
