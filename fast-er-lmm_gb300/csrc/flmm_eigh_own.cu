@@ -30,6 +30,7 @@
 #include <math.h>
 
 #include <algorithm>
+#include <mutex>
 #include <stdint.h>
 
 #include "flmm_common.cuh"
@@ -38,8 +39,11 @@ using namespace flmm;
 
 namespace {
 
-constexpr int kMaxClusterCtas = 8;
+constexpr int kMaxClusterCtas = 16;  // beyond 8 the size is not portable
+constexpr int kMaxParts = 8;         // partial sums of p^T v
 constexpr int kSytrdThreads = 512;
+// a column's cycles at N = 1,000: its row pass in one CTA, what every CTA repeats, and the barrier's share per CTA
+constexpr double kRowPassCycles = 100e3, kColumnCycles = 5e3, kCtaCycles = 50;
 constexpr int kRowsPerWarp = 4;    // rows a warp of the tridiagonalisation works on at once
 constexpr int kLoadsPerRow = 8;    // loads of each of them a lane has in flight
 constexpr int kWy = 16;            // reflectors per WY block
@@ -134,7 +138,7 @@ __device__ Reflector make_reflector(float d, float alpha, float ss_partial, floa
 }
 
 __global__ void __launch_bounds__(kSytrdThreads, 1)
-k_sytrd_cluster(float* __restrict__ W, int N, float* __restrict__ d_out, float* __restrict__ e_out,
+k_sytrd_cluster(float* __restrict__ W, int N, int parts, float* __restrict__ d_out, float* __restrict__ e_out,
                 float* __restrict__ tau_out) {
     extern __shared__ float sm[];
     const int Np = (N + 3) & ~3;
@@ -142,8 +146,8 @@ k_sytrd_cluster(float* __restrict__ W, int N, float* __restrict__ d_out, float* 
     float* wbuf[2] = {sm + 2 * Np, sm + 3 * Np};
     float* pbuf[2] = {sm + 4 * Np, sm + 5 * Np};
     float* red = sm + 6 * Np;        // 32 floats
-    float* part = red + 32;          // partial p^T v of every CTA of the cluster, [parity][rank]
-    float* scal2 = part + 2 * kMaxClusterCtas;  // d and alpha of the next reflector
+    float* part = red + 32;          // partial sums of p^T v
+    float* scal2 = part + kMaxParts;  // d and alpha of the next reflector
     const int C = static_cast<int>(cluster_size());
     const int b = static_cast<int>(cluster_index());
     const int r = static_cast<int>(cta_rank());
@@ -173,7 +177,6 @@ k_sytrd_cluster(float* __restrict__ W, int N, float* __restrict__ d_out, float* 
         // (B) rows i > k of this CTA: column k-1's update (lazy), then p_i = tau W[i, k+1:] . v.  A warp takes
         // kRowsPerWarp rows at a time and a lane issues kLoadsPerRow loads of each before using any, so the pass
         // keeps enough L2 reads in flight to run at bandwidth rather than at L2 latency.
-        float dot = 0.0f;
         const int first = k + 1 + ((r - (k + 1)) % C + C) % C;
         const int n_own = first < N ? (N - 1 - first) / C + 1 : 0;
         const bool lazy = k > 0;
@@ -225,18 +228,28 @@ k_sytrd_cluster(float* __restrict__ W, int N, float* __restrict__ d_out, float* 
                     const float pi = tau * a;
                     // p_i into every CTA's copy of p (lane l to CTA l): after the barrier all of p is local
                     if (lane < C) st_remote(&pb[i], static_cast<uint32_t>(lane), pi);
-                    dot = fmaf(pi, vc[i], dot);
                 }
             }
         }
-        // lanes of a warp hold the same dot; sum one lane per warp
-        const float dsum = block_sum(lane == 0 ? dot : 0.0f, red);
-        if (threadIdx.x < static_cast<unsigned>(C))
-            st_remote(&part[cur * kMaxClusterCtas + r], threadIdx.x, dsum);
-        cluster_barrier();  // every CTA's p, p^T v and updated rows are visible
-        // (C) w = p - (tau / 2) (p^T v) v over the whole trailing range (p^T v summed in rank order)
+        cluster_barrier();  // every CTA's p and updated rows are visible
+        // (C) w = p - (tau / 2) (p^T v) v over the whole trailing range.  Every CTA adds up p^T v from its copy of p in one
+        // order whatever the cluster size: `parts` interleaved row sets, each in 16 chains of four rows at a time.
+        if (threadIdx.x < 16 * kMaxParts) {
+            const int q = threadIdx.x >> 4, chain = threadIdx.x & 15;
+            float dot = 0.0f;
+            if (q < parts) {
+                const int f = k + 1 + ((q - (k + 1)) % parts + parts) % parts;
+                const int n = f < N ? (N - 1 - f) / parts + 1 : 0;
+                for (int t0 = chain * kRowsPerWarp; t0 < n; t0 += 16 * kRowsPerWarp)
+                    for (int t = t0; t < min(t0 + kRowsPerWarp, n); ++t) dot = fmaf(pb[f + t * parts], vc[f + t * parts], dot);
+            }
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+            if (chain == 0) part[q] = dot;
+        }
+        __syncthreads();
         float s = 0.0f;
-        for (int q = 0; q < C; ++q) s += part[cur * kMaxClusterCtas + q];
+        for (int q = 0; q < parts; ++q) s += part[q];
         const float c = -0.5f * tau * s;
         for (int j = k + 1 + threadIdx.x; j < N; j += kSytrdThreads) wc[j] = fmaf(c, vc[j], pb[j]);
         __syncthreads();
@@ -723,6 +736,54 @@ struct OwnLayout {
     int nblocks;
 };
 
+// Clusters of each size that fit on the device at once (one CTA per SM; a cluster lies within one GPC, so 7 CTAs fit 15
+// times on 152 SMs where 6 fit 23 times), and the size with the least time for a batch: waves of clusters times the
+// column's row pass, shared by the cluster, plus what does not shrink (barrier, reductions, the next reflector).
+int cluster_ctas(int dev, int N, int batch, int* out) {
+    static std::mutex mu;
+    static int active[64][kMaxClusterCtas + 1];
+    static bool known[64];
+    std::lock_guard<std::mutex> lock(mu);
+    if (dev < 0 || dev >= 64) return fail(FLMM_ERR_ARG, "eigh: device %d", dev);
+    if (!known[dev]) {
+        FLMM_CUDA(cudaFuncSetAttribute(k_sytrd_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
+        FLMM_CUDA(cudaFuncSetAttribute(k_sytrd_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        for (int c = 2; c <= kMaxClusterCtas; ++c) {
+            cudaLaunchConfig_t cfg = {};
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = static_cast<unsigned>(c);
+            attr[0].val.clusterDim.y = 1;
+            attr[0].val.clusterDim.z = 1;
+            cfg.gridDim = dim3(static_cast<unsigned>(c * 64));
+            cfg.blockDim = dim3(kSytrdThreads);
+            cfg.dynamicSmemBytes = 96 * 1024;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            int n = 0;
+            if (cudaOccupancyMaxActiveClusters(&n, k_sytrd_cluster, &cfg) != cudaSuccess) {
+                cudaGetLastError();
+                n = 0;
+            }
+            active[dev][c] = n;
+        }
+        known[dev] = true;
+    }
+    const double rows = kRowPassCycles * (N / 1000.0) * (N / 1000.0);
+    double best = 0.0;
+    *out = 0;
+    for (int c = 2; c <= kMaxClusterCtas; ++c) {
+        if (active[dev][c] < 1) continue;
+        const double waves = (batch + active[dev][c] - 1) / active[dev][c];
+        const double cost = waves * (rows / c + kColumnCycles + kCtaCycles * c);
+        if (*out == 0 || cost < best) {
+            best = cost;
+            *out = c;
+        }
+    }
+    return *out ? FLMM_OK : fail(FLMM_ERR_CUDA, "eigh: no cluster of the tridiagonalisation fits on the device");
+}
+
 size_t up256(size_t x) { return (x + 255) / 256 * 256; }
 
 OwnLayout own_layout(int N, int batch) {
@@ -766,14 +827,16 @@ int eigh_own_f32(float* A, int N, int batch, float* evals, void* work, cudaStrea
     FLMM_CUDA(cudaMemcpyAsync(W, A, 4 * NN * batch, cudaMemcpyDeviceToDevice, st));
     // 1. tridiagonalisation, one cluster per matrix
     const int Np = (N + 3) & ~3;
-    const size_t smem1 = sizeof(float) * (6 * static_cast<size_t>(Np) + 32 + 2 * kMaxClusterCtas + 2);
-    // cluster size: as many CTAs per matrix as fill the SMs once (one CTA per SM), 2 to 8
+    const size_t smem1 = sizeof(float) * (6 * static_cast<size_t>(Np) + 32 + kMaxParts + 2);
     int dev = 0, sms = 0;
     FLMM_CUDA(cudaGetDevice(&dev));
     FLMM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const int C = std::max(2, std::min(kMaxClusterCtas, sms / std::max(batch, 1)));
+    // the row sets that p^T v is added up in: part of the result, so they follow the batch and not the cluster
+    const int parts = std::max(2, std::min(kMaxParts, sms / std::max(batch, 1)));
+    int C = 0;
+    int rc = cluster_ctas(dev, N, batch, &C);
+    if (rc) return rc;
     // (per device, so set on every call; the call is cheap)
-    FLMM_CUDA(cudaFuncSetAttribute(k_sytrd_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
     FLMM_CUDA(cudaFuncSetAttribute(k_backtransform, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
@@ -787,9 +850,8 @@ int eigh_own_f32(float* A, int N, int batch, float* evals, void* work, cudaStrea
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    FLMM_CUDA(cudaLaunchKernelEx(&cfg, k_sytrd_cluster, W, N, d, e, tau));
-    int rc = check_launch("k_sytrd_cluster");
-    if (rc) return rc;
+    FLMM_CUDA(cudaLaunchKernelEx(&cfg, k_sytrd_cluster, W, N, parts, d, e, tau));
+    if ((rc = check_launch("k_sytrd_cluster"))) return rc;
     // 2. eigenvalues
     k_tridiag_bisect<<<dim3(ceil_div(N, kBisectThreads), batch), kBisectThreads,
                        sizeof(float) * 2 * static_cast<size_t>(N), st>>>(
