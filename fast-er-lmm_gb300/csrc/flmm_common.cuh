@@ -42,6 +42,15 @@ int refine_m_tc(const float* R, int N, int batch, float* M, void* work, cudaStre
 int refine_update_tc(const float* T, const float* Ut, float* scratch, int N, int batch, float* U_out, void* work,
                      cudaStream_t st);
 
+// flmm_project_kinship of n_units stacked kinships in place (csrc/flmm_prep.cu).
+size_t project_kinships_bytes(int N, int D, int n_units);
+int project_kinships(double* K, const double* Qx, int N, int D, int n_units, void* work, cudaStream_t st);
+
+// flmm_mean_f32 and flmm_wald_interp_nodes of n_units stacked spectra: shat (n_units), W (n_units, R, Neff)
+// (csrc/flmm_fast.cu).
+int interp_units(const double* s, int Neff, int n_units, float* shat, double x0, double h, int R, double* W,
+                 cudaStream_t st);
+
 inline unsigned ceil_div(int64_t a, int64_t b) { return static_cast<unsigned>((a + b - 1) / b); }
 
 #define FLMM_REQUIRE(cond, ...)                                                       \

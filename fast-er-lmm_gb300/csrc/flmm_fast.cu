@@ -945,21 +945,23 @@ k_wald_prep_columns(const float* __restrict__ s32, int Neff, const float* __rest
     }
 }
 
-// normalised weights at the interpolation nodes: W~[r, n] = (shat + e^{x_r}) / (s_n + e^{x_r}), FP64
+// normalised weights at the interpolation nodes: W~[r, n] = (shat + e^{x_r}) / (s_n + e^{x_r}), FP64; grid.y spectra
 __global__ void k_interp_nodes(const double* __restrict__ s, int Neff, const float* __restrict__ shat_p, double x0,
                                double h, int R, double* __restrict__ W) {
     const int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
     if (t >= static_cast<int64_t>(R) * Neff) return;
     const int r = static_cast<int>(t / Neff), n = static_cast<int>(t % Neff);
     const double delta = exp(x0 + r * h);
-    W[t] = (static_cast<double>(*shat_p) + delta) / (s[n] + delta);
+    const int64_t u = blockIdx.y;
+    W[u * R * Neff + t] = (static_cast<double>(shat_p[u]) + delta) / (s[u * Neff + n] + delta);
 }
 
 __global__ void k_mean(const double* __restrict__ x, int n, float* __restrict__ out) {
+    const double* xu = x + static_cast<int64_t>(blockIdx.x) * n;
     double acc = 0.0;
-    for (int i = threadIdx.x; i < n; i += 32) acc += x[i];
+    for (int i = threadIdx.x; i < n; i += 32) acc += xu[i];
     acc = warp_sum(acc);
-    if (threadIdx.x == 0) *out = static_cast<float>(acc / n);
+    if (threadIdx.x == 0) out[blockIdx.x] = static_cast<float>(acc / n);
 }
 
 // Wald variant side: B1 = US, B2 = US o US, each row split.  One warp per variant m.
@@ -1358,6 +1360,15 @@ extern "C" int flmm_mean_f32(const double* x, int n, float* out, void* stream) {
     FLMM_REQUIRE(x && out && n > 0, "flmm_mean_f32: bad arguments");
     k_mean<<<1, 32, 0, as_stream(stream)>>>(x, n, out);
     return check_launch("k_mean");
+}
+
+int flmm::interp_units(const double* s, int Neff, int n_units, float* shat, double x0, double h, int R, double* W,
+                       cudaStream_t st) {
+    k_mean<<<n_units, 32, 0, st>>>(s, Neff, shat);
+    int rc = check_launch("k_mean");
+    if (rc) return rc;
+    k_interp_nodes<<<dim3(ceil_div(static_cast<int64_t>(R) * Neff, 256), n_units), 256, 0, st>>>(s, Neff, shat, x0, h, R, W);
+    return check_launch("k_interp_nodes");
 }
 
 extern "C" int flmm_wald_interp_nodes(const double* s, int Neff, const float* shat, double x0, double h, int R,

@@ -178,31 +178,33 @@ __global__ void k_loco_kinship(const double* __restrict__ Gtot, const double* __
 }
 
 // ---- covariate projection of K + I -------------------------------------------------------------------------
+// grid.y stacked kinships, each with its own W, C and VmW.
 // W (N, D): W[i, k] = sum_j (K + I)[i, j] Q[k, j]; one warp per (i, k).
 __global__ void k_proj_W(const double* __restrict__ K, int64_t ldk, const double* __restrict__ Q, int N, int D,
                          double* __restrict__ W) {
     const int lane = threadIdx.x & 31;
-    const int64_t w = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5;
+    const int64_t u = blockIdx.y, w = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5;
     if (w >= static_cast<int64_t>(N) * D) return;
     const int i = static_cast<int>(w / D), k = static_cast<int>(w % D);
-    const double* krow = K + static_cast<int64_t>(i) * ldk;
+    const double* krow = K + u * N * ldk + static_cast<int64_t>(i) * ldk;
     const double* q = Q + static_cast<int64_t>(k) * N;
     double acc = 0.0;
     for (int j = lane; j < N; j += 32) acc += krow[j] * q[j];
     acc = warp_sum(acc);
-    if (lane == 0) W[static_cast<int64_t>(i) * D + k] = acc + q[i];
+    if (lane == 0) W[u * N * D + static_cast<int64_t>(i) * D + k] = acc + q[i];
 }
 
-// C (D, D) = Q W, then V (N, D) = Q^T C; one block
+// C (D, D) = Q W; one block
 __global__ void k_proj_C(const double* __restrict__ Q, const double* __restrict__ W, int N, int D,
                          double* __restrict__ C) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const double* Wu = W + static_cast<int64_t>(blockIdx.y) * N * D;
     for (int e = warp; e < D * D; e += nw) {
         int k = e / D, l = e % D;
         double acc = 0.0;
-        for (int i = lane; i < N; i += 32) acc += Q[static_cast<int64_t>(k) * N + i] * W[static_cast<int64_t>(i) * D + l];
+        for (int i = lane; i < N; i += 32) acc += Q[static_cast<int64_t>(k) * N + i] * Wu[static_cast<int64_t>(i) * D + l];
         acc = warp_sum(acc);
-        if (lane == 0) C[e] = acc;
+        if (lane == 0) C[static_cast<int64_t>(blockIdx.y) * D * D + e] = acc;
     }
 }
 
@@ -210,27 +212,46 @@ __global__ void k_proj_V(const double* __restrict__ Q, const double* __restrict_
                          int N, int D, double* __restrict__ VmW) {
     int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
     if (t >= static_cast<int64_t>(N) * D) return;
+    const int64_t u = blockIdx.y;
     int i = static_cast<int>(t / D), l = static_cast<int>(t % D);
     double acc = 0.0;
-    for (int k = 0; k < D; ++k) acc += Q[static_cast<int64_t>(k) * N + i] * C[k * D + l];
-    VmW[t] = acc - W[t];  // (Q^T C - W)[i, l]
+    for (int k = 0; k < D; ++k) acc += Q[static_cast<int64_t>(k) * N + i] * C[u * D * D + k * D + l];
+    VmW[u * N * D + t] = acc - W[u * N * D + t];  // (Q^T C - W)[i, l]
 }
 
-// Kp[i, j] = (K + I)[i, j] - sum_k Q[k, i] W[j, k] + sum_k (V - W)[i, k] Q[k, j]
-__global__ void k_proj_apply(const double* __restrict__ K, int64_t ldk, const double* __restrict__ Q,
-                             const double* __restrict__ W, const double* __restrict__ VmW, int N, int D,
-                             double* __restrict__ Kp, int64_t ldkp) {
+// Kp[i, j] = (K + I)[i, j] - sum_k Q[k, i] W[j, k] + sum_k (V - W)[i, k] Q[k, j]; Kp may be K
+__global__ void k_proj_apply(const double* K, int64_t ldk, const double* __restrict__ Q, const double* __restrict__ W,
+                             const double* __restrict__ VmW, int N, int D, double* Kp, int64_t ldkp) {
     int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
     if (t >= static_cast<int64_t>(N) * N) return;
+    const int64_t u = blockIdx.y;
     int i = static_cast<int>(t / N), j = static_cast<int>(t % N);
-    double a = K[static_cast<int64_t>(i) * ldk + j] + (i == j ? 1.0 : 0.0);
+    double a = K[u * N * ldk + static_cast<int64_t>(i) * ldk + j] + (i == j ? 1.0 : 0.0);
     double acc = 0.0;
     for (int k = 0; k < D; ++k) {
         const double qki = Q[static_cast<int64_t>(k) * N + i];
         const double qkj = Q[static_cast<int64_t>(k) * N + j];
-        acc += VmW[static_cast<int64_t>(i) * D + k] * qkj - qki * W[static_cast<int64_t>(j) * D + k];
+        acc += VmW[u * N * D + static_cast<int64_t>(i) * D + k] * qkj - qki * W[u * N * D + static_cast<int64_t>(j) * D + k];
     }
-    Kp[static_cast<int64_t>(i) * ldkp + j] = a + acc;
+    Kp[u * N * ldkp + static_cast<int64_t>(i) * ldkp + j] = a + acc;
+}
+
+int launch_project(const double* K, int64_t ldk, const double* Qx, int N, int D, int n_units, double* Kp, int64_t ldkp,
+                   void* work, cudaStream_t st) {
+    const size_t nd = static_cast<size_t>(N) * D, U = n_units;
+    double* W = static_cast<double*>(work);
+    double* VmW = W + U * nd;
+    double* C = VmW + U * nd;
+    const unsigned y = static_cast<unsigned>(n_units);
+    int rc;
+    k_proj_W<<<dim3(ceil_div(nd * 32, 256), y), 256, 0, st>>>(K, ldk, Qx, N, D, W);
+    if ((rc = check_launch("k_proj_W"))) return rc;
+    k_proj_C<<<dim3(1, y), 512, 0, st>>>(Qx, W, N, D, C);
+    if ((rc = check_launch("k_proj_C"))) return rc;
+    k_proj_V<<<dim3(ceil_div(nd, 256), y), 256, 0, st>>>(Qx, C, W, N, D, VmW);
+    if ((rc = check_launch("k_proj_V"))) return rc;
+    k_proj_apply<<<dim3(ceil_div(static_cast<int64_t>(N) * N, 256), y), 256, 0, st>>>(K, ldk, Qx, W, VmW, N, D, Kp, ldkp);
+    return check_launch("k_proj_apply");
 }
 
 template <typename T>
@@ -395,20 +416,15 @@ extern "C" int flmm_project_kinship(const double* K, int64_t ldk, const double* 
     flmm_project_kinship_workspace_bytes(N, D, &need);
     if (work_bytes < need)
         return fail(FLMM_ERR_WORKSPACE, "flmm_project_kinship: need %zu bytes, got %zu", need, work_bytes);
-    double* W = static_cast<double*>(work);
-    double* VmW = W + static_cast<size_t>(N) * D;
-    double* C = VmW + static_cast<size_t>(N) * D;
-    cudaStream_t st = as_stream(stream);
-    int64_t nd = static_cast<int64_t>(N) * D;
-    int rc;
-    k_proj_W<<<ceil_div(nd * 32, 256), 256, 0, st>>>(K, ldk, Qx, N, D, W);
-    if ((rc = check_launch("k_proj_W"))) return rc;
-    k_proj_C<<<1, 512, 0, st>>>(Qx, W, N, D, C);
-    if ((rc = check_launch("k_proj_C"))) return rc;
-    k_proj_V<<<ceil_div(nd, 256), 256, 0, st>>>(Qx, C, W, N, D, VmW);
-    if ((rc = check_launch("k_proj_V"))) return rc;
-    k_proj_apply<<<ceil_div(static_cast<int64_t>(N) * N, 256), 256, 0, st>>>(K, ldk, Qx, W, VmW, N, D, Kp, ldkp);
-    return check_launch("k_proj_apply");
+    return launch_project(K, ldk, Qx, N, D, 1, Kp, ldkp, work, as_stream(stream));
+}
+
+size_t flmm::project_kinships_bytes(int N, int D, int n_units) {
+    return sizeof(double) * n_units * (2 * static_cast<size_t>(N) * D + static_cast<size_t>(D) * D);
+}
+
+int flmm::project_kinships(double* K, const double* Qx, int N, int D, int n_units, void* work, cudaStream_t st) {
+    return launch_project(K, N, Qx, N, D, n_units, K, N, work, st);
 }
 
 extern "C" int flmm_compat_spectrum(const double* evals, int N, int D, double* s, void* stream) {

@@ -18,6 +18,23 @@ _i, _i64, _d, _p, _sz, _s = C.c_int, C.c_int64, C.c_double, C.c_void_p, C.c_size
 _pi32 = C.POINTER(C.c_int32)
 _psz = C.POINTER(C.c_size_t)
 
+class ScanOpts(C.Structure):
+    """flmm_scan_opts of include/fasterlmm_gb300.h."""
+    _fields_ = [("n_grid", C.c_int), ("log_delta_min", C.c_double), ("log_delta_max", C.c_double),
+                ("refine", C.c_int), ("eigh_refine_steps", C.c_int), ("f_refine", C.c_double), ("pipeline", C.c_int)]
+
+
+class Units(C.Structure):
+    """flmm_units of include/fasterlmm_gb300.h."""
+    _fields_ = [("N", C.c_int), ("D", C.c_int), ("P", C.c_int), ("n_real", C.c_int), ("n_units", C.c_int),
+                ("refine_cap", C.c_int), ("Yh", C.c_void_p), ("Yl", C.c_void_p), ("Yscale", C.c_void_p),
+                ("ldY", C.c_int64), ("Zh", C.c_void_p), ("Zl", C.c_void_p), ("Zscale", C.c_void_p), ("ldZ", C.c_int64),
+                ("unit_start", C.POINTER(C.c_int64)), ("unit_count", C.POINTER(C.c_int)), ("rows", C.c_void_p),
+                ("U", C.c_void_p), ("evals", C.c_void_p), ("opts", ScanOpts), ("f", C.c_void_p), ("beta", C.c_void_p),
+                ("se", C.c_void_p), ("sfve", C.c_void_p), ("nullh2", C.c_void_p), ("ldo", C.c_int64),
+                ("max_F", C.c_void_p), ("log_delta", C.c_void_p)]
+
+
 # name -> argument types (all return int status unless listed in _RESTYPE)
 SIGNATURES: dict[str, list] = {
     "flmm_version": [],
@@ -125,6 +142,10 @@ SIGNATURES: dict[str, list] = {
     "flmm_lr_interp_nodes": [_p, _i, _p, C.c_double, C.c_double, _i, _p, _i64, _p],
     "flmm_wald_refine_f32": [_p, _p, _p, _i, C.c_float, _p, _i64, _p, _i64, _p, _p, _i, _i, _i, _p, _p, _p, _p, _p,
                              _i64, _p, _p],
+    "flmm_loco_kinships_f32_workspace_bytes": [_i, _i, _i, C.POINTER(C.c_int), _i, _psz],
+    "flmm_loco_kinships_f32": [_p, _p, _i, C.POINTER(C.c_int), _i, C.POINTER(C.c_int), _i, _p, _i, _p, _p, _sz, _p],
+    "flmm_scan_units_workspace_bytes": [C.POINTER(Units), _psz],
+    "flmm_scan_units": [_p, C.POINTER(Units), _p, _sz, _p, _p],
     "flmm_scan_opts_default": [_p],
     "flmm_scan_create": [_i, _i, _i, _p, C.POINTER(_p)],
     "flmm_scan_destroy": [_p],
@@ -138,12 +159,6 @@ SIGNATURES: dict[str, list] = {
     "flmm_loco_kinship_f32": [_p, _p, _i, _d, _p, _p],
 }
 _RESTYPE = {"flmm_status_string": C.c_char_p, "flmm_last_error": C.c_char_p, "flmm_kernel_launches": C.c_uint64}
-
-
-class ScanOpts(C.Structure):
-    """flmm_scan_opts of include/fasterlmm_gb300.h."""
-    _fields_ = [("n_grid", C.c_int), ("log_delta_min", C.c_double), ("log_delta_max", C.c_double),
-                ("refine", C.c_int), ("eigh_refine_steps", C.c_int), ("f_refine", C.c_double), ("pipeline", C.c_int)]
 
 
 class FlmmError(RuntimeError):

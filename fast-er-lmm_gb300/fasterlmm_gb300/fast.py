@@ -10,7 +10,7 @@ O(Neff P M) products on the tensor cores:
 * the kinship eigendecomposition, the covariate SVD and the projection of K + I stay FP64.
 
 Device layouts: tested variants are grouped by chromosome (a stable reorder, undone by the output row map), so every
-chromosome is one contiguous row block of the split variant matrix; the kinship panel is also kept sample-major
+chromosome is one contiguous row block of the split variant matrix; the kinship panel is also formed sample-major
 with each chromosome's columns starting on a 64-column boundary, so the Gram of a chromosome is one K range.
 """
 
@@ -23,8 +23,7 @@ import torch
 from torch import Tensor
 
 from . import _lib
-from .core import F64, CovariateBasis, ScanResult, _alloc_outputs, _ptr, _stream, _work, compat_spectrum, \
-    eigh_batched, project_kinship
+from .core import F64, CovariateBasis, ScanResult, _alloc_outputs, _ptr, _stream, _work, compat_spectrum, eigh_batched
 
 F16 = torch.float16
 F32 = torch.float32
@@ -144,46 +143,23 @@ def _chrom_order(chrom: np.ndarray) -> tuple[np.ndarray | None, list]:
     return (None if np.array_equal(order, np.arange(chrom.size)) else order), blocks
 
 
-class KinshipPanel:
-    """Sample-major split of a standardised panel with 64-aligned chromosome column blocks, and its Grams."""
-
-    def __init__(self, Zt: Tensor, chrom: np.ndarray, ctx):
-        dev = Zt.device
-        M, N = Zt.shape
-        order, blocks = _chrom_order(chrom)
-        offs, off = [], 0
-        for _, _, n in blocks:
-            offs.append(off)
-            off += _pad(n, 64)
-        Mpad = max(off, 64)
-        Zg = torch.zeros((N, Mpad), dtype=F64, device=dev)
-        st = _stream(dev)
-        src = Zt if order is None else Zt.index_select(0, torch.from_numpy(order).to(dev))
-        for (c, a, n), o in zip(blocks, offs):
-            if n:
-                _lib.call("flmm_transpose_f64", _ptr(src[a:a + n]), N, n, N, _ptr(Zg[:, o:]), Mpad, st)
-        del src
-        self.split = SplitRows.of(Zg)
-        del Zg
-        self.M = M
-        self.counts = {c: n for (c, _, n) in blocks}
-        self.grams: dict = {}
-        self.Gtot = torch.zeros((N, N), dtype=F64, device=dev)
-        for (c, a, n), o in zip(blocks, offs):
-            G = torch.empty((N, N), dtype=F32, device=dev)
-            v = self.split.view(0, N, o, n)
-            gemm_split(ctx, v, v, G)
-            self.grams[c] = G
-            _lib.call("flmm_accumulate_f32_f64", N * N, _ptr(G), _ptr(self.Gtot), st)
-
-    def kinship(self, c) -> Tensor:
-        """LOCO kinship without chromosome c (c = None: all chromosomes)."""
-        N = self.Gtot.shape[0]
-        K = torch.empty((N, N), dtype=F64, device=self.Gtot.device)
-        Gc = self.grams.get(c) if c is not None else None
-        m = self.M - (self.counts.get(c, 0) if c is not None else 0)
-        _lib.call("flmm_loco_kinship_f32", _ptr(self.Gtot), _ptr(Gc), N, float(m), _ptr(K), _stream(K.device))
-        return K
+def loco_kinships(Zt: Tensor, chrom: np.ndarray, units: list, basis: CovariateBasis, ctx) -> Tensor:
+    """Projected kinships Kp (units, N, N) FP64 of the standardised panel Zt (M, N) without each unit's chromosome
+    (None: of the whole panel), from one Gram per chromosome."""
+    dev = Zt.device
+    N = Zt.shape[1]
+    D = basis.X.shape[1]
+    order, blocks = _chrom_order(chrom)
+    src = Zt.contiguous() if order is None else Zt.index_select(0, torch.from_numpy(order).to(dev))
+    at = {c: i for i, (c, _, _) in enumerate(blocks)}
+    counts = (C.c_int * max(len(blocks), 1))(*(n for _, _, n in blocks))
+    own = (C.c_int * len(units))(*(at.get(c, -1) if c is not None else -1 for c in units))
+    Kp = torch.empty((len(units), N, N), dtype=F64, device=dev)
+    nbytes = _lib.query_bytes("flmm_loco_kinships_f32_workspace_bytes", N, D, len(blocks), counts, len(units))
+    work = torch.empty(nbytes, dtype=torch.uint8, device=dev)  # (not the shared scratch: it is the size of the panel)
+    _lib.call("flmm_loco_kinships_f32", ctx, _ptr(src), N, counts, len(blocks), own, len(units), _ptr(basis.Qx), D,
+              _ptr(Kp), _ptr(work), nbytes, _stream(dev))
+    return Kp
 
 
 # sWs interpolation nodes in log delta: spacing and points of the local Lagrange rule (see csrc/flmm_fast.cu)
@@ -328,20 +304,17 @@ def scan_t(Zt: Tensor, X: Tensor, Yt: Tensor, chrom: np.ndarray, *, n_real: int,
     Zs = SplitRows.of(Zt if order_t is None else Zt.index_select(0, order_t))
     row_map = torch.arange(M, dtype=torch.int64, device=dev) if order_t is None else order_t.to(torch.int64)
 
-    kin = KinshipPanel(Zt if Zt_kin is None else Zt_kin, np.asarray(chrom if Zt_kin is None else chrom_kin), ctx)
     units = [(c, a, n) for (c, a, n) in blocks] if loco else [(None, 0, M)]
-    ops = WaldOperands(dev)
     log_deltas = {}
     D = X.shape[1]
     if N <= D:
         raise ValueError(f"need more samples than covariate columns (N={N}, D={D})")
     Neff = N - D
     ldk = _pad(Neff)
-    # all projected LOCO kinships first, so their FP64 eigendecompositions run side by side
+    # all projected LOCO kinships first, so their eigendecompositions run as one batch
+    Kp = loco_kinships(Zt if Zt_kin is None else Zt_kin, np.asarray(chrom if Zt_kin is None else chrom_kin),
+                       [c for c, _, _ in units], basis, ctx)
     slot = mark("eigh")
-    Kp = torch.empty((len(units), N, N), dtype=F64, device=dev)
-    for k_idx, (c, _, _) in enumerate(units):
-        project_kinship(kin.kinship(c), basis, Kp[k_idx])
     if EIGH_PRECISION == "f32r":
         Kp, evals = _eigh_batched_f32_refined(ctx, Kp)
     elif EIGH_PRECISION == "f32":
@@ -349,6 +322,16 @@ def scan_t(Zt: Tensor, X: Tensor, Yt: Tensor, chrom: np.ndarray, *, n_real: int,
     else:
         evals = eigh_batched(Kp, mode=EIGH_MODE)
     done(slot)
+    plain_loop = timers is None and sink is None and on_chrom is None
+    if plain_loop and EIGH_PRECISION == "f32r" and DELTA_PROPOSAL == "grid" and (REFINE_F is None or REFINE_F > 0):
+        lds = _scan_units(ctx, units, Ys, Zs, row_map, Kp, evals, D, n_real, out, max_F, n_grid=n_grid,
+                          log_delta_min=log_delta_min, log_delta_max=log_delta_max, refine=refine)
+        _lib.call("flmm_context_check", ctx, st)
+        for k, (c, _, _) in enumerate(units):
+            log_deltas[c if c is not None else 0] = lds[k]
+        return ScanResult(max_F=max_F, log_delta=log_deltas, **out)
+    # The same loop from Python: progress calls, stage timers, streamed results and the learned proposal hook into it.
+    ops = WaldOperands(dev)
     # Column side of chromosome k (its spectrum, eigenvector split, UY rotation and delta fit) runs on a side stream
     # one chromosome ahead of the variant side (US rotation, Wald operand prep, fused Wald) on the main stream, so
     # the delta fit's FP32 work shares the SMs with the tensor-core Wald kernel of the previous chromosome.  Two UY
@@ -413,6 +396,33 @@ def scan_t(Zt: Tensor, X: Tensor, Yt: Tensor, chrom: np.ndarray, *, n_real: int,
     if sink is not None:
         return sink.finish(max_F, log_deltas)
     return ScanResult(max_F=max_F, log_delta=log_deltas, **out)
+
+
+def _scan_units(ctx, units: list, Ys: SplitRows, Zs: SplitRows, row_map: Tensor, U: Tensor, evals: Tensor, D: int,
+                n_real: int, out: dict, max_F: Tensor, *, n_grid: int, log_delta_min: float, log_delta_max: float,
+                refine: bool) -> Tensor:
+    """The chromosome loop of scan_t in native code (flmm_scan_units): every unit's column and variant side into ``out``
+    and ``max_F``; returns log delta (units, P)."""
+    dev = U.device
+    n, N = U.shape[0], U.shape[1]
+    P = Ys.rows
+    lds = torch.empty((n, P), dtype=F64, device=dev)
+    at = lambda t: t.data_ptr() or None
+    q = _lib.Units(
+        N=N, D=D, P=P, n_real=n_real, n_units=n, refine_cap=REFINE_CAP, Yh=at(Ys.hi), Yl=at(Ys.lo), Yscale=at(Ys.scale),
+        ldY=Ys.ld, Zh=at(Zs.hi), Zl=at(Zs.lo), Zscale=at(Zs.scale), ldZ=Zs.ld,
+        unit_start=(C.c_int64 * n)(*(a for _, a, _ in units)), unit_count=(C.c_int * n)(*(m for _, _, m in units)),
+        rows=at(row_map), U=at(U), evals=at(evals),
+        opts=_lib.ScanOpts(n_grid=n_grid, log_delta_min=log_delta_min, log_delta_max=log_delta_max,
+                           refine=int(bool(refine)), f_refine=-1.0 if REFINE_F is None else REFINE_F),
+        **{k: at(out[k]) for k in ("f", "beta", "se", "sfve", "nullh2")}, ldo=n_real, max_F=at(max_F), log_delta=at(lds))
+    nbytes = _lib.query_bytes("flmm_scan_units_workspace_bytes", C.byref(q))
+    work = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+    main = torch.cuda.current_stream(dev)
+    side = torch.cuda.Stream(device=dev) if PIPELINE else main
+    _lib.call("flmm_scan_units", ctx, C.byref(q), _ptr(work), nbytes, C.c_void_p(main.cuda_stream),
+              C.c_void_p(side.cuda_stream))
+    return lds
 
 
 def _eigh_batched_f32(ctx, Kp: Tensor) -> tuple[Tensor, Tensor]:

@@ -595,6 +595,42 @@ int flmm_fill_rows_host_f64(double* dst, int64_t ld, int64_t rows, const double*
 int flmm_host_alloc_mapped(size_t bytes, void** host_ptr, void** dev_ptr);
 int flmm_host_free_mapped(void* host_ptr);
 
+/* ---- a scan's chromosome work on caller-owned buffers ---------------------------------------------------------- *
+ *
+ * flmm_loco_kinships_f32: projected LOCO kinships Kp (n_units, N, N) of a standardised panel Zt (M, N) whose rows are
+ * grouped into n_blocks chromosomes of counts[c] variants (host); unit u leaves out block unit_block[u] (-1: none).
+ * The steps of flmm_gemm_split_f16 Grams, flmm_loco_kinship_f32 and flmm_project_kinship, for all units.
+ *
+ * flmm_scan_units: every unit of a fast-form scan on `stream`, its column side (UY, delta fit) one unit ahead on
+ * `side_stream` (the same stream: one after another).  All pointers are device memory but unit_start and unit_count. */
+int flmm_loco_kinships_f32_workspace_bytes(int N, int D, int n_blocks, const int* counts, int n_units, size_t* bytes);
+int flmm_loco_kinships_f32(flmm_context* ctx, const double* Zt, int N, const int* counts, int n_blocks,
+                           const int* unit_block, int n_units, const double* Qx, int D, double* Kp, void* work,
+                           size_t work_bytes, void* stream);
+typedef struct flmm_units {
+    int N, D, P, n_real, n_units;
+    int refine_cap;             /* entries of the strong-test list at most */
+    const void *Yh, *Yl;        /* (P, ldY) regressed scan columns, split */
+    const float* Yscale;
+    int64_t ldY;
+    const void *Zh, *Zl;        /* (M, ldZ) tested variants grouped by unit, split */
+    const float* Zscale;
+    int64_t ldZ;
+    const int64_t* unit_start;  /* first grouped variant of each unit */
+    const int* unit_count;
+    const int64_t* rows;        /* (M,) output row of each grouped variant */
+    const float* U;             /* (n_units, N, N) eigenvector rows, ascending */
+    const double* evals;        /* (n_units, N) */
+    flmm_scan_opts opts;        /* (eigh_refine_steps and pipeline are not read) */
+    double *f, *beta, *se, *sfve, *nullh2;
+    int64_t ldo;
+    double* max_F;              /* (P,), raised */
+    double* log_delta;          /* (n_units, P) */
+} flmm_units;
+int flmm_scan_units_workspace_bytes(const flmm_units* units, size_t* bytes);
+int flmm_scan_units(flmm_context* ctx, const flmm_units* units, void* work, size_t work_bytes, void* stream,
+                    void* side_stream);
+
 #ifdef __cplusplus
 }
 #endif
