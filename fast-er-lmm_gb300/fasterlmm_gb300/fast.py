@@ -335,10 +335,11 @@ def scan_t(Zt: Tensor, X: Tensor, Yt: Tensor, chrom: np.ndarray, *, n_real: int,
     # Column side of chromosome k (its spectrum, eigenvector split, UY rotation and delta fit) runs on a side stream
     # one chromosome ahead of the variant side (US rotation, Wald operand prep, fused Wald) on the main stream, so
     # the delta fit's FP32 work shares the SMs with the tensor-core Wald kernel of the previous chromosome.  Two UY
-    # buffers alternate; the side stream reuses one only after the main stream's Wald prep has read it.
+    # buffers alternate (also on one stream, where k + 1's rotation is issued before k's Wald scan); the side stream
+    # reuses one only after the main stream's Wald prep has read it.
     main = torch.cuda.current_stream(dev)
     side = torch.cuda.Stream(device=dev) if PIPELINE else main
-    UY_bufs = [torch.empty((P, ldk), dtype=F32, device=dev) for _ in range(2 if PIPELINE else 1)]
+    UY_bufs = [torch.empty((P, ldk), dtype=F32, device=dev) for _ in range(2)]
     buf_free = [None] * len(UY_bufs)
     # made on the main stream and read on the side stream: their memory is not reused before the side stream's work
     # is done, also when an error ends the scan early
