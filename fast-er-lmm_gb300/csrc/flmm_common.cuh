@@ -51,6 +51,71 @@ int project_kinships(double* K, const double* Qx, int N, int D, int n_units, voi
 int interp_units(const double* s, int Neff, int n_units, float* shat, double x0, double h, int R, double* W,
                  cudaStream_t st);
 
+// One unit of a grouped split product: tiles of A rows [a_row0, a_row0 + a_rows) against B rows [b_row0, b_row0 + b_rows),
+// numbered from tile0 on (256 A rows x 128 B rows, csrc/flmm_fast.cu).
+struct UnitTiles {
+    int tile0, a_row0, a_rows, b_row0, b_rows;
+};
+constexpr int kUnitTileA = 256, kUnitTileB = 128;
+
+// Grouped launches over the units of a scan (csrc/flmm_fast.cu).  units: device array of n_units; total: all tiles.
+// units_pair_ok: whether grouped launches may run (the pair kernels are available and no other form is forced).
+bool units_pair_ok();
+// C[a row][b row - b_row0] = A B^T for every unit's rows, over K.
+int gemm_units(flmm_context* ctx, const void* Ah, const void* Al, const float* sa, int64_t lda, int a_total, const void* Bh,
+               const void* Bl, const float* sb, int64_t ldb, int b_total, int K, float* C, int64_t ldc,
+               const UnitTiles* units, int n_units, int total, cudaStream_t st);
+// The fused Wald of flmm_wald_split_f16 with the columns of unit u in rows u P .. of the column operands and variants in
+// rows of their own; listed tests hold the variant's row.  largest: the unit whose shape the tile order is tuned on.
+struct WaldUnits {
+    const void *A1h, *A1l;
+    int64_t lda;
+    const float* sa1;
+    const void *Lh, *Ll;
+    int64_t ldl;
+    const float *sl, *rWr, *rWr0;
+    int P, n_real, n_units;
+    const void *B1h, *B1l;
+    int64_t ldb;
+    const float* sb1;
+    const void *Fh, *Fl;
+    int64_t ldf;
+    const float* sf;
+    int M, Neff, R;
+    const int64_t* rows;
+    double *f, *beta, *se, *sfve;
+    int64_t ldo;
+    double* max_F;
+    float f_refine;
+    int32_t *flag_count, *flags;
+    int flag_cap;
+};
+int wald_units(flmm_context* ctx, const WaldUnits& w, const UnitTiles* units, int total, const UnitTiles& largest,
+               cudaStream_t st);
+// flmm_split_rows_f16 of n_units stacked FP32 matrices: rows of X from x_stride entries apart into rows dst_rows apart.
+int split_units(const float* X, int64_t ldx, int64_t x_stride, int rows, int K, int n_units, void* hi, void* lo, int64_t ldo,
+                int dst_rows, float* scale, cudaStream_t st);
+// flmm_wald_split_prep_columns of every unit: s32 (n_units, Neff), UY uy_stride entries apart, log delta (n_units, P),
+// outputs with unit u's columns from row u P on.
+int prep_columns_units(const float* s32, int Neff, const float* UYt, int64_t ldu, int64_t uy_stride, const double* log_delta,
+                       int P, int n_units, const float* shat, double x0, double h, int R, void* A1h, void* A1l, int64_t lda,
+                       void* Lh, void* Ll, int64_t ldl, float* sa1, float* sl, float* rWr, float* rWr0, cudaStream_t st);
+// flmm_fit_delta_fast of every unit (csrc/flmm_delta_fast.cu): s (n_units, Neff), log_delta and idx (n_units, P).
+size_t fit_units_bytes(int Neff, int n_grid, int n_units);
+int fit_delta_units(const double* s, int Neff, const float* UYt, int64_t ldu, int64_t uy_stride, int P, int n_units,
+                    int n_grid, double lo, double hi, int refine, double* log_delta, int32_t* idx, void* work,
+                    cudaStream_t st);
+// flmm_wald_refine_f32 of every unit (csrc/flmm_wald_refine.cu): variant rows over all units, unit u's from start[u] on
+// (device, n_units + 1 entries).
+int wald_refine_units(flmm_context* ctx, const int32_t* flags, const int32_t* flag_count, int flag_cap, float f_refine,
+                      const float* US, int64_t ldus, const float* UYt, int64_t ldu, int64_t uy_stride, const float* s32,
+                      const double* log_delta, int P, int Neff, int M, int n_real, const int* start, int n_units,
+                      const int64_t* rows, double* f, double* beta, double* se, double* sfve, int64_t ldo, double* max_F,
+                      cudaStream_t st);
+// flmm_fill_nullh2 of every unit (csrc/flmm_prep.cu).
+int fill_nullh2_units(const double* log_delta, int P, int n_real, const int64_t* rows, const int* start, int n_units,
+                      int most, double* out, int64_t ldo, cudaStream_t st);
+
 inline unsigned ceil_div(int64_t a, int64_t b) { return static_cast<unsigned>((a + b - 1) / b); }
 
 #define FLMM_REQUIRE(cond, ...)                                                       \

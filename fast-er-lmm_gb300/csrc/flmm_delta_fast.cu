@@ -28,6 +28,10 @@ __global__ void k_grid_weights_f32(const double* __restrict__ s, int Neff, const
                                    float* __restrict__ Wg, float* __restrict__ sum_log) {
     __shared__ double red[32];
     const int g = blockIdx.x;
+    // grid.y spectra
+    s += static_cast<int64_t>(blockIdx.y) * Neff;
+    Wg += static_cast<int64_t>(blockIdx.y) * gridDim.x * Neff;
+    sum_log += static_cast<int64_t>(blockIdx.y) * gridDim.x;
     const double delta = exp(grid[g]);
     double acc = 0.0;
     for (int n = threadIdx.x; n < Neff; n += blockDim.x) {
@@ -59,7 +63,7 @@ template <bool kList>
 __global__ void __launch_bounds__(NT)
 k_grid_argmin_f32(const float* __restrict__ Wg, const float* __restrict__ sum_log, const float* __restrict__ UYt,
                   int64_t ldu, int Neff, int P, int G, int32_t* __restrict__ idx_out, const int32_t* __restrict__ cols,
-                  const int32_t* __restrict__ count) {
+                  const int32_t* __restrict__ count, int64_t uy_stride) {
     __shared__ __align__(16) float Ws[TK * WS_LD];
     __shared__ __align__(16) float Us[TK * US_LD];
     __shared__ float red_v[8][TP];
@@ -68,6 +72,11 @@ k_grid_argmin_f32(const float* __restrict__ Wg, const float* __restrict__ sum_lo
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     const int lane = tid & 31, warp = tid >> 5;
     const int p0 = blockIdx.x * TP;
+    // grid.y units
+    Wg += static_cast<int64_t>(blockIdx.y) * G * Neff;
+    sum_log += static_cast<int64_t>(blockIdx.y) * G;
+    UYt += blockIdx.y * uy_stride;
+    idx_out += static_cast<int64_t>(blockIdx.y) * P;
     if (kList) {
         const int n = min(*count, P);
         if (p0 >= n) return;
@@ -173,6 +182,11 @@ k_grid_argmin_f32(const float* __restrict__ Wg, const float* __restrict__ sum_lo
 __global__ void k_spectrum_prep(const double* __restrict__ s, int Neff, float* __restrict__ s32,
                                 float* __restrict__ dsb, float* __restrict__ sbar_out) {
     __shared__ double red[32];
+    // a block per spectrum
+    const int64_t u0 = static_cast<int64_t>(blockIdx.x) * Neff;
+    s += u0;
+    s32 += u0;
+    dsb += u0;
     double acc = 0.0;
     for (int n = threadIdx.x; n < Neff; n += blockDim.x) acc += s[n];
     acc = warp_sum(acc);
@@ -190,7 +204,7 @@ __global__ void k_spectrum_prep(const double* __restrict__ s, int Neff, float* _
         s32[n] = sn;
         dsb[n] = sbar - sn;
     }
-    if (threadIdx.x == 0) *sbar_out = sbar;
+    if (threadIdx.x == 0) sbar_out[blockIdx.x] = sbar;
 }
 
 // Lanes per column of the refinement: two columns per warp (see group_sum).
@@ -201,13 +215,17 @@ constexpr int kNewtonLanes = 16;
 __global__ void k_newton_refine(const float* __restrict__ s32, const float* __restrict__ dsb,
                                 const float* __restrict__ sbar_p, int Neff, const float* __restrict__ UYt, int64_t ldu,
                                 int P, const double* __restrict__ grid, int G, const int32_t* __restrict__ idx,
-                                int refine, double* __restrict__ log_delta) {
+                                int refine, double* __restrict__ log_delta, int64_t uy_stride) {
     constexpr int W = kNewtonLanes;
     const int lane = threadIdx.x & (W - 1);
-    const int64_t p = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) / W;
-    if (p >= P) return;
-    const float* u = UYt + p * ldu;
-    const float sbar = *sbar_p;
+    const int64_t col = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) / W;
+    if (col >= P) return;
+    // grid.y units
+    const int64_t unit = blockIdx.y, p = unit * P + col;
+    s32 += unit * Neff;
+    dsb += unit * Neff;
+    const float* u = UYt + unit * uy_stride + col * ldu;
+    const float sbar = sbar_p[unit];
     const int i = idx[p];
     // one pass gives the column's sum of squares and the evaluations at the grid argmin and its two neighbours (the
     // bracket test of the usual case), sharing the loads of the column and the spectrum
@@ -243,21 +261,28 @@ __global__ void k_newton_refine(const float* __restrict__ s32, const float* __re
     if (lane == 0) log_delta[p] = out;
 }
 
+// Every unit's fit; one unit with uy_stride 0 is the plain call.  The tables of all units stand one after another.
+int launch_fits(const double* s, int Neff, const float* UYt, int64_t ldu, int64_t uy_stride, int P, int units, int G,
+                double lo, double hi, int refine, double* log_delta, int32_t* idx, const FastWs& w, cudaStream_t st) {
+    const unsigned y = static_cast<unsigned>(units);
+    int rc = flmm_delta_grid_nodes(lo, hi, G, w.grid, st);
+    if (rc) return rc;
+    k_grid_weights_f32<<<dim3(G, y), 256, 0, st>>>(s, Neff, w.grid, w.Wg, w.sum_log);
+    if ((rc = check_launch("k_grid_weights_f32"))) return rc;
+    k_grid_argmin_f32<false><<<dim3(ceil_div(P, TP), y), NT, 0, st>>>(w.Wg, w.sum_log, UYt, ldu, Neff, P, G, idx, nullptr,
+                                                                      nullptr, uy_stride);
+    if ((rc = check_launch("k_grid_argmin_f32"))) return rc;
+    k_spectrum_prep<<<y, 256, 0, st>>>(s, Neff, w.s32, w.dsb, w.sbar);
+    if ((rc = check_launch("k_spectrum_prep"))) return rc;
+    k_newton_refine<<<dim3(ceil_div(static_cast<int64_t>(P) * kNewtonLanes, 256), y), 256, 0, st>>>(
+        w.s32, w.dsb, w.sbar, Neff, UYt, ldu, P, w.grid, G, idx, refine, log_delta, uy_stride);
+    return check_launch("k_newton_refine");
+}
+
 int launch_fast_fit(const double* s, int Neff, const float* UYt, int64_t ldu, int P, int n_grid, double lo,
                     double hi, int refine, double* log_delta, int32_t* grid_idx, void* scratch, cudaStream_t st) {
-    const FastWs w = carve_fast(scratch, Neff, n_grid);
-    int rc = flmm_delta_grid_nodes(lo, hi, n_grid, w.grid, st);
-    if (rc) return rc;
-    k_grid_weights_f32<<<n_grid, 256, 0, st>>>(s, Neff, w.grid, w.Wg, w.sum_log);
-    if ((rc = check_launch("k_grid_weights_f32"))) return rc;
-    k_grid_argmin_f32<false><<<ceil_div(P, TP), NT, 0, st>>>(w.Wg, w.sum_log, UYt, ldu, Neff, P, n_grid, grid_idx,
-                                                             nullptr, nullptr);
-    if ((rc = check_launch("k_grid_argmin_f32"))) return rc;
-    k_spectrum_prep<<<1, 256, 0, st>>>(s, Neff, w.s32, w.dsb, w.sbar);
-    if ((rc = check_launch("k_spectrum_prep"))) return rc;
-    k_newton_refine<<<ceil_div(static_cast<int64_t>(P) * kNewtonLanes, 256), 256, 0, st>>>(
-        w.s32, w.dsb, w.sbar, Neff, UYt, ldu, P, w.grid, n_grid, grid_idx, refine, log_delta);
-    return check_launch("k_newton_refine");
+    return launch_fits(s, Neff, UYt, ldu, 0, P, 1, n_grid, lo, hi, refine, log_delta, grid_idx,
+                       carve_fast(scratch, Neff, n_grid), st);
 }
 
 }  // namespace
@@ -291,7 +316,7 @@ int launch_grid_tables(const double* s, int Neff, double lo, double hi, int G, c
 
 int launch_grid_argmin_list(const FastWs& w, const float* UYt, int64_t ldu, int Neff, int P, int G,
                             const int32_t* cols, const int32_t* count, int32_t* idx, cudaStream_t st) {
-    k_grid_argmin_f32<true><<<ceil_div(P, TP), NT, 0, st>>>(w.Wg, w.sum_log, UYt, ldu, Neff, P, G, idx, cols, count);
+    k_grid_argmin_f32<true><<<ceil_div(P, TP), NT, 0, st>>>(w.Wg, w.sum_log, UYt, ldu, Neff, P, G, idx, cols, count, 0);
     return check_launch("k_grid_argmin_f32 (column list)");
 }
 
@@ -301,12 +326,32 @@ int launch_refine(const double* s, int Neff, const float* UYt, int64_t ldu, int 
     int rc = check_launch("k_spectrum_prep");
     if (rc) return rc;
     k_newton_refine<<<ceil_div(static_cast<int64_t>(P) * kNewtonLanes, 256), 256, 0, st>>>(
-        w.s32, w.dsb, w.sbar, Neff, UYt, ldu, P, w.grid, G, idx, refine, log_delta);
+        w.s32, w.dsb, w.sbar, Neff, UYt, ldu, P, w.grid, G, idx, refine, log_delta, 0);
     return check_launch("k_newton_refine");
 }
 
 }  // namespace dfit
 }  // namespace flmm
+
+size_t flmm::fit_units_bytes(int Neff, int n_grid, int n_units) {
+    const size_t G = n_grid, n = Neff, u = n_units;
+    return sizeof(double) * G + sizeof(float) * u * (G * n + G + 2 * n + 1) + 512;
+}
+
+int flmm::fit_delta_units(const double* s, int Neff, const float* UYt, int64_t ldu, int64_t uy_stride, int P, int n_units,
+                          int n_grid, double lo, double hi, int refine, double* log_delta, int32_t* idx, void* work,
+                          cudaStream_t st) {
+    if (P == 0) return FLMM_OK;
+    const size_t G = n_grid, n = Neff, u = n_units;
+    FastWs w;
+    w.grid = static_cast<double*>(work);
+    w.Wg = reinterpret_cast<float*>(w.grid + G);
+    w.sum_log = w.Wg + u * G * n;
+    w.s32 = w.sum_log + u * G;
+    w.dsb = w.s32 + u * n;
+    w.sbar = w.dsb + u * n;
+    return launch_fits(s, Neff, UYt, ldu, uy_stride, P, n_units, n_grid, lo, hi, refine, log_delta, idx, w, st);
+}
 
 extern "C" int flmm_fit_delta_fast_workspace_bytes(int Neff, int n_grid, size_t* bytes) {
     FLMM_REQUIRE(bytes && Neff > 0 && n_grid > 0, "flmm_fit_delta_fast_workspace_bytes: bad arguments");

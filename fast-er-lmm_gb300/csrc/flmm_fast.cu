@@ -117,6 +117,9 @@ struct TcArgs {
     int group;
     // k-blocks per chunk accumulator of product 0 (>= 1)
     int chunk_kb;
+    // grouped launch (pair kernel): the tiles of n_units units, each with its own row ranges of both operands
+    const UnitTiles* units;
+    int n_units, total_tiles;
 };
 
 // Tile t of the persistent schedule -> (A block ta, B block tb).  Tiles are visited in groups of `group` A blocks;
@@ -131,6 +134,27 @@ __device__ __forceinline__ void tile_coords(int t, int tiles_a, int tiles_b, int
     const int ga = min(g, tiles_a - k * g);
     tb = tl / ga;
     ta = k * g + tl % ga;
+}
+
+// The pair kernel's tile t: block coordinates within its unit and the unit's row ranges (the whole operands when the
+// launch is not grouped).  `u` is the unit of an earlier tile of the caller's schedule.
+struct PairTile {
+    int ta, tb, a_row0, a_rows, b_row0, b_rows;
+};
+
+__device__ __forceinline__ PairTile pair_tile(const TcArgs& args, int t, int& u) {
+    PairTile r{0, 0, 0, args.Mr, 0, args.Nr};
+    if (args.units != nullptr) {
+        while (u + 1 < args.n_units && t >= args.units[u + 1].tile0) ++u;
+        const UnitTiles q = args.units[u];
+        t -= q.tile0;
+        r.a_row0 = q.a_row0;
+        r.a_rows = q.a_rows;
+        r.b_row0 = q.b_row0;
+        r.b_rows = q.b_rows;
+    }
+    tile_coords(t, (r.a_rows + kUnitTileA - 1) / kUnitTileA, (r.b_rows + kUnitTileB - 1) / kUnitTileB, args.group, r.ta, r.tb);
+    return r;
 }
 
 // hardware reciprocal (relative error ~2^-23); arguments here are clamped to normal numbers
@@ -556,7 +580,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_pair(const __grid_constant_
     const int cl = static_cast<int>(cluster_id_x()), n_cl = static_cast<int>(cluster_count_x());
     const int tiles_b = (args.Nr + kBN - 1) / kBN;
     const int tiles_a = (args.Mr + kPairRows - 1) / kPairRows;
-    const int n_tiles = tiles_a * tiles_b;
+    const int n_tiles = args.units != nullptr ? args.total_tiles : tiles_a * tiles_b;
     const int n_kb0 = (args.K + C::kBK - 1) / C::kBK;
     const int n_kb = n_kb0 + (NG == 2 ? (args.K2 + C::kBK - 1) / C::kBK : 0);
     constexpr uint32_t idesc = idesc_f16_f32(kPairRows, kBN);
@@ -590,16 +614,15 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_pair(const __grid_constant_
         // ---- TMA producer (both CTAs): this CTA's halves of the tile, counted on the even CTA's full[] ----
         if (lane == 0) {
             const uint32_t full0 = map_to_rank(smem_u32(full), 0);
-            int stage = 0;
+            int stage = 0, unit = 0;
             uint32_t phase = 0;
             bool armed[C::kStages] = {};
             uint32_t armed_phase[C::kStages] = {};
             bool ok = true;
             for (int t = cl; t < n_tiles && ok; t += n_cl) {
-                int ta, tb;
-                tile_coords(t, tiles_a, tiles_b, args.group, ta, tb);
-                const int arow = ta * kPairRows + static_cast<int>(rank) * 128;
-                const int brow = tb * kBN + static_cast<int>(rank) * (kBN / 2);
+                const PairTile pt = pair_tile(args, t, unit);
+                const int arow = pt.a_row0 + pt.ta * kPairRows + static_cast<int>(rank) * 128;
+                const int brow = pt.b_row0 + pt.tb * kBN + static_cast<int>(rank) * (kBN / 2);
                 for (int kb = 0; kb < n_kb; ++kb) {
                     if (!mbar_wait(&empty[stage], phase ^ 1u, args.err, 1)) { ok = false; break; }
                     if (leader) {
@@ -682,24 +705,38 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_pair(const __grid_constant_
         int64_t* rws = reinterpret_cast<int64_t*>(sc2 + kPairCols);
         const uint32_t slot_empty0 = map_to_rank(smem_u32(slot_empty), 0);
         const uint32_t tl0 = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(cbeg);
-        int slot = 0;
+        int slot = 0, unit = 0;
         uint32_t sphase = 0;
         bool ok = true;
         for (int t = cl; t < n_tiles && ok; t += n_cl) {
-            int ta, tb;
-            tile_coords(t, tiles_a, tiles_b, args.group, ta, tb);
-            const int nvalid = min(kBN, args.Nr - tb * kBN);
+            const PairTile pt = pair_tile(args, t, unit);
+            const int ta = pt.ta, tb = pt.tb;
+            const int nvalid = min(kBN, pt.b_rows - tb * kBN);
             const int row0 = ta * kPairRows + static_cast<int>(rank) * 128;
+            // the unit's own rows of the scales and outputs
+            TcArgs ua = args;
+            ua.Mr = pt.a_rows;
+            ua.sa += pt.a_row0;
+            ua.sb += pt.b_row0;
+            if constexpr (NG == 2) {
+                ua.sa2 += pt.a_row0;
+                ua.rWr += pt.a_row0;
+                ua.rWr0 += pt.a_row0;
+                ua.sb2 += pt.b_row0;
+                ua.rows += pt.b_row0;
+            } else {
+                ua.C += static_cast<int64_t>(pt.a_row0) * args.ldc;
+            }
             const bool real_tile = NG == 2 && row0 < args.n_real;  // uniform over the CTA
             __syncwarp();
             for (int k = lane; k < kPairCols; k += 32) {
                 const int c = cbeg + k;
                 const int m = tb * kBN + c;
                 const bool okc = c < nvalid;
-                sc1[k] = okc ? args.sb[m] : 0.0f;
+                sc1[k] = okc ? ua.sb[m] : 0.0f;
                 if constexpr (NG == 2) {
-                    sc2[k] = okc ? args.sb2[m] : 0.0f;
-                    if (real_tile) rws[k] = okc ? args.rows[m] : 0;
+                    sc2[k] = okc ? ua.sb2[m] : 0.0f;
+                    if (real_tile) rws[k] = okc ? ua.rows[m] : 0;
                 }
             }
             __syncwarp();
@@ -720,14 +757,14 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_pair(const __grid_constant_
             }
             if (!ok) break;
             if constexpr (NG == 1) {
-                gemm_rows(args, acc0, row0 + r, tb * kBN, nvalid, cbeg, sc1);
+                gemm_rows(ua, acc0, row0 + r, tb * kBN, nvalid, cbeg, sc1);
             } else {
                 // product 1 (one chunk) is read from its slot by the statistics, then the slot is handed back
                 const bool got = mbar_wait(&slot_full[slot], sphase, args.err, 4);
                 if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
                 fence_after_sync();
-                wald_rows(args, acc0, tl0 + static_cast<uint32_t>(slot * kBN), row0 + r, real_tile, nvalid, cbeg,
-                          tb * kBN, sc1, sc2, rws);
+                wald_rows(ua, acc0, tl0 + static_cast<uint32_t>(slot * kBN), row0 + r, real_tile, nvalid, cbeg,
+                          pt.b_row0 + tb * kBN, sc1, sc2, rws);
                 fence_before_sync();
                 __syncwarp();
                 if (lane == 0) mbar_arrive_cluster_relaxed(slot_empty0 + static_cast<uint32_t>(slot * 8));
@@ -755,11 +792,13 @@ constexpr int kSplitCache = 32;  // per-lane register cache of k_split_rows: row
 template <typename T>
 __global__ void __launch_bounds__(256)
 k_split_rows(const T* __restrict__ X, int64_t ldx, int rows, int K, __half* __restrict__ hi,
-             __half* __restrict__ lo, int64_t ldo, float* __restrict__ scale) {
+             __half* __restrict__ lo, int64_t ldo, float* __restrict__ scale, int64_t x_stride, int dst_rows) {
     const int lane = threadIdx.x & 31;
-    const int64_t r = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5;
-    if (r >= rows) return;
-    const T* x = X + r * ldx;
+    const int64_t rx = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5;
+    if (rx >= rows) return;
+    // (grid.y stacked matrices)
+    const T* x = X + blockIdx.y * x_stride + rx * ldx;
+    const int64_t r = rx + static_cast<int64_t>(blockIdx.y) * dst_rows;
     // rows of up to 32 * kSplitCache entries are read and rounded once, into registers, for both passes
     float xv[kSplitCache];
     const bool cached = K <= 32 * kSplitCache;
@@ -849,12 +888,15 @@ k_wald_prep_columns(const float* __restrict__ s32, int Neff, const float* __rest
                     const double* __restrict__ ld, int P, const float* __restrict__ shat_p, double x0, double h,
                     double inv_h, int R, __half* __restrict__ A1h, __half* __restrict__ A1l, int64_t lda,
                     __half* __restrict__ Lh, __half* __restrict__ Ll, int64_t ldl, float* __restrict__ sa1,
-                    float* __restrict__ sl, float* __restrict__ rWr, float* __restrict__ rWr0) {
+                    float* __restrict__ sl, float* __restrict__ rWr, float* __restrict__ rWr0, int64_t uy_stride) {
     __shared__ float lw[kPrepCols][kInterpPoints];
     __shared__ int lbase[kPrepCols];
     const int lane = threadIdx.x & 31, j = threadIdx.x >> 5;
-    const int64_t p = static_cast<int64_t>(blockIdx.x) * kPrepCols + j;
-    if (p >= P) return;
+    const int64_t col = static_cast<int64_t>(blockIdx.x) * kPrepCols + j;
+    if (col >= P) return;
+    // grid.y units; p is the column's row of the outputs
+    const int64_t unit = blockIdx.y, p = unit * P + col;
+    s32 += unit * Neff;
     const double x = ld[p];
     // Lagrange weights of the column's warp on nodes base .. base + 9 around x, by its lanes 0..9:
     // w_k = prod_{m != k} (t - m) / prod_{m != k} (k - m), the denominators' reciprocals being constants (the FP64
@@ -875,8 +917,8 @@ k_wald_prep_columns(const float* __restrict__ s32, int Neff, const float* __rest
     const float xh = static_cast<float>(x);
     const float xl = static_cast<float>(x - static_cast<double>(xh));
     const float delta = expf(xh) * (1.0f + xl);
-    const float num = *shat_p + delta;
-    const float* u = UYt + p * ldu;
+    const float num = shat_p[unit] + delta;
+    const float* u = UYt + unit * uy_stride + col * ldu;
     float m1 = 0.0f, acc = 0.0f, comp = 0.0f;
     // a column of up to 32 * kPrepCache entries is read once and its weighted values kept in registers for the split
     float av[kPrepCache];
@@ -1082,7 +1124,7 @@ int pair_clusters(int device) {
 
 template <int NG>
 int launch_pair(const TcMaps& maps, const TcArgs& args, int n_clusters_max, cudaStream_t st) {
-    const int tiles = ((args.Mr + kPairRows - 1) / kPairRows) * ((args.Nr + kBN - 1) / kBN);
+    const int tiles = args.units ? args.total_tiles : ((args.Mr + kPairRows - 1) / kPairRows) * ((args.Nr + kBN - 1) / kBN);
     if (tiles == 0 || args.K <= 0) return FLMM_OK;
     const int n_cl = tiles < n_clusters_max ? tiles : n_clusters_max;
     cudaLaunchConfig_t cfg = {};
@@ -1187,12 +1229,11 @@ int time_choice(const TcMaps& maps_tc, const TcMaps& maps_pair, const TcArgs& a,
     return FLMM_OK;
 }
 
-// Launch one split product with the configured choice (see above).  maps_pair holds the pair kernel's half-height B
-// maps; n_cl = 0 when the device cannot run the pair kernel.
+// The configured choice for one split product (see above), tuned on its operands if need be.  maps_pair holds the pair
+// kernel's half-height B maps; n_cl = 0 when the device cannot run the pair kernel.
 template <int NG>
-int launch_product(const TcMaps& maps_tc, const TcMaps& maps_pair, const TcArgs& a, int n_cl, int sm_count,
-                   bool rerunnable, cudaStream_t st) {
-    if (!use_pair_kernel()) n_cl = 0;  // FLMM_TC_PAIR=0: single-CTA kernels only
+int choose_product(const TcMaps& maps_tc, const TcMaps& maps_pair, const TcArgs& a, int n_cl, int sm_count,
+                   bool rerunnable, cudaStream_t st, TcChoice* out) {
     const TcChoice def = {n_cl > 0, 1};
     TcChoice choice = def;
     std::unique_lock<std::mutex> lock(g_tune_mu);
@@ -1257,7 +1298,18 @@ int launch_product(const TcMaps& maps_tc, const TcMaps& maps_pair, const TcArgs&
         }
     }
     if (lock.owns_lock()) lock.unlock();
-    return launch_choice<NG>(maps_tc, maps_pair, a, choice, n_cl, sm_count, st);
+    *out = choice;
+    return FLMM_OK;
+}
+
+// Launch one split product with its choice.
+template <int NG>
+int launch_product(const TcMaps& maps_tc, const TcMaps& maps_pair, const TcArgs& a, int n_cl, int sm_count,
+                   bool rerunnable, cudaStream_t st) {
+    if (!use_pair_kernel()) n_cl = 0;  // FLMM_TC_PAIR=0: single-CTA kernels only
+    TcChoice choice;
+    int rc = choose_product<NG>(maps_tc, maps_pair, a, n_cl, sm_count, rerunnable, st, &choice);
+    return rc ? rc : launch_choice<NG>(maps_tc, maps_pair, a, choice, n_cl, sm_count, st);
 }
 
 }  // namespace
@@ -1314,9 +1366,9 @@ extern "C" int flmm_split_rows_f16(const void* X, int x_is_f64, int64_t ldx, int
     }
     const unsigned grid = ceil_div(static_cast<int64_t>(rows) * 32, 256);  // one warp per row
     if (x_is_f64)
-        k_split_rows<double><<<grid, 256, 0, st>>>(static_cast<const double*>(X), ldx, rows, K, h, l, ldo, scale);
+        k_split_rows<double><<<grid, 256, 0, st>>>(static_cast<const double*>(X), ldx, rows, K, h, l, ldo, scale, 0, 0);
     else
-        k_split_rows<float><<<grid, 256, 0, st>>>(static_cast<const float*>(X), ldx, rows, K, h, l, ldo, scale);
+        k_split_rows<float><<<grid, 256, 0, st>>>(static_cast<const float*>(X), ldx, rows, K, h, l, ldo, scale, 0, 0);
     return check_launch("k_split_rows");
 }
 
@@ -1389,7 +1441,7 @@ extern "C" int flmm_wald_split_prep_columns(const float* s32, int Neff, const fl
     if (P == 0) return FLMM_OK;
     k_wald_prep_columns<<<ceil_div(P, kPrepCols), 32 * kPrepCols, 0, as_stream(stream)>>>(
         s32, Neff, UYt, ldu, log_delta, P, shat, x0, h, 1.0 / h, R, static_cast<__half*>(A1h), static_cast<__half*>(A1l), lda,
-        static_cast<__half*>(Lh), static_cast<__half*>(Ll), ldl, sa1, sl, rWr, rWr0);
+        static_cast<__half*>(Lh), static_cast<__half*>(Ll), ldl, sa1, sl, rWr, rWr0, 0);
     return check_launch("k_wald_prep_columns");
 }
 
@@ -1485,4 +1537,139 @@ extern "C" int flmm_wald_split_f16_df(flmm_context* ctx, const void* A1h, const 
         if ((rc = make_map(&maps_pair.m[7], Fl, Mc, R, ldf, kBK, kBN / 2))) return rc;
     }
     return launch_product<2>(maps, maps_pair, a, n_cl, flmm_ctx_sm_count(ctx), true, as_stream(stream));
+}
+
+// ---- grouped launches over a scan's units ---------------------------------------------------------------------------
+
+namespace {
+
+int pair_count(int* n_cl1, int* n_cl2) {
+    int dev = 0;
+    FLMM_CUDA(cudaGetDevice(&dev));
+    *n_cl1 = use_pair_kernel() ? pair_clusters<1>(dev) : 0;
+    *n_cl2 = use_pair_kernel() ? pair_clusters<2>(dev) : 0;
+    return FLMM_OK;
+}
+
+}  // namespace
+
+bool flmm::units_pair_ok() {
+    int a = 0, b = 0;
+    if (pair_count(&a, &b) || a <= 0 || b <= 0) return false;
+    std::lock_guard<std::mutex> lock(g_tune_mu);
+    return tune_mode_locked() != 2 || g_forced.pair;
+}
+
+int flmm::gemm_units(flmm_context* ctx, const void* Ah, const void* Al, const float* sa, int64_t lda, int a_total,
+                     const void* Bh, const void* Bl, const float* sb, int64_t ldb, int b_total, int K, float* Cout,
+                     int64_t ldc, const UnitTiles* units, int n_units, int total, cudaStream_t st) {
+    int n1 = 0, n2 = 0;
+    int rc = pair_count(&n1, &n2);
+    if (rc || total == 0) return rc;
+    TcMaps maps;
+    std::memset(&maps, 0, sizeof(maps));
+    if ((rc = make_map(&maps.m[0], Ah, a_total, K, lda, kBK))) return rc;
+    if ((rc = make_map(&maps.m[1], Al, a_total, K, lda, kBK))) return rc;
+    if ((rc = make_map(&maps.m[2], Bh, b_total, K, ldb, kBK, kBN / 2))) return rc;
+    if ((rc = make_map(&maps.m[3], Bl, b_total, K, ldb, kBK, kBN / 2))) return rc;
+    TcArgs a;
+    std::memset(&a, 0, sizeof(a));
+    a.K = K;
+    a.err = flmm_ctx_err_flag(ctx);
+    a.sa = sa;
+    a.sb = sb;
+    a.C = Cout;
+    a.ldc = ldc;
+    a.group = 1;
+    a.chunk_kb = chunk_kb_for<1>();
+    a.units = units;
+    a.n_units = n_units;
+    a.total_tiles = total;
+    return launch_pair<1>(maps, a, n1, st);
+}
+
+int flmm::wald_units(flmm_context* ctx, const WaldUnits& w, const UnitTiles* units, int total, const UnitTiles& largest,
+                     cudaStream_t st) {
+    int n1 = 0, n2 = 0;
+    int rc = pair_count(&n1, &n2);
+    if (rc) return rc;
+    if (w.flag_count != nullptr) FLMM_CUDA(cudaMemsetAsync(w.flag_count, 0, sizeof(int32_t), st));
+    if (total == 0) return FLMM_OK;
+    // maps over the column rows [a0, a0 + na) and variant rows [b0, b0 + nb), with boxes of `box` variant rows
+    auto make = [&](TcMaps* m, int a0, int na, int b0, int nb, int box) -> int {
+        std::memset(m, 0, sizeof(*m));
+        const __half* p[8] = {static_cast<const __half*>(w.A1h) + a0 * w.lda, static_cast<const __half*>(w.A1l) + a0 * w.lda,
+                              static_cast<const __half*>(w.B1h) + b0 * w.ldb, static_cast<const __half*>(w.B1l) + b0 * w.ldb,
+                              static_cast<const __half*>(w.Lh) + a0 * w.ldl,  static_cast<const __half*>(w.Ll) + a0 * w.ldl,
+                              static_cast<const __half*>(w.Fh) + b0 * w.ldf,  static_cast<const __half*>(w.Fl) + b0 * w.ldf};
+        const int64_t ld[4] = {w.lda, w.ldb, w.ldl, w.ldf};
+        for (int i = 0; i < 8; ++i) {
+            const bool var = i & 2;
+            int r2 = make_map(&m->m[i], p[i], var ? nb : na, i < 4 ? w.Neff : w.R, ld[i / 2], kBK, var ? box : kBM);
+            if (r2) return r2;
+        }
+        return FLMM_OK;
+    };
+    TcArgs a;
+    std::memset(&a, 0, sizeof(a));
+    a.K = w.Neff;
+    a.K2 = w.R;
+    a.err = flmm_ctx_err_flag(ctx);
+    a.n_real = w.n_real;
+    a.var_df = static_cast<float>(w.Neff - 1);
+    a.f = w.f;
+    a.beta = w.beta;
+    a.se = w.se;
+    a.sfve = w.sfve;
+    a.ldo = w.ldo;
+    a.max_F = w.max_F;
+    a.f_refine = w.f_refine;
+    a.flag_count = w.flag_count;
+    a.flags = reinterpret_cast<int2*>(w.flags);
+    a.flag_cap = w.flag_cap;
+    auto rows_at = [&](TcArgs* q, int a0, int b0) {
+        q->sa = w.sa1 + a0;
+        q->sa2 = w.sl + a0;
+        q->rWr = w.rWr + a0;
+        q->rWr0 = w.rWr0 + a0;
+        q->sb = w.sb1 + b0;
+        q->sb2 = w.sf + b0;
+        q->rows = w.rows + b0;
+    };
+    // the tile order of the largest unit's shape, tuned on it (a unit's launch writes what the grouped one writes again)
+    TcMaps tc, pair;
+    TcArgs one = a;
+    one.Mr = largest.a_rows;
+    one.Nr = largest.b_rows;
+    rows_at(&one, largest.a_row0, largest.b_row0);
+    if ((rc = make(&tc, largest.a_row0, largest.a_rows, largest.b_row0, largest.b_rows, kBM))) return rc;
+    if ((rc = make(&pair, largest.a_row0, largest.a_rows, largest.b_row0, largest.b_rows, kBN / 2))) return rc;
+    TcChoice choice;
+    if ((rc = choose_product<2>(tc, pair, one, n2, flmm_ctx_sm_count(ctx), true, st, &choice))) return rc;
+    // a unit by itself may be too small to fill the CTA pairs; the units together go over them in either case
+    if (!choice.pair) choice = {true, 1};
+    if ((rc = make(&pair, 0, w.P * w.n_units, 0, w.M, kBN / 2))) return rc;
+    rows_at(&a, 0, 0);
+    a.units = units;
+    a.n_units = w.n_units;
+    a.total_tiles = total;
+    return launch_choice<2>(pair, pair, a, choice, n2, flmm_ctx_sm_count(ctx), st);
+}
+
+int flmm::split_units(const float* X, int64_t ldx, int64_t x_stride, int rows, int K, int n_units, void* hi, void* lo,
+                      int64_t ldo, int dst_rows, float* scale, cudaStream_t st) {
+    k_split_rows<float><<<dim3(ceil_div(static_cast<int64_t>(rows) * 32, 256), n_units), 256, 0, st>>>(
+        X, ldx, rows, K, static_cast<__half*>(hi), static_cast<__half*>(lo), ldo, scale, x_stride, dst_rows);
+    return check_launch("k_split_rows");
+}
+
+int flmm::prep_columns_units(const float* s32, int Neff, const float* UYt, int64_t ldu, int64_t uy_stride,
+                             const double* log_delta, int P, int n_units, const float* shat, double x0, double h, int R,
+                             void* A1h, void* A1l, int64_t lda, void* Lh, void* Ll, int64_t ldl, float* sa1, float* sl,
+                             float* rWr, float* rWr0, cudaStream_t st) {
+    if (P == 0) return FLMM_OK;
+    k_wald_prep_columns<<<dim3(ceil_div(P, kPrepCols), n_units), 32 * kPrepCols, 0, st>>>(
+        s32, Neff, UYt, ldu, log_delta, P, shat, x0, h, 1.0 / h, R, static_cast<__half*>(A1h), static_cast<__half*>(A1l), lda,
+        static_cast<__half*>(Lh), static_cast<__half*>(Ll), ldl, sa1, sl, rWr, rWr0, uy_stride);
+    return check_launch("k_wald_prep_columns");
 }

@@ -337,6 +337,17 @@ __global__ void k_fill_nullh2(const double* __restrict__ ld, int n_real, const i
     }
 }
 
+// the same over units: unit blockIdx.z's rows start[u] .. start[u + 1] and log deltas ld + u P
+__global__ void k_fill_nullh2_units(const double* __restrict__ ld, int P, int n_real, const int64_t* __restrict__ rows,
+                                    const int* __restrict__ start, double* __restrict__ out, int64_t ldo) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x, u = blockIdx.z;
+    const int m1 = start[u + 1];
+    int m = start[u] + blockIdx.y * kNullh2Rows;
+    if (p >= n_real || m >= m1) return;
+    const double h2 = 1.0 / (1.0 + exp(ld[static_cast<int64_t>(u) * P + p]));
+    for (const int end = min(m1, m + kNullh2Rows); m < end; ++m) out[rows[m] * ldo + p] = h2;
+}
+
 __global__ void k_axpy(int64_t n, double alpha, const double* __restrict__ x, double* __restrict__ y) {
     int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
     if (t < n) y[t] += alpha * x[t];
@@ -476,6 +487,15 @@ extern "C" int flmm_fill_nullh2(const double* log_delta, int n_real, const int64
                     static_cast<unsigned>(row_blocks < 65535 ? row_blocks : 65535));
     k_fill_nullh2<<<grid, 128, 0, as_stream(stream)>>>(log_delta, n_real, rows, Mc, nullh2, ldo);
     return check_launch("k_fill_nullh2");
+}
+
+int flmm::fill_nullh2_units(const double* log_delta, int P, int n_real, const int64_t* rows, const int* start, int n_units,
+                            int most, double* out, int64_t ldo, cudaStream_t st) {
+    FLMM_REQUIRE(log_delta && rows && out && ldo >= n_real, "flmm_fill_nullh2: bad arguments");
+    if (n_real <= 0 || most <= 0) return FLMM_OK;
+    const dim3 grid(ceil_div(n_real, 128), ceil_div(most, kNullh2Rows), n_units);
+    k_fill_nullh2_units<<<grid, 128, 0, st>>>(log_delta, P, n_real, rows, start, out, ldo);
+    return check_launch("k_fill_nullh2_units");
 }
 
 extern "C" int flmm_fill_f64(double* x, int64_t n, double value, void* stream) {

@@ -7,14 +7,18 @@
 //                            unit u + 1 on a second stream beside the variant side of unit u
 //
 // Each unit is ~20 launches of a few microseconds for ordinary studies, and issuing them from Python cost 10-20 us each:
-// 150 samples x 1,500 variants on 16 chromosomes took 10.2 ms in 505 launches, 4.35 here.  What depends on the spectra
+// 150 samples x 1,500 variants on 16 chromosomes took 10.2 ms in 505 launches, 4.35 unit by unit and 3.00 grouped.  What depends on the spectra
 // alone (mean, FP32 copies, sWs node weights and their split) and the projections run for all units in one launch each.
-// The launches and their arithmetic are otherwise those of the C entry points called one by one.
+// Where every unit's column operands fit kGroupBytes together, so does the rest (run_grouped): the launches then take all
+// units' rows, the split products with the units' tiles one after another.  The arithmetic is in every form that of the
+// C entry points called one by one.
 #include <cuda_fp16.h>
+#include <limits.h>
 #include <math.h>
 
 #include <algorithm>
 #include <cmath>
+#include <vector>
 
 #include "flmm_common.cuh"
 
@@ -70,6 +74,31 @@ __global__ void k_sum_grams(const float* __restrict__ x, int64_t len, int n, dou
     double s = 0.0;
     for (int i = 0; i < n; ++i) s += static_cast<double>(x[i * len + t]);
     y[t] = s;
+}
+
+constexpr int kPut = 256;
+template <typename T>
+struct Put {
+    T x[kPut];
+};
+template <typename T>
+__global__ void k_put(Put<T> p, int n, T* __restrict__ to) {
+    if (static_cast<int>(threadIdx.x) < n) to[threadIdx.x] = p.x[threadIdx.x];
+}
+
+// A host table into device memory, as launch parameters: it needs no buffer that outlives the call, also under capture.
+template <typename T>
+int put(const T* from, int n, T* to, cudaStream_t st) {
+    static_assert(sizeof(Put<T>) <= 24000, "launch parameters");
+    for (int i = 0; i < n; i += kPut) {
+        Put<T> p = {};
+        const int k = std::min(kPut, n - i);
+        std::copy(from + i, from + i + k, p.x);
+        k_put<T><<<1, kPut, 0, st>>>(p, k, to + i);
+        int rc = check_launch("k_put");
+        if (rc) return rc;
+    }
+    return FLMM_OK;
 }
 
 struct UnitGram {
@@ -155,15 +184,10 @@ extern "C" int flmm_loco_kinships_f32(flmm_context* ctx, const double* Zt, int N
     }
     k_sum_grams<<<ceil_div(nn, 256), 256, 0, st>>>(grams, nn, n_blocks, Gtot);
     if ((rc = check_launch("k_sum_grams"))) return rc;
-    UnitGram host[256];
-    for (int u0 = 0; u0 < n_units; u0 += 256) {  // (pageable copies of a few hundred bytes are staged at once)
-        const int n = std::min(256, n_units - u0);
-        for (int u = 0; u < n; ++u) {
-            const int b = unit_block[u0 + u];
-            host[u] = UnitGram{b, static_cast<double>(M - (b >= 0 ? counts[b] : 0))};
-        }
-        FLMM_CUDA(cudaMemcpyAsync(units + u0, host, sizeof(UnitGram) * n, cudaMemcpyHostToDevice, st));
-    }
+    std::vector<UnitGram> host(n_units);
+    for (int u = 0; u < n_units; ++u)
+        host[u] = UnitGram{unit_block[u], static_cast<double>(M - (unit_block[u] >= 0 ? counts[unit_block[u]] : 0))};
+    if ((rc = put(host.data(), n_units, units, st))) return rc;
     k_unit_kinships<<<dim3(ceil_div(nn, 256), n_units), 256, 0, st>>>(Gtot, grams, nn, units, Kp);
     if ((rc = check_launch("k_unit_kinships"))) return rc;
     return project_kinships(Kp, Qx, N, D, n_units, proj, st);
@@ -173,7 +197,13 @@ extern "C" int flmm_loco_kinships_f32(flmm_context* ctx, const double* Zt, int N
 
 namespace {
 
+// Grouped launches when every unit's column operands (eigenvectors, rotated phenotypes and their weighted rows) take at
+// most this much: 150 x 1,500 on 16 chromosomes 4.35 -> 3.00 ms, 563 x 20,011 on 22 15.1 -> 12.5, 1,600 x 6,000 on 8
+// 169 -> 162.  With more columns a unit's launches fill the device for many waves, and the second stream hides the rest.
+constexpr size_t kGroupBytes = size_t{1} << 30;
+
 struct UnitBufs {
+    bool grouped;
     double* s;       // (units, Neff)
     float *s32, *shat;
     double* W;       // (units, R, Neff) sWs node weights
@@ -185,6 +215,9 @@ struct UnitBufs {
         void* fit;
     } slot[2];
     size_t fit_bytes;
+    // grouped: every unit's tiles of the three products and first variant row; rotated phenotypes are (P, units ldk)
+    UnitTiles *tiles_us, *tiles_f, *tiles_w;
+    int* start;
     float* US;
     __half *A1h, *A1l, *Lh, *Ll, *B1h, *B1l, *B2h, *B2l;
     float *sa1, *sl, *rWr, *rWr0, *sb1, *sb2, *F;
@@ -195,7 +228,7 @@ struct UnitBufs {
     double x0;
 };
 
-int carve_units(Arena& a, const flmm_units* q, UnitBufs* b) {
+int carve_units(Arena& a, const flmm_units* q, bool group, UnitBufs* b) {
     const int Neff = q->N - q->D;
     const size_t P = q->P, U = q->n_units;
     int mc = 0;
@@ -210,25 +243,46 @@ int carve_units(Arena& a, const flmm_units* q, UnitBufs* b) {
     b->Ws = take_split(a, static_cast<int64_t>(U) * b->R, b->ldk);
     int rc = flmm_fit_delta_fast_workspace_bytes(Neff, q->opts.n_grid, &b->fit_bytes);
     if (rc) return rc;
-    for (auto& s : b->slot) {
-        s.Us = take_split(a, Neff, pad8(q->N));
-        s.UY = a.of<float>(P * b->ldk);
-        s.idx = a.of<int32_t>(P);
-        s.fit = a.take(b->fit_bytes);
+    // one unit's row after another's, and few enough columns
+    int64_t total = 0;
+    bool dense = group && U > 1 && U <= 32767;  // (grid.y)
+    for (int u = 0; u < q->n_units; ++u) {
+        dense = dense && q->unit_start[u] == total;
+        total += q->unit_count[u];
     }
-    const size_t M = mc;
+    const size_t columns = U * b->ldk * 4 * (pad8(q->N) + 2 * P);
+    b->grouped = dense && total < (int64_t{1} << 30) && U * std::max<size_t>(P, b->ldk) < (size_t{1} << 30) &&
+                 columns <= kGroupBytes;
+    if (b->grouped) {
+        UnitBufs::Slot& s = b->slot[0];
+        s.Us = take_split(a, static_cast<int64_t>(U) * b->ldk, pad8(q->N));
+        s.UY = a.of<float>(U * P * b->ldk);
+        s.idx = a.of<int32_t>(U * P);
+        s.fit = a.take(fit_units_bytes(Neff, q->opts.n_grid, q->n_units));
+        for (UnitTiles** t : {&b->tiles_us, &b->tiles_f, &b->tiles_w}) *t = a.of<UnitTiles>(U);
+        b->start = a.of<int>(U + 1);
+    } else {
+        for (auto& s : b->slot) {
+            s.Us = take_split(a, Neff, pad8(q->N));
+            s.UY = a.of<float>(P * b->ldk);
+            s.idx = a.of<int32_t>(P);
+            s.fit = a.take(b->fit_bytes);
+        }
+    }
+    const size_t M = b->grouped ? total : mc;
+    const size_t PA = b->grouped ? U * P : P;
     b->US = a.of<float>(M * b->ldk);
-    b->A1h = a.of<__half>(P * b->ldk);
-    b->A1l = a.of<__half>(P * b->ldk);
-    b->Lh = a.of<__half>(P * b->ldr);
-    b->Ll = a.of<__half>(P * b->ldr);
-    for (float** x : {&b->sa1, &b->sl, &b->rWr, &b->rWr0}) *x = a.of<float>(P);
+    b->A1h = a.of<__half>(PA * b->ldk);
+    b->A1l = a.of<__half>(PA * b->ldk);
+    b->Lh = a.of<__half>(PA * b->ldr);
+    b->Ll = a.of<__half>(PA * b->ldr);
+    for (float** x : {&b->sa1, &b->sl, &b->rWr, &b->rWr0}) *x = a.of<float>(PA);
     for (__half** x : {&b->B1h, &b->B1l, &b->B2h, &b->B2l}) *x = a.of<__half>(M * b->ldk);
     for (float** x : {&b->sb1, &b->sb2}) *x = a.of<float>(M);
     b->F = a.of<float>(M * b->ldr);
-    b->Fs = take_split(a, mc, pad8(b->R));
-    const int64_t tests = static_cast<int64_t>(mc) * q->n_real;
-    b->cap = q->opts.f_refine > 0.0 ? static_cast<int>(std::min<int64_t>(tests, q->refine_cap)) : 0;
+    b->Fs = take_split(a, M, pad8(b->R));
+    const int64_t tests = static_cast<int64_t>(M) * q->n_real;
+    b->cap = q->opts.f_refine > 0.0 ? static_cast<int>(std::min<int64_t>({tests, q->refine_cap * (b->grouped ? int64_t{q->n_units} : 1), INT_MAX / 2})) : 0;
     b->flags = a.of<int32_t>(2 * static_cast<size_t>(b->cap));
     b->flag_count = a.of<int32_t>(1);
     return FLMM_OK;
@@ -322,16 +376,116 @@ int unit_variants(flmm_context* ctx, const flmm_units* q, const UnitBufs& b, int
     return flmm_fill_nullh2(ld, q->n_real, rows, Mc, q->nullh2, q->ldo, st);
 }
 
+// Every unit at once: the rotated phenotypes and the fits on `side`, beside the rotated variants and their operands.
+int run_grouped(flmm_context* ctx, const flmm_units* q, const UnitBufs& b, cudaStream_t main, cudaStream_t side, Events& ev) {
+    const int N = q->N, Neff = N - q->D, P = q->P, U = q->n_units, R = b.R;
+    const UnitBufs::Slot& s = b.slot[0];
+    const int ldk = static_cast<int>(b.ldk);
+    const bool pipe = side != main;
+    auto after = [&](cudaEvent_t e, cudaStream_t first, cudaStream_t then) -> int {
+        if (!pipe) return FLMM_OK;
+        FLMM_CUDA(cudaEventRecord(e, first));
+        FLMM_CUDA(cudaStreamWaitEvent(then, e, 0));
+        return FLMM_OK;
+    };
+    std::vector<UnitTiles> us(U), f(U), w(U);
+    std::vector<int> start(U + 1);
+    int n_us = 0, n_f = 0, n_w = 0, big = 0, most = 0;
+    auto tiles = [](int a, int rows_b) {
+        return ((a + kUnitTileA - 1) / kUnitTileA) * ((rows_b + kUnitTileB - 1) / kUnitTileB);
+    };
+    for (int u = 0; u < U; ++u) {
+        const int m0 = static_cast<int>(q->unit_start[u]), m = q->unit_count[u];
+        start[u] = m0;
+        start[u + 1] = m0 + m;
+        us[u] = {n_us, m0, m, u * ldk, Neff};
+        f[u] = {n_f, m0, m, u * R, R};
+        w[u] = {n_w, u * P, P, m0, m};
+        n_us += tiles(m, Neff);
+        n_f += tiles(m, R);
+        n_w += tiles(P, m);
+        if (m > most) {
+            most = m;
+            big = u;
+        }
+    }
+    const int M = start[U];
+    int rc;
+    if ((rc = put(us.data(), U, b.tiles_us, main)) || (rc = put(f.data(), U, b.tiles_f, main)) ||
+        (rc = put(w.data(), U, b.tiles_w, main)) || (rc = put(start.data(), U + 1, b.start, main)))
+        return rc;
+    // every unit's eigenvector rows from a multiple of ldk on, zeros between
+    const size_t pad = ldk - Neff, row = sizeof(__half) * s.Us.ld;
+    if (pad) {
+        for (__half* h : {s.Us.hi, s.Us.lo})
+            FLMM_CUDA(cudaMemset2DAsync(h + Neff * s.Us.ld, ldk * row, 0, pad * row, U, main));
+        FLMM_CUDA(cudaMemset2DAsync(s.Us.scale + Neff, ldk * sizeof(float), 0, pad * sizeof(float), U, main));
+    }
+    if ((rc = split_units(q->U + static_cast<int64_t>(q->D) * N, N, static_cast<int64_t>(N) * N, Neff, N, U, s.Us.hi, s.Us.lo,
+                          s.Us.ld, ldk, s.Us.scale, main)))
+        return rc;
+    if ((rc = after(ev.e[0], main, side))) return rc;
+    if (P > 0) {
+        const int64_t ldu = static_cast<int64_t>(U) * ldk;
+        if ((rc = flmm_gemm_split_f16(ctx, q->Yh, q->Yl, q->Yscale, q->ldY, P, s.Us.hi, s.Us.lo, s.Us.scale, s.Us.ld,
+                                      U * ldk, N, s.UY, ldu, 0, side)))
+            return rc;
+        if ((rc = fit_delta_units(b.s, Neff, s.UY, ldu, ldk, P, U, q->opts.n_grid, q->opts.log_delta_min,
+                                  q->opts.log_delta_max, q->opts.refine, q->log_delta, s.idx, s.fit, side)))
+            return rc;
+        if ((rc = prep_columns_units(b.s32, Neff, s.UY, ldu, ldk, q->log_delta, P, U, b.shat, b.x0, kInterpH, R, b.A1h, b.A1l,
+                                     b.ldk, b.Lh, b.Ll, b.ldr, b.sa1, b.sl, b.rWr, b.rWr0, side)))
+            return rc;
+    }
+    if (M > 0) {
+        if ((rc = gemm_units(ctx, q->Zh, q->Zl, q->Zscale, q->ldZ, M, s.Us.hi, s.Us.lo, s.Us.scale, s.Us.ld, U * ldk, N, b.US,
+                             b.ldk, b.tiles_us, U, n_us, main)))
+            return rc;
+        if ((rc = flmm_wald_split_prep_variants(b.US, b.ldk, M, Neff, b.B1h, b.B1l, b.B2h, b.B2l, b.ldk, b.sb1, b.sb2, main)))
+            return rc;
+        // node values of sWs~: F (M, R) = (US o US) W~^T, every variant with its unit's weights
+        if ((rc = gemm_units(ctx, b.B2h, b.B2l, b.sb2, b.ldk, M, b.Ws.hi, b.Ws.lo, b.Ws.scale, b.ldk, U * R, Neff, b.F, b.ldr,
+                             b.tiles_f, U, n_f, main)))
+            return rc;
+        if ((rc = flmm_split_rows_f16(b.F, 0, b.ldr, M, R, b.Fs.hi, b.Fs.lo, b.Fs.ld, b.Fs.scale, main))) return rc;
+    }
+    if ((rc = after(ev.e[1], side, main)) || M == 0 || P == 0) return rc;
+    const bool refine = q->opts.f_refine > 0.0 && q->n_real > 0;
+    WaldUnits x;
+    x.A1h = b.A1h, x.A1l = b.A1l, x.lda = b.ldk, x.sa1 = b.sa1;
+    x.Lh = b.Lh, x.Ll = b.Ll, x.ldl = b.ldr, x.sl = b.sl, x.rWr = b.rWr, x.rWr0 = b.rWr0;
+    x.P = P, x.n_real = q->n_real, x.n_units = U;
+    x.B1h = b.B1h, x.B1l = b.B1l, x.ldb = b.ldk, x.sb1 = b.sb1;
+    x.Fh = b.Fs.hi, x.Fl = b.Fs.lo, x.ldf = b.Fs.ld, x.sf = b.Fs.scale;
+    x.M = M, x.Neff = Neff, x.R = R, x.rows = q->rows;
+    x.f = q->f, x.beta = q->beta, x.se = q->se, x.sfve = q->sfve, x.ldo = q->ldo, x.max_F = q->max_F;
+    x.f_refine = refine ? static_cast<float>(q->opts.f_refine) : INFINITY;
+    x.flag_count = refine ? b.flag_count : nullptr;
+    x.flags = refine ? b.flags : nullptr;
+    x.flag_cap = refine ? b.cap : 0;
+    if ((rc = wald_units(ctx, x, b.tiles_w, n_w, w[big], main))) return rc;
+    if (refine && (rc = wald_refine_units(ctx, b.flags, b.flag_count, b.cap, x.f_refine, b.US, b.ldk, s.UY,
+                                          static_cast<int64_t>(U) * ldk, ldk, b.s32, q->log_delta, P, Neff, M, q->n_real,
+                                          b.start, U, q->rows, q->f, q->beta, q->se, q->sfve, q->ldo, q->max_F, main)))
+        return rc;
+    if (q->n_real == 0) return FLMM_OK;
+    return fill_nullh2_units(q->log_delta, P, q->n_real, q->rows, b.start, U, most, q->nullh2, q->ldo, main);
+}
+
 }  // namespace
 
 extern "C" int flmm_scan_units_workspace_bytes(const flmm_units* q, size_t* bytes) {
     FLMM_REQUIRE(bytes, "flmm_scan_units_workspace_bytes: bytes is NULL");
     int rc = check_units(q);
     if (rc) return rc;
-    Arena a(nullptr);
-    UnitBufs b;
-    if ((rc = carve_units(a, q, &b))) return rc;
-    *bytes = a.off + 2048;
+    // enough for either form, whichever is configured when the scan runs
+    *bytes = 0;
+    for (const bool group : {false, true}) {
+        Arena a(nullptr);
+        UnitBufs b;
+        if ((rc = carve_units(a, q, group, &b))) return rc;
+        *bytes = std::max(*bytes, a.off + 2048);
+    }
     return FLMM_OK;
 }
 
@@ -348,7 +502,7 @@ extern "C" int flmm_scan_units(flmm_context* ctx, const flmm_units* q, void* wor
     if (work_bytes < need) return fail(FLMM_ERR_WORKSPACE, "flmm_scan_units: need %zu bytes, got %zu", need, work_bytes);
     Arena a(work);
     UnitBufs b;
-    if ((rc = carve_units(a, q, &b))) return rc;
+    if ((rc = carve_units(a, q, units_pair_ok(), &b))) return rc;
     const int Neff = q->N - q->D, U = q->n_units;
     cudaStream_t main = as_stream(stream), side = as_stream(side_stream);
     Events ev;
@@ -359,6 +513,11 @@ extern "C" int flmm_scan_units(flmm_context* ctx, const flmm_units* q, void* wor
     if ((rc = interp_units(b.s, Neff, U, b.shat, b.x0, kInterpH, b.R, b.W, main))) return rc;
     if ((rc = flmm_split_rows_f16(b.W, 1, Neff, U * b.R, Neff, b.Ws.hi, b.Ws.lo, b.ldk, b.Ws.scale, main))) return rc;
     const bool pipe = side != main;
+    if (b.grouped) {
+        rc = run_grouped(ctx, q, b, main, side, ev);
+        if (rc && pipe && cudaEventRecord(ev.e[0], side) == cudaSuccess) cudaStreamWaitEvent(main, ev.e[0], 0);
+        return rc;
+    }
     auto record = [&](cudaEvent_t e, cudaStream_t s) { return !pipe || cudaEventRecord(e, s) == cudaSuccess; };
     auto wait = [&](cudaStream_t s, cudaEvent_t e) { return !pipe || cudaStreamWaitEvent(s, e, 0) == cudaSuccess; };
     // slot 0 and 1 alternate; e[1 + slot]: its column side is done, e[3 + slot]: its variant side is

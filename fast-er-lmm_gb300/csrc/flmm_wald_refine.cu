@@ -46,6 +46,11 @@ struct RefineArgs {
     int64_t ldo;
     double* max_F;
     float f_refine;
+    // a scan's units in one launch: unit u's variants are rows start[u] .. start[u + 1], its rotated columns start at
+    // UY + u uy_stride, its spectrum at s32 + u Neff and its log deltas at log_delta + u P (n_units = 1: one unit)
+    const int* start;
+    int n_units, P;
+    int64_t uy_stride;
 };
 
 __device__ __forceinline__ void acc2(float& s, float& c, float x) {
@@ -63,14 +68,23 @@ __device__ __forceinline__ double warp_sum_d(double v) {
 
 // Recompute test (m, p) of the chromosome; called by all 32 lanes of a warp with the same (m, p).
 __device__ void refine_one(const RefineArgs& a, int m, int p) {
+    int unit = 0;
+    if (a.n_units > 1) {  // the last unit that starts at or before m
+        int hi = a.n_units;
+        while (hi - unit > 1) {
+            const int mid = (unit + hi) >> 1;
+            if (a.start[mid] <= m) unit = mid; else hi = mid;
+        }
+    }
     const float* u = a.US + static_cast<int64_t>(m) * a.ldus;
-    const float* r = a.UY + static_cast<int64_t>(p) * a.lduy;
+    const float* r = a.UY + unit * a.uy_stride + static_cast<int64_t>(p) * a.lduy;
+    const float* s32 = a.s32 + static_cast<int64_t>(unit) * a.Neff;
     const int64_t o = a.rows[m] * a.ldo + p;
     const float b = static_cast<float>(a.beta[o]);
-    const float dl = static_cast<float>(exp(a.log_delta[p]));
+    const float dl = static_cast<float>(exp(a.log_delta[static_cast<int64_t>(unit) * a.P + p]));
     float s0 = 0.f, c0 = 0.f, s1 = 0.f, c1 = 0.f, s2 = 0.f, c2 = 0.f, s3 = 0.f, c3 = 0.f;
     for (int n = threadIdx.x & 31; n < a.Neff; n += 32) {
-        const float w = __frcp_rn(a.s32[n] + dl);
+        const float w = __frcp_rn(s32[n] + dl);
         const float un = u[n];
         const float rn = r[n];
         const float e = fmaf(-b, un, rn);
@@ -136,6 +150,26 @@ __global__ void __launch_bounds__(256) k_wald_refine_scan(const int* count, int 
 
 int flmm_ctx_sm_count(flmm_context* ctx);
 
+namespace {
+
+int launch_refine(flmm_context* ctx, const int32_t* flags, const int32_t* flag_count, int flag_cap, const RefineArgs& a,
+                  cudaStream_t st) {
+    // A small grid: the launch usually finds few or no strong tests, and it must get onto the SMs quickly while the
+    // next chromosome's delta fit runs beside it on another stream (a grid of several CTAs per SM waited there for
+    // whole waves of that fit and held the Wald stream back ~1 ms per chromosome).
+    const int sms = flmm_ctx_sm_count(ctx);
+    const unsigned grid = static_cast<unsigned>(sms < 32 ? sms : 32);
+    if (flag_cap > 0) {
+        k_wald_refine_list<<<grid, 256, 0, st>>>(reinterpret_cast<const int2*>(flags), flag_count, flag_cap, a);
+        int rc = check_launch("k_wald_refine_list");
+        if (rc) return rc;
+    }
+    k_wald_refine_scan<<<grid, 256, 0, st>>>(flag_count, flag_cap, a);
+    return check_launch("k_wald_refine_scan");
+}
+
+}  // namespace
+
 extern "C" int flmm_wald_refine_f32(flmm_context* ctx, const int32_t* flags, const int32_t* flag_count, int flag_cap,
                                     float f_refine, const float* USt, int64_t ldus, const float* UYt, int64_t lduy,
                                     const float* s32, const double* log_delta, int Neff, int Mc, int n_real,
@@ -165,17 +199,20 @@ extern "C" int flmm_wald_refine_f32(flmm_context* ctx, const int32_t* flags, con
     a.ldo = ldo;
     a.max_F = max_F;
     a.f_refine = f_refine;
-    cudaStream_t st = as_stream(stream);
-    // A small grid: the launch usually finds few or no strong tests, and it must get onto the SMs quickly while the
-    // next chromosome's delta fit runs beside it on another stream (a grid of several CTAs per SM waited there for
-    // whole waves of that fit and held the Wald stream back ~1 ms per chromosome).
-    const int sms = flmm_ctx_sm_count(ctx);
-    const unsigned grid = static_cast<unsigned>(sms < 32 ? sms : 32);
-    if (flag_cap > 0) {
-        k_wald_refine_list<<<grid, 256, 0, st>>>(reinterpret_cast<const int2*>(flags), flag_count, flag_cap, a);
-        int rc = check_launch("k_wald_refine_list");
-        if (rc) return rc;
-    }
-    k_wald_refine_scan<<<grid, 256, 0, st>>>(flag_count, flag_cap, a);
-    return check_launch("k_wald_refine_scan");
+    a.start = nullptr;
+    a.n_units = 1;
+    a.P = 0;
+    a.uy_stride = 0;
+    return launch_refine(ctx, flags, flag_count, flag_cap, a, as_stream(stream));
+}
+
+int flmm::wald_refine_units(flmm_context* ctx, const int32_t* flags, const int32_t* flag_count, int flag_cap,
+                            float f_refine, const float* US, int64_t ldus, const float* UYt, int64_t ldu,
+                            int64_t uy_stride, const float* s32, const double* log_delta, int P, int Neff, int M,
+                            int n_real, const int* start, int n_units, const int64_t* rows, double* f, double* beta,
+                            double* se, double* sfve, int64_t ldo, double* max_F, cudaStream_t st) {
+    if (M == 0 || n_real == 0) return FLMM_OK;
+    const RefineArgs a{US, ldus, UYt, ldu, s32, log_delta, Neff, M, n_real, rows, f, beta, se, sfve, ldo, max_F, f_refine,
+                       start, n_units, P, uy_stride};
+    return launch_refine(ctx, flags, flag_count, flag_cap, a, st);
 }

@@ -55,6 +55,25 @@ def test_native_loop_gives_the_python_loops_bits(monkeypatch, case):
     assert all(torch.equal(a.log_delta[c], b.log_delta[c]) for c in a.log_delta)
 
 
+@pytest.mark.parametrize("choice", [(2, 0, 1), (2, 1, 3)])
+@pytest.mark.parametrize("shape,sizes", [((40, 30, 1, 5, 2), [1, 28, 1]), ((300, 700, 3, 270, 130), [129, 256, 0, 315]),
+                                         ((129, 301, 1, 257, 257), [128, 127, 46])])
+def test_units_together_and_one_by_one_give_the_same_bits(monkeypatch, shape, sizes, choice):
+    """Every unit in one launch (CTA pairs) and unit by unit (single-CTA products forced), at the edges of a unit's tiles."""
+    from fasterlmm_gb300 import _lib, build
+    build()
+    kw = dict(shape=shape, chrom=np.repeat(np.arange(len(sizes)), sizes), patch=dict(REFINE_F=1.0))
+    a, _ = _scan(monkeypatch, False, **{**kw})
+    try:
+        _lib.tc_config(*choice)
+        b, _ = _scan(monkeypatch, False, **{**kw})
+        c, _ = _scan(monkeypatch, True, **{**kw})
+    finally:
+        _lib.tc_config(1)
+    for k in ("f", "beta", "se", "sfve", "nullh2", "max_F"):
+        assert torch.equal(getattr(a, k), getattr(b, k)) and torch.equal(getattr(a, k), getattr(c, k)), k
+
+
 def test_a_chromosome_that_holds_every_variant_is_refused(monkeypatch):
     from fasterlmm_gb300 import _lib
     with pytest.raises(_lib.FlmmError):
