@@ -142,6 +142,32 @@ __device__ __forceinline__ float warp_sum(float v) {
     return v;
 }
 
+// The golden-section bracket of the reference (fasterlmm/core.py:545-558), in its operations; [grid[i-1], grid[i+1]] first.
+struct Bracket {
+    double a, b, inv_phi, inv_phi2;
+
+    __device__ Bracket(const double* grid, int G, int i)
+        : a(grid[max(i - 1, 0)]), b(grid[min(i + 1, G - 1)]), inv_phi(2.0 / (1.0 + sqrt(5.0))) {
+        inv_phi2 = __dmul_rn(inv_phi, inv_phi);
+    }
+    __device__ double c() const { return __dadd_rn(a, __dmul_rn(inv_phi2, __dadd_rn(b, -a))); }
+    __device__ double d() const { return __dadd_rn(a, __dmul_rn(inv_phi, __dadd_rn(b, -a))); }
+    __device__ void narrow(bool left) {
+        const double nc = c(), nd = d();
+        b = left ? nd : b;
+        a = left ? a : nc;
+    }
+    // The step after losses (c, d).  Of the next two points one is an old one but for its rounding: whether point e is the
+    // old one to the bit, and its loss.
+    __device__ bool narrow_kept(const double* loss, int e, double* kept) {
+        const double oc = c(), od = d(), lc = loss[0], ld = loss[1];
+        const bool left = lc < ld;
+        narrow(left);
+        *kept = left ? lc : ld;
+        return left ? e == 1 && d() == oc : e == 0 && c() == od;
+    }
+};
+
 // Neumaier-compensated running sum: comp collects the rounding error of every addition, so sum + comp is the sum of
 // the added terms without the accumulated FP32 rounding
 __device__ __forceinline__ void neumaier(float& sum, float& comp, float x) {

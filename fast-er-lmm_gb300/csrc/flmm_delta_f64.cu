@@ -146,12 +146,119 @@ __global__ void k_grid_pick(const double* __restrict__ grid, const int32_t* __re
     if (p < P) log_delta[p] = grid[idx[p]];
 }
 
-// Golden-section search, one block per column (fasterlmm/core.py:545-558, :577-595).  The terms of a step's two
-// evaluations, a division and a logarithm per eigenvalue, are formed by all threads into shared memory, kTermChunk
-// eigenvalues at a time; one warp per sum then adds them, lane l the terms l, l + 32, ... in order and the lanes by a
-// butterfly.  The search stops at the rounding noise of the loss, so this order is part of the result.  Bound by the FP64
-// pipe (~60 operations a term); a warp per column had few columns wait for 2 Neff / 32 terms one after another on few
-// SMs: 176 columns x 450 eigenvalues 5.6 -> 1.8 ms, 220 x 880 8.7 -> 2.8 ms, 2,100 x 596 12.7 -> 11.0 ms.
+// Golden-section search (fasterlmm/core.py:545-558, :577-595), 50 steps that each compare two losses.  Its value is the
+// list of those comparisons: the last third of them compare rounding noise, so every loss that decides one has to keep its
+// bits (k_golden), but the first half compare losses that are far apart, and those need only be good enough to be sure of
+// the sign (k_golden_certain).  The list is handed over in the output word: bit k is step k's answer, the top byte how many
+// steps are decided.
+constexpr int kGoldenSteps = 50;
+
+__device__ __forceinline__ double warp_max(double v) {
+    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+
+// The steps whose answer is certain, one warp per column.  The sums come from groups of up to 16 eigenvalues as one
+// fraction and one logarithm, sum u^2 / x = num / den and sum log x = log den, ~7 operations of the FP64 pipe an eigenvalue
+// for the ~60 of a division and a logarithm each, and the point that a step shares with the one before is not evaluated
+// again.  A step is certain when the two losses differ by more than twice what rounding can make of them here and in
+// k_golden together.  With u = 2^-53 and n eigenvalues, to first order and both sides: sum u^2 / x is a sum of positive
+// terms, relative error below (n / 30 + 58) u; sum log x is off by at most (n / 30 + 20) u sum |log x| + n u; a shared
+// point whose position differs in its last bits moves the loss by at most (neff + n + |n_logd|) times that.  The first step
+// that is not certain ends the list, as does anything out of the range of these bounds.
+// 2,100 columns x 596 eigenvalues: 22 of the 50 steps on average, the whole fit 10.5 -> 7.0 ms.
+constexpr int kCertainWarps = 4, kGroup = 16;
+
+__global__ void __launch_bounds__(32 * kCertainWarps)
+k_golden_certain(const double* __restrict__ s, int Neff, const double* __restrict__ UYt, int64_t ldu, int P,
+                 const double* __restrict__ grid, int G, const int32_t* __restrict__ idx, OffRank off,
+                 double* __restrict__ list) {
+    const int lane = threadIdx.x & 31;
+    const int64_t p = static_cast<int64_t>(blockIdx.x) * kCertainWarps + (threadIdx.x >> 5);
+    if (p >= P) return;
+    const double* u = UYt + p * ldu;
+    const double yy = off.yy ? off.yy[p] : 0.0;
+    Bracket br(grid, G, idx[p]);
+    double smin = INFINITY, smax = -INFINITY;
+    for (int n = lane; n < Neff; n += 32) {
+        smin = fmin(smin, s[n]);
+        smax = fmax(smax, s[n]);
+    }
+    const double xlo = -warp_max(-smin) + exp(br.a), xhi = warp_max(smax) + exp(br.b);
+    const double edge = fmax(fmax(fabs(br.a), fabs(br.b)), 1.0);
+    const double rnd = 0x1p-53, n = Neff, nd = fabs(off.n_logd);
+    // what does not depend on the loss: the logarithms' share, and that of the extra log(delta)
+    const double labs = n * fmax(fabs(log(xlo)), fabs(log(xhi)));
+    const double fixed = labs * (n / 30.0 + 26.0) + n + 12.0 * nd * edge;
+    bool certain = xlo > 0x1p-50 && xhi < 0x1p50 && yy >= 0.0;
+
+    double bound = 0.0;  // of the loss of the latest call
+    auto loss_at = [&](double x) {
+        const double delta = exp(x);
+        double q = 0.0, l = 0.0;
+        for (int n0 = 0; n0 < Neff; n0 += 32 * kGroup) {
+            double num = 0.0, den = 1.0;
+            // pairs of eigenvalues, joined one after another
+#pragma unroll
+            for (int j = 0; j < kGroup; j += 2) {
+                if (n0 + 32 * j >= Neff) break;
+                const int i0 = n0 + 32 * j + lane, i1 = i0 + 32;
+                double x0 = 1.0, x1 = 1.0, u0 = 0.0, u1 = 0.0;
+                if (i0 < Neff) {
+                    x0 = s[i0] + delta;
+                    u0 = u[i0];
+                }
+                if (i1 < Neff) {
+                    x1 = s[i1] + delta;
+                    u1 = u[i1];
+                }
+                const double pn = fma(u0 * u0, x1, u1 * u1 * x0), pd = x0 * x1;
+                num = fma(num, pd, pn * den);
+                den *= pd;
+            }
+            q += num / den;
+            l += log(den);
+        }
+        q = warp_sum(q);
+        l = warp_sum(l);
+        if (off.yy) q += yy / delta;
+        certain = certain && q > 0x1p-200 && q < 0x1p300;
+        const double ls = log(fmax(q, kPosFloor) / off.neff);
+        bound = rnd * (off.neff * (n / 30.0 + 90.0 + 10.0 * fabs(ls)) + fixed);
+        return off.neff * (kLog2Pi + ls + 1.0) + l + off.n_logd * x;
+    };
+
+    unsigned long long bits = 0;
+    int it = 0;
+    double xc = br.c(), xd = br.d();
+    double fc = loss_at(xc), bc = bound, fd = loss_at(xd), bd = bound;
+    while (certain && it < kGoldenSteps) {
+        const double slope = off.neff + n + nd;
+        const double tol = 2.0 * (bc + bd + slope * (fabs(xc - br.c()) + fabs(xd - br.d()) + 16.0 * rnd));
+        const bool left = fd - fc > tol;
+        if (!left && !(fc - fd > tol)) break;
+        if (left) bits |= 1ull << it;
+        ++it;
+        br.narrow(left);
+        if (it == kGoldenSteps) break;
+        if (left) {
+            xd = xc, fd = fc, bd = bc;
+            xc = br.c(), fc = loss_at(xc), bc = bound;
+        } else {
+            xc = xd, fc = fd, bc = bd;
+            xd = br.d(), fd = loss_at(xd), bd = bound;
+        }
+    }
+    if (lane == 0) list[p] = __longlong_as_double(static_cast<long long>(bits | static_cast<unsigned long long>(it) << 56));
+}
+
+// The other steps, one block per column.  The terms of a step's two evaluations, a division and a logarithm per eigenvalue,
+// are formed by all threads into shared memory, kTermChunk eigenvalues at a time; one warp per sum then adds them, lane l
+// the terms l, l + 32, ... in order and the lanes by a butterfly.  A point that is, to the bit, one of the step before keeps
+// its loss (one step in five has one).  The search stops at the rounding noise of the loss, so
+// this order is part of the result.  Bound by the FP64 pipe (~60 operations a term); a warp per column had few columns wait
+// for 2 Neff / 32 terms one after another on few SMs: all steps of 176 columns x 450 eigenvalues 5.6 -> 1.8 ms, 220 x 880
+// 8.7 -> 2.8 ms, 2,100 x 596 12.7 -> 11.0 ms.
 constexpr int kBlockThreads = 256, kTermChunk = 1024;
 
 __global__ void __launch_bounds__(kBlockThreads)
@@ -160,35 +267,37 @@ k_golden(const double* __restrict__ s, int Neff, const double* __restrict__ UYt,
          double* __restrict__ log_delta) {
     __shared__ double term[2][2][kTermChunk];  // [evaluation][w u u, log]
     __shared__ double delta_s[2], sum_s[2][2], loss_s[2];
+    __shared__ int kept_s[2];
     const int64_t p = blockIdx.x;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const double* u = UYt + p * ldu;
     const double yy = off.yy ? off.yy[p] : 0.0;
-    const int i = idx[p];
+    const unsigned long long list = static_cast<unsigned long long>(__double_as_longlong(log_delta[p]));
+    const int done = static_cast<int>(list >> 56);
+    __syncthreads();  // every thread has read the list; thread 0 overwrites it
     // threads 0 and 32 carry the search, one evaluation each
     const bool lead = tid == 0 || tid == 32;
     const int my_e = tid >> 5;
-    double a = grid[max(i - 1, 0)], b = grid[min(i + 1, G - 1)];
-    const double inv_phi = 2.0 / (1.0 + sqrt(5.0));
-    const double inv_phi2 = mul_rn(inv_phi, inv_phi);
-    auto narrow = [&] {
-        const double c = add_rn(a, mul_rn(inv_phi2, add_rn(b, -a))), d = add_rn(a, mul_rn(inv_phi, add_rn(b, -a)));
-        const bool cond = loss_s[0] < loss_s[1];
-        b = cond ? d : b;
-        a = cond ? a : c;
-    };
-    for (int it = 0; it < 50; ++it) {
-        double delta = 0.0;
+    Bracket br(grid, G, idx[p]);
+    if (lead)
+        for (int it = 0; it < done; ++it) br.narrow(list >> it & 1);
+    for (int it = done; it < kGoldenSteps; ++it) {
+        double delta = 0.0, kept_loss = 0.0;
+        bool kept = false;
         if (lead) {
-            if (it > 0) narrow();
-            delta = exp(add_rn(a, mul_rn(my_e ? inv_phi : inv_phi2, add_rn(b, -a))));
+            kept = it > done && br.narrow_kept(loss_s, my_e, &kept_loss);
+            delta = exp(my_e ? br.d() : br.c());
             delta_s[my_e] = delta;
+            kept_s[my_e] = kept;
         }
         __syncthreads();
+        // evaluations e0 .. e1
+        const int e0 = kept_s[0], e1 = 2 - kept_s[1];
         double acc = 0.0;  // warps 0..3: sum (warp & 1) of evaluation warp >> 1
+        const bool sums = warp < 4 && (warp >> 1) >= e0 && (warp >> 1) < e1;
         for (int n0 = 0; n0 < Neff; n0 += kTermChunk) {
             const int m = min(kTermChunk, Neff - n0);
-            for (int t = tid; t < 2 * m; t += kBlockThreads) {
+            for (int t = e0 * m + tid; t < e1 * m; t += kBlockThreads) {
                 const int e = t >= m, n = t - (e ? m : 0);
                 const double sd = s[n0 + n] + delta_s[e];
                 const double w = 1.0 / sd;
@@ -197,23 +306,23 @@ k_golden(const double* __restrict__ s, int Neff, const double* __restrict__ UYt,
                 term[e][1][n] = log(sd);
             }
             __syncthreads();
-            if (warp < 4) {
+            if (sums) {
                 const double* x = term[warp >> 1][warp & 1];
                 for (int n = lane; n < m; n += 32) acc += x[n];
             }
             __syncthreads();
         }
-        if (warp < 4) {
+        if (sums) {
             acc = warp_sum(acc);
             if (lane == 0) sum_s[warp >> 1][warp & 1] = acc;
         }
         __syncthreads();
-        if (lead) loss_s[my_e] = ml_loss(sum_s[my_e][0], sum_s[my_e][1], delta, yy, off);
+        if (lead) loss_s[my_e] = kept ? kept_loss : ml_loss(sum_s[my_e][0], sum_s[my_e][1], delta, yy, off);
         __syncthreads();
     }
     if (tid == 0) {
-        narrow();
-        log_delta[p] = fmin(fmax(mul_rn(0.5, add_rn(a, b)), lo), hi);
+        if (done < kGoldenSteps) br.narrow(loss_s[0] < loss_s[1]);
+        log_delta[p] = fmin(fmax(mul_rn(0.5, add_rn(br.a, br.b)), lo), hi);
     }
 }
 
@@ -251,6 +360,9 @@ int fit_delta_impl(const double* s, int Neff, const double* UYt, int64_t ldu, in
         k_grid_argmin<1><<<ceil_div(P, 16), NT, 0, st>>>(Wg, sum_log, grid, UYt, ldu, Neff, P, n_grid, off, grid_idx);
     if ((rc = check_launch("k_grid_argmin"))) return rc;
     if (refine) {
+        k_golden_certain<<<ceil_div(P, kCertainWarps), 32 * kCertainWarps, 0, st>>>(s, Neff, UYt, ldu, P, grid, n_grid, grid_idx,
+                                                                                   off, log_delta);
+        if ((rc = check_launch("k_golden_certain"))) return rc;
         k_golden<<<P, kBlockThreads, 0, st>>>(s, Neff, UYt, ldu, grid, n_grid, grid_idx, lo, hi, off, log_delta);
         return check_launch("k_golden");
     }

@@ -323,7 +323,8 @@ __global__ void k_gls_golden(const double* __restrict__ s, int N, const double* 
 // The same search with one block per column: both evaluations of a step share the block, whose threads form the weights
 // (one division per eigenvalue; a warp of k_gls_golden forms them again for every eight products of its Gram) and
 // logarithms into shared memory, and whose warps then add the Gram's products four at a time, each sum in the order of
-// k_gls_golden's lanes and butterfly, so every loss keeps its bits.  60 columns x 300 samples, C = 5, with the grid:
+// k_gls_golden's lanes and butterfly, so every loss keeps its bits.  A point that is, to the bit, one of the step before
+// keeps its loss.  60 columns x 300 samples, C = 5, with the grid:
 // 7.5 -> 2.3 ms.  Beyond ~6,000 samples the weights no longer fit in shared memory and k_gls_golden runs.
 constexpr int kBlockThreads = 256;
 constexpr int kBlockPairs = 4;
@@ -339,6 +340,7 @@ k_gls_golden_block(const double* __restrict__ s, int N, const double* __restrict
                    const int32_t* __restrict__ idx, int reml, double lo, double hi, double* __restrict__ log_delta) {
     extern __shared__ double sm[];
     __shared__ double delta_s[2], log_s[2], loss_s[2];
+    __shared__ int kept_s[2];
     const int64_t p = blockIdx.x;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int K = C + 1, pairs = K * (K + 1) / 2;
@@ -347,32 +349,28 @@ k_gls_golden_block(const double* __restrict__ s, int N, const double* __restrict
     double* mats = lg + 2 * N;
     const int per = K * K + C * C + K;
     const double* y = Yrt + p * ldy;
-    const int i = idx[p];
     const bool lead = tid == 0 || tid == 32;  // carry the search, one evaluation each
     const int my_e = tid >> 5;
-    double a = grid[max(i - 1, 0)], b = grid[min(i + 1, G - 1)];
-    const double inv_phi = 2.0 / (1.0 + sqrt(5.0));
-    const double inv_phi2 = mul_rn(inv_phi, inv_phi);
-    auto narrow = [&] {
-        const double c = add_rn(a, mul_rn(inv_phi2, add_rn(b, -a))), d = add_rn(a, mul_rn(inv_phi, add_rn(b, -a)));
-        const bool cond = loss_s[0] < loss_s[1];
-        b = cond ? d : b;
-        a = cond ? a : c;
-    };
+    Bracket br(grid, G, idx[p]);
     const int groups = (pairs + kBlockPairs - 1) / kBlockPairs;  // of products; one more sum per evaluation is the log's
     for (int it = 0; it < 50; ++it) {
+        double kept_loss = 0.0;
+        bool kept = false;
         if (lead) {
-            if (it > 0) narrow();
-            delta_s[my_e] = exp(add_rn(a, mul_rn(my_e ? inv_phi : inv_phi2, add_rn(b, -a))));
+            kept = it > 0 && br.narrow_kept(loss_s, my_e, &kept_loss);
+            delta_s[my_e] = exp(my_e ? br.d() : br.c());
+            kept_s[my_e] = kept;
         }
         __syncthreads();
-        for (int t = tid; t < 2 * N; t += kBlockThreads) {
+        // evaluations e0 .. e1
+        const int e0 = kept_s[0], e1 = 2 - kept_s[1];
+        for (int t = e0 * N + tid; t < e1 * N; t += kBlockThreads) {
             const double sd = s[t < N ? t : t - N] + delta_s[t >= N];
             w[t] = 1.0 / sd;
             lg[t] = log(sd);
         }
         __syncthreads();
-        for (int g = warp; g < 2 * (groups + 1); g += kBlockThreads / 32) {
+        for (int g = e0 * (groups + 1) + warp; g < e1 * (groups + 1); g += kBlockThreads / 32) {
             const int e = g > groups, q = g - e * (groups + 1);
             const double* we = w + e * N;
             if (q == groups) {
@@ -408,15 +406,17 @@ k_gls_golden_block(const double* __restrict__ s, int N, const double* __restrict
             }
         }
         __syncthreads();
-        if (lead) {
+        if (kept) {
+            loss_s[my_e] = kept_loss;
+        } else if (lead) {
             double* Gs = mats + my_e * per;
             loss_s[my_e] = gram_loss(Gs, log_s[my_e], N, C, reml != 0, Gs + K * K, Gs + K * K + C * C);
         }
         __syncthreads();
     }
     if (tid == 0) {
-        narrow();
-        log_delta[p] = fmin(fmax(mul_rn(0.5, add_rn(a, b)), lo), hi);
+        br.narrow(loss_s[0] < loss_s[1]);
+        log_delta[p] = fmin(fmax(mul_rn(0.5, add_rn(br.a, br.b)), lo), hi);
     }
 }
 

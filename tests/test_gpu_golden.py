@@ -75,3 +75,40 @@ def test_gls_fit(n, C, P, reml):
     want, i = _golden(loss, P, s.device)
     assert torch.equal(idx.long(), i)
     torch.testing.assert_close(loss(ld), loss(want), rtol=4 * n * 2.0 ** -53, atol=1e-10)
+
+
+@pytest.mark.parametrize("n,P,scale", [(1, 2, 1.0), (33, 40, 1.0), (511, 9, 1.0), (512, 9, 1e-9), (513, 9, 1e5),
+                                       (1537, 5, 1.0)])
+@pytest.mark.parametrize("off", [0, 7])
+def test_steps_taken_from_grouped_sums(n, P, scale, off):
+    """The steps that grouped sums decide (groups of 16 x 32 eigenvalues) are the reference's: the answer lies in the bracket
+    that the search in torch FP64 has while its two losses still differ by more than 1e-8 (rounding there is ~1e-11)."""
+    from fasterlmm_gb300 import build, core, lowrank
+    build()
+    s, UY, rn = _inputs(n, P, 3 * n + off)
+    s = s * scale
+    N = n + off
+    rest = rn(P, 1 + off)
+    yy = rest.square().sum(1)
+    if off:
+        ld, i = lowrank.fit_delta_t(s, UY, rest, N)
+    else:
+        ld, i = core.fit_delta_t(s, UY)
+
+    def loss(x):
+        sd = s[None, :] + x.exp()[:, None]
+        q = (UY * UY / sd).sum(1) + (yy / x.exp() if off else 0.0)
+        return N * (math.log(2 * math.pi) + torch.log(q / N) + 1.0) + torch.log(sd).sum(1) + off * x
+
+    grid = torch.linspace(LO, HI, G, dtype=torch.float64, device=s.device)
+    i = i.long()  # (eigenvalues of 1e-9 leave the loss flat: the node is rounding's choice)
+    a, b = grid[(i - 1).clamp(min=0)], grid[(i + 1).clamp(max=G - 1)]
+    phi = 2.0 / (1.0 + math.sqrt(5.0))
+    sure = torch.ones(P, dtype=torch.bool, device=s.device)
+    for _ in range(50):
+        c, d = a + phi * phi * (b - a), a + phi * (b - a)
+        fc, fd = loss(c), loss(d)
+        sure &= (fc - fd).abs() > 1e-8
+        left = fc < fd
+        b, a = torch.where(sure & left, d, b), torch.where(sure & ~left, c, a)
+    assert ((ld >= a - 1e-12) & (ld <= b + 1e-12)).all()
