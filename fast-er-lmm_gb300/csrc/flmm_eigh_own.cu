@@ -47,9 +47,9 @@ constexpr double kRowPassCycles = 100e3, kColumnCycles = 5e3, kCtaCycles = 50;
 constexpr int kRowsPerWarp = 4;    // rows a warp of the tridiagonalisation works on at once
 constexpr int kLoadsPerRow = 8;    // loads of each of them a lane has in flight
 constexpr int kWy = 16;            // reflectors per WY block
-constexpr int kTile = 16;          // eigenvectors per back-transform CTA
-constexpr int kBtThreads = 256;
-constexpr int kChunk = 128;        // rows of a V block staged at a time in the back-transform
+constexpr int kChunk = 64;         // rows of two V blocks staged at a time in the back-transform
+constexpr int kRing = 3;           // such chunks in shared memory: one read by each phase, one on its way
+static_assert(kWy == 16 && kChunk == 64, "the back-transform's thread layout");
 // the FP32 shift is within ~1e-7 ||T|| of its eigenvalue: at the cluster cut (a gap of 1e-5 ||T||) each solve shrinks
 // the neighbour by ~1e-2, so three solves leave ~1e-6 of it (two left pairs near the cut ~1e-4 from orthogonal)
 constexpr int kInvitSolves = 3;
@@ -643,92 +643,193 @@ k_wy_factors(const float* __restrict__ W, const float* __restrict__ tau_all, int
     Tq[((static_cast<int64_t>(b) * gridDim.x + q) * kWy + a) * kWy + c] = T[a][c];
 }
 
-// grid (ceil(N / kTile), batch): columns c0 .. c0+15 of Z (eigenvectors of T) to eigenvector rows of A in U
-__global__ void __launch_bounds__(kBtThreads)
+// grid (ceil(N / kTile), batch): columns c0 .. c0 + kTile - 1 of Z (eigenvectors of T) to eigenvector rows of A in U.
+//
+// Every entry of S = V^T Z is one chain of multiply-adds down the rows, every entry of Z -= V S' one over the block's
+// reflectors.  Round q goes down the rows once: Z -= V_q S'_q a chunk ahead of S_{q-1} = V_{q-1}^T Z, the one by four
+// warps with the 16 x 4 entries of S' of a thread's columns in registers, the other by two with 2 x 2 chains a thread;
+// both blocks' rows come through a ring of kRing chunks.  Shared-memory reads and a barrier a chunk bound it.  One phase after
+// the other, an operand read per multiply-add and a chunk's loads waited for: 20 x 1,000 x 1,000 4.20 -> 2.61 ms, 8 x 1,600 x
+// 1,600 7.98 -> 4.61.
+template <int kTile>
+struct Bt {
+    static constexpr int kDot = 4 * kTile;             // threads of V^T Z
+    static constexpr int kUpd = 8 * kTile;             // and of Z -= V S'
+    static constexpr int kThreads = kDot + kUpd;
+    static size_t smem(int N) { return sizeof(float) * (static_cast<size_t>(N + kChunk) * kTile + kRing * 2 * kWy * kChunk); }
+};
+
+template <int kTile>
+__global__ void __launch_bounds__(Bt<kTile>::kThreads, kTile == 16 ? 2 : 1)
 k_backtransform(const float* __restrict__ W, const float* __restrict__ Tq_all, const float* __restrict__ Z, int N,
                 int n_refl, int nblocks, float* __restrict__ U) {
-    extern __shared__ float sm[];
-    float* Zt = sm;                          // N x kTile
-    float* Vc = Zt + N * kTile;              // kWy x kChunk: Vc[a * kChunk + ii] = v_{k0+a}[i0 + ii]
+    constexpr int kBtThreads = Bt<kTile>::kThreads, kBtDot = Bt<kTile>::kDot, kUpd = Bt<kTile>::kUpd;
+    extern __shared__ float4 sm4[];
+    float* Zt = reinterpret_cast<float*>(sm4);  // N x kTile, kChunk rows of zeros
+    float* ring = Zt + (N + kChunk) * kTile;    // kRing x [V_q, V_{q-1}] x kWy x kChunk
     __shared__ float Sm[kWy][kTile + 1];
-    __shared__ float Sp[kWy][kTile + 1];
+    __shared__ __align__(16) float Sp[kWy][kTile];  // -S'
     __shared__ float Tm[kWy][kWy + 1];
     const int b = blockIdx.y;
     const int c0 = blockIdx.x * kTile;
     const int64_t NN = static_cast<int64_t>(N) * N;
     const float* Wb = W + b * NN;
     const float* Zb = Z + b * NN;
+    const float* Tb = Tq_all + static_cast<int64_t>(b) * nblocks * kWy * kWy;
     const int ncols = min(kTile, N - c0);
-    for (int t = threadIdx.x; t < N * kTile; t += kBtThreads) {
-        const int i = t / kTile, c = t % kTile;
-        Zt[t] = c < ncols ? Zb[static_cast<int64_t>(i) * N + c0 + c] : 0.0f;
-    }
-    const int a = threadIdx.x / kTile, cc = threadIdx.x % kTile;  // one (reflector, column) pair per thread
-    // V is staged kChunk rows at a time; each thread loads its kPre entries of the next stage into registers while
-    // the current one is used, so the stage's global loads overlap the block's arithmetic instead of preceding it
-    constexpr int kPre = kChunk * kWy / kBtThreads;
-    static_assert(kChunk * kWy % kBtThreads == 0, "stage entries per thread");
+    const int tid = threadIdx.x;
+    // rows base(q) + kChunk j .. of blocks q and q - 1, by the threads of the second phase: into registers, and an iteration
+    // later to ring slot j (rows of a block from its first one on)
+    constexpr int kEntries = 2 * kWy * kChunk, kPre = (kEntries + kUpd - 1) / kUpd;
     float pre[kPre];
-    int pk0 = 0;
-    auto load_stage = [&](int i0) {
+    auto base = [&](int q) { return max(q - 1, 0) * kWy + 1; };
+    constexpr int kStep = kUpd / kChunk;  // reflectors la, la + kStep, ..., of both blocks one after the other, row li
+    static_assert(kUpd % kChunk == 0, "a thread's entries of a chunk are of one row");
+    const int la = (tid - kBtDot) / kChunk, li = (tid - kBtDot) % kChunk;
+    auto load = [&](int q, int j) {
+        const int i0 = base(q) + j * kChunk, i = i0 + li;
+        if (j > 0 && q > 0 && (q + 1) * kWy <= n_refl && i0 + kChunk <= N) {  // nothing to leave out
+#pragma unroll
+            for (int u = 0; u < kPre; ++u) {
+                const int a = min(la + u * kStep, 2 * kWy - 1);
+                pre[u] = Wb[(q * kWy + a - (a < kWy ? 0 : 2 * kWy)) * N + i];
+            }
+            return;
+        }
 #pragma unroll
         for (int u = 0; u < kPre; ++u) {
-            const int t = threadIdx.x + u * kBtThreads;
-            const int aa = t / kChunk, ii = t % kChunk, i = i0 + ii, k = pk0 + aa;
-            pre[u] = (i < N && k < n_refl && i > k) ? Wb[static_cast<int64_t>(k) * N + i] : 0.0f;
+            const int a = la + u * kStep, k = q * kWy + a - (a < kWy ? 0 : 2 * kWy);
+            pre[u] = (a < 2 * kWy && i < N && k >= 0 && k < n_refl && i > k) ? Wb[k * N + i] : 0.0f;
         }
     };
-    auto store_stage = [&]() {
+    auto store = [&](int j) {
+        float* slot = ring + (j % kRing) * kEntries;
 #pragma unroll
-        for (int u = 0; u < kPre; ++u) Vc[threadIdx.x + u * kBtThreads] = pre[u];
-    };
-    for (int q = nblocks - 1; q >= 0; --q) {
-        const int k0 = q * kWy;
-        const int r0 = k0 + 1;  // first row any reflector of the block touches
-        if (threadIdx.x < kWy * kWy)
-            Tm[threadIdx.x / kWy][threadIdx.x % kWy] = Tq_all[(static_cast<int64_t>(b) * nblocks + q) * kWy * kWy + threadIdx.x];
-        float s = 0.0f;
-        pk0 = k0;
-        // S = V^T Z over the block's rows, V staged kChunk rows at a time (V[i][a] = v_{k0+a}[i]; consecutive
-        // threads read one row of W)
-        load_stage(r0);
-        for (int i0 = r0; i0 < N; i0 += kChunk) {
-            __syncthreads();
-            store_stage();
-            __syncthreads();
-            if (i0 + kChunk < N) load_stage(i0 + kChunk);
-            const int iend = min(kChunk, N - i0);
-            for (int ii = 0; ii < iend; ++ii) s = fmaf(Vc[a * kChunk + ii], Zt[(i0 + ii) * kTile + cc], s);
+        for (int u = 0; u < kPre; ++u) {
+            const int t = tid - kBtDot + u * kUpd;
+            if (kEntries % kUpd == 0 || t < kEntries) slot[t] = pre[u];
         }
-        Sm[a][cc] = s;
-        __syncthreads();
-        // S' = T S
-        float sp = 0.0f;
-        for (int m = a; m < kWy; ++m) sp = fmaf(Tm[a][m], Sm[m][cc], sp);
-        Sp[a][cc] = sp;
-        __syncthreads();
-        // Z -= V S'
-        load_stage(r0);
-        for (int i0 = r0; i0 < N; i0 += kChunk) {
-            __syncthreads();
-            store_stage();
-            __syncthreads();
-            if (i0 + kChunk < N) load_stage(i0 + kChunk);
-            const int iend = min(kChunk, N - i0);
-            for (int t = threadIdx.x; t < iend * kTile; t += kBtThreads) {
-                const int ii = t / kTile, c = t % kTile;
-                float acc = Zt[(i0 + ii) * kTile + c];
+    };
+    if (tid >= kBtDot) {
+        load(nblocks, 0);
+        store(0);
+        load(nblocks, 1);
+    }
+    for (int t = tid; t < (N + kChunk) * kTile; t += kBtThreads) {
+        const int i = t / kTile, c = t % kTile;
+        Zt[t] = c < ncols && i < N ? Zb[static_cast<int64_t>(i) * N + c0 + c] : 0.0f;
+    }
+    // S: reflectors sa, sa + 1 and columns sc, sc + 1 of a thread of the first phase
+    const int sa = tid / (kTile / 2) * 2, sc = tid % (kTile / 2) * 2;
+    // Z -= V S': columns zc .. zc + 3 of a chunk's rows zr and zr + 32 of a thread of the other warps
+    constexpr int kQuads = kTile / 4;
+    static_assert(kUpd / kQuads == kChunk / 2, "two rows of four columns a thread");
+    const int zc = (tid - kBtDot) % kQuads * 4, zr = (tid - kBtDot) / kQuads;
+    for (int q = nblocks; q >= 0; --q) {
+        const int i0 = base(q), first = q * kWy + 1;  // first row that V_q touches
+        const int chunks = (N - i0 + kChunk - 1) / kChunk;
+        float s[2][2] = {};
+        float4 ns[kWy] = {};
+        if (tid >= kBtDot && q < nblocks) {
 #pragma unroll
-                for (int m = 0; m < kWy; ++m) acc = fmaf(-Vc[m * kChunk + ii], Sp[m][c], acc);
-                Zt[(i0 + ii) * kTile + c] = acc;
+            for (int m = 0; m < kWy; ++m) ns[m] = *reinterpret_cast<const float4*>(&Sp[m][zc]);
+        }
+        if (q > 0)
+            for (int t = tid; t < kWy * kWy; t += kBtThreads) Tm[t / kWy][t % kWy] = Tb[static_cast<int64_t>(q - 1) * kWy * kWy + t];
+        for (int j = 0; j <= chunks; ++j) {
+            __syncthreads();  // chunk j is staged, and rows of chunk j - 1 are up to date
+            if (tid >= kBtDot) {
+                if (j + 1 < chunks) store(j + 1);
+                if (j + 2 < chunks) load(q, j + 2);
+                else if (j + 2 == max(chunks, 2) && q > 0) load(q - 1, 0);
+                if (j == chunks || q == nblocks) continue;
+                const float* V = ring + (j % kRing) * 2 * kWy * kChunk;
+                const int r = i0 + j * kChunk, end = min(kChunk, N - r);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int ii = zr + h * (kChunk / 2);
+                    if (ii >= end || r + ii < first) continue;
+                    float4* zp = reinterpret_cast<float4*>(Zt + (r + ii) * kTile + zc);
+                    float4 z = *zp;
+#pragma unroll
+                    for (int m = 0; m < kWy; ++m) {
+                        const float v = V[m * kChunk + ii];
+                        z.x = fmaf(v, ns[m].x, z.x);
+                        z.y = fmaf(v, ns[m].y, z.y);
+                        z.z = fmaf(v, ns[m].z, z.z);
+                        z.w = fmaf(v, ns[m].w, z.w);
+                    }
+                    *zp = z;
+                }
+            } else if (j > 0 && q > 0) {
+                // eight rows at a time, the next eight on their way (rows past N are zeros in both operands)
+                const float* v = ring + ((j - 1) % kRing) * 2 * kWy * kChunk + (kWy + sa) * kChunk;
+                const float* z = Zt + (i0 + (j - 1) * kChunk) * kTile + sc;
+                float4 vv[2][2][2];  // [buffer][reflector][rows / 4]
+                float2 zz[2][8];
+                auto fetch = [&](int u, int ii) {
+#pragma unroll
+                    for (int a = 0; a < 2; ++a)
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) vv[u][a][h] = *reinterpret_cast<const float4*>(v + a * kChunk + ii + 4 * h);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) zz[u][e] = *reinterpret_cast<const float2*>(z + (ii + e) * kTile);
+                };
+                fetch(0, 0);
+#pragma unroll
+                for (int g = 0; g < kChunk / 8; ++g) {
+                    if (g + 1 < kChunk / 8) fetch((g + 1) & 1, 8 * (g + 1));
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        const float2 x = zz[g & 1][e];
+#pragma unroll
+                        for (int a = 0; a < 2; ++a) {
+                            const float4 f = vv[g & 1][a][e / 4];
+                            const float y = e % 4 == 0 ? f.x : e % 4 == 1 ? f.y : e % 4 == 2 ? f.z : f.w;
+                            s[a][0] = fmaf(y, x.x, s[a][0]);
+                            s[a][1] = fmaf(y, x.y, s[a][1]);
+                        }
+                    }
+                }
+            }
+        }
+        if (q == 0) break;
+        if (tid < kBtDot) {
+#pragma unroll
+            for (int a = 0; a < 2; ++a) {
+                Sm[sa + a][sc] = s[a][0];
+                Sm[sa + a][sc + 1] = s[a][1];
             }
         }
         __syncthreads();
+        if (tid >= kBtDot) {
+            store(0);
+            load(q - 1, 1);
+        }
+        // S' = T S
+        for (int t = tid; t < kWy * kTile; t += kBtThreads) {
+            const int a = t / kTile, cc = t % kTile;
+            float sp = 0.0f;
+#pragma unroll
+            for (int m = 0; m < kWy; ++m) sp = m >= a ? fmaf(Tm[a][m], Sm[m][cc], sp) : sp;
+            Sp[a][cc] = -sp;
+        }
+        __syncthreads();
     }
+    __syncthreads();
     // eigenvector c0 + c is column c of the tile: one row of U each
     for (int c = 0; c < ncols; ++c)
-        for (int i = threadIdx.x; i < N; i += kBtThreads)
-            U[b * NN + static_cast<int64_t>(c0 + c) * N + i] = Zt[i * kTile + c];
+        for (int i = tid; i < N; i += kBtThreads) U[b * NN + static_cast<int64_t>(c0 + c) * N + i] = Zt[i * kTile + c];
+}
+
+template <int kTile>
+int launch_backtransform(const float* W, const float* Tq, const float* Z, int N, int n_refl, int nblocks, int batch, float* U,
+                         cudaStream_t st) {
+    const size_t smem = Bt<kTile>::smem(N);
+    // (per device, so set on every call; the call is cheap)
+    FLMM_CUDA(cudaFuncSetAttribute(k_backtransform<kTile>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    k_backtransform<kTile><<<dim3(ceil_div(N, kTile), batch), Bt<kTile>::kThreads, smem, st>>>(W, Tq, Z, N, n_refl, nblocks, U);
+    return check_launch("k_backtransform");
 }
 
 struct OwnLayout {
@@ -836,8 +937,6 @@ int eigh_own_f32(float* A, int N, int batch, float* evals, void* work, cudaStrea
     int C = 0;
     int rc = cluster_ctas(dev, N, batch, &C);
     if (rc) return rc;
-    // (per device, so set on every call; the call is cheap)
-    FLMM_CUDA(cudaFuncSetAttribute(k_backtransform, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -868,9 +967,11 @@ int eigh_own_f32(float* A, int N, int batch, float* evals, void* work, cudaStrea
         k_wy_factors<<<dim3(L.nblocks, batch), kWy * kWy, 0, st>>>(W, tau, N, n_refl, Tq);
         if ((rc = check_launch("k_wy_factors"))) return rc;
     }
-    const size_t smem4 = sizeof(float) * (static_cast<size_t>(N) * kTile + kChunk * kWy);
-    k_backtransform<<<dim3(ceil_div(N, kTile), batch), kBtThreads, smem4, st>>>(W, Tq, Z, N, n_refl, L.nblocks, A);
-    return check_launch("k_backtransform");
+    // Two CTAs of 16 columns an SM as long as they fit; then one of 24, as long as that fits (8 x 1,600 x 1,600: 4.61 ms, one
+    // of 16 5.61); then one of 16.
+    if (N <= 1310) return launch_backtransform<16>(W, Tq, Z, N, n_refl, L.nblocks, batch, A, st);
+    if (N <= 1900) return launch_backtransform<24>(W, Tq, Z, N, n_refl, L.nblocks, batch, A, st);
+    return launch_backtransform<16>(W, Tq, Z, N, n_refl, L.nblocks, batch, A, st);
 }
 
 }  // namespace flmm
