@@ -5,15 +5,18 @@
 //
 // Five stages, all matrices of the batch side by side:
 //
-// 1. k_sytrd_cluster: Householder tridiagonalisation A = Q T Q^T, one thread-block cluster of 2 to 8 CTAs per
+// 1. k_sytrd_cluster: Householder tridiagonalisation A = Q T Q^T, one thread-block cluster of 2 to 16 CTAs per
 //    matrix (one CTA per SM).  The FP32 matrix stays in global memory (L2-resident for the batch sizes used), rows
 //    dealt round-robin to the cluster's CTAs.  Column k's reflector is formed redundantly by every CTA, each CTA
-//    computes p = tau W v for its rows and stores it, with its partial p^T v, into every CTA's shared memory
-//    (distributed shared memory), so after the barrier each CTA reads only its own.  The symmetric rank-2 update
-//    W -= v w^T + w v^T is applied lazily, in the same pass that forms the next column's W v, so the trailing
-//    matrix is read and written once per column; the next pivot row gets its last update in registers in every
-//    CTA, which forms the next reflector from it.  Both products of an update term are rounded before the add, so
-//    W stays exactly symmetric.  One cluster barrier per column.
+//    computes p = tau W v for its rows and stores it into every CTA's shared memory (distributed shared memory), so
+//    after the barrier each CTA reads only its own.  The symmetric rank-2 update W -= v w^T + w v^T is applied lazily,
+//    in the passes that form the next columns' W v, and a row is written back with every second update only; the next
+//    pivot row gets what is pending in registers in every CTA, which forms the next reflector from it.  Both products
+//    of an update term are rounded before the add, so W stays exactly symmetric.  One cluster barrier per column.
+//    What bounds it: the write path to L2 (88% of its cycles with a write per column; two updates in a row cost less than
+//    a write), then the chain of a column: barrier, p^T v, w, reflector, whose loads pass during the row pass.  20 x 1,000
+//    11.3 -> 8.2 ms, 8 x 1,600 21.7 -> 16.3, 22 x 563 3.46 -> 2.48.  Keeping rows in shared memory (all of them at 563),
+//    and smaller blocks of loads ahead of the one at work, gave nothing or less.
 // 2. k_tridiag_bisect: each eigenvalue of T by multisection on FP32 Sturm counts (ascending, by index; three points
 //    per step, so 24 steps narrow the bracket as 48 halvings would).
 // 3. k_tridiag_invit: each eigenvector of T by inverse iteration in FP64 (LDL^T of T - lambda I with a pivot floor,
@@ -42,9 +45,12 @@ namespace {
 constexpr int kMaxClusterCtas = 16;  // beyond 8 the size is not portable
 constexpr int kMaxParts = 8;         // partial sums of p^T v
 constexpr int kSytrdThreads = 512;
-// a column's cycles at N = 1,000: its row pass in one CTA, what every CTA repeats, and the barrier's share per CTA
-constexpr double kRowPassCycles = 100e3, kColumnCycles = 5e3, kCtaCycles = 50;
+// a column's cycles on average: its row pass at N = 1,000 in one CTA, what every CTA repeats, and the barrier's share per CTA
+constexpr double kRowPassCycles = 75e3, kColumnCycles = 3e3, kCtaCycles = 50;
+constexpr int kPend = 2;           // column updates that gather before the rows are written
 constexpr int kRowsPerWarp = 4;    // rows a warp of the tridiagonalisation works on at once
+constexpr int kDotRows = 4;        // rows of p^T v that follow one another in a chain (part of the result)
+constexpr int kOwnCols = 5;        // columns of a thread in the vector passes: N <= 512 * 5
 constexpr int kLoadsPerRow = 8;    // loads of each of them a lane has in flight
 constexpr int kWy = 16;            // reflectors per WY block
 constexpr int kChunk = 64;         // rows of two V blocks staged at a time in the back-transform
@@ -106,9 +112,9 @@ __device__ float block_sum(float v, float* red) {
 // reflector scalars (tau[N-2] = tau[N-1] = 0).  The cluster size C is the launch's (%cluster_nctarank); CTA r owns
 // the rows i with i % C == r.
 //
-// Step k: (B) each CTA brings its rows i > k up to date with column k-1's update and forms p_i = tau_k W[i, k+1:] v_k;
-// one cluster barrier; (C) every CTA gathers p and p^T v from the cluster, forms w_k, reads row k+1 (stored by its
-// owner in (B), so it already carries every update but column k's), applies column k's update to it in registers and
+// Step k: (B) each CTA applies its rows' pending updates (one or two columns; stored if two, but for row k + 1) and forms
+// p_i = tau_k W[i, k+1:] v_k; one cluster barrier; (C) every CTA adds up p^T v, forms w_k, applies what is pending and column
+// k's update to row k + 1 in registers (as it was last written: loaded before (B), since nobody writes it in this step) and
 // forms the next reflector v_{k+1} -- redundantly in every CTA, so no second barrier is needed.
 __device__ __forceinline__ uint32_t cluster_size() {
     uint32_t r;
@@ -137,16 +143,104 @@ __device__ Reflector make_reflector(float d, float alpha, float ss_partial, floa
     return R;
 }
 
+// kQ rows i0, i0 + di, ... (rows of N entries from W on) at columns k + 1 ..: the kM pending updates, oldest first, whose
+// vectors start at sm[ov[m]] and sm[ow[m]], stored when kM is kPend (not row k + 1); then p_i = tau row . v into every CTA's copy of p.
+// Every lane adds up its columns k + 1 + lane + 32 t in order.
+extern __shared__ float sytrd_sm[];
+
+template <int kM, int kQ>
+__device__ __forceinline__ void update_rows(float* W, int N, int k, int i0, int di, int oc, const int (&ov)[kPend],
+                                            const int (&ow)[kPend], float tau, int C, float* pb) {
+    const int lane = threadIdx.x & 31, len = N - k - 1;
+    const bool next = i0 == k + 1;
+    float* row0 = W + static_cast<int64_t>(i0) * N + k + 1 + lane;
+    const int64_t dr = static_cast<int64_t>(di) * N;
+    float vi[kM > 0 ? kM : 1][kQ], wi[kM > 0 ? kM : 1][kQ], acc[kQ];
+#pragma unroll
+    for (int q = 0; q < kQ; ++q) {
+        acc[q] = 0.0f;
+#pragma unroll
+        for (int m = 0; m < kM; ++m) {
+            vi[m][q] = sytrd_sm[ov[m] + i0 + q * di];
+            wi[m][q] = sytrd_sm[ow[m] + i0 + q * di];
+        }
+    }
+    const float* v = sytrd_sm + oc + k + 1 + lane;
+    float* at[kQ];
+#pragma unroll
+    for (int q = 0; q < kQ; ++q) at[q] = row0 + q * dr;
+    auto take = [&](const float (&x)[kQ], int u) {
+        const float vj = v[32 * u];
+        float vp[kM > 0 ? kM : 1], wp[kM > 0 ? kM : 1];
+#pragma unroll
+        for (int m = 0; m < kM; ++m) {
+            vp[m] = v[ov[m] - oc + 32 * u];
+            wp[m] = v[ow[m] - oc + 32 * u];
+        }
+#pragma unroll
+        for (int q = 0; q < kQ; ++q) {
+            float y = x[q];
+#pragma unroll
+            for (int m = 0; m < kM; ++m) y -= __fmul_rn(vi[m][q], wp[m]) + __fmul_rn(wi[m][q], vp[m]);
+            if (kM == kPend && !(q == 0 && next)) at[q][32 * u] = y;
+            acc[q] = fmaf(y, vj, acc[q]);
+        }
+    };
+    int rest = len;
+#pragma unroll 1
+    for (; rest >= 32 * kLoadsPerRow; rest -= 32 * kLoadsPerRow) {
+        float x[kLoadsPerRow][kQ];
+#pragma unroll
+        for (int u = 0; u < kLoadsPerRow; ++u)
+#pragma unroll
+            for (int q = 0; q < kQ; ++q) x[u][q] = at[q][32 * u];
+#pragma unroll
+        for (int u = 0; u < kLoadsPerRow; ++u) take(x[u], u);
+        v += 32 * kLoadsPerRow;
+#pragma unroll
+        for (int q = 0; q < kQ; ++q) at[q] += 32 * kLoadsPerRow;
+    }
+    if (rest > 0) {
+        float x[kLoadsPerRow][kQ];
+#pragma unroll
+        for (int u = 0; u < kLoadsPerRow; ++u)
+#pragma unroll
+            for (int q = 0; q < kQ; ++q) x[u][q] = 32 * u + lane < rest ? at[q][32 * u] : 0.0f;
+#pragma unroll
+        for (int u = 0; u < kLoadsPerRow; ++u)
+            if (32 * u + lane < rest) take(x[u], u);
+    }
+#pragma unroll
+    for (int q = 0; q < kQ; ++q) {
+        const float pi = tau * warp_sum(acc[q]);
+        // p_i into every CTA's copy of p (lane l to CTA l): after the barrier all of p is local
+        if (lane < C) st_remote(&pb[i0 + q * di], static_cast<uint32_t>(lane), pi);
+    }
+}
+
+// A warp's rows i0, i0 + di, ..., kRowsPerWarp at a time.
+template <int kM>
+__device__ __forceinline__ void update_all(float* W, int N, int k, int i0, int di, int oc, const int (&ov)[kPend],
+                                           const int (&ow)[kPend], float tau, int C, float* pb) {
+    for (; i0 + (kRowsPerWarp - 1) * di < N; i0 += kRowsPerWarp * di)
+        update_rows<kM, kRowsPerWarp>(W, N, k, i0, di, oc, ov, ow, tau, C, pb);
+    if (i0 + di < N) {
+        update_rows<kM, 2>(W, N, k, i0, di, oc, ov, ow, tau, C, pb);
+        i0 += 2 * di;
+    }
+    if (i0 < N) update_rows<kM, 1>(W, N, k, i0, di, oc, ov, ow, tau, C, pb);
+}
+
 __global__ void __launch_bounds__(kSytrdThreads, 1)
 k_sytrd_cluster(float* __restrict__ W, int N, int parts, float* __restrict__ d_out, float* __restrict__ e_out,
                 float* __restrict__ tau_out) {
-    extern __shared__ float sm[];
+    float* const sm = sytrd_sm;
     const int Np = (N + 3) & ~3;
-    float* vbuf[2] = {sm, sm + Np};
-    float* wbuf[2] = {sm + 2 * Np, sm + 3 * Np};
-    float* pbuf[2] = {sm + 4 * Np, sm + 5 * Np};
-    float* red = sm + 6 * Np;        // 32 floats
-    float* part = red + 32;          // partial sums of p^T v
+    float* const vbuf = sm;                        // v_k in slot k % (kPend + 1)
+    float* const wbuf = sm + (kPend + 1) * Np;     // w_k likewise
+    float* const pbuf = wbuf + (kPend + 1) * Np;         // p of column k in slot k % 2
+    float* red = pbuf + 2 * Np;      // 2 x 32 floats
+    float* part = red + 64;          // partial sums of p^T v
     float* scal2 = part + kMaxParts;  // d and alpha of the next reflector
     const int C = static_cast<int>(cluster_size());
     const int b = static_cast<int>(cluster_index());
@@ -156,147 +250,151 @@ k_sytrd_cluster(float* __restrict__ W, int N, int parts, float* __restrict__ d_o
     float* db = d_out + static_cast<int64_t>(b) * N;
     float* eb = e_out + static_cast<int64_t>(b) * N;
     float* tb = tau_out + static_cast<int64_t>(b) * N;
+    int first = r > 0 ? r : C;  // first row of this CTA past row k
+    int first_dot = 1 % parts;  // k + 1 modulo parts
     Reflector R{0.0f, 0.0f, 0.0f};
     if (N >= 3) {  // reflector of column 0 from the untouched row 0
         float ss = 0.0f;
         for (int j = 2 + threadIdx.x; j < N; j += kSytrdThreads) {
             const float x = Wb[j];
-            vbuf[0][j] = x;
+            vbuf[j] = x;
             ss = fmaf(x, x, ss);
         }
-        R = make_reflector(Wb[0], Wb[1], ss, vbuf[0], 0, N, red);
+        R = make_reflector(Wb[0], Wb[1], ss, vbuf, 0, N, red);
     }
     for (int k = 0; k + 2 < N; ++k) {
-        const int cur = k & 1;
-        float* vc = vbuf[cur];
-        float* wc = wbuf[cur];
-        float* vn = vbuf[cur ^ 1];        // v_{k-1} until (B) is done, then v_{k+1}
-        const float* wp = wbuf[cur ^ 1];  // w_{k-1}
-        float* pb = pbuf[cur];
+        const float* vc = vbuf + k % (kPend + 1) * Np;
+        float* vn = vbuf + (k + 1) % (kPend + 1) * Np;  // v_{k - kPend}, then v_{k+1}
+        float* wc = wbuf + k % (kPend + 1) * Np;
+        float* pb = pbuf + (k & 1) * Np;
         const float tau = R.tau;
-        // (B) rows i > k of this CTA: column k-1's update (lazy), then p_i = tau W[i, k+1:] . v.  A warp takes
-        // kRowsPerWarp rows at a time and a lane issues kLoadsPerRow loads of each before using any, so the pass
-        // keeps enough L2 reads in flight to run at bandwidth rather than at L2 latency.
-        const int first = k + 1 + ((r - (k + 1)) % C + C) % C;
-        const int n_own = first < N ? (N - 1 - first) / C + 1 : 0;
-        const bool lazy = k > 0;
-        for (int t0 = wid * kRowsPerWarp; t0 < n_own; t0 += nw * kRowsPerWarp) {
-            float* rows[kRowsPerWarp];
-            float vi[kRowsPerWarp], wi[kRowsPerWarp], acc[kRowsPerWarp];
+        // (B) rows i > k of this CTA: the pending updates of the columns k - pend .. k - 1, then p_i = tau W[i, k+1:] . v.
+        // A warp takes kRowsPerWarp rows at a time and a lane issues kLoadsPerRow loads of each before using any, so the
+        // pass keeps enough L2 reads in flight to run at bandwidth rather than at L2 latency.
+        const int pend = k > 0 ? (k - 1) % kPend + 1 : 0;
+        int ov[kPend], ow[kPend];
 #pragma unroll
-            for (int q = 0; q < kRowsPerWarp; ++q) {
-                const int t = t0 + q;
-                const int i = first + t * C;
-                rows[q] = t < n_own ? Wb + static_cast<int64_t>(i) * N : nullptr;
-                vi[q] = (t < n_own && lazy) ? vn[i] : 0.0f;
-                wi[q] = (t < n_own && lazy) ? wp[i] : 0.0f;
-                acc[q] = 0.0f;
-            }
-            for (int j0 = k + 1; j0 < N; j0 += 32 * kLoadsPerRow) {
-                float x[kRowsPerWarp][kLoadsPerRow];
-#pragma unroll
-                for (int q = 0; q < kRowsPerWarp; ++q)
-#pragma unroll
-                    for (int u = 0; u < kLoadsPerRow; ++u) {
-                        const int j = j0 + lane + 32 * u;
-                        x[q][u] = (rows[q] != nullptr && j < N) ? rows[q][j] : 0.0f;
-                    }
-#pragma unroll
-                for (int u = 0; u < kLoadsPerRow; ++u) {
-                    const int j = j0 + lane + 32 * u;
-                    if (j < N) {
-                        const float vj = vc[j];
-                        const float vpj = lazy ? vn[j] : 0.0f, wpj = lazy ? wp[j] : 0.0f;
-#pragma unroll
-                        for (int q = 0; q < kRowsPerWarp; ++q) {
-                            if (rows[q] == nullptr) continue;
-                            float xv = x[q][u];
-                            if (lazy) {
-                                xv -= __fmul_rn(vi[q], wpj) + __fmul_rn(wi[q], vpj);
-                                rows[q][j] = xv;
-                            }
-                            acc[q] = fmaf(xv, vj, acc[q]);
-                        }
-                    }
-                }
-            }
-#pragma unroll
-            for (int q = 0; q < kRowsPerWarp; ++q) {
-                const float a = warp_sum(acc[q]);
-                if (rows[q] != nullptr) {
-                    const int i = first + (t0 + q) * C;
-                    const float pi = tau * a;
-                    // p_i into every CTA's copy of p (lane l to CTA l): after the barrier all of p is local
-                    if (lane < C) st_remote(&pb[i], static_cast<uint32_t>(lane), pi);
-                }
-            }
+        for (int m = 0; m < kPend; ++m) {
+            const int c = max(k - pend + m, 0);
+            ov[m] = c % (kPend + 1) * Np;
+            ow[m] = (kPend + 1 + c % (kPend + 1)) * Np;
         }
+        const int oc = k % (kPend + 1) * Np;
+        // row k + 1 as it was last written: nobody writes it in this step, so its loads pass while the rows are at work
+        const float* rown = Wb + static_cast<int64_t>(k + 1) * N;
+        const int j0 = k + 1 + threadIdx.x;
+        float x[kOwnCols];
+#pragma unroll
+        for (int u = 0; u < kOwnCols; ++u) x[u] = j0 + kSytrdThreads * u < N ? __ldcg(rown + j0 + kSytrdThreads * u) : 0.0f;
+        const int i0 = first + wid * C;
+        if (pend == 0) update_all<0>(Wb, N, k, i0, nw * C, oc, ov, ow, tau, C, pb);
+        else if (pend == kPend) update_all<kPend>(Wb, N, k, i0, nw * C, oc, ov, ow, tau, C, pb);
+        else update_all<1>(Wb, N, k, i0, nw * C, oc, ov, ow, tau, C, pb);
+        if (first == k + 1) first += C;
+        static_assert(kPend == 2, "the cases above");
         cluster_barrier();  // every CTA's p and updated rows are visible
-        // (C) w = p - (tau / 2) (p^T v) v over the whole trailing range.  Every CTA adds up p^T v from its copy of p in one
-        // order whatever the cluster size: `parts` interleaved row sets, each in 16 chains of four rows at a time.
+        // (C) w = p - (tau / 2) (p^T v) v over the whole trailing range, and row k + 1 with what is pending and column k's
+        // update: the next reflector.  Thread t has the columns k + 1 + t + 512 u of both.
+        // Every CTA adds up p^T v from its copy of p in one order whatever the cluster size: `parts` interleaved row sets,
+        // each in 16 chains of four rows at a time.
         if (threadIdx.x < 16 * kMaxParts) {
             const int q = threadIdx.x >> 4, chain = threadIdx.x & 15;
             float dot = 0.0f;
             if (q < parts) {
-                const int f = k + 1 + ((q - (k + 1)) % parts + parts) % parts;
-                const int n = f < N ? (N - 1 - f) / parts + 1 : 0;
-                for (int t0 = chain * kRowsPerWarp; t0 < n; t0 += 16 * kRowsPerWarp)
-                    for (int t = t0; t < min(t0 + kRowsPerWarp, n); ++t) dot = fmaf(pb[f + t * parts], vc[f + t * parts], dot);
+                // set q: rows f, f + parts, ... with f % parts == q
+                const int f = k + 1 + (q >= first_dot ? q - first_dot : q - first_dot + parts);
+                for (int i = f + chain * kDotRows * parts; i < N; i += 16 * kDotRows * parts) {
+                    float pv[kDotRows], vv[kDotRows];
+#pragma unroll
+                    for (int e = 0; e < kDotRows; ++e) {
+                        const int ie = i + e * parts < N ? i + e * parts : i;
+                        pv[e] = pb[ie];
+                        vv[e] = vc[ie];
+                    }
+#pragma unroll
+                    for (int e = 0; e < kDotRows; ++e)
+                        if (i + e * parts < N) dot = fmaf(pv[e], vv[e], dot);
+                }
             }
 #pragma unroll
             for (int o = 8; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
             if (chain == 0) part[q] = dot;
         }
+        if (++first_dot == parts) first_dot = 0;
         __syncthreads();
         float s = 0.0f;
-        for (int q = 0; q < parts; ++q) s += part[q];
+#pragma unroll
+        for (int q = 0; q < kMaxParts; ++q) {
+            const float v = part[q];
+            if (q < parts) s += v;
+        }
         const float c = -0.5f * tau * s;
-        for (int j = k + 1 + threadIdx.x; j < N; j += kSytrdThreads) wc[j] = fmaf(c, vc[j], pb[j]);
-        __syncthreads();
+        const float vk1 = vc[k + 1], wk1 = fmaf(c, vk1, pb[k + 1]);
+        float vp[kPend], wp[kPend];
+#pragma unroll
+        for (int m = 0; m < kPend; ++m) {
+            vp[m] = sm[ov[m] + k + 1];
+            wp[m] = sm[ow[m] + k + 1];
+        }
+        float ss = 0.0f;
+#pragma unroll
+        for (int u = 0; u < kOwnCols; ++u) {
+            const int j = j0 + kSytrdThreads * u;
+            if (j >= N) break;
+            const float v = vc[j], w = fmaf(c, v, pb[j]);
+            wc[j] = w;
+#pragma unroll
+            for (int m = 0; m < kPend; ++m)
+                if (m < pend) x[u] -= __fmul_rn(vp[m], sm[ow[m] + j]) + __fmul_rn(wp[m], sm[ov[m] + j]);
+            x[u] -= __fmul_rn(vk1, w) + __fmul_rn(wk1, v);
+            if (j == k + 1) scal2[0] = x[u];
+            else if (j == k + 2) scal2[1] = x[u];
+            else ss = fmaf(x[u], x[u], ss);
+        }
         if (r == 0) {  // row k is read by nobody any more: it keeps the reflector
             float* rowv = Wb + static_cast<int64_t>(k) * N;
-            for (int j = k + 1 + threadIdx.x; j < N; j += kSytrdThreads) rowv[j] = vc[j];
+            for (int j = j0; j < N; j += kSytrdThreads) rowv[j] = vc[j];
             if (threadIdx.x == 0) {
                 db[k] = R.d;
                 eb[k] = R.beta;
                 tb[k] = tau;
             }
         }
-        // row k + 1 with column k's update, in registers: the next reflector (or, after the last one, T's trailing
-        // 2 x 2 block)
-        const float* rown = Wb + static_cast<int64_t>(k + 1) * N;
-        const float vk1 = vc[k + 1], wk1 = wc[k + 1];
+        // sum of squares in every thread: the warps' sums, then theirs, as block_sum adds them
+        ss = warp_sum(ss);
+        float* red_k = red + (k & 1) * 32;
+        if (lane == 0) red_k[wid] = ss;
+        __syncthreads();
+        const float sig = warp_sum(lane < nw ? red_k[lane] : 0.0f);
         if (k + 3 < N) {
-            float ss = 0.0f;
-            for (int j = k + 1 + threadIdx.x; j < N; j += kSytrdThreads) {
-                const float x = __ldcg(rown + j) - (__fmul_rn(vk1, wc[j]) + __fmul_rn(wk1, vc[j]));
-                if (j == k + 1) scal2[0] = x;
-                else if (j == k + 2) scal2[1] = x;
-                else {
-                    vn[j] = x;
-                    ss = fmaf(x, x, ss);
-                }
-            }
-            // the reduction synchronises the CTA before scal2 is read
-            const float sig = block_sum(ss, red);
-            const float dn = scal2[0], alpha = scal2[1];
-            Reflector Rn{dn, alpha, 0.0f};
-            float scl = 0.0f;
+            const float alpha = scal2[1];
+            Reflector Rn{scal2[0], alpha, 0.0f};
+            float scl = 1.0f;
             if (sig > 0.0f) {
                 Rn.beta = -copysignf(sqrtf(fmaf(alpha, alpha, sig)), alpha);
                 Rn.tau = (Rn.beta - alpha) / Rn.beta;
                 scl = 1.0f / (alpha - Rn.beta);
+            } else {
+                scl = 0.0f;
             }
-            for (int j = k + 3 + threadIdx.x; j < N; j += kSytrdThreads) vn[j] *= scl;
+#pragma unroll
+            for (int u = 0; u < kOwnCols; ++u) {
+                const int j = j0 + kSytrdThreads * u;
+                if (j < N && j > k + 2) vn[j] = x[u] * scl;
+            }
             if (threadIdx.x == 0) vn[k + 2] = 1.0f;
             __syncthreads();
             R = Rn;
-        } else if (r == 0 && threadIdx.x == 0) {  // k = N - 3: rows N - 2 and N - 1 get column k's update
-            const float* rowl = Wb + static_cast<int64_t>(N - 1) * N;
-            const float vl = vc[N - 1], wl = wc[N - 1];
-            db[N - 2] = __ldcg(rown + N - 2) - (__fmul_rn(vk1, wc[N - 2]) + __fmul_rn(wk1, vc[N - 2]));
-            eb[N - 2] = __ldcg(rown + N - 1) - (__fmul_rn(vk1, wc[N - 1]) + __fmul_rn(wk1, vc[N - 1]));
-            db[N - 1] = __ldcg(rowl + N - 1) - (__fmul_rn(vl, wc[N - 1]) + __fmul_rn(wl, vc[N - 1]));
+        } else if (r == 0 && threadIdx.x == 0) {  // k = N - 3: rows N - 2 and N - 1 get column k's update: T's trailing 2 x 2
+            auto update = [&](float y, int i, int j, int pending) {
+#pragma unroll
+                for (int m = 0; m < kPend; ++m)
+                    if (m < pending) y -= __fmul_rn(sm[ov[m] + i], sm[ow[m] + j]) + __fmul_rn(sm[ow[m] + i], sm[ov[m] + j]);
+                return y - (__fmul_rn(vc[i], wc[j]) + __fmul_rn(wc[i], vc[j]));
+            };
+            db[N - 2] = update(__ldcg(rown + N - 2), N - 2, N - 2, pend);
+            eb[N - 2] = update(__ldcg(rown + N - 1), N - 2, N - 1, pend);
+            db[N - 1] = update(__ldcg(Wb + static_cast<int64_t>(N - 1) * N + N - 1), N - 1, N - 1, pend == kPend ? 0 : pend);
         }
     }
     if (r == 0 && threadIdx.x == 0) {
@@ -928,7 +1026,7 @@ int eigh_own_f32(float* A, int N, int batch, float* evals, void* work, cudaStrea
     FLMM_CUDA(cudaMemcpyAsync(W, A, 4 * NN * batch, cudaMemcpyDeviceToDevice, st));
     // 1. tridiagonalisation, one cluster per matrix
     const int Np = (N + 3) & ~3;
-    const size_t smem1 = sizeof(float) * (6 * static_cast<size_t>(Np) + 32 + kMaxParts + 2);
+    const size_t smem1 = sizeof(float) * ((2 * kPend + 4) * static_cast<size_t>(Np) + 64 + kMaxParts + 2);
     int dev = 0, sms = 0;
     FLMM_CUDA(cudaGetDevice(&dev));
     FLMM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
