@@ -419,7 +419,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc(const __grid_constant__ TcMa
         }
     } else if (warp == 1) {
         // ---- MMA issuer: every chunk starts afresh in the next slot of the ring ----
-        if (lane == 0) {
+        {
+            const uint32_t elected = elect_one();
             int stage = 0;
             uint32_t phase = 0;
             int slot = 0;
@@ -428,11 +429,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc(const __grid_constant__ TcMa
             for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
                 for (int kc = 0, kc_end = 0; kc < n_kb && ok; kc = kc_end) {
                     kc_end = kc < n_kb0 ? min(kc + args.chunk_kb, n_kb0) : n_kb;
-                    if (!mbar_wait(&slot_empty[slot], sphase ^ 1u, args.err, 2)) { ok = false; break; }
+                    if (!mbar_wait_warp(&slot_empty[slot], sphase ^ 1u, args.err, 2)) { ok = false; break; }
                     fence_after_sync();
                     const uint32_t d = tmem_base + static_cast<uint32_t>(slot * kBN);
                     for (int kb = kc; kb < kc_end; ++kb) {
-                        if (!mbar_wait(&full[stage], phase, args.err, 3)) { ok = false; break; }
+                        if (!mbar_wait_warp(&full[stage], phase, args.err, 3)) { ok = false; break; }
                         fence_after_sync();
                         const uint32_t sbase = smem_u32(smem + stage * C::kStageBytes);
 #pragma unroll
@@ -441,20 +442,20 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc(const __grid_constant__ TcMa
                             const uint64_t al = smem_desc(sbase + 1 * C::kTileBytes, C::kSBO, C::kSwizzle) + 2u * kk;
                             const uint64_t bh = smem_desc(sbase + 2 * C::kTileBytes, C::kSBO, C::kSwizzle) + 2u * kk;
                             const uint64_t bl = smem_desc(sbase + 3 * C::kTileBytes, C::kSBO, C::kSwizzle) + 2u * kk;
-                            mma_f16(d, ah, bh, idesc, (kb != kc || kk) ? 1u : 0u);
-                            mma_f16(d, ah, bl, idesc, 1u);
-                            mma_f16(d, al, bh, idesc, 1u);
+                            mma_f16(elected, d, ah, bh, idesc, (kb != kc || kk) ? 1u : 0u);
+                            mma_f16(elected, d, ah, bl, idesc, 1u);
+                            mma_f16(elected, d, al, bh, idesc, 1u);
                         }
-                        mma_commit(&empty[stage]);
+                        if (elected) mma_commit(&empty[stage]);
                         if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
                     }
                     if (!ok) break;
-                    mma_commit(&slot_full[slot]);
+                    if (elected) mma_commit(&slot_full[slot]);
                     if (++slot == kSlots) { slot = 0; sphase ^= 1u; }
                 }
             }
             // every MMA this thread issued has completed before tensor memory is released
-            mma_commit(final_bar);
+            if (elected) mma_commit(final_bar);
             mbar_drain(final_bar, 0);
         }
     } else {
@@ -651,8 +652,9 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_pair(const __grid_constant_
             }
         }
     } else if (warp == 1) {
-        if (leader && lane == 0) {
+        if (leader) {
             // ---- MMA issuer (even CTA): every chunk starts afresh in the next slot of the ring ----
+            const uint32_t elected = elect_one();
             int stage = 0;
             uint32_t phase = 0;
             int slot = 0;
@@ -661,11 +663,11 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_pair(const __grid_constant_
             for (int t = cl; t < n_tiles && ok; t += n_cl) {
                 for (int kc = 0, kc_end = 0; kc < n_kb && ok; kc = kc_end) {
                     kc_end = kc < n_kb0 ? min(kc + args.chunk_kb, n_kb0) : n_kb;
-                    if (!mbar_wait_cluster(&slot_empty[slot], sphase ^ 1u, args.err, 2)) { ok = false; break; }
+                    if (!mbar_wait_cluster_warp(&slot_empty[slot], sphase ^ 1u, args.err, 2)) { ok = false; break; }
                     fence_after_sync();
                     const uint32_t d = tmem_base + static_cast<uint32_t>(slot * kBN);
                     for (int kb = kc; kb < kc_end; ++kb) {
-                        if (!mbar_wait(&full[stage], phase, args.err, 3)) { ok = false; break; }
+                        if (!mbar_wait_warp(&full[stage], phase, args.err, 3)) { ok = false; break; }
                         fence_after_sync();
                         const uint32_t sbase = smem_u32(smem + stage * C::kStageBytes);
 #pragma unroll
@@ -675,19 +677,19 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_pair(const __grid_constant_
                             const uint64_t bh = smem_desc(sbase + 2 * C::kATileBytes, C::kSBO, C::kSwizzle) + 2u * kk;
                             const uint64_t bl =
                                 smem_desc(sbase + 2 * C::kATileBytes + C::kBTileBytes, C::kSBO, C::kSwizzle) + 2u * kk;
-                            mma_f16_pair(d, ah, bh, idesc, (kb != kc || kk) ? 1u : 0u);
-                            mma_f16_pair(d, ah, bl, idesc, 1u);
-                            mma_f16_pair(d, al, bh, idesc, 1u);
+                            mma_f16_pair(elected, d, ah, bh, idesc, (kb != kc || kk) ? 1u : 0u);
+                            mma_f16_pair(elected, d, ah, bl, idesc, 1u);
+                            mma_f16_pair(elected, d, al, bh, idesc, 1u);
                         }
-                        mma_commit_pair(&empty[stage], 3);
+                        if (elected) mma_commit_pair(&empty[stage], 3);
                         if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
                     }
                     if (!ok) break;
-                    mma_commit_pair(&slot_full[slot], 3);
+                    if (elected) mma_commit_pair(&slot_full[slot], 3);
                     if (++slot == kSlots) { slot = 0; sphase ^= 1u; }
                 }
             }
-            mma_commit_pair(final_bar, 3);
+            if (elected) mma_commit_pair(final_bar, 3);
             mbar_drain(final_bar, 0);
         } else if (lane == 0) {
             // odd CTA: its shared and tensor memory stay live until the even CTA's last MMA has completed

@@ -18,17 +18,19 @@
 // ratios exceeds quality_limit(K), and any row that is not finite or whose exponent is out of range, is left to
 // k_marked_f64, which forms those tiles on the FP64 pipe as before.
 //
-// Kernel: persistent, one CTA per SM; tiles of 128 A rows x 64 B rows, 8 levels x 64 columns = all of tensor memory.
-// Warp 0 issues the TMA loads: a stage is 16 deep, 8 x 4 KB + 8 x 2 KB = 48 KB in four boxes of 128-byte rows that hold
-// four planes each, four stages.  Warp 1 issues the 36 MMAs of a stage (M = 128, N = 64, K = 16), warps 2..17 drain the
-// levels; tensor memory is handed back before the outputs are rounded and stored, so only the drain itself (8 x 64
-// columns per 512 terms, 4,300 cycles) interrupts the MMAs.  Shared memory is the bound: an MMA reads 6 KB of operands
-// in at least 48 cycles (32 of tensor work), and with the copies' writes it takes 73; waits for loads and for the
-// epilogue are 7 % (cycle counts around the waits, 1,100 x 4,096 x 995 twice, 743 us).
+// Kernel: persistent CTA pairs; tiles of 256 A rows (128 a CTA) x 64 B rows, 8 levels x 64 columns = all of tensor memory.
+// Warp 0 of each CTA issues its TMA loads: a stage is 16 deep, 8 x 4 KB of its own A rows and 8 x 1 KB of half the B rows =
+// 40 KB in four boxes of 128-byte rows that hold four planes each, five stages.  Warp 1 of the even CTA issues the 36 MMAs
+// of a stage (M = 256, N = 64, K = 16 over both), warps 2..17 drain the levels; tensor memory is handed back before the
+// outputs are rounded and stored, so only the drain itself (8 x 64 columns per 512 terms, 4,300 cycles) interrupts the
+// MMAs.  A pair's MMA reads 5 KB of operands a CTA where a CTA by itself reads 6 for half the work; and see elect_one: with
+// an MMA's operands moved to uniform registers one by one, neither form went below 73 cycles an MMA.  Both products of 660
+// columns x 4,000 variants x 800 samples with 5 covariates: 1.19 -> 0.78 ms (pairs by themselves 1.24).
 #include <cuda.h>
 #include <float.h>
 #include <math.h>
 
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 
@@ -44,9 +46,9 @@ constexpr int kLevels = 8;
 constexpr int kChunk = 512;  // terms of one exact accumulation
 constexpr int kBK = 16;      // depth of one stage: a row's eight planes of 16 elements are 256 bytes, two 128-byte boxes
 constexpr int kRowElems = kOzPlanes * kBK;            // elements of a row in one stage
-constexpr int kABox = kOzRowsA * 128, kBBox = kOzRowsB * 128;
+constexpr int kABox = kOzRowsA * 128, kBBox = kOzRowsB / 2 * 128;
 constexpr int kStageBytes = 2 * (kABox + kBBox);
-constexpr int kStages = 4;
+constexpr int kStages = 5;
 constexpr uint32_t kSBO = 1024;     // bytes between 8-row groups
 constexpr uint32_t kSwizzle128 = 2u;
 constexpr int kTmemCols = kLevels * kOzRowsB;
@@ -68,7 +70,8 @@ struct OzMaps {
 
 struct OzArgs {
     int Ma, Nb, K, batches;
-    int tiles_i, tiles_m;
+    int tiles_i, tiles_m;  // of 128 A rows, of 64 B rows
+    int pairs_i;           // of 256 A rows
     const int* ea;
     const int* eb;
     const float* qa;
@@ -181,12 +184,12 @@ __global__ void k_zero_f32(float* __restrict__ x, int n) {
 
 // ---- the product ------------------------------------------------------------------------------------------------
 
-// Tile t of the schedule: groups of at most kGroup A blocks, inside a group the A block fastest, so that the ~152
+// Tile t of the schedule: groups of at most kGroup pairs of A blocks, inside a group the pair fastest, so that the ~76
 // tiles in flight share few A and B blocks in L2.
-constexpr int kGroup = 12;
+constexpr int kGroup = 6;
 
 struct Tile {
-    int b, ti, tm;
+    int b, ti, tm;  // ti: of 256 A rows in the schedule, of 128 for a CTA
 };
 
 __device__ __forceinline__ Tile tile_at(int t, int tiles_i, int tiles_m) {
@@ -204,7 +207,12 @@ __device__ __forceinline__ Tile tile_at(int t, int tiles_i, int tiles_m) {
 
 __device__ __forceinline__ bool tile_good(const OzArgs& a, const Tile& t) {
     // (an infinite quality makes the product infinite: qualities are at least 1, or 0 for tiles past the rows)
-    return a.qa[t.b * a.tiles_i + t.ti] * a.qb[t.b * a.tiles_m + t.tm] <= a.limit[t.b];
+    return t.ti < a.tiles_i && a.qa[t.b * a.tiles_i + t.ti] * a.qb[t.b * a.tiles_m + t.tm] <= a.limit[t.b];
+}
+
+// The pair's tile: formed if either half is good (digits of rows that are not finite are zeros).
+__device__ __forceinline__ bool pair_good(const OzArgs& a, const Tile& t) {
+    return tile_good(a, Tile{t.b, 2 * t.ti, t.tm}) || tile_good(a, Tile{t.b, 2 * t.ti + 1, t.tm});
 }
 
 // Descriptors differ in their low words only (the tile's address in 16-byte units): plane t lies in box t / 4, 32 bytes
@@ -214,31 +222,34 @@ __device__ __forceinline__ uint64_t plane_desc(uint32_t lo, uint32_t hi) {
 }
 
 template <int I, int J>
-__device__ __forceinline__ void mma_pair(uint32_t tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t acc0,
-                                         uint32_t idesc) {
-    mma_f16(tmem + static_cast<uint32_t>((I + J) * kOzRowsB),
+__device__ __forceinline__ void mma_pair(uint32_t elected, uint32_t tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi,
+                                         uint32_t acc0, uint32_t idesc) {
+    mma_f16_pair(elected, tmem + static_cast<uint32_t>((I + J) * kOzRowsB),
             plane_desc(a_lo + (I / 4) * (kABox / 16) + 2 * (I % 4), hi),
             plane_desc(b_lo + (J / 4) * (kBBox / 16) + 2 * (J % 4), hi), idesc, I == 0 ? acc0 : 1u);
-    if constexpr (J < kLevels - 1 - I) mma_pair<I, J + 1>(tmem, a_lo, b_lo, hi, acc0, idesc);
-    else if constexpr (I < kOzPlanes - 1) mma_pair<I + 1, 0>(tmem, a_lo, b_lo, hi, acc0, idesc);
+    if constexpr (J < kLevels - 1 - I) mma_pair<I, J + 1>(elected, tmem, a_lo, b_lo, hi, acc0, idesc);
+    else if constexpr (I < kOzPlanes - 1) mma_pair<I + 1, 0>(elected, tmem, a_lo, b_lo, hi, acc0, idesc);
 }
 
 __global__ void __launch_bounds__(kThreads, 1) k_oz64(const __grid_constant__ OzMaps maps, const OzArgs args) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023u)) & 1023u);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStages * kStageBytes);
-    uint64_t* full = bars;                  // [kStages]
+    uint64_t* full = bars;                  // [kStages], used in the even CTA
     uint64_t* empty = bars + kStages;       // [kStages]
     uint64_t* acc_full = empty + kStages;   // chunk accumulated (MMA -> epilogue)
-    uint64_t* acc_empty = acc_full + 1;     // chunk drained (epilogue -> MMA)
+    uint64_t* acc_empty = acc_full + 1;     // chunk drained (both epilogues -> MMA), used in the even CTA
     uint64_t* final_bar = acc_empty + 1;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(final_bar + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n_tiles = args.batches * args.tiles_i * args.tiles_m;
+    const uint32_t rank = cluster_ctarank();
+    const bool leader = rank == 0;
+    const int cl = static_cast<int>(cluster_id_x()), n_cl = static_cast<int>(cluster_count_x());
+    const int n_tiles = args.batches * args.pairs_i * args.tiles_m;
     const int n_kb = (args.K + kBK - 1) / kBK;
     constexpr int kChunkKb = kChunk / kBK;
-    constexpr uint32_t idesc = idesc_f16_f32(kOzRowsA, kOzRowsB);
+    constexpr uint32_t idesc = idesc_f16_f32(2 * kOzRowsA, kOzRowsB);
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
@@ -246,7 +257,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz64(const __grid_constant__ Oz
             mbar_init(&empty[s], 1);
         }
         mbar_init(acc_full, 1);
-        mbar_init(acc_empty, kEpiWarps);
+        mbar_init(acc_empty, 2 * kEpiWarps);
         mbar_init(final_bar, 1);
         fence_barrier_init();
     }
@@ -255,71 +266,87 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz64(const __grid_constant__ Oz
         tma_prefetch_desc(&maps.b);
     }
     if (warp == 1) {
-        tmem_alloc(tmem_slot, kTmemCols);
-        tmem_relinquish();
+        tmem_alloc_pair(tmem_slot, kTmemCols);
+        tmem_relinquish_pair();
     }
     fence_before_sync();
-    __syncthreads();
+    __syncwarp();
+    cluster_sync();  // barriers initialised and tensor memory allocated in both CTAs
     fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0) {
         if (lane == 0) {
+            const uint32_t full0 = map_to_rank(smem_u32(full), 0);
             int stage = 0;
             uint32_t phase = 0;
             bool armed[kStages] = {};
             uint32_t armed_phase[kStages] = {};
             bool ok = true;
-            for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
-                const Tile tl = tile_at(t, args.tiles_i, args.tiles_m);
-                if (!tile_good(args, tl)) continue;
-                const int ya = tl.b * args.Ma + tl.ti * kOzRowsA, yb = tl.b * args.Nb + tl.tm * kOzRowsB;
+            for (int t = cl; t < n_tiles && ok; t += n_cl) {
+                const Tile tl = tile_at(t, args.pairs_i, args.tiles_m);
+                if (!pair_good(args, tl)) continue;
+                const int ya = tl.b * args.Ma + (2 * tl.ti + static_cast<int>(rank)) * kOzRowsA;
+                const int yb = tl.b * args.Nb + tl.tm * kOzRowsB + static_cast<int>(rank) * (kOzRowsB / 2);
                 for (int kb = 0; kb < n_kb; ++kb) {
                     if (!mbar_wait(&empty[stage], phase ^ 1u, args.err, 21)) { ok = false; break; }
-                    mbar_arrive_expect_tx(&full[stage], kStageBytes);
-                    armed[stage] = true;
-                    armed_phase[stage] = phase;
+                    if (leader) {
+                        mbar_arrive_expect_tx(&full[stage], 2 * kStageBytes);
+                        armed[stage] = true;
+                        armed_phase[stage] = phase;
+                    }
+                    const uint32_t bar = full0 + static_cast<uint32_t>(stage * 8);
                     uint8_t* base = smem + stage * kStageBytes;
                     const int x = kb * kRowElems;
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
-                        tma_load_2d(base + h * kABox, &maps.a, x + h * (kRowElems / 2), ya, &full[stage]);
-                        tma_load_2d(base + 2 * kABox + h * kBBox, &maps.b, x + h * (kRowElems / 2), yb, &full[stage]);
+                        tma_load_2d_pair(base + h * kABox, &maps.a, x + h * (kRowElems / 2), ya, bar);
+                        tma_load_2d_pair(base + 2 * kABox + h * kBBox, &maps.b, x + h * (kRowElems / 2), yb, bar);
                     }
                     if (++stage == kStages) { stage = 0; phase ^= 1u; }
                 }
             }
-            for (int s = 0; s < kStages; ++s)
-                if (armed[s]) mbar_drain(&full[s], armed_phase[s]);
+            if (leader) {
+                // the pair's copies of every armed phase have landed before the CTAs leave
+                for (int s = 0; s < kStages; ++s)
+                    if (armed[s]) mbar_drain(&full[s], armed_phase[s]);
+            } else if (*reinterpret_cast<volatile int*>(args.err) != 0) {
+                // the even CTA may have stopped waiting on this CTA's last copies: give them time to land
+                for (int i = 0; i < 100; ++i) __nanosleep(1000);
+            }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (leader) {
+            const uint32_t elected = elect_one();
             int stage = 0;
             uint32_t phase = 0, tphase = 0;
             bool ok = true;
-            for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
-                if (!tile_good(args, tile_at(t, args.tiles_i, args.tiles_m))) continue;
+            for (int t = cl; t < n_tiles && ok; t += n_cl) {
+                if (!pair_good(args, tile_at(t, args.pairs_i, args.tiles_m))) continue;
                 for (int kb = 0; kb < n_kb && ok; ++kb) {
                     const bool first = kb % kChunkKb == 0;
                     if (first) {
-                        if (!mbar_wait(acc_empty, tphase ^ 1u, args.err, 22)) { ok = false; break; }
+                        if (!mbar_wait_cluster_warp(acc_empty, tphase ^ 1u, args.err, 22)) { ok = false; break; }
                         fence_after_sync();
                     }
-                    if (!mbar_wait(&full[stage], phase, args.err, 23)) { ok = false; break; }
+                    if (!mbar_wait_warp(&full[stage], phase, args.err, 23)) { ok = false; break; }
                     fence_after_sync();
                     const uint64_t d0 = smem_desc(smem_u32(smem + stage * kStageBytes), kSBO, kSwizzle128);
                     const uint32_t lo = static_cast<uint32_t>(d0);
-                    mma_pair<0, 0>(tmem_base, lo, lo + 2 * (kABox / 16), static_cast<uint32_t>(d0 >> 32), first ? 0u : 1u,
+                    mma_pair<0, 0>(elected, tmem_base, lo, lo + 2 * (kABox / 16), static_cast<uint32_t>(d0 >> 32), first ? 0u : 1u,
                                    idesc);
-                    mma_commit(&empty[stage]);
+                    if (elected) mma_commit_pair(&empty[stage], 3);
                     if (++stage == kStages) { stage = 0; phase ^= 1u; }
                     if ((kb + 1) % kChunkKb == 0 || kb + 1 == n_kb) {
-                        mma_commit(acc_full);
+                        if (elected) mma_commit_pair(acc_full, 3);
                         tphase ^= 1u;
                     }
                 }
             }
-            mma_commit(final_bar);
+            if (elected) mma_commit_pair(final_bar, 3);
+            mbar_drain(final_bar, 0);
+        } else if (lane == 0) {
+            // odd CTA: its shared and tensor memory stay live until the even CTA's last MMA has completed
             mbar_drain(final_bar, 0);
         }
     } else {
@@ -328,16 +355,18 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz64(const __grid_constant__ Oz
         const int q = warp & 3;
         const int c0 = ((warp - 2) >> 2) * kEpiCols;
         const uint32_t tl0 = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(c0);
+        const uint32_t acc_empty0 = map_to_rank(smem_u32(acc_empty), 0);
         uint32_t tphase = 0;
         bool ok = true;
-        for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
-            const Tile tl = tile_at(t, args.tiles_i, args.tiles_m);
-            if (!tile_good(args, tl)) continue;
+        for (int t = cl; t < n_tiles && ok; t += n_cl) {
+            const Tile tl = tile_at(t, args.pairs_i, args.tiles_m);
+            if (!pair_good(args, tl)) continue;
             long long hi[kEpiCols], lo[kEpiCols];
 #pragma unroll
             for (int c = 0; c < kEpiCols; ++c) hi[c] = lo[c] = 0;
             for (int kb = 0; kb < n_kb; kb += kChunkKb) {
-                if (!mbar_wait(acc_full, tphase, args.err, 24)) { ok = false; break; }
+                const bool got = mbar_wait(acc_full, tphase, args.err, 24);
+                if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
                 fence_after_sync();
                 float v[kEpiCols];
 #pragma unroll
@@ -356,12 +385,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz64(const __grid_constant__ Oz
                 }
                 fence_before_sync();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(acc_empty);
+                if (lane == 0) mbar_arrive_cluster_relaxed(acc_empty0);
                 tphase ^= 1u;
             }
             if (!ok) break;
-            const int i = tl.ti * kOzRowsA + q * 32 + lane;
-            if (i < args.Ma) {
+            const Tile half{tl.b, 2 * tl.ti + static_cast<int>(rank), tl.tm};
+            const int i = half.ti * kOzRowsA + q * 32 + lane;
+            if (i < args.Ma && tile_good(args, half)) {
                 const int ea = args.ea[tl.b * args.Ma + i];
                 const int m0 = tl.tm * kOzRowsB + c0;
                 const int* eb = args.eb + tl.b * args.Nb + m0;
@@ -380,10 +410,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz64(const __grid_constant__ Oz
     }
 
     fence_before_sync();
-    __syncthreads();
+    __syncwarp();
+    cluster_sync();  // no CTA leaves while its peer may still signal its barriers or read its operands
     if (warp == 1) {
         fence_after_sync();
-        tmem_dealloc(tmem_base, kTmemCols);
+        tmem_dealloc_pair(tmem_base, kTmemCols);
     }
 }
 
@@ -506,16 +537,11 @@ int oz_gemm(const OzOperand& A, const OzOperand& B, const OzProduct& p, cudaStre
     int rc;
     const int w = static_cast<int>(A.ldp);
     if ((rc = tc::make_map_f16(&maps.a, A.planes, static_cast<int>(ra), w, A.ldp, kRowElems / 2, kOzRowsA))) return rc;
-    if ((rc = tc::make_map_f16(&maps.b, B.planes, static_cast<int>(rb), w, B.ldp, kRowElems / 2, kOzRowsB))) return rc;
-    static std::once_flag once;
-    static cudaError_t attr_rc = cudaSuccess;
-    std::call_once(once, [] {
-        attr_rc = cudaFuncSetAttribute(k_oz64, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-    });
-    if (attr_rc != cudaSuccess) return fail(FLMM_ERR_CUDA, "k_oz64: %s", cudaGetErrorString(attr_rc));
-    int dev = 0, sm = 0;
+    if ((rc = tc::make_map_f16(&maps.b, B.planes, static_cast<int>(rb), w, B.ldp, kRowElems / 2, kOzRowsB / 2))) return rc;
+    static PairCache cache;
+    int dev = 0, pairs = 0;
     FLMM_CUDA(cudaGetDevice(&dev));
-    FLMM_CUDA(cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev));
+    if ((rc = pair_count(k_oz64, kThreads, kSmemBytes, cache, &pairs))) return rc;
     OzArgs a{};
     a.err = device_err_flag(dev);
     if (!a.err) return fail(FLMM_ERR_CUDA, "oz_gemm: cannot allocate the device error flag");
@@ -525,6 +551,7 @@ int oz_gemm(const OzOperand& A, const OzOperand& B, const OzProduct& p, cudaStre
     a.batches = A.batches < B.batches ? A.batches : B.batches;
     a.tiles_i = A.tiles();
     a.tiles_m = B.tiles();
+    a.pairs_i = (a.tiles_i + 1) / 2;
     a.ea = A.expo;
     a.eb = B.expo;
     a.qa = A.qual;
@@ -537,8 +564,8 @@ int oz_gemm(const OzOperand& A, const OzOperand& B, const OzProduct& p, cudaStre
     a.c_stride = p.c_stride;
     a.D = p.D;
     a.ldd = p.ldd;
-    const int64_t tiles = static_cast<int64_t>(a.batches) * a.tiles_i * a.tiles_m;
-    k_oz64<<<static_cast<int>(tiles < sm ? tiles : sm), kThreads, kSmemBytes, st>>>(maps, a);
+    const int64_t tiles = static_cast<int64_t>(a.batches) * a.pairs_i * a.tiles_m;
+    if ((rc = launch_pairs(k_oz64, static_cast<int>(std::min<int64_t>(tiles, pairs)), kThreads, kSmemBytes, st, maps, a))) return rc;
     if ((rc = check_launch("k_oz64"))) return rc;
     const dim3 grid(ceil_div(B.rows, kST), ceil_div(A.rows, kST), a.batches);
     k_marked_f64<<<grid, kSThreads, 0, st>>>(a, p.Xa, p.lda, p.xa_stride, p.Xb, p.ldb, p.square[0], p.square[1]);

@@ -16,26 +16,27 @@
 // rounded U~, which the refinement then uses in place of U (it is an equally good iterate, and the residuals must
 // belong to the vectors they correct).  A (FP64) takes 7 planes (48 bits).  Plane pairs (i, j) of equal level
 // l = i + j carry the same weight 2^(-7 l) and share one accumulator in tensor memory; levels 0..7 are kept (25
-// pairs; the first dropped level weighs 2^-56).  Levels 0..3 are exact by the bound above; levels 4..7 weigh at
-// most 2^-28 and round at 2^-18 of themselves over 1,024 terms.  The leading digits of most elements are small
+// pairs; the first dropped level weighs 2^-56).  No level has more than four pairs, so all are exact by the bound above.
+// The leading digits of most elements are small
 // (off-diagonal kinship entries and most eigenvector entries lie well below their row's maximum), so the
 // lower levels carry more than their nominal weight: on a 600 x 600 kinship-like test the product's error was
 // 1.3e-14 of sum |u||a| with eight levels and 8e-14 with seven, against 3.2e-13 for double-FP32.  Per output,
 //     W = 2^(e_i + e_m - 12) sum_l 2^(-7 l) C_l
-// is combined in double-FP32 (TwoSum) and stored in FP64.  Reductions longer than 1,024 run as several launches
-// that add into W.
+// is combined in double-FP32 (TwoSum) and stored in FP64; of reductions longer than 1,024 the chunks' W are added.
 //
-// Kernel: persistent, one CTA per SM, 320 threads -- warp 0 issues the TMA loads (per 32-deep k-block the 4 U
-// planes of 128 rows and the 7 A planes of 64 rows, 60 KB, three stages), warp 1 owns tensor memory and issues the
-// 50 MMAs of a k-block (M = 128, N = 64, K = 16, kind::f16), warps 2..9 combine the 8 level accumulators of a tile
-// (all 512 columns) and store it.  Tiles are (matrix, 128 U rows, 64 A rows).
+// Kernel: persistent CTA pairs -- warp 0 of each CTA issues its TMA loads (per 32-deep k-block the U planes of its 128 rows
+// and the A planes of half the tile's A rows), warp 1 of the even CTA the MMAs of the pair (M = 256, N = 64 to 128, K = 16,
+// kind::f16; 50 of a k-block for the product), warps 2..17 combine the level accumulators of a tile and store it.  Tiles
+// are (matrix, 256 U rows, 64 to 128 A rows).  The 12 refinement steps of 1,057 to 1,600 rows, 8 matrices each, with 4 x 7,
+// 3 x 3 and 4 x 4 planes: 17.4, 7.6 and 10.5 ms with single CTAs, a launch per 1,024 terms, an MMA's operands moved to
+// uniform registers one by one, and outputs stored (and read again) by lanes that went down a column; 11.8, 2.6 and 4.5 here.
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <math.h>
 
-#include <cstdlib>
+#include <algorithm>
 #include <cstring>
-#include <mutex>
+#include <type_traits>
 
 #include "flmm_common.cuh"
 #include "flmm_tc.cuh"
@@ -46,25 +47,32 @@ using namespace flmm::tc;
 namespace {
 
 constexpr int kDigitShift = 7;    // bits per digit below the first
-constexpr int kMaxChunk = 1024;   // reduction of one launch (exact accumulation bound)
+constexpr int kMaxChunk = 1024;   // reduction of one exact accumulation (four pairs of 12-bit products a level)
 constexpr int kBM = 128;          // A-side rows per tile (TMEM lanes)
-constexpr int kBN = 64;           // B-side rows per tile (columns of one level accumulator)
 constexpr int kBK = 32;           // reduction depth of one stage (64-byte rows, 64-byte swizzle)
 constexpr int kATile = kBM * kBK * 2;                                   // 8 KB: one A-side plane
-constexpr int kBTile = kBN * kBK * 2;                                   // 4 KB: one B-side plane
 constexpr uint32_t kSBO = 8u * kBK * 2u;                                // bytes between 8-row groups
 constexpr uint32_t kSwizzle64 = 4u;
-constexpr int kThreads = 320;
-constexpr int kEpilogueThreads = 256;
 
-// One configuration of the digit-plane product: PA planes on the A side (128 rows per tile), PB on the B side (64),
-// levels 0 .. LV - 1 kept, FP64 output (the refinement's A U) or FP32 output (its corrections).
+// One configuration of the digit-plane product: PA planes on the A side (256 rows per tile, 128 a CTA), PB on the B side,
+// levels 0 .. LV - 1 kept, FP64 output (the refinement's A U) or FP32 output (its corrections).  A tile has as many B rows
+// as tensor memory holds columns per level: with few planes the copies would otherwise be the bound (a stage of 3 + 3
+// planes is 30 KB for 540 cycles of MMAs at 64 rows, 36 KB for 770 at 128).
 template <int PA, int PB, int LV, bool F64>
 struct OzCfg {
+    static constexpr int kBN = LV <= 4 ? 128 : (LV == 5 ? 96 : 64);
+    static constexpr int kBTile = kBN / 2 * kBK * 2;  // a CTA's half of one B-side plane
     static constexpr int kStageBytes = PA * kATile + PB * kBTile;
-    static constexpr int kStages = (192 * 1024) / kStageBytes < 4 ? (192 * 1024) / kStageBytes : 4;
-    static constexpr int kTmemCols = LV * kBN <= 256 ? 256 : 512;
-    static constexpr int kSmemBytes = kStages * kStageBytes + 256 + 1024;
+    // (8 warps have the registers for FP64 sums over several chunks)
+    static constexpr int kEpiWarps = F64 ? 8 : 16;
+    static constexpr int kThreads = 64 + 32 * kEpiWarps;
+    // a warp's 32 rows of 16 outputs pass through shared memory on their way out, one padding entry a row
+    static constexpr int kOutBytes = 32 * 17 * (F64 ? 8 : 4);
+    static constexpr int kFixedBytes = kEpiWarps * kOutBytes + 256 + 1024;
+    static constexpr int kFit = (227 * 1024 - kFixedBytes) / kStageBytes;
+    static constexpr int kStages = kFit < 4 ? kFit : 4;
+    static constexpr int kTmemCols = 512;
+    static constexpr int kSmemBytes = kStages * kStageBytes + kFixedBytes;
     static_assert(LV * kBN <= kTmemCols && kTmemCols <= 512, "tensor memory budget");
     static_assert(kStages >= 2, "pipeline depth");
     static_assert(kSmemBytes <= 227 * 1024, "shared memory budget");
@@ -83,13 +91,11 @@ struct OzMaps {
 
 struct OzArgs {
     int N, batch;
-    int k0, klen;        // reduction range of this launch
     const int* eU;       // (batch N) row exponents of the A side
     const int* eA;       // (batch N) row exponents of the B side
     double* W;           // (batch, N, N), FP64 output
     float* C;            // (batch, N, N), FP32 output
     const float* D;      // (batch, N, N) added to the FP32 output, or null
-    int accumulate;      // add into the output (launches after the first)
     int* err;
 };
 
@@ -166,28 +172,34 @@ __global__ void k_digits_a(const double* __restrict__ A, int64_t rows, int N, __
 // ---- the tensor-core product ----------------------------------------------------------------------------------
 
 template <int PA, int PB, int LV, bool F64>
-__global__ void __launch_bounds__(kThreads, 1) k_ozaki(const __grid_constant__ OzMaps maps, const OzArgs args) {
+__global__ void __launch_bounds__(OzCfg<PA, PB, LV, F64>::kThreads, 1) k_ozaki(const __grid_constant__ OzMaps maps, const OzArgs args) {
     using Cfg = OzCfg<PA, PB, LV, F64>;
+    constexpr int kBN = Cfg::kBN, kBTile = Cfg::kBTile, kEpiWarps = Cfg::kEpiWarps;
     constexpr int kStages = Cfg::kStages;
     constexpr int kStageBytes = Cfg::kStageBytes;
     constexpr int kTmemCols = Cfg::kTmemCols;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023u)) & 1023u);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStages * kStageBytes);
-    uint64_t* full = bars;                  // [kStages]
+    uint64_t* full = bars;                  // [kStages], used in the even CTA
     uint64_t* empty = bars + kStages;       // [kStages]
     uint64_t* acc_full = empty + kStages;   // tile accumulated (MMA -> epilogue)
-    uint64_t* acc_empty = acc_full + 1;     // tile combined (epilogue -> MMA)
+    uint64_t* acc_empty = acc_full + 1;     // tile combined (both epilogues -> MMA), used in the even CTA
     uint64_t* final_bar = acc_empty + 1;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(final_bar + 1);
+    uint8_t* out_smem = smem + kStages * kStageBytes + 256;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_ctarank();
+    const bool leader = rank == 0;
+    const int cl = static_cast<int>(cluster_id_x()), n_cl = static_cast<int>(cluster_count_x());
     const int N = args.N;
-    const int tiles_i = (N + kBM - 1) / kBM, tiles_m = (N + kBN - 1) / kBN;
+    const int tiles_i = (N + 2 * kBM - 1) / (2 * kBM), tiles_m = (N + kBN - 1) / kBN;
     const int per = tiles_i * tiles_m;
     const int n_tiles = args.batch * per;
-    const int n_kb = (args.klen + kBK - 1) / kBK;
-    constexpr uint32_t idesc = idesc_f16_f32(kBM, kBN);
+    const int n_kb = (N + kBK - 1) / kBK;
+    constexpr int kChunkKb = kMaxChunk / kBK;
+    constexpr uint32_t idesc = idesc_f16_f32(2 * kBM, kBN);
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
@@ -195,7 +207,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_ozaki(const __grid_constant__ O
             mbar_init(&empty[s], 1);
         }
         mbar_init(acc_full, 1);
-        mbar_init(acc_empty, kEpilogueThreads);
+        mbar_init(acc_empty, 2 * kEpiWarps);
         mbar_init(final_bar, 1);
         fence_barrier_init();
     }
@@ -204,58 +216,74 @@ __global__ void __launch_bounds__(kThreads, 1) k_ozaki(const __grid_constant__ O
         tma_prefetch_desc(&maps.a);
     }
     if (warp == 1) {
-        tmem_alloc(tmem_slot, kTmemCols);
-        tmem_relinquish();
+        tmem_alloc_pair(tmem_slot, kTmemCols);
+        tmem_relinquish_pair();
     }
     fence_before_sync();
-    __syncthreads();
+    __syncwarp();
+    cluster_sync();  // barriers initialised and tensor memory allocated in both CTAs
     fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0) {
         // ---- TMA producer ----
         if (lane == 0) {
+            const uint32_t full0 = map_to_rank(smem_u32(full), 0);
             int stage = 0;
             uint32_t phase = 0;
             bool armed[kStages] = {};
             uint32_t armed_phase[kStages] = {};
             bool ok = true;
-            for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
+            for (int t = cl; t < n_tiles && ok; t += n_cl) {
                 const int b = t / per, rem = t - b * per;
                 const int ti = rem / tiles_m, tm = rem - ti * tiles_m;
                 for (int kb = 0; kb < n_kb; ++kb) {
                     if (!mbar_wait(&empty[stage], phase ^ 1u, args.err, 11)) { ok = false; break; }
-                    mbar_arrive_expect_tx(&full[stage], kStageBytes);
-                    armed[stage] = true;
-                    armed_phase[stage] = phase;
+                    if (leader) {
+                        mbar_arrive_expect_tx(&full[stage], 2 * kStageBytes);
+                        armed[stage] = true;
+                        armed_phase[stage] = phase;
+                    }
+                    const uint32_t bar = full0 + static_cast<uint32_t>(stage * 8);
                     uint8_t* base = smem + stage * kStageBytes;
-                    const int x = args.k0 + kb * kBK;
+                    const int x = kb * kBK;
 #pragma unroll
                     for (int p = 0; p < PA; ++p)
-                        tma_load_2d(base + p * kATile, &maps.u, x, (p * args.batch + b) * N + ti * kBM, &full[stage]);
+                        tma_load_2d_pair(base + p * kATile, &maps.u, x,
+                                         (p * args.batch + b) * N + (2 * ti + static_cast<int>(rank)) * kBM, bar);
 #pragma unroll
                     for (int p = 0; p < PB; ++p)
-                        tma_load_2d(base + PA * kATile + p * kBTile, &maps.a, x,
-                                    (p * args.batch + b) * N + tm * kBN, &full[stage]);
+                        tma_load_2d_pair(base + PA * kATile + p * kBTile, &maps.a, x,
+                                         (p * args.batch + b) * N + tm * kBN + static_cast<int>(rank) * (kBN / 2), bar);
                     if (++stage == kStages) { stage = 0; phase ^= 1u; }
                 }
             }
-            for (int s = 0; s < kStages; ++s)
-                if (armed[s]) mbar_drain(&full[s], armed_phase[s]);
+            if (leader) {
+                // the pair's copies of every armed phase have landed before the CTAs leave
+                for (int s = 0; s < kStages; ++s)
+                    if (armed[s]) mbar_drain(&full[s], armed_phase[s]);
+            } else if (*reinterpret_cast<volatile int*>(args.err) != 0) {
+                // the even CTA may have stopped waiting on this CTA's last copies: give them time to land
+                for (int i = 0; i < 100; ++i) __nanosleep(1000);
+            }
         }
     } else if (warp == 1) {
         // ---- MMA issuer: the plane pairs (i, j) with i + j < LV of every 16-deep step, each into its level's
         // accumulator ----
-        if (lane == 0) {
+        if (leader) {
+            const uint32_t elected = elect_one();
             int stage = 0;
             uint32_t phase = 0;
             uint32_t tphase = 0;
             bool ok = true;
-            for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
-                if (!mbar_wait(acc_empty, tphase ^ 1u, args.err, 12)) break;
-                fence_after_sync();
+            for (int t = cl; t < n_tiles && ok; t += n_cl) {
                 for (int kb = 0; kb < n_kb; ++kb) {
-                    if (!mbar_wait(&full[stage], phase, args.err, 13)) { ok = false; break; }
+                    const bool first = kb % kChunkKb == 0;
+                    if (first) {
+                        if (!mbar_wait_cluster_warp(acc_empty, tphase ^ 1u, args.err, 12)) { ok = false; break; }
+                        fence_after_sync();
+                    }
+                    if (!mbar_wait_warp(&full[stage], phase, args.err, 13)) { ok = false; break; }
                     fence_after_sync();
                     const uint32_t sbase = smem_u32(smem + stage * kStageBytes);
 #pragma unroll
@@ -270,105 +298,153 @@ __global__ void __launch_bounds__(kThreads, 1) k_ozaki(const __grid_constant__ O
                                 const uint64_t ad = smem_desc(sbase + i * kATile, kSBO, kSwizzle64) + 2u * kk;
                                 const uint64_t bd =
                                     smem_desc(sbase + PA * kATile + j * kBTile, kSBO, kSwizzle64) + 2u * kk;
-                                const uint32_t acc = (kb > 0 || kk > 0 || i > i_lo) ? 1u : 0u;
-                                mma_f16(tmem_base + static_cast<uint32_t>(l * kBN), ad, bd, idesc, acc);
+                                const uint32_t acc = (!first || kk > 0 || i > i_lo) ? 1u : 0u;
+                                mma_f16_pair(elected, tmem_base + static_cast<uint32_t>(l * kBN), ad, bd, idesc, acc);
                             }
                         }
                     }
-                    mma_commit(&empty[stage]);
+                    if (elected) mma_commit_pair(&empty[stage], 3);
                     if (++stage == kStages) { stage = 0; phase ^= 1u; }
+                    if ((kb + 1) % kChunkKb == 0 || kb + 1 == n_kb) {
+                        if (elected) mma_commit_pair(acc_full, 3);
+                        tphase ^= 1u;
+                    }
                 }
-                if (!ok) break;
-                mma_commit(acc_full);
-                tphase ^= 1u;
             }
-            mma_commit(final_bar);
+            if (elected) mma_commit_pair(final_bar, 3);
+            mbar_drain(final_bar, 0);
+        } else if (lane == 0) {
+            // odd CTA: its shared and tensor memory stay live until the even CTA's last MMA has completed
             mbar_drain(final_bar, 0);
         }
     } else {
-        // ---- epilogue: warp w reads TMEM lanes 32 (w % 4) .. +31 (thread = one U row) and half (w - 2) / 4 of the
-        // tile's 64 columns, in two groups of 16 ----
+        // ---- epilogue: warp w reads TMEM lanes 32 (w % 4) .. +31 (thread = one U row of this CTA's half) and groups
+        // (w - 2) / 4, + kStep, ... of 16 columns of the tile; what it adds and stores passes through shared memory, so that
+        // lanes go along the rows of global memory ----
+        using Out = typename std::conditional<F64, double, float>::type;
+        constexpr int kStep = kEpiWarps / 4, kGroups = (kBN / 16 + kStep - 1) / kStep;
         const int q = warp & 3;
-        const int half = (warp - 2) >> 2;
-        const int r = q * 32 + lane;
-        const uint32_t tl0 =
-            tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(half * (kBN / 2));
+        const int g0 = (warp - 2) >> 2;
+        const uint32_t tl0 = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
+        const uint32_t acc_empty0 = map_to_rank(smem_u32(acc_empty), 0);
+        Out* buf = reinterpret_cast<Out*>(out_smem + (warp - 2) * Cfg::kOutBytes);
         uint32_t tphase = 0;
-        for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
-            if (!mbar_wait(acc_full, tphase, args.err, 14)) break;
-            fence_after_sync();
+        bool ok = true;
+        for (int t = cl; t < n_tiles && ok; t += n_cl) {
             const int b = t / per, rem = t - b * per;
             const int ti = rem / tiles_m, tm = rem - ti * tiles_m;
-            const int i = ti * kBM + r;
-            const bool row_ok = i < N;
-            const int eu = row_ok ? args.eU[static_cast<int64_t>(b) * N + i] : 0;
-            const int64_t orow = (static_cast<int64_t>(b) * N + (row_ok ? i : 0)) * N;
-#pragma unroll 1
-            for (int g = 0; g < 2; ++g) {
-                const int c0 = tm * kBN + half * (kBN / 2) + g * 16;
-                const uint32_t ta = tl0 + static_cast<uint32_t>(g * 16);
-                float hi[16], lo[16], v[16];
-                if constexpr (F64) {
-                    // double-FP32 sum of the levels, stored in FP64
-                    tmem_ld16_wait(ta, hi);
+            const int row0 = (2 * ti + static_cast<int>(rank)) * kBM + q * 32;
+            const int eu = row0 + lane < N ? args.eU[static_cast<int64_t>(b) * N + row0 + lane] : 0;
+            const int64_t at = static_cast<int64_t>(b) * N * N;
+            Out acc[kGroups][16] = {};
+            bool add = !F64 && args.D != nullptr;
+            if constexpr (!F64) {
+                if (add) {
 #pragma unroll
-                    for (int c = 0; c < 16; ++c) lo[c] = 0.0f;
+                    for (int gi = 0; gi < kGroups; ++gi) {
+                        const int c0 = tm * kBN + (g0 + kStep * gi) * 16;
+                        __syncwarp();
 #pragma unroll
-                    for (int l = 1; l < LV; ++l) {
-                        tmem_ld16_wait(ta + static_cast<uint32_t>(l * kBN), v);
-                        const float w = ldexpf(1.0f, -kDigitShift * l);
-#pragma unroll
-                        for (int c = 0; c < 16; ++c) {
-                            float s, err;
-                            two_sum(hi[c], v[c] * w, s, err);
-                            hi[c] = s;
-                            lo[c] += err;
+                        for (int u = 0; u < 16; ++u) {
+                            const int rr = 2 * u + lane / 16, c = lane % 16;
+                            const bool in = row0 + rr < N && c0 + c < N && g0 + kStep * gi < kBN / 16;
+                            buf[rr * 17 + c] = in ? args.D[at + static_cast<int64_t>(row0 + rr) * N + c0 + c] : 0.0f;
                         }
-                    }
-                } else {
-                    // FP32 sum of the levels, smallest first
-                    tmem_ld16_wait(ta + static_cast<uint32_t>((LV - 1) * kBN), hi);
-                    const float wl = ldexpf(1.0f, -kDigitShift * (LV - 1));
+                        __syncwarp();
 #pragma unroll
-                    for (int c = 0; c < 16; ++c) hi[c] *= wl;
-#pragma unroll
-                    for (int l = LV - 2; l >= 0; --l) {
-                        tmem_ld16_wait(ta + static_cast<uint32_t>(l * kBN), v);
-                        const float w = ldexpf(1.0f, -kDigitShift * l);
-#pragma unroll
-                        for (int c = 0; c < 16; ++c) hi[c] = fmaf(v[c], w, hi[c]);
-                    }
-                }
-                if (row_ok) {
-#pragma unroll
-                    for (int c = 0; c < 16; ++c) {
-                        const int m = c0 + c;
-                        if (m < N) {
-                            const int ex = eu + args.eA[static_cast<int64_t>(b) * N + m] - 12;
-                            if constexpr (F64) {
-                                const double x = ldexp(static_cast<double>(hi[c]) + static_cast<double>(lo[c]), ex);
-                                args.W[orow + m] = args.accumulate ? args.W[orow + m] + x : x;
-                            } else {
-                                float x = ldexpf(hi[c], ex);
-                                if (args.accumulate) x += args.C[orow + m];
-                                else if (args.D) x += args.D[orow + m];
-                                args.C[orow + m] = x;
-                            }
-                        }
+                        for (int c = 0; c < 16; ++c) acc[gi][c] = buf[lane * 17 + c];
                     }
                 }
             }
-            fence_before_sync();
-            mbar_arrive(acc_empty);
-            tphase ^= 1u;
+            for (int kb = 0; kb < n_kb; kb += kChunkKb) {
+                const bool got = mbar_wait(acc_full, tphase, args.err, 14);
+                if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
+                fence_after_sync();
+#pragma unroll
+                for (int gi = 0; gi < kGroups; ++gi) {
+                    if (g0 + kStep * gi >= kBN / 16) continue;
+                    const int c0 = tm * kBN + (g0 + kStep * gi) * 16;
+                    const uint32_t ta = tl0 + static_cast<uint32_t>((g0 + kStep * gi) * 16);
+                    float hi[16], lo[16], v[16];
+                    if constexpr (F64) {
+                        // double-FP32 sum of the levels, stored in FP64
+                        tmem_ld16_wait(ta, hi);
+#pragma unroll
+                        for (int c = 0; c < 16; ++c) lo[c] = 0.0f;
+#pragma unroll
+                        for (int l = 1; l < LV; ++l) {
+                            tmem_ld16_wait(ta + static_cast<uint32_t>(l * kBN), v);
+                            const float w = ldexpf(1.0f, -kDigitShift * l);
+#pragma unroll
+                            for (int c = 0; c < 16; ++c) {
+                                float s, err;
+                                two_sum(hi[c], v[c] * w, s, err);
+                                hi[c] = s;
+                                lo[c] += err;
+                            }
+                        }
+                    } else {
+                        // FP32 sum of the levels, smallest first
+                        tmem_ld16_wait(ta + static_cast<uint32_t>((LV - 1) * kBN), hi);
+                        const float wl = ldexpf(1.0f, -kDigitShift * (LV - 1));
+#pragma unroll
+                        for (int c = 0; c < 16; ++c) hi[c] *= wl;
+#pragma unroll
+                        for (int l = LV - 2; l >= 0; --l) {
+                            tmem_ld16_wait(ta + static_cast<uint32_t>(l * kBN), v);
+                            const float w = ldexpf(1.0f, -kDigitShift * l);
+#pragma unroll
+                            for (int c = 0; c < 16; ++c) hi[c] = fmaf(v[c], w, hi[c]);
+                        }
+                    }
+                    if (gi + 1 == kGroups || g0 + kStep * (gi + 1) >= kBN / 16) {  // the chunk's last read of tensor memory
+                        fence_before_sync();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive_cluster_relaxed(acc_empty0);
+                    }
+#pragma unroll
+                    for (int c = 0; c < 16; ++c) {
+                        const int ex = eu + (c0 + c < N ? args.eA[static_cast<int64_t>(b) * N + c0 + c] : 0) - 12;
+                        Out x;
+                        if constexpr (F64) {
+                            // (one multiplication on the FP64 pipe where ldexp takes several)
+                            x = static_cast<double>(hi[c]) + static_cast<double>(lo[c]);
+                            x = abs(ex) < 1000 ? x * __hiloint2double((1023 + ex) << 20, 0) : ldexp(x, ex);
+                        } else {
+                            x = ldexpf(hi[c], ex);
+                        }
+                        if (add) acc[gi][c] += x;
+                        else acc[gi][c] = x;
+                    }
+                }
+                add = true;
+                tphase ^= 1u;
+            }
+            if (!ok) break;
+            Out* dst = F64 ? reinterpret_cast<Out*>(args.W) : reinterpret_cast<Out*>(args.C);
+#pragma unroll
+            for (int gi = 0; gi < kGroups; ++gi) {
+                if (g0 + kStep * gi >= kBN / 16) continue;
+                const int c0 = tm * kBN + (g0 + kStep * gi) * 16;
+                __syncwarp();
+#pragma unroll
+                for (int c = 0; c < 16; ++c) buf[lane * 17 + c] = acc[gi][c];
+                __syncwarp();
+#pragma unroll
+                for (int u = 0; u < 16; ++u) {
+                    const int rr = 2 * u + lane / 16, c = lane % 16;
+                    if (row0 + rr < N && c0 + c < N) dst[at + static_cast<int64_t>(row0 + rr) * N + c0 + c] = buf[rr * 17 + c];
+                }
+            }
         }
     }
 
     fence_before_sync();
-    __syncthreads();
+    __syncwarp();
+    cluster_sync();  // no CTA leaves while its peer may still signal its barriers or read its operands
     if (warp == 1) {
         fence_after_sync();
-        tmem_dealloc(tmem_base, kTmemCols);
+        tmem_dealloc_pair(tmem_base, kTmemCols);
     }
 }
 
@@ -403,13 +479,6 @@ OzWs carve_oz(void* base, int N, int batch) {
     return w;
 }
 
-int sm_count_current() {
-    int dev = 0, sm = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-        return 0;
-    return sm;
-}
-
 // FP32 rows (rows, pitch N) -> 4 digit planes at `planes` (plane stride w.plane) and row exponents; Ut (optional) the
 // rounding the planes represent.
 int digits_f32(const float* X, int64_t rows, int N, __half* planes, const OzWs& w, int* expo, float* Ut,
@@ -419,8 +488,7 @@ int digits_f32(const float* X, int64_t rows, int N, __half* planes, const OzWs& 
 }
 
 // The digit-plane product of configuration <PA, PB, LV, F64>: out[b][i][m] = sum over pairs of A-side planes (rows i)
-// and B-side planes (rows m), scaled by the row exponents; FP64 into W or FP32 into C (+ D).  Reductions longer than
-// kMaxChunk run as several launches that add into the output.
+// and B-side planes (rows m), scaled by the row exponents; FP64 into W or FP32 into C (+ D).
 template <int PA, int PB, int LV, bool F64>
 int launch_oz(const __half* aplanes, const int* ea_side, const __half* bplanes, const int* eb_side, int N, int batch,
               const OzWs& w, double* W, float* C, const float* D, cudaStream_t st) {
@@ -432,39 +500,28 @@ int launch_oz(const __half* aplanes, const int* ea_side, const __half* bplanes, 
     std::memset(&maps, 0, sizeof(maps));
     int rc;
     if ((rc = tc::make_map_f16(&maps.u, aplanes, static_cast<int>(PA * rows), N, w.ldp, kBK, kBM))) return rc;
-    if ((rc = tc::make_map_f16(&maps.a, bplanes, static_cast<int>(PB * rows), N, w.ldp, kBK, kBN))) return rc;
-    static std::once_flag attr_once;
-    static cudaError_t attr_rc = cudaSuccess;
-    std::call_once(attr_once, [] {
-        attr_rc = cudaFuncSetAttribute(k_ozaki<PA, PB, LV, F64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       Cfg::kSmemBytes);
-    });
-    if (attr_rc != cudaSuccess) return fail(FLMM_ERR_CUDA, "k_ozaki: %s", cudaGetErrorString(attr_rc));
+    if ((rc = tc::make_map_f16(&maps.a, bplanes, static_cast<int>(PB * rows), N, w.ldp, kBK, Cfg::kBN / 2))) return rc;
+    static PairCache cache;
+    int pairs = 0;
+    if ((rc = pair_count(k_ozaki<PA, PB, LV, F64>, Cfg::kThreads, Cfg::kSmemBytes, cache, &pairs))) return rc;
     int dev = 0;
     FLMM_CUDA(cudaGetDevice(&dev));
     int* err = device_err_flag(dev);
     if (!err) return fail(FLMM_ERR_CUDA, "refine product: cannot allocate the device error flag");
-    const int sm = sm_count_current();
-    const int64_t tiles = static_cast<int64_t>(batch) * ((N + kBM - 1) / kBM) * ((N + kBN - 1) / kBN);
-    const int grid = static_cast<int>(tiles < sm ? tiles : sm);
-    if (grid <= 0) return FLMM_OK;
-    for (int k0 = 0; k0 < N; k0 += kMaxChunk) {
-        OzArgs a;
-        a.N = N;
-        a.batch = batch;
-        a.k0 = k0;
-        a.klen = N - k0 < kMaxChunk ? N - k0 : kMaxChunk;
-        a.eU = ea_side;
-        a.eA = eb_side;
-        a.W = W;
-        a.C = C;
-        a.D = D;
-        a.accumulate = k0 > 0;
-        a.err = err;
-        k_ozaki<PA, PB, LV, F64><<<grid, kThreads, Cfg::kSmemBytes, st>>>(maps, a);
-        if ((rc = check_launch("k_ozaki"))) return rc;
-    }
-    return FLMM_OK;
+    const int64_t tiles = static_cast<int64_t>(batch) * ((N + 2 * kBM - 1) / (2 * kBM)) * ((N + Cfg::kBN - 1) / Cfg::kBN);
+    pairs = static_cast<int>(std::min<int64_t>(tiles, pairs));
+    if (pairs <= 0) return FLMM_OK;
+    OzArgs a;
+    a.N = N;
+    a.batch = batch;
+    a.eU = ea_side;
+    a.eA = eb_side;
+    a.W = W;
+    a.C = C;
+    a.D = D;
+    a.err = err;
+    if ((rc = launch_pairs(k_ozaki<PA, PB, LV, F64>, pairs, Cfg::kThreads, Cfg::kSmemBytes, st, maps, a))) return rc;
+    return check_launch("k_ozaki");
 }
 
 // batched (N, N) FP32 transpose, 32 x 32 tiles through shared memory

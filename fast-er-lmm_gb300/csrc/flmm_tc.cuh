@@ -7,6 +7,10 @@
 #include <cuda.h>
 #include <stdint.h>
 
+#include <mutex>
+
+#include "flmm_common.cuh"
+
 namespace flmm {
 namespace tc {
 
@@ -128,14 +132,30 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t sbo_bytes
     return d;
 }
 
-// D[tmem] (+)= A[smem] * B[smem]^T, issued by one thread.
-__device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+// One lane of a converged warp.  The MMA warps run their loops as a whole and leave the instructions themselves to this
+// lane: the loops are then uniform, and descriptors and addresses live in uniform registers.  Behind `if (lane == 0)` each of
+// an MMA's operands was moved there for every MMA, ~73 cycles between one and the next, where M = 128 x N = 64 x 16 takes 48
+// and a CTA pair's 256 x 128 x 16 takes 64.
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+    return e;
+}
+
+// a converged warp's wait (mbar_wait in every lane): true if all lanes saw the phase complete
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int* err, int code) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, err, code));
+}
+
+// D[tmem] (+)= A[smem] * B[smem]^T, issued by the elected lane of a converged warp.
+__device__ __forceinline__ void mma_f16(uint32_t elected, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                         uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p, e;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        "setp.ne.b32 e, %5, 0;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(elected)
         : "memory");
 }
 
@@ -285,14 +305,20 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 
-// D (+)= A B^T over the pair, issued by one thread of the even CTA
-__device__ __forceinline__ void mma_f16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                             uint32_t accumulate) {
+// a converged warp's wait for a barrier whose arrivals come from the peer CTA
+__device__ __forceinline__ bool mbar_wait_cluster_warp(uint64_t* bar, uint32_t parity, int* err, int code) {
+    return __all_sync(0xffffffffu, mbar_wait_cluster(bar, parity, err, code));
+}
+
+// D (+)= A B^T over the pair, issued by the elected lane of a converged warp of the even CTA
+__device__ __forceinline__ void mma_f16_pair(uint32_t elected, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
+                                             uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p, e;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        "setp.ne.b32 e, %5, 0;\n\t"
+        "@e tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(elected)
         : "memory");
 }
 
@@ -308,6 +334,60 @@ __device__ __forceinline__ void mma_commit_pair(uint64_t* bar, uint16_t cta_mask
 // FP16 matrix (rows, K) with row pitch ld elements (a multiple of 8, base 16-byte aligned) -> tiled TMA map with box
 // {BK, box_rows}, BK 32 (64-byte swizzle) or 64 (128-byte swizzle); rows and columns outside the matrix read as zero.
 int make_map_f16(CUtensorMap* map, const void* base, int rows, int K, int64_t ld, int BK, int box_rows);
+
+// CTA pairs of a kernel (one CTA per SM) that the current device runs at once; sets its shared-memory limit.  `cache` is
+// the kernel's own, by device.
+struct PairCache {
+    std::mutex mu;
+    int pairs[64] = {};
+};
+
+template <typename Kernel>
+int pair_count(Kernel* kernel, int threads, int smem_bytes, PairCache& cache, int* out) {
+    int dev = 0, sm = 0, n = 0;
+    FLMM_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return fail(FLMM_ERR_ARG, "pair_count: device %d", dev);
+    std::lock_guard<std::mutex> lock(cache.mu);
+    if (cache.pairs[dev] == 0) {
+        FLMM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
+        FLMM_CUDA(cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev));
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 2;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.gridDim = dim3(static_cast<unsigned>(sm & ~1));
+        cfg.blockDim = dim3(static_cast<unsigned>(threads));
+        cfg.dynamicSmemBytes = static_cast<size_t>(smem_bytes);
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        FLMM_CUDA(cudaOccupancyMaxActiveClusters(&n, kernel, &cfg));
+        if (n < 1) return fail(FLMM_ERR_CUDA, "pair_count: no CTA pair fits on the device");
+        cache.pairs[dev] = n;
+    }
+    *out = cache.pairs[dev];
+    return FLMM_OK;
+}
+
+// `pairs` CTA pairs of a kernel
+template <typename... Params, typename... Args>
+int launch_pairs(void (*kernel)(Params...), int pairs, int threads, int smem_bytes, cudaStream_t st, const Args&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(static_cast<unsigned>(2 * pairs));
+    cfg.blockDim = dim3(static_cast<unsigned>(threads));
+    cfg.dynamicSmemBytes = static_cast<size_t>(smem_bytes);
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    FLMM_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+    return FLMM_OK;
+}
 
 // Bounded wait that ignores the kernel's error flag: used at teardown to drain TMA copies still in flight.
 __device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {
