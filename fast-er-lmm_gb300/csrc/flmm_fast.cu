@@ -272,6 +272,19 @@ __device__ __forceinline__ void gemm_rows(const TcArgs& args, const float (&v)[N
         const float* sc = sc1 + 16 * qd;
         const float* vv = v + 16 * qd;
         float* dst = crow + c0;
+        if (c0 + 16 <= nvalid && !args.accumulate && (reinterpret_cast<uintptr_t>(dst) & 31u) == 0) {
+            // the thread's 16 outputs are two whole sectors: two 32-byte stores, so that L2 merges no halves
+#pragma unroll
+            for (int h = 0; h < 16; h += 8) {
+                float x[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) x[j] = vv[h + j] * sa * sc[h + j];
+                asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst + h), "f"(x[0]), "f"(x[1]),
+                             "f"(x[2]), "f"(x[3]), "f"(x[4]), "f"(x[5]), "f"(x[6]), "f"(x[7])
+                             : "memory");
+            }
+            continue;
+        }
         if (c0 + 16 <= nvalid && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {
             // a thread owns 16 consecutive outputs of its row: four 16-byte stores
             float4* d4 = reinterpret_cast<float4*>(dst);

@@ -20,7 +20,7 @@
 //
 // Kernel: persistent CTA pairs; tiles of 256 A rows (128 a CTA) x 64 B rows, 8 levels x 64 columns = all of tensor memory.
 // Warp 0 of each CTA issues its TMA loads: a stage is 16 deep, 8 x 4 KB of its own A rows and 8 x 1 KB of half the B rows =
-// 40 KB in four boxes of 128-byte rows that hold four planes each, five stages.  Warp 1 of the even CTA issues the 36 MMAs
+// 40 KB in four boxes of 128-byte rows that hold four planes each, four stages.  Warp 1 of the even CTA issues the 36 MMAs
 // of a stage (M = 256, N = 64, K = 16 over both), warps 2..17 drain the levels; tensor memory is handed back before the
 // outputs are rounded and stored, so only the drain itself (8 x 64 columns per 512 terms, 4,300 cycles) interrupts the
 // MMAs.  A pair's MMA reads 5 KB of operands a CTA where a CTA by itself reads 6 for half the work; and see elect_one: with
@@ -48,14 +48,16 @@ constexpr int kBK = 16;      // depth of one stage: a row's eight planes of 16 e
 constexpr int kRowElems = kOzPlanes * kBK;            // elements of a row in one stage
 constexpr int kABox = kOzRowsA * 128, kBBox = kOzRowsB / 2 * 128;
 constexpr int kStageBytes = 2 * (kABox + kBBox);
-constexpr int kStages = 5;
+constexpr int kStages = 4;
 constexpr uint32_t kSBO = 1024;     // bytes between 8-row groups
 constexpr uint32_t kSwizzle128 = 2u;
 constexpr int kTmemCols = kLevels * kOzRowsB;
 constexpr int kEpiWarps = 16;
 constexpr int kThreads = 64 + 32 * kEpiWarps;
 constexpr int kEpiCols = kOzRowsB / (kEpiWarps / 4);  // output columns per epilogue thread
-constexpr int kSmemBytes = kStages * kStageBytes + 256 + 1024;
+constexpr int kOutCols = 8;                           // outputs of a row that pass through shared memory together
+constexpr int kOutBytes = 32 * (kOutCols + 1) * 8;    // of a warp
+constexpr int kSmemBytes = kStages * kStageBytes + kEpiWarps * kOutBytes + 256 + 1024;
 constexpr int kMaxExp = 450;  // |e| beyond this: the scale 2^(e_a + e_b - 61) could leave FP64's range
 static_assert(kTmemCols == 512 && kSmemBytes <= 227 * 1024 && kEpiCols == 16, "budgets");
 
@@ -356,6 +358,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz64(const __grid_constant__ Oz
         const int c0 = ((warp - 2) >> 2) * kEpiCols;
         const uint32_t tl0 = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(c0);
         const uint32_t acc_empty0 = map_to_rank(smem_u32(acc_empty), 0);
+        double* buf = reinterpret_cast<double*>(smem + kStages * kStageBytes + 256 + (warp - 2) * kOutBytes);
         uint32_t tphase = 0;
         bool ok = true;
         for (int t = cl; t < n_tiles && ok; t += n_cl) {
@@ -390,19 +393,31 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz64(const __grid_constant__ Oz
             }
             if (!ok) break;
             const Tile half{tl.b, 2 * tl.ti + static_cast<int>(rank), tl.tm};
-            const int i = half.ti * kOzRowsA + q * 32 + lane;
-            if (i < args.Ma && tile_good(args, half)) {
-                const int ea = args.ea[tl.b * args.Ma + i];
-                const int m0 = tl.tm * kOzRowsB + c0;
-                const int* eb = args.eb + tl.b * args.Nb + m0;
-                double* out = args.C + tl.b * args.c_stride + static_cast<int64_t>(i) * args.ldc + m0;
-                const double* d = args.D ? args.D + static_cast<int64_t>(i) * args.ldd + m0 : nullptr;
+            if (!tile_good(args, half)) continue;
+            // the outputs leave through shared memory, so that lanes go along the rows of C (and D)
+            const int i0 = half.ti * kOzRowsA + q * 32;
+            const int ea = i0 + lane < args.Ma ? args.ea[tl.b * args.Ma + i0 + lane] : 0;
+            double* C = args.C + tl.b * args.c_stride;
 #pragma unroll
-                for (int c = 0; c < kEpiCols; ++c) {
-                    if (m0 + c < args.Nb) {
-                        const double s = __longlong_as_double(static_cast<long long>(1023 + ea + eb[c] - 61) << 52);
-                        const double v = fma(static_cast<double>(hi[c]), 0x1p28, static_cast<double>(lo[c])) * s;
-                        out[c] = d ? d[c] - v : v;
+            for (int h = 0; h < kEpiCols; h += kOutCols) {
+                const int m0 = tl.tm * kOzRowsB + c0 + h;
+                const int* eb = args.eb + tl.b * args.Nb + m0;
+                __syncwarp();
+#pragma unroll
+                for (int c = 0; c < kOutCols; ++c) {
+                    const int e = ea + (m0 + c < args.Nb ? eb[c] : 0);
+                    const double s = __longlong_as_double(static_cast<long long>(1023 + e - 61) << 52);
+                    buf[lane * (kOutCols + 1) + c] =
+                        fma(static_cast<double>(hi[h + c]), 0x1p28, static_cast<double>(lo[h + c])) * s;
+                }
+                __syncwarp();
+#pragma unroll
+                for (int u = 0; u < kOutCols; ++u) {
+                    const int rr = (32 / kOutCols) * u + lane / kOutCols, c = lane % kOutCols;
+                    if (i0 + rr < args.Ma && m0 + c < args.Nb) {
+                        const double v = buf[rr * (kOutCols + 1) + c];
+                        const int64_t i = i0 + rr;
+                        C[i * args.ldc + m0 + c] = args.D ? args.D[i * args.ldd + m0 + c] - v : v;
                     }
                 }
             }
