@@ -250,6 +250,7 @@ k_sytrd_cluster(float* __restrict__ W, int N, int parts, float* __restrict__ d_o
     float* db = d_out + static_cast<int64_t>(b) * N;
     float* eb = e_out + static_cast<int64_t>(b) * N;
     float* tb = tau_out + static_cast<int64_t>(b) * N;
+    cluster_barrier();          // every CTA runs: its shared memory may be written
     int first = r > 0 ? r : C;  // first row of this CTA past row k
     int first_dot = 1 % parts;  // k + 1 modulo parts
     Reflector R{0.0f, 0.0f, 0.0f};

@@ -15,6 +15,7 @@
 
 #include "flmm_common.cuh"
 #include "flmm_oz64.cuh"
+#include "flmm_tc.cuh"
 
 using namespace flmm;
 
@@ -135,8 +136,10 @@ __device__ double gram_loss(const double* Gs, double sum_log, int N, int C, bool
     const bool ok = chol_lower(A, C);
     if (!ok) set_identity(A, C);
     double logdet = 0.0;
-    for (int i = 0; i < C; ++i) logdet += log(A[i * C + i]);
-    logdet = 2.0 * logdet;
+    if (reml) {
+        for (int i = 0; i < C; ++i) logdet += log(A[i * C + i]);
+        logdet = 2.0 * logdet;
+    }
     forward_solve(A, C, z);
     double uAu = 0.0;
     for (int i = 0; i < C; ++i) uAu += z[i] * z[i];
@@ -320,102 +323,107 @@ __global__ void k_gls_golden(const double* __restrict__ s, int N, const double* 
     if ((threadIdx.x & 31) == 0) log_delta[p] = fmin(fmax(mul_rn(0.5, add_rn(a, b)), lo), hi);
 }
 
-// The same search with one block per column: both evaluations of a step share the block, whose threads form the weights
-// (one division per eigenvalue; a warp of k_gls_golden forms them again for every eight products of its Gram) and
-// logarithms into shared memory, and whose warps then add the Gram's products four at a time, each sum in the order of
-// k_gls_golden's lanes and butterfly, so every loss keeps its bits.  A point that is, to the bit, one of the step before
-// keeps its loss.  60 columns x 300 samples, C = 5, with the grid:
-// 7.5 -> 2.3 ms.  Beyond ~6,000 samples the weights no longer fit in shared memory and k_gls_golden runs.
+// The same search with a cluster of two blocks per column, one for each evaluation of a step: the FP64 pipe of an SM bounds
+// a step, and a study of tens of columns leaves most SMs idle otherwise.  A block's threads form the weights (one division
+// per eigenvalue; a warp of k_gls_golden forms them again for every eight products of its Gram) and logarithms into shared
+// memory, its warps add the Gram's products four at a time, each sum in the order of k_gls_golden's lanes and butterfly, so
+// every loss keeps its bits; thread 0 puts the loss into both blocks, and both carry the search.  A point that is, to the
+// bit, one of the step before keeps its loss.  60 columns x 300 samples, C = 5, with the grid: 7.5 ms with a warp per column,
+// 2.3 with one block, 1.5 here.  Beyond ~12,000 samples the weights no longer fit in shared memory and k_gls_golden runs.
 constexpr int kBlockThreads = 256;
 constexpr int kBlockPairs = 4;
 
 size_t golden_block_smem(int N, int C) {
-    return sizeof(double) * (4 * static_cast<size_t>(N) +
-                             2 * (static_cast<size_t>(C + 1) * (C + 1) + static_cast<size_t>(C) * C + (C + 1)));
+    return sizeof(double) * (2 * static_cast<size_t>(N) + static_cast<size_t>(C + 1) * (C + 1) + static_cast<size_t>(C) * C +
+                             (C + 1));
 }
 
-__global__ void __launch_bounds__(kBlockThreads)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBlockThreads)
 k_gls_golden_block(const double* __restrict__ s, int N, const double* __restrict__ Xrt, int64_t ldx, int C,
                    const double* __restrict__ Yrt, int64_t ldy, const double* __restrict__ grid, int G,
                    const int32_t* __restrict__ idx, int reml, double lo, double hi, double* __restrict__ log_delta) {
     extern __shared__ double sm[];
-    __shared__ double delta_s[2], log_s[2], loss_s[2];
-    __shared__ int kept_s[2];
-    const int64_t p = blockIdx.x;
+    __shared__ double delta_s, log_s, loss_s[2][2];  // loss_s[step % 2][evaluation]
+    __shared__ int kept_s;
+    const int64_t p = blockIdx.x >> 1;
+    const int my_e = static_cast<int>(tc::cluster_ctarank());
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int K = C + 1, pairs = K * (K + 1) / 2;
-    double* w = sm;           // [2][N]
-    double* lg = w + 2 * N;   // [2][N]
-    double* mats = lg + 2 * N;
-    const int per = K * K + C * C + K;
+    double* w = sm;        // [N]
+    double* lg = w + N;    // [N]
+    double* Gs = lg + N;   // Gram, then the factor and a vector
     const double* y = Yrt + p * ldy;
-    const bool lead = tid == 0 || tid == 32;  // carry the search, one evaluation each
-    const int my_e = tid >> 5;
     Bracket br(grid, G, idx[p]);
-    const int groups = (pairs + kBlockPairs - 1) / kBlockPairs;  // of products; one more sum per evaluation is the log's
+    const int groups = (pairs + kBlockPairs - 1) / kBlockPairs;  // of products; one more sum is the logarithms'
+    tc::cluster_sync();  // the other block runs: its shared memory may be written
     for (int it = 0; it < 50; ++it) {
         double kept_loss = 0.0;
-        bool kept = false;
-        if (lead) {
-            kept = it > 0 && br.narrow_kept(loss_s, my_e, &kept_loss);
-            delta_s[my_e] = exp(my_e ? br.d() : br.c());
-            kept_s[my_e] = kept;
+        if (tid == 0) {
+            kept_s = it > 0 && br.narrow_kept(loss_s[(it - 1) & 1], my_e, &kept_loss);
+            delta_s = exp(my_e ? br.d() : br.c());
         }
         __syncthreads();
-        // evaluations e0 .. e1
-        const int e0 = kept_s[0], e1 = 2 - kept_s[1];
-        for (int t = e0 * N + tid; t < e1 * N; t += kBlockThreads) {
-            const double sd = s[t < N ? t : t - N] + delta_s[t >= N];
-            w[t] = 1.0 / sd;
-            lg[t] = log(sd);
-        }
-        __syncthreads();
-        for (int g = e0 * (groups + 1) + warp; g < e1 * (groups + 1); g += kBlockThreads / 32) {
-            const int e = g > groups, q = g - e * (groups + 1);
-            const double* we = w + e * N;
-            if (q == groups) {
-                double sl = 0.0;
-                for (int n = lane; n < N; n += 32) sl += lg[e * N + n];
-                sl = warp_sum(sl);
-                if (lane == 0) log_s[e] = sl;
-                continue;
+        const bool kept = kept_s != 0;
+        if (!kept) {
+            for (int n = tid; n < N; n += kBlockThreads) {
+                const double sd = s[n] + delta_s;
+                w[n] = 1.0 / sd;
+                lg[n] = log(sd);
             }
-            const double *ai[kBlockPairs], *aj[kBlockPairs];
-            int at[kBlockPairs];
+            __syncthreads();
+            for (int q = warp; q <= groups; q += kBlockThreads / 32) {
+                if (q == groups) {
+                    double sl = 0.0;
+                    for (int n = lane; n < N; n += 32) sl += lg[n];
+                    sl = warp_sum(sl);
+                    if (lane == 0) log_s = sl;
+                    continue;
+                }
+                const double *ai[kBlockPairs], *aj[kBlockPairs];
+                int at[kBlockPairs];
 #pragma unroll
-            for (int k = 0; k < kBlockPairs; ++k) {
-                const int r = min(q * kBlockPairs + k, pairs - 1);
-                int pi = static_cast<int>((sqrtf(8.0f * r + 1.0f) - 1.0f) * 0.5f);
-                if (pi * (pi + 1) / 2 > r) --pi;
-                if ((pi + 1) * (pi + 2) / 2 <= r) ++pi;
-                const int pj = r - pi * (pi + 1) / 2;
-                at[k] = pi * K + pj;
-                ai[k] = pi < C ? Xrt + pi * ldx : y;
-                aj[k] = pj < C ? Xrt + pj * ldx : y;
-            }
-            double acc[kBlockPairs] = {};
-            for (int n = lane; n < N; n += 32) {
-                const double wn = we[n];
+                for (int k = 0; k < kBlockPairs; ++k) {
+                    const int r = min(q * kBlockPairs + k, pairs - 1);
+                    int pi = static_cast<int>((sqrtf(8.0f * r + 1.0f) - 1.0f) * 0.5f);
+                    if (pi * (pi + 1) / 2 > r) --pi;
+                    if ((pi + 1) * (pi + 2) / 2 <= r) ++pi;
+                    const int pj = r - pi * (pi + 1) / 2;
+                    at[k] = pi * K + pj;
+                    ai[k] = pi < C ? Xrt + pi * ldx : y;
+                    aj[k] = pj < C ? Xrt + pj * ldx : y;
+                }
+                double acc[kBlockPairs] = {};
+                for (int n = lane; n < N; n += 32) {
+                    const double wn = w[n];
+                    double wa = 0.0;
 #pragma unroll
-                for (int k = 0; k < kBlockPairs; ++k) acc[k] += mul_rn(mul_rn(wn, ai[k][n]), aj[k][n]);
-            }
+                    for (int k = 0; k < kBlockPairs; ++k) {
+                        if (k == 0 || ai[k] != ai[k - 1]) wa = mul_rn(wn, ai[k][n]);
+                        acc[k] += mul_rn(wa, aj[k][n]);
+                    }
+                }
 #pragma unroll
-            for (int k = 0; k < kBlockPairs; ++k) {
-                const double v = warp_sum(acc[k]);
-                if (lane == 0 && q * kBlockPairs + k < pairs) mats[e * per + at[k]] = v;
+                for (int k = 0; k < kBlockPairs; ++k) {
+                    const double v = warp_sum(acc[k]);
+                    if (lane == 0 && q * kBlockPairs + k < pairs) Gs[at[k]] = v;
+                }
             }
+            __syncthreads();
         }
-        __syncthreads();
-        if (kept) {
-            loss_s[my_e] = kept_loss;
-        } else if (lead) {
-            double* Gs = mats + my_e * per;
-            loss_s[my_e] = gram_loss(Gs, log_s[my_e], N, C, reml != 0, Gs + K * K, Gs + K * K + C * C);
+        if (tid == 0) {
+            const double loss = kept ? kept_loss : gram_loss(Gs, log_s, N, C, reml != 0, Gs + K * K, Gs + K * K + C * C);
+            const uint32_t at = tc::smem_u32(&loss_s[it & 1][my_e]);
+#pragma unroll
+            for (uint32_t r = 0; r < 2; ++r)
+                asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(tc::map_to_rank(at, r)), "d"(loss) : "memory");
         }
-        __syncthreads();
+        // (two buffers: a block can be one step ahead of the other's read, not two; and after the last step neither leaves
+        // before the other has written)
+        tc::cluster_sync();
     }
-    if (tid == 0) {
-        br.narrow(loss_s[0] < loss_s[1]);
+    if (tid == 0 && my_e == 0) {
+        const double* loss = loss_s[49 & 1];
+        br.narrow(loss[0] < loss[1]);
         log_delta[p] = fmin(fmax(mul_rn(0.5, add_rn(br.a, br.b)), lo), hi);
     }
 }
@@ -747,7 +755,7 @@ extern "C" int flmm_fit_delta_gls_f64(const double* s, int N, const double* Xrt,
     if (refine && block_smem <= 200 * 1024) {
         if (block_smem > 48 * 1024)
             FLMM_CUDA(cudaFuncSetAttribute(k_gls_golden_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)block_smem));
-        k_gls_golden_block<<<P, kBlockThreads, block_smem, st>>>(s, N, Xrt, ldx, C, Yrt, ldy, ws.grid, n_grid, grid_idx,
+        k_gls_golden_block<<<2 * P, kBlockThreads, block_smem, st>>>(s, N, Xrt, ldx, C, Yrt, ldy, ws.grid, n_grid, grid_idx,
                                                                  reml, lo, hi, log_delta);
         return check_launch("k_gls_golden_block");
     }
