@@ -144,8 +144,8 @@ __device__ Reflector make_reflector(float d, float alpha, float ss_partial, floa
 }
 
 // kQ rows i0, i0 + di, ... (rows of N entries from W on) at columns k + 1 ..: the kM pending updates, oldest first, whose
-// vectors start at sm[ov[m]] and sm[ow[m]], stored when kM is kPend (not row k + 1); then p_i = tau row . v into every CTA's copy of p.
-// Every lane adds up its columns k + 1 + lane + 32 t in order.
+// vectors start at sm[ov[m]] and sm[ow[m]], stored when kM is kPend (not row k + 1); then p_i = tau row . v into every CTA's
+// copy of p.  Every lane adds up its columns k + 1 + lane + 32 t in order.
 extern __shared__ float sytrd_sm[];
 
 template <int kM, int kQ>
@@ -834,7 +834,8 @@ k_backtransform(const float* __restrict__ W, const float* __restrict__ Tq_all, c
             for (int m = 0; m < kWy; ++m) ns[m] = *reinterpret_cast<const float4*>(&Sp[m][zc]);
         }
         if (q > 0)
-            for (int t = tid; t < kWy * kWy; t += kBtThreads) Tm[t / kWy][t % kWy] = Tb[static_cast<int64_t>(q - 1) * kWy * kWy + t];
+            for (int t = tid; t < kWy * kWy; t += kBtThreads)
+                Tm[t / kWy][t % kWy] = Tb[static_cast<int64_t>(q - 1) * kWy * kWy + t];
         for (int j = 0; j <= chunks; ++j) {
             __syncthreads();  // chunk j is staged, and rows of chunk j - 1 are up to date
             if (tid >= kBtDot) {

@@ -14,8 +14,8 @@
 // What is lost is the rounding to 55 bits and the levels from 8 on (weight 2^-56 against the row maxima).  For rows
 // whose largest entry is a few times their rms this is several times smaller than the rounding of an FP64 sum of K
 // terms (~0.4 * 2^-53 * K times the rms product; measured against exact sums in tests/test_gpu_oz64.py).  The loss
-// grows with max/rms of both rows (after balancing, oz_balance), so every tile of rows carries its largest ratio; a tile pair whose product of
-// ratios exceeds quality_limit(K), and any row that is not finite or whose exponent is out of range, is left to
+// grows with max/rms of both rows (after balancing, oz_balance), so every tile of rows carries its largest ratio; a tile
+// pair whose product of ratios exceeds quality_limit(K), and any row that is not finite or whose exponent is out of range, is left to
 // k_marked_f64, which forms those tiles on the FP64 pipe as before.
 //
 // Kernel: persistent CTA pairs; tiles of 256 A rows (128 a CTA) x 64 B rows, 8 levels x 64 columns = all of tensor memory.
@@ -335,8 +335,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz64(const __grid_constant__ Oz
                     fence_after_sync();
                     const uint64_t d0 = smem_desc(smem_u32(smem + stage * kStageBytes), kSBO, kSwizzle128);
                     const uint32_t lo = static_cast<uint32_t>(d0);
-                    mma_pair<0, 0>(elected, tmem_base, lo, lo + 2 * (kABox / 16), static_cast<uint32_t>(d0 >> 32), first ? 0u : 1u,
-                                   idesc);
+                    mma_pair<0, 0>(elected, tmem_base, lo, lo + 2 * (kABox / 16), static_cast<uint32_t>(d0 >> 32),
+                                   first ? 0u : 1u, idesc);
                     if (elected) mma_commit_pair(&empty[stage], 3);
                     if (++stage == kStages) { stage = 0; phase ^= 1u; }
                     if ((kb + 1) % kChunkKb == 0 || kb + 1 == n_kb) {
@@ -580,7 +580,8 @@ int oz_gemm(const OzOperand& A, const OzOperand& B, const OzProduct& p, cudaStre
     a.D = p.D;
     a.ldd = p.ldd;
     const int64_t tiles = static_cast<int64_t>(a.batches) * a.pairs_i * a.tiles_m;
-    if ((rc = launch_pairs(k_oz64, static_cast<int>(std::min<int64_t>(tiles, pairs)), kThreads, kSmemBytes, st, maps, a))) return rc;
+    pairs = static_cast<int>(std::min<int64_t>(tiles, pairs));
+    if ((rc = launch_pairs(k_oz64, pairs, kThreads, kSmemBytes, st, maps, a))) return rc;
     if ((rc = check_launch("k_oz64"))) return rc;
     const dim3 grid(ceil_div(B.rows, kST), ceil_div(A.rows, kST), a.batches);
     k_marked_f64<<<grid, kSThreads, 0, st>>>(a, p.Xa, p.lda, p.xa_stride, p.Xb, p.ldb, p.square[0], p.square[1]);

@@ -79,8 +79,8 @@ struct OzCfg {
 };
 // Configurations used: the refinement's A U as <4, 7, 8, FP64> (U~ in 4 planes, A in 7, levels 0..7, 25 pairs); the
 // corrections u_i . r_j as <3, 3, 3, FP32> (6 pairs on planes 0..2 of either side: the coefficients E_ij are
-// themselves corrections and need ~1e-3 relative accuracy) and T U~ as <4, 4, 5, FP32> (13 pairs: FP32 accuracy against the row's largest rotation, which
-// reaches 0.25 for nearly degenerate pairs).
+// themselves corrections and need ~1e-3 relative accuracy) and T U~ as <4, 4, 5, FP32> (13 pairs: FP32 accuracy
+// against the row's largest rotation, which reaches 0.25 for nearly degenerate pairs).
 constexpr int kUPlanes = 4;
 constexpr int kAPlanes = 7;
 static_assert(kMaxChunk % kBK == 0, "chunks must start on a k-block");
@@ -172,7 +172,8 @@ __global__ void k_digits_a(const double* __restrict__ A, int64_t rows, int N, __
 // ---- the tensor-core product ----------------------------------------------------------------------------------
 
 template <int PA, int PB, int LV, bool F64>
-__global__ void __launch_bounds__(OzCfg<PA, PB, LV, F64>::kThreads, 1) k_ozaki(const __grid_constant__ OzMaps maps, const OzArgs args) {
+__global__ void __launch_bounds__(OzCfg<PA, PB, LV, F64>::kThreads, 1)
+k_ozaki(const __grid_constant__ OzMaps maps, const OzArgs args) {
     using Cfg = OzCfg<PA, PB, LV, F64>;
     constexpr int kBN = Cfg::kBN, kBTile = Cfg::kBTile, kEpiWarps = Cfg::kEpiWarps;
     constexpr int kStages = Cfg::kStages;

@@ -7,8 +7,8 @@
 //                            unit u + 1 on a second stream beside the variant side of unit u
 //
 // Each unit is ~20 launches of a few microseconds for ordinary studies, and issuing them from Python cost 10-20 us each:
-// 150 samples x 1,500 variants on 16 chromosomes took 10.2 ms in 505 launches, 4.35 unit by unit and 3.00 grouped.  What depends on the spectra
-// alone (mean, FP32 copies, sWs node weights and their split) and the projections run for all units in one launch each.
+// 150 samples x 1,500 variants on 16 chromosomes took 10.2 ms in 505 launches, 4.35 unit by unit and 3.00 grouped.  What
+// depends on the spectra alone (mean, FP32 copies, sWs node weights and their split) and the projections run for all units in one launch each.
 // Where every unit's column operands fit kGroupBytes together, so does the rest (run_grouped): the launches then take all
 // units' rows, the split products with the units' tiles one after another.  The arithmetic is in every form that of the
 // C entry points called one by one.
@@ -282,7 +282,8 @@ int carve_units(Arena& a, const flmm_units* q, bool group, UnitBufs* b) {
     b->F = a.of<float>(M * b->ldr);
     b->Fs = take_split(a, M, pad8(b->R));
     const int64_t tests = static_cast<int64_t>(M) * q->n_real;
-    b->cap = q->opts.f_refine > 0.0 ? static_cast<int>(std::min<int64_t>({tests, q->refine_cap * (b->grouped ? int64_t{q->n_units} : 1), INT_MAX / 2})) : 0;
+    const int64_t most = q->refine_cap * (b->grouped ? int64_t{q->n_units} : 1);
+    b->cap = q->opts.f_refine > 0.0 ? static_cast<int>(std::min<int64_t>({tests, most, INT_MAX / 2})) : 0;
     b->flags = a.of<int32_t>(2 * static_cast<size_t>(b->cap));
     b->flag_count = a.of<int32_t>(1);
     return FLMM_OK;
@@ -495,7 +496,8 @@ extern "C" int flmm_scan_units(flmm_context* ctx, const flmm_units* q, void* wor
     if (rc) return rc;
     FLMM_REQUIRE(ctx && work && q->U && q->evals && q->rows && q->max_F && q->log_delta &&
                      (q->P == 0 || (q->Yh && q->Yl && q->Yscale && q->ldY >= q->N)) && q->Zh && q->Zl && q->Zscale &&
-                     q->ldZ >= q->N && (q->n_real == 0 || (q->f && q->beta && q->se && q->sfve && q->nullh2 && q->ldo >= q->n_real)),
+                     q->ldZ >= q->N &&
+                     (q->n_real == 0 || (q->f && q->beta && q->se && q->sfve && q->nullh2 && q->ldo >= q->n_real)),
                  "flmm_scan_units: operands or outputs missing");
     size_t need = 0;
     if ((rc = flmm_scan_units_workspace_bytes(q, &need))) return rc;

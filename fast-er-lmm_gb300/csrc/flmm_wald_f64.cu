@@ -159,9 +159,8 @@ constexpr int kFinP = 32, kFinTile = 64, kFinM = 256;
 template <bool GLS>
 __global__ void __launch_bounds__(256)
 k_wald_finish(const double* __restrict__ Gy, const double* __restrict__ Gs, const double* __restrict__ Gq, int nq,
-              int64_t ldg,
-              const double* __restrict__ rWr, double var_df, int P, int n_real, int Mc, const int64_t* __restrict__ rows, double* __restrict__ f,
-              double* __restrict__ beta, double* __restrict__ se, double* __restrict__ sfve, int64_t ldo,
+              int64_t ldg, const double* __restrict__ rWr, double var_df, int P, int n_real, int Mc,
+              const int64_t* __restrict__ rows, double* __restrict__ f, double* __restrict__ beta, double* __restrict__ se, double* __restrict__ sfve, int64_t ldo,
               double* __restrict__ max_F) {
     __shared__ double sy[kFinP][kFinTile + 1];
     __shared__ double ss[kFinP][kFinTile + 1];
