@@ -149,12 +149,13 @@ __device__ __forceinline__ Test wald_test(double swy, double sws, double rwr, do
 }
 
 // Epilogue over the sums of a block of columns and variants (layout: flmm_oz64.cuh): a thread block takes 32 columns x
-// kFinM variants in tiles of 64, transposed through shared memory so that the reads run along the
-// variants and the detail stores along the columns.  Real columns get the full epilogue.  A permutation column needs its
+// kFinTile variants, transposed through shared memory so that the reads run along the variants and the detail stores along
+// the columns.  Real columns get the full epilogue; with 256 variants a block, those few blocks' FP64 pipes set the time
+// (1,100 columns, 100 of them real, x 4,096: 265 -> 161 us with one F a block; 660 with covariates, 60 real, x 4,000: 277 -> 138).  A permutation column needs its
 // largest F only, and F grows with q / denom, so its tests are ranked by cross-multiplication (three FP64 operations
-// instead of four divisions; GB300's FP64 pipe is the bound here) and one F is formed per thread; sums outside
+// instead of four divisions; GB300's FP64 pipe is the bound here) and one F is formed per block; sums outside
 // 1e-100 .. 1e100, and NaN, take the full formula.
-constexpr int kFinP = 32, kFinTile = 64, kFinM = 256;
+constexpr int kFinP = 32, kFinTile = 64;
 
 template <bool GLS>
 __global__ void __launch_bounds__(256)
@@ -164,62 +165,56 @@ k_wald_finish(const double* __restrict__ Gy, const double* __restrict__ Gs, cons
               double* __restrict__ max_F) {
     __shared__ double sy[kFinP][kFinTile + 1];
     __shared__ double ss[kFinP][kFinTile + 1];
-    __shared__ double red[8][kFinP];
+    __shared__ double red[8][kFinP], red_q[8][kFinP], red_den[8][kFinP], red_sy[8][kFinP];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int p0 = blockIdx.y * kFinP, p = p0 + lane;
     const bool p_ok = p < P, real = p < n_real;
     const double rwr = p_ok ? rWr[p] : 1.0;
     double best = -INFINITY, bq = -1.0, bden = 1.0, bsy = 0.0;
     bool any_nan = false;
-    const int m_end = min(Mc, (static_cast<int>(blockIdx.x) + 1) * kFinM);
-    for (int m0 = blockIdx.x * kFinM; m0 < m_end; m0 += kFinTile) {
-        __syncthreads();
+    const int m0 = blockIdx.x * kFinTile, m_end = min(Mc, m0 + kFinTile);
 #pragma unroll
-        for (int l = 0; l < kFinP * kFinTile / 256; ++l) {
-            const int t = tid + l * 256, r = t / kFinTile, c = t % kFinTile;
-            if (p0 + r < P && m0 + c < m_end) {
-                const int64_t o = static_cast<int64_t>(p0 + r) * ldg + m0 + c;
-                sy[r][c] = Gy[o];
-                double w = Gs[o];
-                if (GLS) {
-                    const double* g = Gq + static_cast<int64_t>(p0 + r) * nq * ldg + m0 + c;
-                    double quad = 0.0;
-                    for (int k = 0; k < nq; ++k) quad = fma(g[k * ldg], g[k * ldg], quad);
-                    w = add_rn(w, -quad);
-                }
-                ss[r][c] = w;
+    for (int l = 0; l < kFinP * kFinTile / 256; ++l) {
+        const int t = tid + l * 256, r = t / kFinTile, c = t % kFinTile;
+        if (p0 + r < P && m0 + c < m_end) {
+            const int64_t o = static_cast<int64_t>(p0 + r) * ldg + m0 + c;
+            sy[r][c] = Gy[o];
+            double w = Gs[o];
+            if (GLS) {
+                const double* g = Gq + static_cast<int64_t>(p0 + r) * nq * ldg + m0 + c;
+                double quad = 0.0;
+                for (int k = 0; k < nq; ++k) quad = fma(g[k * ldg], g[k * ldg], quad);
+                w = add_rn(w, -quad);
             }
-        }
-        __syncthreads();
-        if (!p_ok) continue;
-        for (int c = warp; c < kFinTile && m0 + c < m_end; c += 8) {
-            const double swy = sy[lane][c], den = fmax(ss[lane][c], kPosFloor), q = mul_rn(swy, swy);
-            if (!real && q < 1e100 && den < 1e100 && den > 1e-100) {
-                if (q * bden > bq * den) {
-                    bq = q;
-                    bden = den;
-                    bsy = swy;
-                }
-                continue;
-            }
-            const Test t = wald_test(swy, ss[lane][c], rwr, var_df);
-            best = fmax(best, t.F);
-            any_nan |= isnan(t.F);
-            if (real) {
-                const int64_t o = rows[m0 + c] * ldo + p;
-                f[o] = t.F;
-                beta[o] = t.b;
-                se[o] = sqrt(t.var_b);
-                sfve[o] = sqrt(fmax(t.q / mul_rn(t.denom, rwr), 0.0));
-            }
+            ss[r][c] = w;
         }
     }
-    if (bq >= 0.0) {
-        const double F = wald_test(bsy, bden, rwr, var_df).F;
-        best = fmax(best, F);
-        any_nan |= isnan(F);
+    __syncthreads();
+    for (int c = warp; p_ok && c < kFinTile && m0 + c < m_end; c += 8) {
+        const double swy = sy[lane][c], den = fmax(ss[lane][c], kPosFloor), q = mul_rn(swy, swy);
+        if (!real && q < 1e100 && den < 1e100 && den > 1e-100) {
+            if (q * bden > bq * den) {
+                bq = q;
+                bden = den;
+                bsy = swy;
+            }
+            continue;
+        }
+        const Test t = wald_test(swy, ss[lane][c], rwr, var_df);
+        best = fmax(best, t.F);
+        any_nan |= isnan(t.F);
+        if (real) {
+            const int64_t o = rows[m0 + c] * ldo + p;
+            f[o] = t.F;
+            beta[o] = t.b;
+            se[o] = sqrt(t.var_b);
+            sfve[o] = sqrt(fmax(t.q / mul_rn(t.denom, rwr), 0.0));
+        }
     }
     red[warp][lane] = any_nan ? NAN : best;
+    red_q[warp][lane] = bq;
+    red_den[warp][lane] = bden;
+    red_sy[warp][lane] = bsy;
     __syncthreads();
     if (warp == 0 && p_ok) {
         double v = -INFINITY;
@@ -227,6 +222,20 @@ k_wald_finish(const double* __restrict__ Gy, const double* __restrict__ Gs, cons
         for (int r = 0; r < 8; ++r) {
             nan |= isnan(red[r][lane]);
             v = fmax(v, red[r][lane]);
+        }
+        // one F a column for its best ranked test
+        for (int r = 1; r < 8; ++r) {
+            const double q = red_q[r][lane], den = red_den[r][lane];
+            if (q * bden > bq * den) {
+                bq = q;
+                bden = den;
+                bsy = red_sy[r][lane];
+            }
+        }
+        if (bq >= 0.0) {
+            const double F = wald_test(bsy, bden, rwr, var_df).F;
+            v = fmax(v, F);
+            nan |= isnan(F);
         }
         if (nan) v = NAN;
         if (v >= 0.0 || isnan(v)) atomic_max_nonneg(max_F + p, v);
@@ -282,7 +291,7 @@ size_t wald_ws(int P, int Neff) { return carve_wald(nullptr, P, Neff).bytes; }
 int flmm::wald_finish(const double* Gy, const double* Gs, const double* Gq, int nq, int64_t ldg, const double* rWr,
                       double var_df, int P, int n_real, int Mc, const int64_t* rows, double* f, double* beta, double* se,
                       double* sfve, int64_t ldo, double* max_F, cudaStream_t st) {
-    const dim3 grid(ceil_div(Mc, kFinM), ceil_div(P, kFinP));
+    const dim3 grid(ceil_div(Mc, kFinTile), ceil_div(P, kFinP));
     auto* k = nq > 0 ? k_wald_finish<true> : k_wald_finish<false>;
     k<<<grid, 256, 0, st>>>(Gy, Gs, Gq, nq, ldg, rWr, var_df, P, n_real, Mc, rows, f, beta, se, sfve, ldo, max_F);
     return check_launch("k_wald_finish");
