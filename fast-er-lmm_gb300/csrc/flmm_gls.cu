@@ -83,9 +83,10 @@ __device__ void back_solve(const double* L, int C, double* x) {
 }
 
 // Weighted Gram of the augmented columns a_0..a_C = (x~_0 .. x~_{C-1}, y) at one delta, by one warp:
-// Gs[i * (C + 1) + j] = sum_n a_i[n] a_j[n] / (s[n] + delta) for j <= i.  Returns sum_n log(s[n] + delta).
+// Gs[i * (C + 1) + j] = sum_n a_i[n] a_j[n] / (s[n] + delta) for j <= i, over the lane's samples first, first + step, ...
+// Returns sum_n log(s[n] + delta).
 __device__ double warp_gram(const double* __restrict__ s, int N, const double* __restrict__ Xrt, int64_t ldx, int C,
-                            const double* __restrict__ y, double delta, double* Gs) {
+                            const double* __restrict__ y, double delta, double* Gs, int first, int step) {
     const int lane = threadIdx.x & 31;
     const int K = C + 1;
     const int pairs = K * (K + 1) / 2;
@@ -103,7 +104,7 @@ __device__ double warp_gram(const double* __restrict__ s, int N, const double* _
         i0 = i;
         j0 = j;
         double acc[kPairChunk] = {};
-        for (int n = lane; n < N; n += 32) {
+        for (int n = first; n < N; n += step) {
             const double sd = s[n] + delta;
             const double w = 1.0 / sd;
             if (q0 == 0) sl += log(sd);
@@ -152,7 +153,7 @@ __device__ double warp_pheno_loss(const double* __restrict__ s, int N, const dou
                                   int C, const double* __restrict__ y, double ld, bool reml, double* Gs, double* A,
                                   double* z) {
     const int lane = threadIdx.x & 31;
-    const double sum_log = warp_gram(s, N, Xrt, ldx, C, y, exp(ld), Gs);
+    const double sum_log = warp_gram(s, N, Xrt, ldx, C, y, exp(ld), Gs, lane, 32);
     double loss = 0.0;
     if (lane == 0) loss = gram_loss(Gs, sum_log, N, C, reml, A, z);
     __syncwarp();
@@ -433,24 +434,32 @@ k_gls_golden_block(const double* __restrict__ s, int N, const double* __restrict
 // Null fit of column p at its log delta (fasterlmm/core.py:328-341): A_p, L_p (identity when the Cholesky fails),
 // beta_x = A^-1 u, r = y~ - X~ beta_x, rWr = sum w r^2, and the left operands of the scan, rows of N entries: w o r at
 // Rv, w at Wv (column pitch rv_stride), and C rows at Qv (column pitch qv_stride): w o x~_c, or with `solved` the rows
-// of L^-1 X~^T W, whose products with a variant are the terms of B^T A^-1 B as squares.
-__global__ void k_gls_wald_prep(const double* __restrict__ s, int N, const double* __restrict__ Xrt, int64_t ldx,
-                                int C, const double* __restrict__ Yrt, int64_t ldy, int P,
-                                const double* __restrict__ ld, int solved, double* __restrict__ Rv,
-                                double* __restrict__ Wv, int64_t rv_stride, double* __restrict__ Qv, int64_t qv_stride,
-                                double* __restrict__ Lp, double* __restrict__ rWr) {
+// of L^-1 X~^T W, whose products with a variant are the terms of B^T A^-1 B as squares.  A block a column: a warp's
+// chains of FP64 operations are slow on this pipe, so four share a column's samples (660 columns x 800 samples, C = 5: 0.28
+// ms with four columns a block, a warp each, 0.24 with one; 0.18 here).
+constexpr int kPrepThreads = 128;
+
+__global__ void __launch_bounds__(kPrepThreads)
+k_gls_wald_prep(const double* __restrict__ s, int N, const double* __restrict__ Xrt, int64_t ldx, int C,
+                const double* __restrict__ Yrt, int64_t ldy, const double* __restrict__ ld, int solved,
+                double* __restrict__ Rv, double* __restrict__ Wv, int64_t rv_stride, double* __restrict__ Qv,
+                int64_t qv_stride, double* __restrict__ Lp, double* __restrict__ rWr) {
     extern __shared__ double sm[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t p = static_cast<int64_t>(blockIdx.x) * kEvalWarps + warp;
-    if (p >= P) return;
-    double* Gs = sm + warp * eval_smem_doubles(C);
-    double* A = Gs + (C + 1) * (C + 1);
+    __shared__ double red[kPrepThreads / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, K = C + 1;
+    const int64_t p = blockIdx.x;
+    double* Gs = sm;  // a Gram of each warp's samples, added into the first
+    double* A = Gs + (kPrepThreads / 32) * K * K;
     double* z = A + C * C;
     const double* y = Yrt + p * ldy;
     const double delta = exp(ld[p]);
-    warp_gram(s, N, Xrt, ldx, C, y, delta, Gs);
-    if (lane == 0) {
-        const int K = C + 1;
+    warp_gram(s, N, Xrt, ldx, C, y, delta, Gs + warp * K * K, tid, kPrepThreads);
+    __syncthreads();
+    for (int e = tid; e < K * K; e += kPrepThreads)
+        if (e % K <= e / K)
+            for (int w = 1; w < kPrepThreads / 32; ++w) Gs[e] += Gs[w * K * K + e];
+    __syncthreads();
+    if (tid == 0) {
         for (int i = 0; i < C; ++i) {
             for (int j = 0; j <= i; ++j) A[i * C + j] = Gs[i * K + j];
             z[i] = Gs[C * K + i];
@@ -465,11 +474,11 @@ __global__ void k_gls_wald_prep(const double* __restrict__ s, int N, const doubl
             for (int i = 0; i < C * C; ++i) L[i] = A[i];
         }
     }
-    __syncwarp();
+    __syncthreads();
     double* rv = Rv + p * rv_stride;
     double* wv = Wv + p * rv_stride;
     double acc = 0.0;
-    for (int n = lane; n < N; n += 32) {
+    for (int n = tid; n < N; n += kPrepThreads) {
         const double w = 1.0 / (s[n] + delta);
         double fit = 0.0;
         for (int c = 0; c < C; ++c) fit = fma(Xrt[c * ldx + n], z[c], fit);
@@ -489,7 +498,12 @@ __global__ void k_gls_wald_prep(const double* __restrict__ s, int N, const doubl
         wv[n] = w;
     }
     acc = warp_sum(acc);
-    if (lane == 0) rWr[p] = acc;
+    if (lane == 0) red[warp] = acc;
+    __syncthreads();
+    if (tid == 0) {
+        for (int w = 1; w < kPrepThreads / 32; ++w) acc += red[w];
+        rWr[p] = acc;
+    }
 }
 
 constexpr int WP = 16, WM = 16, WK = 8, WT = 256;
@@ -791,9 +805,8 @@ extern "C" int flmm_wald_gls_f64(const double* s, int N, const double* Xrt, int6
         return fail(FLMM_ERR_WORKSPACE, "flmm_wald_gls_f64: need %zu bytes, got %zu", wald_ws(N, C, P), work_bytes);
     if (P == 0 || M == 0) return FLMM_OK;
     cudaStream_t st = as_stream(stream);
-    const size_t smem_prep = eval_smem_bytes(C);
-    if (smem_prep > 48 * 1024)
-        FLMM_CUDA(cudaFuncSetAttribute(k_gls_wald_prep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_prep));
+    const size_t smem_prep = sizeof(double) * ((kPrepThreads / 32) * static_cast<size_t>(C + 1) * (C + 1) +
+                                               static_cast<size_t>(C) * C + (C + 1));
     // Large scans: the products (w o r)^T s, w^T (s o s) and (L^-1 X~^T W) s on the tensor cores from digit planes.  The
     // tile kernel reads two shared-memory operands per FP64 multiply-add and reached 0.87 TFLOP/s (660 columns x 4,000
     // variants x 800 samples, C = 5: 33.9 ms).
@@ -806,8 +819,8 @@ extern "C" int flmm_wald_gls_f64(const double* s, int N, const double* Xrt, int6
             const int pc = P - p0 < w.pc ? P - p0 : w.pc;
             const int nr = n_real > p0 ? (n_real - p0 < pc ? n_real - p0 : pc) : 0;
             const int64_t half = static_cast<int64_t>(pc) * N, gs = static_cast<int64_t>(pc) * (M < w.mc ? M : w.mc);
-            k_gls_wald_prep<<<ceil_div(pc, kEvalWarps), 32 * kEvalWarps, smem_prep, st>>>(
-                s, N, Xrt, ldx, C, Yrt + static_cast<int64_t>(p0) * ldy, ldy, pc, log_delta + p0, 1, w.RW, w.RW + half, N,
+            k_gls_wald_prep<<<pc, kPrepThreads, smem_prep, st>>>(
+                s, N, Xrt, ldx, C, Yrt + static_cast<int64_t>(p0) * ldy, ldy, log_delta + p0, 1, w.RW, w.RW + half, N,
                 w.Q, static_cast<int64_t>(C) * N, nullptr, w.rWr);
             if ((rc = check_launch("k_gls_wald_prep"))) return rc;
             const OzOperand rw = oz_carve(w.rw_op, pc, N, 2, kOzRowsA), qo = oz_carve(w.q_op, pc * C, N, 1, kOzRowsA);
@@ -840,8 +853,8 @@ extern "C" int flmm_wald_gls_f64(const double* s, int N, const double* Xrt, int6
         double* Lv = static_cast<double*>(work);
         double* Lp = Lv + static_cast<size_t>(pc) * (C + 2) * N;
         double* rWr = Lp + static_cast<size_t>(pc) * C * C;
-        k_gls_wald_prep<<<ceil_div(pc, kEvalWarps), 32 * kEvalWarps, smem_prep, st>>>(
-            s, N, Xrt, ldx, C, Yrt + static_cast<int64_t>(q0) * ldy, ldy, pc, log_delta + q0, 0, Lv,
+        k_gls_wald_prep<<<pc, kPrepThreads, smem_prep, st>>>(
+            s, N, Xrt, ldx, C, Yrt + static_cast<int64_t>(q0) * ldy, ldy, log_delta + q0, 0, Lv,
             Lv + static_cast<int64_t>(C + 1) * N, static_cast<int64_t>(C + 2) * N, Lv + N,
             static_cast<int64_t>(C + 2) * N, Lp, rWr);
         if ((rc = check_launch("k_gls_wald_prep"))) return rc;
