@@ -63,7 +63,9 @@ constexpr int kInvitBlock = 16;     // elements whose loads a recurrence pass is
 constexpr double kClusterTol = 1e-5;
 constexpr int kSectPts = 3;        // points per multisection step of the eigenvalue brackets (its quarters)
 constexpr int kBisectSteps = 24;   // 4^-24 = 2^-48 of the Gershgorin interval
-constexpr int kBisectThreads = 128;
+// one warp a block: the eigenvalues' warps spread over all SMs (20 x 1,000 with blocks of 128: 0.67 -> 0.60 and, inverse
+// iteration, 2.32 -> 2.02 ms; 8 x 1,600 0.88 -> 0.74 and 2.95 -> 2.90)
+constexpr int kBisectThreads = 32, kInvitThreads = 32;
 
 __device__ __forceinline__ uint32_t cta_rank() {
     uint32_t r;
@@ -1057,7 +1059,7 @@ int eigh_own_f32(float* A, int N, int batch, float* evals, void* work, cudaStrea
         d, e, N, evals, tn);
     if ((rc = check_launch("k_tridiag_bisect"))) return rc;
     // 3. eigenvectors of T
-    k_tridiag_invit<<<dim3(ceil_div(N, 128), batch), 128, 0, st>>>(d, e, evals, tn, N, S, Z);
+    k_tridiag_invit<<<dim3(ceil_div(N, kInvitThreads), batch), kInvitThreads, 0, st>>>(d, e, evals, tn, N, S, Z);
     if ((rc = check_launch("k_tridiag_invit"))) return rc;
     k_cluster_orth<<<dim3(ceil_div(N, kOrthCols), batch), kOrthThreads, sizeof(float) * N, st>>>(evals, tn, N, Z);
     if ((rc = check_launch("k_cluster_orth"))) return rc;
