@@ -8,8 +8,9 @@
 //
 // Each unit is ~20 launches of a few microseconds for ordinary studies, and issuing them from Python cost 10-20 us each:
 // 150 samples x 1,500 variants on 16 chromosomes took 10.2 ms in 505 launches, 4.35 unit by unit and 3.00 grouped.  What
-// depends on the spectra alone (mean, FP32 copies, sWs node weights and their split) and the projections run for all units in one launch each.
-// Where every unit's column operands fit kGroupBytes together, so does the rest (run_grouped): the launches then take all
+// depends on the spectra alone (mean, FP32 copies, sWs node weights and their split) and the projections run for all units
+// in one launch each.  Where every unit's operands fit kGroupBytes together, so does the rest (run_grouped): the launches
+// then take all
 // units' rows, the split products with the units' tiles one after another.  The arithmetic is in every form that of the
 // C entry points called one by one.
 #include <cuda_fp16.h>
@@ -198,8 +199,8 @@ extern "C" int flmm_loco_kinships_f32(flmm_context* ctx, const double* Zt, int N
 namespace {
 
 // Grouped launches when every unit's column operands (eigenvectors, rotated phenotypes and their weighted rows) take at
-// most this much: 150 x 1,500 on 16 chromosomes 4.35 -> 3.00 ms, 563 x 20,011 on 22 15.1 -> 12.5, 1,600 x 6,000 on 8
-// 169 -> 162.  With more columns a unit's launches fill the device for many waves, and the second stream hides the rest.
+// most this much together, and the variants' (rotations and their halves) too: 150 x 1,500 on 16 chromosomes 4.35 -> 3.00
+// ms, 563 x 20,011 on 22 15.1 -> 12.5, 1,600 x 6,000 on 8 169 -> 162.  With more columns a unit's launches fill the device for many waves, and the second stream hides the rest.
 constexpr size_t kGroupBytes = size_t{1} << 30;
 
 struct UnitBufs {
@@ -251,8 +252,9 @@ int carve_units(Arena& a, const flmm_units* q, bool group, UnitBufs* b) {
         total += q->unit_count[u];
     }
     const size_t columns = U * b->ldk * 4 * (pad8(q->N) + 2 * P);
+    const size_t variants = static_cast<size_t>(total) * (12 * b->ldk + 4 * (b->ldr + pad8(b->R)));
     b->grouped = dense && total < (int64_t{1} << 30) && U * std::max<size_t>(P, b->ldk) < (size_t{1} << 30) &&
-                 columns <= kGroupBytes;
+                 columns <= kGroupBytes && variants <= kGroupBytes;
     if (b->grouped) {
         UnitBufs::Slot& s = b->slot[0];
         s.Us = take_split(a, static_cast<int64_t>(U) * b->ldk, pad8(q->N));
@@ -282,7 +284,7 @@ int carve_units(Arena& a, const flmm_units* q, bool group, UnitBufs* b) {
     b->F = a.of<float>(M * b->ldr);
     b->Fs = take_split(a, M, pad8(b->R));
     const int64_t tests = static_cast<int64_t>(M) * q->n_real;
-    const int64_t most = q->refine_cap * (b->grouped ? int64_t{q->n_units} : 1);
+    const int64_t most = q->refine_cap * (b->grouped ? std::min<int64_t>(q->n_units, 16) : 1);
     b->cap = q->opts.f_refine > 0.0 ? static_cast<int>(std::min<int64_t>({tests, most, INT_MAX / 2})) : 0;
     b->flags = a.of<int32_t>(2 * static_cast<size_t>(b->cap));
     b->flag_count = a.of<int32_t>(1);
