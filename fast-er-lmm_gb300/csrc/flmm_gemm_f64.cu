@@ -179,7 +179,7 @@ extern "C" int flmm_gemm_nt_f64_tc(const double* A, int64_t lda, const double* B
         for (int i0 = 0; i0 < Mr; i0 += ra) {
             const OzOperand a = oz_carve(wa, Mr - i0 < ra ? Mr - i0 : ra, K, 1, kOzRowsA);
             if ((rc = oz_digits(a, 0, A + i0 * lda, lda, false, nullptr, 0, st))) return rc;
-            const OzProduct p{A + i0 * lda, lda, 0, B + j0 * ldb, ldb, {false, false}, false, C + i0 * ldc + j0, ldc, 0,
+            const OzProduct p{A + i0 * lda, lda, 0, B + j0 * ldb, ldb, {false, false}, OzGate::kPlain, C + i0 * ldc + j0, ldc, 0,
                               D ? D + i0 * ldd + j0 : nullptr, ldd};
             if ((rc = oz_gemm(a, b, p, st))) return rc;
         }

@@ -638,7 +638,7 @@ struct WaldWs {
     double *RW, *Q, *rWr;   // w o r and w (2, pc, N), L^-1 X~^T W (pc, C, N)
     double *G, *Gq;         // sums: num and sWs (2, pc, mc), the quadratic form's terms (pc, C, mc)
     char *rw_op, *q_op, *s_op;
-    int* bal;               // balancing exponents, N
+    int* bal;               // balancing exponents and their scratch
     size_t bytes;
 };
 
@@ -666,7 +666,7 @@ WaldWs carve_wald(void* base, int N, int C, int P) {
     w.rw_op = reinterpret_cast<char*>(take(oz_operand_bytes(w.pc, N, 2, kOzRowsA)));
     w.q_op = reinterpret_cast<char*>(take(oz_operand_bytes(w.pc * C, N, 1, kOzRowsA)));
     w.s_op = reinterpret_cast<char*>(take(oz_operand_bytes(w.mc, N, 2, kOzRowsB)));
-    w.bal = reinterpret_cast<int*>(take(sizeof(int) * n));
+    w.bal = reinterpret_cast<int*>(take(sizeof(int) * oz_balance_ints(N)));
     w.bytes = off + 1024;
     return w;
 }
@@ -826,7 +826,8 @@ extern "C" int flmm_wald_gls_f64(const double* s, int N, const double* Xrt, int6
             const OzOperand rw = oz_carve(w.rw_op, pc, N, 2, kOzRowsA), qo = oz_carve(w.q_op, pc * C, N, 1, kOzRowsA);
             if ((rc = oz_digits(rw, 0, w.RW, N, false, w.bal, 1, st))) return rc;
             if ((rc = oz_digits(rw, 1, w.RW + half, N, false, w.bal, 2, st))) return rc;
-            if ((rc = oz_digits(qo, 0, w.Q, N, false, w.bal, 1, st))) return rc;
+            // (L^-1 X~^T W W^-1/2 has orthonormal rows: a term is at most sqrt(w^T (s o s)), so its rows are held against w)
+            if ((rc = oz_digits(qo, 0, w.Q, N, false, w.bal, 1, st, OzWeights{&rw, C}))) return rc;
             auto out = [&](double* x) { return nr > 0 ? x + p0 : nullptr; };
             for (int m0 = 0; m0 < M; m0 += w.mc) {
                 const int mc = M - m0 < w.mc ? M - m0 : w.mc;
@@ -834,9 +835,8 @@ extern "C" int flmm_wald_gls_f64(const double* s, int N, const double* Xrt, int6
                 const OzOperand so = oz_carve(w.s_op, mc, N, 2, kOzRowsB);
                 if ((rc = oz_digits(so, 0, S, lds, false, w.bal, -1, st))) return rc;
                 if ((rc = oz_digits(so, 1, S, lds, true, w.bal, -2, st))) return rc;
-                const OzProduct g{w.RW, N, half, S, lds, {false, true}, false, w.G, mc, gs, nullptr, 0};
-                // what is left of the intercept's row is rounding of either input: any ratio will do
-                const OzProduct gq{w.Q, N, 0, S, lds, {false, false}, true, w.Gq, mc, 0, nullptr, 0};
+                const OzProduct g{w.RW, N, half, S, lds, {false, true}, OzGate::kBalanced, w.G, mc, gs, nullptr, 0};
+                const OzProduct gq{w.Q, N, 0, S, lds, {false, false}, OzGate::kTerms, w.Gq, mc, 0, nullptr, 0};
                 if ((rc = oz_gemm(rw, so, g, st))) return rc;
                 if ((rc = oz_gemm(qo, so, gq, st))) return rc;
                 if ((rc = wald_finish(w.G, w.G + gs, w.Gq, C, mc, w.rWr, static_cast<double>(N - C - 1), pc, nr, mc,

@@ -11,12 +11,13 @@
 // 8 * 512 * 2^12 = 2^24 in magnitude: every accumulation is exact.  The epilogue converts the level sums to integers
 // and adds them into two 64-bit integers per output (levels 0..3 and 4..7), exactly, over all chunks, and rounds once:
 //     C = 2^(e_a + e_b - 61) (2^28 hi + lo).
-// What is lost is the rounding to 55 bits and the levels from 8 on (weight 2^-56 against the row maxima).  For rows
-// whose largest entry is a few times their rms this is several times smaller than the rounding of an FP64 sum of K
-// terms (~0.4 * 2^-53 * K times the rms product; measured against exact sums in tests/test_gpu_oz64.py).  The loss
-// grows with max/rms of both rows (after balancing, oz_balance), so every tile of rows carries its largest ratio; a tile
-// pair whose product of ratios exceeds quality_limit(K), and any row that is not finite or whose exponent is out of range, is left to
-// k_marked_f64, which forms those tiles on the FP64 pipe as before.
+// What is lost is the rounding to 55 bits and the levels from 8 on (weight 2^-56 against the row maxima): fixed-point
+// operands, whose entries far below their row's largest hold fewer bits than FP64's.  For rows whose largest entry is a few
+// times their usual one this is smaller than the rounding of an FP64 sum of K terms (at K = 800 a scan's sums are 0.1 to 0.4
+// of it off, at K = 100 0.3 to 0.9; measured against exact sums in tests/test_gpu_oz64.py).  The loss grows with the spread
+// of both rows (after balancing, oz_balance), so every tile of rows carries its largest ratio; a tile pair whose product of
+// ratios exceeds quality_limit, and any row that is not finite or whose exponent is out of range, is left to k_marked_f64,
+// which forms those tiles on the FP64 pipe.
 //
 // Kernel: persistent CTA pairs; tiles of 256 A rows (128 a CTA) x 64 B rows, 8 levels x 64 columns = all of tensor memory.
 // Warp 0 of each CTA issues its TMA loads: a stage is 16 deep, 8 x 4 KB of its own A rows and 8 x 1 KB of half the B rows =
@@ -27,7 +28,6 @@
 // an MMA's operands moved to uniform registers one by one, neither form went below 73 cycles an MMA.  Both products of 660
 // columns x 4,000 variants x 800 samples with 5 covariates: 1.19 -> 0.78 ms (pairs by themselves 1.24).
 #include <cuda.h>
-#include <float.h>
 #include <math.h>
 
 #include <algorithm>
@@ -61,10 +61,24 @@ constexpr int kSmemBytes = kStages * kStageBytes + kEpiWarps * kOutBytes + 256 +
 constexpr int kMaxExp = 450;  // |e| beyond this: the scale 2^(e_a + e_b - 61) could leave FP64's range
 static_assert(kTmemCols == 512 && kSmemBytes <= 227 * 1024 && kEpiCols == 16, "budgets");
 
-// Largest product of two tiles' max/rms ratios that the digits take.  Measured on a scan's operands at K = 1,000 (rms
-// against exact sums, relative to the row norms): ratios 10 x 5 leave 1.1e-17 where the FP64 sum leaves 3.9e-17, so the
-// two meet near a product of 150, and both errors scale so that the line goes with sqrt(K).
-__host__ __device__ inline float quality_limit(int K) { return 4.0f * sqrtf(static_cast<float>(K)); }
+// Largest product of two tiles' qualities that the digits take.  The loss of a sum is ~2^-56 sqrt(K) of the product of the
+// row maxima.
+//   kPlain (max/rms): an FP64 sum of terms of either sign is off by ~2^-53 K / 5 of the rms product, so the line goes with
+//   sqrt(K).  Measured on a scan's operands at K = 1,000, relative to the row norms: ratios 10 x 5 leave 1.1e-17 where the
+//   FP64 sum leaves 3.9e-17, so the two meet near a product of 150.
+//   kBalanced (max/mean, which unlike max/rms keeps growing when one entry dominates a row: balancing can put a row's
+//   largest entry where the other row is small, and max/rms of such a row is sqrt(K) at most): normal rows have 1.6 times the
+//   ratio, hence 6 sqrt(K).  With one entry of A 16 times and that of B a sixteenth of the others (K = 400, product 2.8
+//   sqrt(K)) the digits lose 2.1 times what the FP64 sum does, and 4 times at 5.3 sqrt(K) (K = 100).  A sum of
+//   non-negative terms is off by 2^-53 K^1.5 / 6 of the product of means: the two meet near 0.7 K.
+//   kTerms: with A over sqrt(mean w) the loss of a term is 2^-56 of the product against sqrt(sum w b^2), twice that of the
+//   term's square against sum w b^2, whose own FP64 sum is off by 2^-53 sqrt(K) / 6.
+__host__ inline float quality_limit(OzGate gate, bool square, int K) {
+    const float k = static_cast<float>(K), root = sqrtf(k);
+    if (gate == OzGate::kPlain) return 4.0f * root;
+    if (gate == OzGate::kTerms) return 0.7f * root;
+    return square ? 0.75f * k : 6.0f * root;
+}
 
 struct OzMaps {
     CUtensorMap a, b;
@@ -90,21 +104,46 @@ struct OzArgs {
 
 constexpr int kMaxBalance = 150;  // |e_k| used at most
 
-// bal[k] = largest high word of |X[., k]| (k_balance), then its exponent (k_balance_exp).  A block reads 32 columns of a
-// range of rows.
+// most[g][k] = largest high word of the finite |X[., k]| over the rows of group g (k_balance), then the exponent of the
+// groups' median (k_balance_exp).  A block reads 32 columns of a group.
 __global__ void __launch_bounds__(256)
-k_balance(const double* __restrict__ X, int64_t ldx, int rows, int K, int* __restrict__ bal) {
-    const int k = blockIdx.x * 32 + (threadIdx.x & 31);
-    if (k >= K) return;
+k_balance(const double* __restrict__ X, int64_t ldx, int rows, int K, int* __restrict__ most) {
+    __shared__ int red[8][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int k = blockIdx.x * 32 + lane, g = blockIdx.y;
+    const int r1 = static_cast<int>(static_cast<int64_t>(rows) * (g + 1) / gridDim.y);
     int m = 0;
-    for (int64_t r = blockIdx.y * 8 + (threadIdx.x >> 5); r < rows; r += gridDim.y * 8)
-        m = max(m, __double2hiint(X[r * ldx + k]) & 0x7fffffff);
-    atomicMax(bal + k, m);
+    if (k < K) {
+        const int* x = reinterpret_cast<const int*>(X) + 1;  // high words
+#pragma unroll 8
+        for (int r = static_cast<int>(static_cast<int64_t>(rows) * g / gridDim.y) + warp; r < r1; r += 8) {
+            const int h = x[2 * (r * ldx + k)] & 0x7fffffff;
+            m = h < 0x7ff00000 ? max(m, h) : m;
+        }
+    }
+    red[warp][lane] = m;
+    __syncthreads();
+    if (warp == 0 && k < K) {
+        for (int w = 1; w < 8; ++w) m = max(m, red[w][lane]);
+        most[static_cast<int64_t>(g) * K + k] = m;
+    }
 }
 
-__global__ void k_balance_exp(int* __restrict__ bal, int K) {
+__global__ void k_balance_exp(const int* __restrict__ most, int groups, int* __restrict__ bal, int K) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < K) bal[k] = max(-kMaxBalance, min(kMaxBalance, (bal[k] >> 20) - 1023));
+    if (k >= K) return;
+    int x[kOzBalanceGroups];
+#pragma unroll
+    for (int g = 0; g < kOzBalanceGroups; ++g) x[g] = g < groups ? most[static_cast<int64_t>(g) * K + k] : 0x7fffffff;
+    int mid = 0;
+#pragma unroll
+    for (int g = 0; g < kOzBalanceGroups; ++g) {
+        int below = 0;  // groups before this one in order
+#pragma unroll
+        for (int h = 0; h < kOzBalanceGroups; ++h) below += x[h] < x[g] || (x[h] == x[g] && h < g);
+        if (below == (groups - 1) / 2) mid = x[g];
+    }
+    bal[k] = max(-kMaxBalance, min(kMaxBalance, (mid >> 20) - 1023));
 }
 
 // One warp per row.  Pass 1: the row's largest |x 2^c| (c = times bal_k) as its bit pattern (integer maximum); pass 2: the
@@ -113,7 +152,8 @@ __global__ void k_balance_exp(int* __restrict__ bal, int K) {
 template <bool SQ>
 __global__ void __launch_bounds__(256)
 k_digits64(const double* __restrict__ X, int64_t ldx, int rows, int K, const int* __restrict__ bal, int times,
-           __half* __restrict__ planes, int64_t ldp, int* __restrict__ expo, float* __restrict__ qual, int tile_rows) {
+           __half* __restrict__ planes, int64_t ldp, int* __restrict__ expo, float* __restrict__ mean,
+           float* __restrict__ qual, int tile_rows, const int* __restrict__ w_expo, const float* __restrict__ w_mean, int per) {
     const int lane = threadIdx.x & 31;
     const int64_t j = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5;
     if (j >= rows) return;
@@ -138,7 +178,7 @@ k_digits64(const double* __restrict__ X, int64_t ldx, int rows, int K, const int
     const int e = mb == 0 ? 0 : static_cast<int>(mb >> 52) - 1022;  // max = f 2^e, f in [0.5, 1)
     const bool bad = e > kMaxExp || e < -kMaxExp;                   // includes infinities, NaN and denormals
     __half* out = planes + j * ldp;
-    float ss = 0.0f;
+    float ss = 0.0f, sa = 0.0f;
     for (int n = 2 * lane; n < (K + kBK - 1) / kBK * kBK; n += 64) {
         long long v[2] = {0, 0};
         if (!bad) {
@@ -151,6 +191,7 @@ k_digits64(const double* __restrict__ X, int64_t ldx, int rows, int K, const int
                 v[h] = __double2ll_rn(y * __longlong_as_double(static_cast<long long>(up) << 52));
                 const float t = static_cast<float>(static_cast<int>(v[h] >> 32)) * 0x1p-23f;
                 ss = fmaf(t, t, ss);
+                sa += fabsf(t);
             }
         }
 #pragma unroll
@@ -171,10 +212,20 @@ k_digits64(const double* __restrict__ X, int64_t ldx, int rows, int K, const int
         }
     }
     ss = warp_sum(ss);
+    sa = warp_sum(sa);
     if (lane == 0) {
         expo[j] = bad ? 0 : e;
-        const float top = mb == 0 ? 1.0f : static_cast<float>(__longlong_as_double((mb & 0xfffffffffffffull) | (1022ull << 52)));
-        const float q = bad ? INFINITY : (mb == 0 ? 1.0f : fmaxf(1.0f, top * sqrtf(static_cast<float>(K) / ss)));
+        const float n = static_cast<float>(K), m = sa / n;
+        mean[j] = m;
+        const float top = static_cast<float>(__longlong_as_double((mb & 0xfffffffffffffull) | (1022ull << 52)));  // over 2^e
+        float q;
+        if (mb == 0) q = 1.0f;  // zeros
+        else if (w_expo != nullptr) {
+            const int ew = w_expo[j / per];
+            q = ldexpf(top * rsqrtf(ldexpf(w_mean[j / per], ew & 1)), e - (ew >> 1));
+        }
+        else q = bal != nullptr ? top / m : top * sqrtf(n / ss);
+        q = !bad && q < INFINITY ? fmaxf(w_expo != nullptr ? 0.0f : 1.0f, q) : INFINITY;
         atomicMax(reinterpret_cast<int*>(qual) + j / tile_rows, __float_as_int(q));
     }
 }
@@ -208,7 +259,7 @@ __device__ __forceinline__ Tile tile_at(int t, int tiles_i, int tiles_m) {
 }
 
 __device__ __forceinline__ bool tile_good(const OzArgs& a, const Tile& t) {
-    // (an infinite quality makes the product infinite: qualities are at least 1, or 0 for tiles past the rows)
+    // (an infinite quality makes the product infinite, or NaN with a zero one: neither is within the limit)
     return t.ti < a.tiles_i && a.qa[t.b * a.tiles_i + t.ti] * a.qb[t.b * a.tiles_m + t.tm] <= a.limit[t.b];
 }
 
@@ -497,7 +548,8 @@ namespace flmm {
 size_t oz_operand_bytes(int rows, int K, int batches, int tile_rows) {
     const size_t ldp = (static_cast<size_t>(K) + kBK - 1) / kBK * kRowElems, n = static_cast<size_t>(rows) * batches;
     const size_t tiles = static_cast<size_t>((rows + tile_rows - 1) / tile_rows) * batches;
-    return align_up(sizeof(__half) * n * ldp) + align_up(sizeof(int) * n) + align_up(sizeof(float) * tiles);
+    return align_up(sizeof(__half) * n * ldp) + align_up(sizeof(int) * n) + align_up(sizeof(float) * n) +
+           align_up(sizeof(float) * tiles);
 }
 
 OzOperand oz_carve(void* base, int rows, int K, int batches, int tile_rows) {
@@ -513,31 +565,35 @@ OzOperand oz_carve(void* base, int rows, int K, int batches, int tile_rows) {
     p += align_up(sizeof(__half) * n * op.ldp);
     op.expo = reinterpret_cast<int*>(p);
     p += align_up(sizeof(int) * n);
+    op.mean = reinterpret_cast<float*>(p);
+    p += align_up(sizeof(float) * n);
     op.qual = reinterpret_cast<float*>(p);
     return op;
 }
 
 int oz_balance(const double* X, int64_t ldx, int rows, int K, int* bal, cudaStream_t st) {
-    FLMM_CUDA(cudaMemsetAsync(bal, 0, sizeof(int) * K, st));
-    const int by = (rows + 63) / 64;
-    k_balance<<<dim3(ceil_div(K, 32), by < 1 ? 1 : (by < 64 ? by : 64)), 256, 0, st>>>(X, ldx, rows, K, bal);
+    const int groups = std::max(1, std::min(rows, kOzBalanceGroups));
+    int* most = bal + K;
+    k_balance<<<dim3(ceil_div(K, 32), groups), 256, 0, st>>>(X, ldx, rows, K, most);
     int rc = check_launch("k_balance");
     if (rc) return rc;
-    k_balance_exp<<<ceil_div(K, 256), 256, 0, st>>>(bal, K);
+    k_balance_exp<<<ceil_div(K, 128), 128, 0, st>>>(most, groups, bal, K);
     return check_launch("k_balance_exp");
 }
 
 int oz_digits(const OzOperand& op, int b, const double* X, int64_t ldx, bool square, const int* bal, int times,
-              cudaStream_t st) {
+              cudaStream_t st, OzWeights weights) {
     if (op.rows == 0) return FLMM_OK;
     const int64_t off = static_cast<int64_t>(b) * op.rows;
     float* qual = op.qual + static_cast<int64_t>(b) * op.tiles();
     k_zero_f32<<<ceil_div(op.tiles(), 256), 256, 0, st>>>(qual, op.tiles());
     int rc = check_launch("k_zero_f32");
     if (rc) return rc;
+    const int64_t w_off = weights.op ? weights.op->rows : 0;  // (batch 1)
     auto* k = square ? k_digits64<true> : k_digits64<false>;
     k<<<ceil_div(static_cast<int64_t>(op.rows) * 32, 256), 256, 0, st>>>(
-        X, ldx, op.rows, op.K, bal, times, op.planes + off * op.ldp, op.ldp, op.expo + off, qual, op.tile_rows);
+        X, ldx, op.rows, op.K, bal, times, op.planes + off * op.ldp, op.ldp, op.expo + off, op.mean + off, qual, op.tile_rows,
+        weights.op ? weights.op->expo + w_off : nullptr, weights.op ? weights.op->mean + w_off : nullptr, weights.per);
     return check_launch("k_digits64");
 }
 
@@ -571,9 +627,7 @@ int oz_gemm(const OzOperand& A, const OzOperand& B, const OzProduct& p, cudaStre
     a.eb = B.expo;
     a.qa = A.qual;
     a.qb = B.qual;
-    // a sum of products of non-negative numbers grows with its length, and with it an FP64 sum's own rounding
-    for (int b = 0; b < 2; ++b)
-        a.limit[b] = p.any_ratio ? FLT_MAX : quality_limit(A.K) * (p.square[b] ? 4.0f : 1.0f);
+    for (int b = 0; b < 2; ++b) a.limit[b] = quality_limit(p.gate, p.square[b], A.K);
     a.C = p.C;
     a.ldc = p.ldc;
     a.c_stride = p.c_stride;

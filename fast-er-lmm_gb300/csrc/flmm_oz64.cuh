@@ -18,7 +18,8 @@ constexpr int kOzRowsB = 64;      // B rows per tile
 struct OzOperand {
     __half* planes;   // [batch][row][ldp]
     int* expo;        // [batch][row]
-    float* qual;      // [batch][tile]: largest max|x| / rms(x) of a tile's rows, infinity where digits cannot hold a row
+    float* mean;      // [batch][row]: mean |x| over 2^expo
+    float* qual;      // [batch][tile]: largest quality of a tile's rows (oz_digits), infinity where digits cannot hold a row
     int64_t ldp;
     int rows, K, batches, tile_rows;
     int tiles() const { return (rows + tile_rows - 1) / tile_rows; }
@@ -27,19 +28,36 @@ struct OzOperand {
 size_t oz_operand_bytes(int rows, int K, int batches, int tile_rows);
 OzOperand oz_carve(void* base, int rows, int K, int batches, int tile_rows);
 
-// Balancing exponents of a product's reduction: e_k of the largest |X[., k]| over the rows of X (pitch ldx), K ints.  A
-// product's operands may be digitised as A 2^e_k and B 2^-e_k (both squared where B is): the digits then resolve each
-// term against the largest term that the variants leave possible at k, not against an entry of A that meets zeros.
+// Balancing exponents of a product's reduction: e_k of the size that |X[., k]| usually reaches over the rows of X (pitch
+// ldx); bal holds oz_balance_ints(K) ints, e_k in the first K.  A product's operands may be digitised as A 2^e_k and
+// B 2^-e_k (both squared where B is): the digits then resolve each term against the largest term that the variants leave
+// possible at k, not against an entry of A that meets zeros.  e_k is the median of the largest finite entries of
+// kOzBalanceGroups groups of rows: the largest over all rows would let one variant's outlier set the resolution of every
+// column for all the others, and the median entry follows the sample too loosely (rows then spread half as far again).
+constexpr int kOzBalanceGroups = 15;
+inline size_t oz_balance_ints(int K) { return (1 + kOzBalanceGroups) * static_cast<size_t>(K); }
 int oz_balance(const double* X, int64_t ldx, int rows, int K, int* bal, cudaStream_t st);
 
-// Digits of batch `b` of `op` from the rows of X (pitch ldx), or of their squares, times 2^(times bal_k).
+// Digits of batch `b` of `op` from the rows of X (pitch ldx), or of their squares, times 2^(times bal_k).  A row's quality
+// is its largest |x| over the root of its mean square, over its mean |x| where it is balanced, or with `weights` over the
+// root of the mean of row r / per of the weights' batch 1 (balanced by twice `times`).
+struct OzWeights {
+    const OzOperand* op;
+    int per;
+};
 int oz_digits(const OzOperand& op, int b, const double* X, int64_t ldx, bool square, const int* bal, int times,
-              cudaStream_t st);
+              cudaStream_t st, OzWeights weights = {nullptr, 0});
+
+// What a product's tiles must fulfil for their digits to be used (see quality_limit).
+enum class OzGate {
+    kPlain,     // unbalanced operands
+    kBalanced,  // balanced operands; batches of squares are sums of non-negative terms
+    kTerms      // terms whose squares are taken from the weighted sums: A's digits with weights, B's balanced
+};
 
 // C[b] (rows of A, rows of B; pitch ldc, batch stride c_stride) = A[b] B[b]^T, or D - A B^T where D is given (pitch
 // ldd).  Xa, Xb: the FP64 matrices the digits were taken from (Xa with a batch stride; Xb shared by the batches, its
-// elements squared in batch b where square[b] is set), read where a tile's digits are not good enough.  any_ratio: take
-// every finite row whatever its max/rms (for sums whose error only has to be small against the product of the row norms).
+// elements squared in batch b where square[b] is set), read where a tile's digits are not good enough.
 // Operands may hold more batches than the product takes; it takes the smaller count, from batch 0.
 struct OzProduct {
     const double* Xa;
@@ -47,7 +65,7 @@ struct OzProduct {
     const double* Xb;
     int64_t ldb;
     bool square[2];
-    bool any_ratio;
+    OzGate gate;
     double* C;
     int64_t ldc, c_stride;
     const double* D;

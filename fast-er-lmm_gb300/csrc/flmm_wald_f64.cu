@@ -256,7 +256,7 @@ struct WaldWs {
     int pc, mc;                // columns and variants of a block
     double *rWr, *A1, *W, *G;  // A1 and W adjacent (pc, Neff) matrices; G (2, pc, mc)
     char *cols, *vars;         // digit operands of [A1 | W] and [US | US^2]
-    int* bal;                  // balancing exponents, Neff
+    int* bal;                  // balancing exponents and their scratch
     size_t bytes;
 };
 
@@ -279,7 +279,7 @@ WaldWs carve_wald(void* base, int P, int Neff) {
     w.G = reinterpret_cast<double*>(take(2 * sizeof(double) * static_cast<size_t>(w.pc) * w.mc));
     w.cols = reinterpret_cast<char*>(take(oz_operand_bytes(w.pc, Neff, 2, kOzRowsA)));
     w.vars = reinterpret_cast<char*>(take(oz_operand_bytes(w.mc, Neff, 2, kOzRowsB)));
-    w.bal = reinterpret_cast<int*>(take(sizeof(int) * static_cast<size_t>(Neff)));
+    w.bal = reinterpret_cast<int*>(take(sizeof(int) * oz_balance_ints(Neff)));
     w.bytes = off + 1024;
     return w;
 }
@@ -355,8 +355,8 @@ int wald_impl(const double* s, int Neff, const double* UYt, int64_t ldu, const d
             if ((rc = oz_digits(vars, 0, US, ldus, false, w.bal, -1, st))) return rc;
             if ((rc = oz_digits(vars, 1, US, ldus, true, w.bal, -2, st))) return rc;
             const int64_t gs = static_cast<int64_t>(pc) * mc;
-            const OzProduct prod{w.A1, Neff, static_cast<int64_t>(pc) * Neff, US, ldus, {false, true}, false, w.G, mc, gs,
-                                 nullptr, 0};
+            const OzProduct prod{w.A1, Neff, static_cast<int64_t>(pc) * Neff, US, ldus, {false, true},
+                                 OzGate::kBalanced, w.G, mc, gs, nullptr, 0};
             if ((rc = oz_gemm(cols, vars, prod, st))) return rc;
             if ((rc = wald_finish(w.G, w.G + gs, nullptr, 0, mc, w.rWr, var_df, pc, nr, mc, rows ? rows + m0 : rows, out(f),
                                   out(beta), out(se), out(sfve), ldo, max_F + p0, st)))

@@ -190,3 +190,50 @@ def test_weights_that_meet_zeros():
     num, den, rwr = (w * UY) @ US.T, w @ (US * US).T, (w * UY * UY).sum(1)
     se = ((rwr[:, None] - num * num / den) / (Neff - 1) / den).sqrt()
     torch.testing.assert_close(out["se"], se.T, rtol=1e-14, atol=0)
+
+
+def _one_entry_scan(entry, K, M, P, C, bad_at, bad_k):
+    """beta / se (M, P) with the covariates projected out (C = 0) or in the model, variant bad_at[0] holding `entry` at
+    bad_k, and the same in the formulas."""
+    from fasterlmm_gb300 import build, core, gls
+    build()
+    g = torch.Generator(device="cuda").manual_seed(K + C)
+    dev = torch.device("cuda", torch.cuda.current_device())
+    rn = lambda *s: torch.randn(*s, generator=g, device=dev, dtype=torch.float64)
+    s, Y, S, ld, X = rn(K).abs() + 0.05, rn(P, K), rn(M, K), rn(P), rn(max(C, 1), K)
+    if entry is not None:
+        S[bad_at, bad_k] = entry
+    out, max_F = core._alloc_outputs(M, P, P, dev)
+    rows = torch.arange(M, device=dev)
+    w = 1.0 / (s[None, :] + ld.exp()[:, None])
+    if C:
+        gls.wald_t(s, X, Y, ld, S, P, rows, out, max_F)
+        L = torch.linalg.cholesky(torch.einsum("pn,cn,dn->pcd", w, X, X))
+        u = torch.einsum("pn,cn,pn->pc", w, X, Y)
+        r = Y - torch.cholesky_solve(u[:, :, None], L)[:, :, 0] @ X
+        z = torch.linalg.solve_triangular(L, torch.einsum("pn,cn,mn->pcm", w, X, S), upper=False)
+        num, den, rwr, df = (w * r) @ S.T, (w @ (S * S).T) - (z * z).sum(1), (w * r * r).sum(1), K - C - 1
+    else:
+        core.wald_t(s, Y, ld, S, P, rows, out, max_F)
+        num, den, rwr, df = (w * Y) @ S.T, w @ (S * S).T, (w * Y * Y).sum(1), K - 1
+    t = num / ((rwr[:, None] - num * num / den) / df * den).sqrt()
+    return out["beta"] / out["se"], t.T, max_F
+
+
+@pytest.mark.parametrize("entry", [float("nan"), float("inf"), -float("inf"), 1e12, 1e6, 1e3])
+@pytest.mark.parametrize("K,C", [(160, 0), (800, 0), (160, 5), (800, 5)])
+def test_one_entry_of_one_variant(entry, K, C):
+    """A variant that is not finite, or far off, at one index costs the other variants nothing: their statistic
+    t = beta / se is what an FP64 sum of K terms allows.  The sums' rounding is at most K 2^-53 of the row norms on either
+    side, and t = sWy / sqrt(sWs rss / df) takes it times sqrt(df), once for sWy and at |t| / sqrt(df) < 1 for the others."""
+    P, M, at = 260, 700, 333
+    t, ref, max_F = _one_entry_scan(entry, K, M, P, C, at, K // 3)
+    others = torch.ones(M, dtype=torch.bool, device=t.device)
+    others[at] = False
+    atol = 8 * K ** 0.5 * K * 2.0 ** -53
+    torch.testing.assert_close(t[others], ref[others], rtol=0, atol=atol)
+    if abs(entry) < 1e4:  # (further off, one term of the variant's sums is nearly all there is of rss)
+        torch.testing.assert_close(t[at], ref[at], rtol=0, atol=64 * atol)
+    finite = torch.full_like(max_F, abs(entry) < float("inf"), dtype=torch.bool)
+    assert torch.equal(torch.isfinite(t[at]), finite)
+    assert torch.equal(torch.isfinite(max_F), finite)
