@@ -237,3 +237,31 @@ def test_one_entry_of_one_variant(entry, K, C):
     finite = torch.full_like(max_F, abs(entry) < float("inf"), dtype=torch.bool)
     assert torch.equal(torch.isfinite(t[at]), finite)
     assert torch.equal(torch.isfinite(max_F), finite)
+
+
+def _loss_of_digits(a, b):
+    """rms error of a product of rows a and b from the method, over the row norms: the rounding of both to 55 bits, the
+    plane pairs of level 8 (seven, of uniform digits), and the rounding of the result at its own size."""
+    na, nb = np.linalg.norm(a), np.linalg.norm(b)
+    ea, eb = (2.0 ** np.frexp(np.abs(x).max())[1] for x in (a, b))
+    digits = 2.0 ** -56 / 3 ** 0.5 * np.hypot(ea / na, eb / nb)
+    level = 2.0 ** -56 * ea * eb / (na * nb) * (7 * a.size) ** 0.5 * (37.0 ** 2 / 2 ** 12)
+    return np.sqrt(digits ** 2 + level ** 2 + (2.0 ** -53 / 3 ** 0.5 * abs(a @ b) / (na * nb)) ** 2)
+
+
+@pytest.mark.parametrize("K", [48, 160, 400, 1000, 2500])
+def test_products_no_further_off_than_sums(K):
+    """Against exact sums: no further off than the FP64 pipe's chains, or, where those are short, than the method's own loss
+    (1.5: the spread of an rms over 300 samples and digits that are not quite uniform)."""
+    g = torch.Generator(device="cuda").manual_seed(K)
+    A, B = (torch.randn(n, K, generator=g, device="cuda", dtype=torch.float64) for n in (200, 2600))
+    tc, ref = _products(A, B)
+    a, b, tc, ref = (t.cpu().numpy() for t in (A, B, tc, ref))
+    rng = np.random.default_rng(1)
+    at = [(int(rng.integers(200)), int(rng.integers(2600))) for _ in range(300)]
+    scale = lambda i, j: np.linalg.norm(a[i]) * np.linalg.norm(b[j])
+    ex = {ij: _exact(a[ij[0]], b[ij[1]]) for ij in at}
+    err = lambda c: _rms([(c[ij] - ex[ij]) / scale(*ij) for ij in at])
+    loss = _rms([_loss_of_digits(a[i], b[j]) for i, j in at])
+    assert err(tc) <= (err(ref) if K >= 400 else max(err(ref), 1.5 * loss))
+    assert err(tc) <= 1.5 * loss
