@@ -757,8 +757,12 @@ struct Bt {
     static constexpr int kDot = 4 * kTile;             // threads of V^T Z
     static constexpr int kUpd = 8 * kTile;             // and of Z -= V S'
     static constexpr int kThreads = kDot + kUpd;
-    static size_t smem(int N) { return sizeof(float) * (static_cast<size_t>(N + kChunk) * kTile + kRing * 2 * kWy * kChunk); }
+    static constexpr int kMaxN = kTile == 16 ? kSytrdThreads * kOwnCols : 1900;
+    static constexpr size_t smem(int N) {
+        return sizeof(float) * (static_cast<size_t>(N + kChunk) * kTile + kRing * 2 * kWy * kChunk);
+    }
 };
+static_assert(Bt<16>::smem(Bt<16>::kMaxN) <= 222 * 1024 && Bt<24>::smem(Bt<24>::kMaxN) <= 222 * 1024, "shared memory budget");
 
 template <int kTile>
 __global__ void __launch_bounds__(Bt<kTile>::kThreads, kTile == 16 ? 2 : 1)
@@ -928,8 +932,10 @@ template <int kTile>
 int launch_backtransform(const float* W, const float* Tq, const float* Z, int N, int n_refl, int nblocks, int batch, float* U,
                          cudaStream_t st) {
     const size_t smem = Bt<kTile>::smem(N);
-    // (per device, so set on every call; the call is cheap)
-    FLMM_CUDA(cudaFuncSetAttribute(k_backtransform<kTile>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    // (per device, so set on every call, to one bound whatever N, so that another host thread's call never lowers it under
+    // this launch; the call is cheap)
+    FLMM_CUDA(cudaFuncSetAttribute(k_backtransform<kTile>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   static_cast<int>(Bt<kTile>::smem(Bt<kTile>::kMaxN))));
     k_backtransform<kTile><<<dim3(ceil_div(N, kTile), batch), Bt<kTile>::kThreads, smem, st>>>(W, Tq, Z, N, n_refl, nblocks, U);
     return check_launch("k_backtransform");
 }
@@ -1072,7 +1078,7 @@ int eigh_own_f32(float* A, int N, int batch, float* evals, void* work, cudaStrea
     // Two CTAs of 16 columns an SM as long as they fit; then one of 24, as long as that fits (8 x 1,600 x 1,600: 4.61 ms, one
     // of 16 5.61); then one of 16.
     if (N <= 1310) return launch_backtransform<16>(W, Tq, Z, N, n_refl, L.nblocks, batch, A, st);
-    if (N <= 1900) return launch_backtransform<24>(W, Tq, Z, N, n_refl, L.nblocks, batch, A, st);
+    if (N <= Bt<24>::kMaxN) return launch_backtransform<24>(W, Tq, Z, N, n_refl, L.nblocks, batch, A, st);
     return launch_backtransform<16>(W, Tq, Z, N, n_refl, L.nblocks, batch, A, st);
 }
 

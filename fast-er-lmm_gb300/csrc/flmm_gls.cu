@@ -333,6 +333,7 @@ __global__ void k_gls_golden(const double* __restrict__ s, int N, const double* 
 // 2.3 with one block, 1.5 here.  Beyond ~12,000 samples the weights no longer fit in shared memory and k_gls_golden runs.
 constexpr int kBlockThreads = 256;
 constexpr int kBlockPairs = 4;
+constexpr size_t kBlockSmemMax = 200 * 1024;
 
 size_t golden_block_smem(int N, int C) {
     return sizeof(double) * (2 * static_cast<size_t>(N) + static_cast<size_t>(C + 1) * (C + 1) + static_cast<size_t>(C) * C +
@@ -766,9 +767,9 @@ extern "C" int flmm_fit_delta_gls_f64(const double* s, int N, const double* Xrt,
     k_gls_argmin<<<ceil_div(P, 256), 256, 0, st>>>(ws.loss, n_grid, P, grid_idx);
     if ((rc = check_launch("k_gls_argmin"))) return rc;
     const size_t block_smem = golden_block_smem(N, C);
-    if (refine && block_smem <= 200 * 1024) {
-        if (block_smem > 48 * 1024)
-            FLMM_CUDA(cudaFuncSetAttribute(k_gls_golden_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)block_smem));
+    if (refine && block_smem <= kBlockSmemMax) {
+        // (one bound whatever N: another host thread's call must not lower it under this launch)
+        FLMM_CUDA(cudaFuncSetAttribute(k_gls_golden_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBlockSmemMax));
         k_gls_golden_block<<<2 * P, kBlockThreads, block_smem, st>>>(s, N, Xrt, ldx, C, Yrt, ldy, ws.grid, n_grid, grid_idx,
                                                                  reml, lo, hi, log_delta);
         return check_launch("k_gls_golden_block");

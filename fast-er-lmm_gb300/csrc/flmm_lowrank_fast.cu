@@ -211,6 +211,7 @@ k_lr_prep_variants(const float* __restrict__ USt, int64_t ldus, const double* __
 // is what it spent its time on: 24,576 variants x 20,000 samples in four calls 49 ms, 2.0 here (9 GB of traffic).  The sum of
 // squares stays one warp's compensated sum in the lanes' order.
 constexpr int kPrepThreads = 512;
+constexpr size_t kPrepRowMax = 220 * 1024;  // bytes of a row in shared memory
 
 __global__ void __launch_bounds__(kPrepThreads)
 k_lr_prep_rows(const float* __restrict__ USt, int64_t ldus, const double* __restrict__ Sr, int64_t lds,
@@ -479,10 +480,10 @@ extern "C" int flmm_lr_prep_variants(const float* USt, int64_t ldus, const doubl
                  "flmm_lr_prep_variants: bad arguments (at most 16 covariate columns)");
     if (Mc == 0) return FLMM_OK;
     const size_t row_bytes = sizeof(float) * static_cast<size_t>(N);
-    if (D == 0 && row_bytes <= 220 * 1024) {
-        if (row_bytes > 40 * 1024)
-            FLMM_CUDA(cudaFuncSetAttribute(k_lr_prep_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           static_cast<int>(row_bytes)));
+    if (D == 0 && row_bytes <= kPrepRowMax) {
+        // (one bound whatever N: another host thread's call must not lower it under this launch)
+        FLMM_CUDA(cudaFuncSetAttribute(k_lr_prep_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       static_cast<int>(kPrepRowMax)));
         k_lr_prep_rows<<<Mc, kPrepThreads, row_bytes, as_stream(stream)>>>(
             USt, ldus, Zt, ldz, Ct, ldc, k, N, static_cast<__half*>(B1h), static_cast<__half*>(B1l), ldb, sb1,
             static_cast<__half*>(B2h), static_cast<__half*>(B2l), ldb2, sb2);
