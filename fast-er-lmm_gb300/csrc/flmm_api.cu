@@ -155,6 +155,14 @@ int* flmm::device_err_flag(int device) {
     return flags[device];
 }
 
+bool flmm::use_pair_kernels() {
+    static const bool on = [] {
+        const char* e = std::getenv("FLMM_TC_PAIR");
+        return !(e && e[0] == '0');
+    }();
+    return on;
+}
+
 // both error flags into the context's mapped host buffer
 __global__ void k_read_flags(const int* __restrict__ ctx_flag, const int* __restrict__ dev_flag, int* out) {
     if (threadIdx.x == 0) {

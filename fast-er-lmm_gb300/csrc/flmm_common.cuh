@@ -26,6 +26,9 @@ int* device_err_flag(int device);
 
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
+// tcgen05 kernel form: CTA pairs unless FLMM_TC_PAIR=0 asks for the single-CTA kernels (kept for cross-checks).
+bool use_pair_kernels();
+
 // The library's own batched FP32 eigensolver (csrc/flmm_eigh_own.cu): A (batch, N, N) symmetric in, one eigenvector
 // per row out, evals (batch, N) ascending; work of eigh_own_workspace_bytes(N, batch) bytes.
 size_t eigh_own_workspace_bytes(int N, int batch);

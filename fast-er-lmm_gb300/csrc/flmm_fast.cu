@@ -1169,14 +1169,6 @@ int chunk_kb_for() {
     return v;
 }
 
-// tcgen05 kernel form: CTA pairs unless FLMM_TC_PAIR=0 asks for the single-CTA kernels (kept for cross-checks)
-bool use_pair_kernel() {
-    static const bool on = [] {
-        const char* e = std::getenv("FLMM_TC_PAIR");
-        return !(e && e[0] == '0');
-    }();
-    return on;
-}
 
 // ---- kernel form and tile order: fixed, forced or autotuned ------------------------------------------------------
 //
@@ -1321,7 +1313,7 @@ int choose_product(const TcMaps& maps_tc, const TcMaps& maps_pair, const TcArgs&
 template <int NG>
 int launch_product(const TcMaps& maps_tc, const TcMaps& maps_pair, const TcArgs& a, int n_cl, int sm_count,
                    bool rerunnable, cudaStream_t st) {
-    if (!use_pair_kernel()) n_cl = 0;  // FLMM_TC_PAIR=0: single-CTA kernels only
+    if (!use_pair_kernels()) n_cl = 0;  // FLMM_TC_PAIR=0: single-CTA kernels only
     TcChoice choice;
     int rc = choose_product<NG>(maps_tc, maps_pair, a, n_cl, sm_count, rerunnable, st, &choice);
     return rc ? rc : launch_choice<NG>(maps_tc, maps_pair, a, choice, n_cl, sm_count, st);
@@ -1561,8 +1553,8 @@ namespace {
 int pair_count(int* n_cl1, int* n_cl2) {
     int dev = 0;
     FLMM_CUDA(cudaGetDevice(&dev));
-    *n_cl1 = use_pair_kernel() ? pair_clusters<1>(dev) : 0;
-    *n_cl2 = use_pair_kernel() ? pair_clusters<2>(dev) : 0;
+    *n_cl1 = use_pair_kernels() ? pair_clusters<1>(dev) : 0;
+    *n_cl2 = use_pair_kernels() ? pair_clusters<2>(dev) : 0;
     return FLMM_OK;
 }
 

@@ -17,7 +17,8 @@
 // of it off, at K = 100 0.3 to 0.9; measured against exact sums in tests/test_gpu_oz64.py).  The loss grows with the spread
 // of both rows (after balancing, oz_balance), so every tile of rows carries its largest ratio; a tile pair whose product of
 // ratios exceeds quality_limit, and any row that is not finite or whose exponent is out of range, is left to k_marked_f64,
-// which forms those tiles on the FP64 pipe.
+// which forms those tiles on the FP64 pipe; and all of them where k_oz64 gave up a bounded wait, so that its callers need
+// not wait for the device to see whether it did.
 //
 // Kernel: persistent CTA pairs; tiles of 256 A rows (128 a CTA) x 64 B rows, 8 levels x 64 columns = all of tensor memory.
 // Warp 0 of each CTA issues its TMA loads: a stage is 16 deep, 8 x 4 KB of its own A rows and 8 x 1 KB of half the B rows =
@@ -230,9 +231,10 @@ k_digits64(const double* __restrict__ X, int64_t ldx, int rows, int K, const int
     }
 }
 
-__global__ void k_zero_f32(float* __restrict__ x, int n) {
+__global__ void k_zero_f32(float* __restrict__ x, int n, int* __restrict__ flag) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) x[i] = 0.0f;
+    if (i == 0 && flag) *flag = 0;
 }
 
 // ---- the product ------------------------------------------------------------------------------------------------
@@ -487,14 +489,18 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz64(const __grid_constant__ Oz
 // ---- tiles left to the FP64 pipe ----------------------------------------------------------------------------------
 
 constexpr int kST = 64, kSK = 16, kSThreads = 256;
+constexpr int kNoPairs = 0x01010101;  // error word of a product that k_oz64 was not launched for
 
-// The 64 x 64 tiles of C whose digit tiles are not good, in FP64 (one block per tile; the others leave at once).
+// The 64 x 64 tiles of C whose digit tiles are not good, or all after an error, in FP64 (one block per tile; the others
+// leave at once).  Where D is C and k_oz64 gave up, some of D is gone: all NaN.
 __global__ void __launch_bounds__(kSThreads)
 k_marked_f64(const OzArgs args, const double* __restrict__ Xa, int64_t lda, int64_t xa_stride,
              const double* __restrict__ Xb, int64_t ldb, int square0, int square1) {
     const int b = blockIdx.z;
     const int i0 = blockIdx.y * kST, j0 = blockIdx.x * kST;
-    if (tile_good(args, Tile{b, i0 / kOzRowsA, j0 / kOzRowsB})) return;
+    const int err = *args.err;
+    if (err == 0 && tile_good(args, Tile{b, i0 / kOzRowsA, j0 / kOzRowsB})) return;
+    const bool lost = args.D == args.C && err != 0 && err != kNoPairs;
     __shared__ double As[kSK][kST + 1];
     __shared__ double Bs[kSK][kST + 1];
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
@@ -533,7 +539,8 @@ k_marked_f64(const OzArgs args, const double* __restrict__ Xa, int64_t lda, int6
             const int j = j0 + tx + 16 * c;
             if (i < args.Ma && j < args.Nb) {
                 double* o = args.C + b * args.c_stride + static_cast<int64_t>(i) * args.ldc + j;
-                *o = args.D ? args.D[static_cast<int64_t>(i) * args.ldd + j] - acc[r][c] : acc[r][c];
+                const double v = args.D ? args.D[static_cast<int64_t>(i) * args.ldd + j] - acc[r][c] : acc[r][c];
+                *o = lost ? NAN : v;
             }
         }
     }
@@ -549,7 +556,7 @@ size_t oz_operand_bytes(int rows, int K, int batches, int tile_rows) {
     const size_t ldp = (static_cast<size_t>(K) + kBK - 1) / kBK * kRowElems, n = static_cast<size_t>(rows) * batches;
     const size_t tiles = static_cast<size_t>((rows + tile_rows - 1) / tile_rows) * batches;
     return align_up(sizeof(__half) * n * ldp) + align_up(sizeof(int) * n) + align_up(sizeof(float) * n) +
-           align_up(sizeof(float) * tiles);
+           align_up(sizeof(float) * (tiles + 1));
 }
 
 OzOperand oz_carve(void* base, int rows, int K, int batches, int tile_rows) {
@@ -568,6 +575,7 @@ OzOperand oz_carve(void* base, int rows, int K, int batches, int tile_rows) {
     op.mean = reinterpret_cast<float*>(p);
     p += align_up(sizeof(float) * n);
     op.qual = reinterpret_cast<float*>(p);
+    op.err = reinterpret_cast<int*>(op.qual + static_cast<size_t>(op.tiles()) * batches);
     return op;
 }
 
@@ -586,7 +594,7 @@ int oz_digits(const OzOperand& op, int b, const double* X, int64_t ldx, bool squ
     if (op.rows == 0) return FLMM_OK;
     const int64_t off = static_cast<int64_t>(b) * op.rows;
     float* qual = op.qual + static_cast<int64_t>(b) * op.tiles();
-    k_zero_f32<<<ceil_div(op.tiles(), 256), 256, 0, st>>>(qual, op.tiles());
+    k_zero_f32<<<ceil_div(op.tiles(), 256), 256, 0, st>>>(qual, op.tiles(), b == 0 ? op.err : nullptr);
     int rc = check_launch("k_zero_f32");
     if (rc) return rc;
     const int64_t w_off = weights.op ? weights.op->rows : 0;  // (batch 1)
@@ -610,12 +618,10 @@ int oz_gemm(const OzOperand& A, const OzOperand& B, const OzProduct& p, cudaStre
     if ((rc = tc::make_map_f16(&maps.a, A.planes, static_cast<int>(ra), w, A.ldp, kRowElems / 2, kOzRowsA))) return rc;
     if ((rc = tc::make_map_f16(&maps.b, B.planes, static_cast<int>(rb), w, B.ldp, kRowElems / 2, kOzRowsB / 2))) return rc;
     static PairCache cache;
-    int dev = 0, pairs = 0;
-    FLMM_CUDA(cudaGetDevice(&dev));
-    if ((rc = pair_count(k_oz64, kThreads, kSmemBytes, cache, &pairs))) return rc;
+    int pairs = 0;
+    if (use_pair_kernels() && (rc = pair_count(k_oz64, kThreads, kSmemBytes, cache, &pairs))) return rc;
     OzArgs a{};
-    a.err = device_err_flag(dev);
-    if (!a.err) return fail(FLMM_ERR_CUDA, "oz_gemm: cannot allocate the device error flag");
+    a.err = A.err;
     a.Ma = A.rows;
     a.Nb = B.rows;
     a.K = A.K;
@@ -635,8 +641,12 @@ int oz_gemm(const OzOperand& A, const OzOperand& B, const OzProduct& p, cudaStre
     a.ldd = p.ldd;
     const int64_t tiles = static_cast<int64_t>(a.batches) * a.pairs_i * a.tiles_m;
     pairs = static_cast<int>(std::min<int64_t>(tiles, pairs));
-    if ((rc = launch_pairs(k_oz64, pairs, kThreads, kSmemBytes, st, maps, a))) return rc;
-    if ((rc = check_launch("k_oz64"))) return rc;
+    if (pairs > 0) {
+        if ((rc = launch_pairs(k_oz64, pairs, kThreads, kSmemBytes, st, maps, a))) return rc;
+        if ((rc = check_launch("k_oz64"))) return rc;
+    } else {
+        FLMM_CUDA(cudaMemsetAsync(a.err, kNoPairs & 0xff, sizeof(int), st));
+    }
     const dim3 grid(ceil_div(B.rows, kST), ceil_div(A.rows, kST), a.batches);
     k_marked_f64<<<grid, kSThreads, 0, st>>>(a, p.Xa, p.lda, p.xa_stride, p.Xb, p.ldb, p.square[0], p.square[1]);
     return check_launch("k_marked_f64");

@@ -20,6 +20,7 @@ struct OzOperand {
     int* expo;        // [batch][row]
     float* mean;      // [batch][row]: mean |x| over 2^expo
     float* qual;      // [batch][tile]: largest quality of a tile's rows (oz_digits), infinity where digits cannot hold a row
+    int* err;         // of an operand A: set once a product with it gave up a wait; zeroed with its batch 0's digits
     int64_t ldp;
     int rows, K, batches, tile_rows;
     int tiles() const { return (rows + tile_rows - 1) / tile_rows; }
@@ -57,7 +58,8 @@ enum class OzGate {
 
 // C[b] (rows of A, rows of B; pitch ldc, batch stride c_stride) = A[b] B[b]^T, or D - A B^T where D is given (pitch
 // ldd).  Xa, Xb: the FP64 matrices the digits were taken from (Xa with a batch stride; Xb shared by the batches, its
-// elements squared in batch b where square[b] is set), read where a tile's digits are not good enough.
+// elements squared in batch b where square[b] is set), read where a tile's digits are not good enough, and for all tiles
+// where the kernel gave up one of its bounded waits or CTA pairs are not to be had (FLMM_TC_PAIR=0, or none fits).
 // Operands may hold more batches than the product takes; it takes the smaller count, from batch 0.
 struct OzProduct {
     const double* Xa;

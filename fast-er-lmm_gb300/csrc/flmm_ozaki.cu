@@ -505,6 +505,7 @@ int launch_oz(const __half* aplanes, const int* ea_side, const __half* bplanes, 
     static PairCache cache;
     int pairs = 0;
     if ((rc = pair_count(k_ozaki<PA, PB, LV, F64>, Cfg::kThreads, Cfg::kSmemBytes, cache, &pairs))) return rc;
+    if (pairs < 1) return fail(FLMM_ERR_CUDA, "k_ozaki: no CTA pair fits on the device");
     int dev = 0;
     FLMM_CUDA(cudaGetDevice(&dev));
     int* err = device_err_flag(dev);

@@ -8,6 +8,10 @@ cannot hold (not finite, exponents out of range, one entry far above the rest) t
 from __future__ import annotations
 
 import math
+import os
+import subprocess
+import sys
+from pathlib import Path
 
 import numpy as np
 import pytest
@@ -265,3 +269,35 @@ def test_products_no_further_off_than_sums(K):
     loss = _rms([_loss_of_digits(a[i], b[j]) for i, j in at])
     assert err(tc) <= (err(ref) if K >= 400 else max(err(ref), 1.5 * loss))
     assert err(tc) <= 1.5 * loss
+
+
+NO_PAIRS = """
+import sys
+sys.path[:0] = [{root!r}, {tests!r}]
+import torch
+from fasterlmm_gb300 import _lib, core
+from test_gpu_oz64 import _one_entry_scan, _products
+from fasterlmm_gb300.core import _ptr, _stream, _work
+g = torch.Generator(device="cuda").manual_seed(4)
+A, B, D = (torch.randn(*s, generator=g, device="cuda", dtype=torch.float64) for s in ((300, 200), (400, 200), (300, 400)))
+tc, ref = _products(A, B)
+assert torch.equal(tc, ref)
+want, _ = _products(A, B, D)
+torch.testing.assert_close(want, D - ref, rtol=0, atol=1e-12)
+w, wb = _work.get(A.device, _lib.query_bytes("flmm_gemm_nt_f64_tc_workspace_bytes", 300, 400, 200))
+_lib.call("flmm_gemm_nt_f64_tc", _ptr(A), 200, _ptr(B), 200, _ptr(D), 400, _ptr(D), 400, 300, 400, 200, w, wb, _stream(A.device))
+assert torch.equal(D, want)
+for C in (0, 3):
+    t, ref, _ = _one_entry_scan(None, 200, 600, 200, C, 0, 0)
+    torch.testing.assert_close(t, ref, rtol=0, atol=8 * 200 ** 1.5 * 2.0 ** -53)
+print("formed on the FP64 pipe")
+"""
+
+
+def test_without_the_tensor_cores():
+    """Every tile on the FP64 pipe, as after a wait that k_oz64 gave up: FLMM_TC_PAIR=0 keeps CTA pairs out of the process."""
+    tests = Path(__file__).resolve().parent
+    code = NO_PAIRS.format(root=str(tests.parent / "fast-er-lmm_gb300"), tests=str(tests))
+    r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, FLMM_TC_PAIR="0"), capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0 and "formed on the FP64 pipe" in r.stdout, r.stderr[-2000:]
