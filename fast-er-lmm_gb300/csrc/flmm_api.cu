@@ -8,9 +8,9 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
-#include <new>
-
+#include <memory>
 #include <mutex>
+#include <new>
 #include <system_error>
 #include <thread>
 
@@ -34,8 +34,8 @@ struct flmm_context {
     cudaStream_t workers[kEighWorkers] = {};
     cusolverDnHandle_t wsolver[kEighWorkers] = {};
     cudaEvent_t fork = nullptr;
-    cudaEvent_t join[kEighWorkers] = {};
-    std::mutex workers_mu;  // one caller at a time on the worker handles
+    cudaEvent_t join[kEighWorkers] = {};  // the last work on each worker handle, on whichever stream
+    std::mutex workers_mu;  // one caller at a time on the worker handles, streams and events
     cusolverDnParams_t params = nullptr;
 };
 
@@ -266,25 +266,30 @@ extern "C" int flmm_eigh_many(flmm_context* ctx, double* const* A, const int* si
     if (count == 1) return flmm_eigh(ctx, A[0], sizes[0], evals[0], work, work_bytes, stream);
     const int slots = count < kEighWorkers ? count : kEighWorkers;
     const size_t slice = need / slots;
-    size_t one[kEighWorkers] = {};
+    // (the queries run on the context's main handle: before the threads, not in them)
+    const std::unique_ptr<size_t[]> one(new (std::nothrow) size_t[count]);
+    if (!one) return fail(FLMM_ERR_ARG, "flmm_eigh_many: out of host memory");
+    for (int b = 0; b < count; ++b)
+        if ((rc = flmm_eigh_workspace_bytes(ctx, sizes[b], &one[b]))) return rc;
+    cudaError_t device[kEighWorkers] = {};
     int status[kEighWorkers] = {};
     std::lock_guard<std::mutex> lock(ctx->workers_mu);
     cudaStream_t st = as_stream(stream);
     FLMM_CUDA(cudaEventRecord(ctx->fork, st));
     for (int w = 0; w < slots; ++w) {
         FLMM_CUDA(cudaStreamWaitEvent(ctx->workers[w], ctx->fork, 0));
+        FLMM_CUDA(cudaStreamWaitEvent(ctx->workers[w], ctx->join[w], 0));
         cusolverDnSetStream(ctx->wsolver[w], ctx->workers[w]);
     }
     auto run = [&](int w) {
-        if (cudaSetDevice(ctx->device) != cudaSuccess) { status[w] = -1; return; }
+        if ((device[w] = cudaSetDevice(ctx->device)) != cudaSuccess) return;
         char* base = static_cast<char*>(work) + slice * static_cast<size_t>(w);
         for (int b = w; b < count && status[w] == 0; b += slots) {
             const int N = sizes[b];
-            if (flmm_eigh_workspace_bytes(ctx, N, &one[w])) { status[w] = -1; return; }
             status[w] = static_cast<int>(cusolverDnDsyevd(
                 ctx->wsolver[w], CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER, N, A[b], N, evals[b],
-                reinterpret_cast<double*>(base), static_cast<int>((one[w] - 256) / sizeof(double)),
-                reinterpret_cast<int*>(base + one[w] - 256)));
+                reinterpret_cast<double*>(base), static_cast<int>((one[b] - 256) / sizeof(double)),
+                reinterpret_cast<int*>(base + one[b] - 256)));
         }
     };
     std::thread threads[kEighWorkers];
@@ -303,6 +308,8 @@ extern "C" int flmm_eigh_many(flmm_context* ctx, double* const* A, const int* si
         if (e == cudaSuccess) e = cudaStreamWaitEvent(st, ctx->join[w], 0);
         if (e != cudaSuccess) joined = e;
     }
+    for (int w = 0; w < slots; ++w)
+        if (device[w] != cudaSuccess) return fail(FLMM_ERR_CUDA, "flmm_eigh_many: %s", cudaGetErrorString(device[w]));
     for (int w = 0; w < slots; ++w)
         if (status[w] != 0) return solver_fail(static_cast<cusolverStatus_t>(status[w]), "cusolverDnDsyevd (worker)");
     if (joined != cudaSuccess) return fail(FLMM_ERR_CUDA, "flmm_eigh_many: %s", cudaGetErrorString(joined));
@@ -366,10 +373,16 @@ extern "C" int flmm_eigh_batched(flmm_context* ctx, double* A, int N, int batch,
         if ((rc = batched_api_sizes(ctx, N, batch, &L))) return rc;
         int* info = reinterpret_cast<int*>(static_cast<char*>(work) + (L.dev_bytes - align_up(sizeof(int) * batch, 256)));
         cusolverDnHandle_t hdl = slot < 0 ? ctx->solver : ctx->wsolver[slot];
+        std::unique_lock<std::mutex> lock(ctx->workers_mu, std::defer_lock);
+        if (slot >= 0) {
+            lock.lock();
+            FLMM_CUDA(cudaStreamWaitEvent(st, ctx->join[slot], 0));
+        }
         cusolverDnSetStream(hdl, st);
         cusolverStatus_t cs = cusolverDnXsyevBatched(hdl, ctx->params, CUSOLVER_EIG_MODE_VECTOR,
                                                      CUBLAS_FILL_MODE_LOWER, N, CUDA_R_64F, A, N, CUDA_R_64F, evals,
                                                      CUDA_R_64F, work, L.dev_bytes, nullptr, 0, info, batch);
+        if (slot >= 0) FLMM_CUDA(cudaEventRecord(ctx->join[slot], st));
         if (cs != CUSOLVER_STATUS_SUCCESS) return solver_fail(cs, "cusolverDnXsyevBatched");
         return check_cuda("cusolverDnXsyevBatched");
     }
@@ -378,8 +391,12 @@ extern "C" int flmm_eigh_batched(flmm_context* ctx, double* A, int N, int batch,
     if ((rc = flmm_eigh_workspace_bytes(ctx, N, &one))) return rc;
     const int slots = batch < kEighWorkers ? batch : kEighWorkers;
     const int lwork = static_cast<int>((one - 256) / sizeof(double));
+    std::lock_guard<std::mutex> lock(ctx->workers_mu);
     FLMM_CUDA(cudaEventRecord(ctx->fork, st));
-    for (int w = 0; w < slots; ++w) FLMM_CUDA(cudaStreamWaitEvent(ctx->workers[w], ctx->fork, 0));
+    for (int w = 0; w < slots; ++w) {
+        FLMM_CUDA(cudaStreamWaitEvent(ctx->workers[w], ctx->fork, 0));
+        FLMM_CUDA(cudaStreamWaitEvent(ctx->workers[w], ctx->join[w], 0));
+    }
     for (int w = 0; w < slots; ++w) cusolverDnSetStream(ctx->wsolver[w], ctx->workers[w]);
     for (int b = 0; b < batch; ++b) {
         const int w = b % slots;

@@ -1,6 +1,8 @@
 """
 Host threads with problems of different sizes on one device: a call's settings of a kernel (its shared-memory limit is one
 value per function and device) must not reach another thread's launch.
+
+The context's worker handles, streams and events serve one caller at a time, whichever entry point takes them.
 """
 from __future__ import annotations
 
@@ -82,3 +84,66 @@ def test_two_sizes_at_once(make, sizes, calls):
     for t in threads:
         t.join()
     assert not errors
+
+
+def test_worker_handles_shared_by_threads():
+    """flmm_eigh_many, flmm_eigh_batched on the workers and on one of their handles, from three host threads on one context:
+    every decomposition has the bits that it has alone."""
+    from fasterlmm_gb300 import _lib, build, core
+    build()
+    dev = torch.device("cuda", torch.cuda.current_device())
+    ctx = _lib.context(dev.index)
+    g = torch.Generator(device=dev).manual_seed(1)
+    src = [torch.randn(5, n, n, generator=g, device=dev, dtype=torch.float64) for n in (150, 180, 200)]
+    src = [x + x.mT for x in src]
+
+    def many(A):
+        n, N = A.shape[0], A.shape[1]
+        ev = torch.empty(n, N, dtype=torch.float64, device=dev)
+        sizes = (_lib.C.c_int * n)(*[N] * n)
+        nbytes = _lib.query_bytes("flmm_eigh_many_workspace_bytes", ctx, sizes, n)
+        work = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+        at = lambda t: (_lib.C.c_void_p * n)(*(x.data_ptr() for x in t))
+        _lib.call("flmm_eigh_many", ctx, at(A), sizes, n, at(ev), core._ptr(work), nbytes, core._stream(dev))
+        return ev
+
+    def batched(mode, slot):
+        def run(A):
+            ev = torch.empty(A.shape[0], A.shape[1], dtype=torch.float64, device=dev)
+            nbytes = _lib.query_bytes("flmm_eigh_batched_workspace_bytes", ctx, A.shape[1], A.shape[0], mode)
+            work = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+            _lib.call("flmm_eigh_batched", ctx, core._ptr(A), A.shape[1], A.shape[0], core._ptr(ev), mode, slot,
+                      core._ptr(work), nbytes, core._stream(dev))
+            return ev
+        return run
+
+    calls = [many, batched(2, -1), batched(1, 2)]
+    alone = []
+    for call, x in zip(calls, src):
+        A = x.clone()
+        alone.append((call(A), A))
+    torch.cuda.synchronize()
+    wrong, errors = [], []
+    start = threading.Barrier(len(calls))
+
+    def work(k):
+        torch.cuda.set_device(dev)
+        stream = torch.cuda.Stream()
+        try:
+            with torch.cuda.stream(stream):
+                start.wait()
+                for _ in range(20):
+                    A = src[k].clone()
+                    ev = calls[k](A)
+                    stream.synchronize()
+                    if not (torch.equal(ev, alone[k][0]) and torch.equal(A, alone[k][1])):
+                        wrong.append(k)
+        except Exception as e:  # (a thread's failure would otherwise pass unseen)
+            errors.append(repr(e))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(len(calls))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors and not wrong
