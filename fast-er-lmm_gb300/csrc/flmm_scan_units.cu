@@ -316,10 +316,15 @@ struct Events {
 };
 
 int check_units(const flmm_units* q) {
-    FLMM_REQUIRE(q && q->N > q->D && q->D >= 1 && q->P >= 0 && q->n_real >= 0 && q->n_real <= q->P && q->n_units > 0 &&
-                     q->unit_start && q->unit_count && q->opts.n_grid >= 1 && q->opts.log_delta_max > q->opts.log_delta_min &&
-                     q->refine_cap >= 0,
+    // (F has N - D - 1 degrees of freedom; a grid of one value, log_delta_min = log_delta_max, fixes delta)
+    FLMM_REQUIRE(q && q->N > q->D + 1 && q->D >= 1 && q->P >= 0 && q->n_real >= 0 && q->n_real <= q->P && q->n_units > 0 &&
+                     q->unit_start && q->unit_count && q->opts.n_grid >= 1 && std::isfinite(q->opts.log_delta_min) &&
+                     std::isfinite(q->opts.log_delta_max) && q->refine_cap >= 0 &&
+                     q->opts.log_delta_max - q->opts.log_delta_min < 1e8,
                  "flmm_scan_units: bad arguments");
+    double x0 = 0.0;
+    FLMM_REQUIRE(interp_nodes(q->opts.log_delta_min, q->opts.log_delta_max, &x0) >= kInterpQ,
+                 "flmm_scan_units: log_delta_max below log_delta_min");
     for (int u = 0; u < q->n_units; ++u)
         FLMM_REQUIRE(q->unit_start[u] >= 0 && q->unit_count[u] >= 0, "flmm_scan_units: bad unit %d", u);
     return FLMM_OK;

@@ -43,6 +43,9 @@ def _scan(monkeypatch, python: bool, **kw):
     dict(shape=(60, 80, 2, 40, 6), chrom=np.repeat([1, 2], 40), patch=dict(PIPELINE=False)),
     dict(shape=(60, 80, 2, 40, 6), chrom=np.repeat([1, 2], 40), patch=dict(REFINE_F=None), n_grid=17, refine=False),
     dict(shape=(60, 80, 2, 40, 6), chrom=np.repeat([1, 2], 40), patch=dict(REFINE_F=0.5, REFINE_CAP=8)),
+    dict(shape=(60, 80, 2, 40, 6), chrom=np.repeat([1, 2], 40), patch=dict(REFINE_CAP=1 << 40)),
+    dict(shape=(60, 80, 2, 40, 6), chrom=np.repeat([1, 2], 40), log_delta_min=0.5, log_delta_max=0.5),
+    dict(shape=(60, 80, 2, 40, 6), chrom=np.repeat([1, 2], 40), log_delta_min=0.5, log_delta_max=0.5, n_grid=1),
 ])
 def test_native_loop_gives_the_python_loops_bits(monkeypatch, case):
     a, none = _scan(monkeypatch, False, **{**case})
@@ -78,3 +81,19 @@ def test_a_chromosome_that_holds_every_variant_is_refused(monkeypatch):
     from fasterlmm_gb300 import _lib
     with pytest.raises(_lib.FlmmError):
         _scan(monkeypatch, False, shape=(40, 30, 1, 5, 2), chrom=np.zeros(30, dtype=int))
+
+
+@pytest.mark.parametrize("python", [False, True])
+def test_one_sample_more_than_covariates_is_refused(monkeypatch, python):
+    """F would have no degrees of freedom."""
+    from fasterlmm_gb300 import _lib
+    with pytest.raises(_lib.FlmmError):
+        _scan(monkeypatch, python, shape=(9, 60, 8, 20, 3), chrom=np.repeat([1, 2, 3], 20))
+
+
+@pytest.mark.parametrize("kw", [dict(log_delta_min=float("nan")), dict(log_delta_max=float("inf")),
+                                dict(log_delta_min=2.0, log_delta_max=-2.0)])
+def test_bad_delta_ranges_are_refused(monkeypatch, kw):
+    from fasterlmm_gb300 import _lib
+    with pytest.raises((_lib.FlmmError, ValueError, OverflowError)):
+        _scan(monkeypatch, False, shape=(60, 80, 2, 40, 6), chrom=np.repeat([1, 2], 40), **kw)
