@@ -84,20 +84,29 @@ def basis_t(Gt: Tensor, basis: CovariateBasis, sv_floor: float = 1e-10) -> tuple
     return _basis_of(evals, V, Gr, sv_floor)
 
 
+def _one_gram_for_all(rows: int, sizes: list[int]) -> bool:
+    """Whether the Gram of all rows should be formed once for selections of these sizes: if that is less work than one each,
+    and at most twice the memory of the largest (a panel that is nearly one chromosome has one small selection and a Gram
+    of its own size squared)."""
+    return bool(sizes) and rows * rows <= min(sum(k * k for k in sizes), 2 * max(sizes) ** 2)
+
+
 def loco_bases(Gt: Tensor, keeps: list[Tensor], basis: CovariateBasis, sv_floor: float = 1e-10):
-    """basis_t(Gt[keep], basis) for every row selection, one at a time.  The rows are regressed once, their Gram is formed
-    once and each selection's is a part of it; the decompositions run side by side, as many as eigh_groups holds."""
+    """basis_t(Gt[keep], basis) for every row selection, one at a time.  The rows are regressed once; where that is the
+    smaller job their Gram is formed once and each selection's is a part of it (the same bits); the decompositions run side
+    by side, as many as eigh_groups holds."""
     N = Gt.shape[1]
     Gr = basis.regress_out(Gt)
-    gram = rotate_rows(Gr, Gr) if any(k.numel() < N for k in keeps) else None
+    gram = rotate_rows(Gr, Gr) if _one_gram_for_all(Gr.shape[0], [k.numel() for k in keeps if k.numel() < N]) else None
     for group in eigh_groups([min(k.numel(), N) for k in keeps]):
         mats = []
         for i in group:
             k = keeps[i]
-            if k.numel() < N:
+            if k.numel() < N and gram is not None:
                 mats.append(gram.index_select(0, k).index_select(1, k))
-            else:
-                mats.append(kinship_from_gram(gram_t(Gr.index_select(0, k)), None, k.numel()))
+                continue
+            rows = Gr.index_select(0, k)
+            mats.append(rotate_rows(rows, rows) if k.numel() < N else kinship_from_gram(gram_t(rows), None, k.numel()))
         for i, V, evals in zip(group, mats, eigh_many(mats)):
             yield _basis_of(evals, V, Gr.index_select(0, keeps[i]), sv_floor)
 

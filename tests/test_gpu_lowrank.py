@@ -88,3 +88,25 @@ def test_lowrank_loco_single_k_and_block_engines_match_golden(golden):
     rs = lowrank.loco_scan_blocks(source, sorted(np.unique(chrom).tolist()), Zs.shape[1], _t(Gs), g["chrom_kin"],
                                   _t(g["X"]), _t(g["Y_all"]), n_real=B, dtype=torch.float64)
     assert_scan_close(_np(rs), g)
+
+
+@pytest.mark.parametrize("sizes,N", [((20, 25, 30, 15), 200), ((30, 31), 100), ((300, 14, 26), 90), ((60, 14, 26), 90),
+                                     ((700, 5), 64)])
+def test_loco_bases_form_no_gram_larger_than_their_selections_need(monkeypatch, sizes, N):
+    """The basis of every selection has basis_t's bits, whether its Gram is its own or a part of one for all rows, and no
+    Gram has over twice the entries of the largest that a basis is taken from."""
+    from fasterlmm_gb300 import lowrank
+    g = torch.Generator(device=DEV).manual_seed(N)
+    rn = lambda *s: torch.randn(*s, generator=g, device=DEV, dtype=torch.float64)
+    chrom = torch.from_numpy(np.repeat(np.arange(len(sizes)), sizes)).to(DEV)
+    Gt = rn(chrom.numel(), N)
+    basis = lowrank.CovariateBasis(torch.cat([torch.ones(N, 1, device=DEV, dtype=torch.float64), rn(N, 2)], 1))
+    keeps = [torch.nonzero(chrom != c).flatten() for c in range(len(sizes))]
+    alone = [lowrank.basis_t(Gt[k], basis) for k in keeps]
+    formed, rotate = [0], lowrank.rotate_rows
+    monkeypatch.setattr(lowrank, "rotate_rows",
+                        lambda A, B: (formed.append(A.shape[0] ** 2 if A is B else 0), rotate(A, B))[1])
+    got = list(lowrank.loco_bases(Gt, keeps, basis))
+    assert max(formed) <= 2 * max(min(k.numel(), N) for k in keeps) ** 2
+    for (s, U), (s1, U1) in zip(got, alone, strict=True):
+        assert torch.equal(s, s1) and torch.equal(U, U1)
