@@ -630,11 +630,13 @@ GridWs carve_grid(void* base, int N, int C, int P, int G) {
 constexpr int kWaldChunk = 4096;  // columns prepared per pass of the FP64 tile kernel
 
 // Blocks of the tensor-core path: (C + 2) operand rows per column, kBlockRows rows and kBlockM variants at most, fewer
-// where their digit planes (16 bytes per element) would pass kPlaneBytes.
+// where their digit planes (16 bytes per element) would pass kPlaneBytes.  A shorter workspace gets smaller blocks, and the
+// FP64 tile kernel's where the smallest do not fit.
 constexpr int kBlockRows = 6144, kBlockM = 4096;
 constexpr size_t kPlaneBytes = size_t(256) << 20;
 
 struct WaldWs {
+    bool tensor;
     int pc, mc;             // columns and variants of a block
     double *RW, *Q, *rWr;   // w o r and w (2, pc, N), L^-1 X~^T W (pc, C, N)
     double *G, *Gq;         // sums: num and sWs (2, pc, mc), the quadratic form's terms (pc, C, mc)
@@ -643,14 +645,11 @@ struct WaldWs {
     size_t bytes;
 };
 
-WaldWs carve_wald(void* base, int N, int C, int P) {
+WaldWs carve_blocks(void* base, int N, int C, int columns, int variants) {
     WaldWs w{};
-    const size_t fit = kPlaneBytes / (16 * static_cast<size_t>(N));
-    const size_t rows = fit < static_cast<size_t>(kBlockRows) ? fit : kBlockRows;
-    w.pc = static_cast<int>(rows / (C + 2));
-    w.pc = w.pc < 1 ? 1 : (P < w.pc ? (P > 0 ? P : 1) : w.pc);
-    w.mc = static_cast<int>(fit / 2 < static_cast<size_t>(kBlockM) ? fit / 2 / kOzRowsB * kOzRowsB : kBlockM);
-    w.mc = w.mc < kOzRowsB ? kOzRowsB : w.mc;
+    w.tensor = true;
+    w.pc = columns;
+    w.mc = variants;
     size_t off = 0;
     const uintptr_t b0 = (reinterpret_cast<uintptr_t>(base) + 1023) / 1024 * 1024;
     auto take = [&](size_t n) {
@@ -672,11 +671,42 @@ WaldWs carve_wald(void* base, int N, int C, int P) {
     return w;
 }
 
-size_t wald_ws(int N, int C, int P) {
-    const size_t pc = static_cast<size_t>(P < kWaldChunk ? P : kWaldChunk);
-    const size_t tiles = sizeof(double) * (pc * (C + 2) * N + pc * C * C + pc) + 1024;
-    const size_t tensor = carve_wald(nullptr, N, C, P).bytes;
-    return tiles > tensor ? tiles : tensor;
+// The FP64 tile kernel's workspace for pc columns: operands of (C + 2) rows, factors, rWr.
+size_t tile_column_bytes(int N, int C) {
+    return sizeof(double) * ((static_cast<size_t>(C) + 2) * N + static_cast<size_t>(C) * C + 1);
+}
+size_t tile_bytes(int N, int C, int P) { return tile_column_bytes(N, C) * (P < kWaldChunk ? P : kWaldChunk) + 1024; }
+
+// The blocks of a scan of P columns x M variants in `bytes` of workspace (pc: columns of a pass also of the tile kernel).
+WaldWs carve_wald(void* base, int N, int C, int P, int M, size_t bytes) {
+    const size_t fit = kPlaneBytes / (16 * static_cast<size_t>(N));
+    const size_t rows = fit < static_cast<size_t>(kBlockRows) ? fit : kBlockRows;
+    int pc = static_cast<int>(rows / (C + 2));
+    pc = pc < 1 ? 1 : (P < pc ? (P > 0 ? P : 1) : pc);
+    int mc = static_cast<int>(fit / 2 < static_cast<size_t>(kBlockM) ? fit / 2 / kOzRowsB * kOzRowsB : kBlockM);
+    mc = mc < kOzRowsB ? kOzRowsB : mc;
+    const int most = (M > 0 ? (M - 1) / kOzRowsB + 1 : 1) * kOzRowsB;
+    if (most < mc) mc = most;
+    for (; oz_worth(static_cast<int64_t>(pc) * (C + 2), M < mc ? M : mc, N);) {
+        const WaldWs w = carve_blocks(base, N, C, pc, mc);
+        if (w.bytes <= bytes) return w;
+        if (mc > 512 || (pc == 1 && mc > kOzRowsB)) mc = (mc / 2 + kOzRowsB - 1) / kOzRowsB * kOzRowsB;
+        else if (pc > 1) pc = (pc + 1) / 2;
+        else break;
+    }
+    WaldWs w{};
+    w.mc = M;
+    const size_t columns = bytes / tile_column_bytes(N, C);
+    w.pc = P < kWaldChunk ? P : kWaldChunk;
+    if (columns < static_cast<size_t>(w.pc)) w.pc = static_cast<int>(columns);
+    w.bytes = tile_bytes(N, C, P);
+    return w;
+}
+
+size_t wald_ws(int N, int C, int P) { return carve_wald(nullptr, N, C, P, kBlockM, SIZE_MAX).bytes; }
+size_t wald_least(int N, int C, int P) {
+    const size_t tiles = tile_bytes(N, C, P), full = wald_ws(N, C, P);
+    return tiles < full ? tiles : full;
 }
 
 __global__ void k_shift_diagonal(double* __restrict__ A, int N, int64_t lda, double v) {
@@ -802,8 +832,8 @@ extern "C" int flmm_wald_gls_f64(const double* s, int N, const double* Xrt, int6
     FLMM_REQUIRE(M == 0 || Srt, "flmm_wald_gls_f64: Srt is NULL");
     int rc = check_c(C, "flmm_wald_gls_f64");
     if (rc) return rc;
-    if (work_bytes < wald_ws(N, C, P))
-        return fail(FLMM_ERR_WORKSPACE, "flmm_wald_gls_f64: need %zu bytes, got %zu", wald_ws(N, C, P), work_bytes);
+    if (work_bytes < wald_least(N, C, P))
+        return fail(FLMM_ERR_WORKSPACE, "flmm_wald_gls_f64: need %zu bytes, got %zu", wald_least(N, C, P), work_bytes);
     if (P == 0 || M == 0) return FLMM_OK;
     cudaStream_t st = as_stream(stream);
     const size_t smem_prep = sizeof(double) * ((kPrepThreads / 32) * static_cast<size_t>(C + 1) * (C + 1) +
@@ -811,8 +841,8 @@ extern "C" int flmm_wald_gls_f64(const double* s, int N, const double* Xrt, int6
     // Large scans: the products (w o r)^T s, w^T (s o s) and (L^-1 X~^T W) s on the tensor cores from digit planes.  The
     // tile kernel reads two shared-memory operands per FP64 multiply-add and reached 0.87 TFLOP/s (660 columns x 4,000
     // variants x 800 samples, C = 5: 33.9 ms).
-    const WaldWs w = carve_wald(work, N, C, P);
-    if (oz_worth(static_cast<int64_t>(w.pc) * (C + 2), M < w.mc ? M : w.mc, N)) {
+    const WaldWs w = carve_wald(work, N, C, P, M, work_bytes);
+    if (w.tensor) {
         // (the rotated intercept is one entry, where every centred variant is ~0 and w largest: balanced, it no longer
         // sets its rows' resolution)
         if ((rc = oz_balance(Srt, lds, M, N, w.bal, st))) return rc;
@@ -849,8 +879,8 @@ extern "C" int flmm_wald_gls_f64(const double* s, int N, const double* Xrt, int6
         return FLMM_OK;
     }
     const size_t smem_wald = sizeof(double) * (static_cast<size_t>(WP) * (C + 2) * WK + WM * WK);
-    for (int q0 = 0; q0 < P; q0 += kWaldChunk) {
-        const int pc = (P - q0 < kWaldChunk) ? P - q0 : kWaldChunk;
+    for (int q0 = 0; q0 < P; q0 += w.pc) {
+        const int pc = P - q0 < w.pc ? P - q0 : w.pc;
         double* Lv = static_cast<double*>(work);
         double* Lp = Lv + static_cast<size_t>(pc) * (C + 2) * N;
         double* rWr = Lp + static_cast<size_t>(pc) * C * C;

@@ -5,6 +5,9 @@
 // variants whose sums an epilogue kernel reads back (16 bytes per test); 1,100 columns x 4,096 variants x 995 with its
 // rotation: 23.9 -> 1.83 ms.  Small products stay in the fused FP64 tile kernel, which needs one launch.
 #include <math.h>
+#include <stdint.h>
+
+#include <algorithm>
 
 #include "flmm_common.cuh"
 #include "flmm_oz64.cuh"
@@ -243,7 +246,8 @@ k_wald_finish(const double* __restrict__ Gy, const double* __restrict__ Gs, cons
 }
 
 // The scan runs over blocks of at most kBlockP columns x kBlockM variants, fewer where their digit planes (32 bytes
-// per element of a column or variant) would pass kPlaneBytes: the workspace does not grow with P or Mc.
+// per element of a column or variant) would pass kPlaneBytes: the workspace does not grow with P or Mc.  A shorter workspace
+// gets smaller blocks, and the FP64 tile kernel's, which has no planes or sums in memory, where the smallest do not fit.
 constexpr int kBlockP = 2048, kBlockM = 4096;
 constexpr size_t kPlaneBytes = size_t(256) << 20;
 
@@ -253,6 +257,7 @@ int block_rows(int most, int unit, int K) {
 }
 
 struct WaldWs {
+    bool tensor;
     int pc, mc;                // columns and variants of a block
     double *rWr, *A1, *W, *G;  // A1 and W adjacent (pc, Neff) matrices; G (2, pc, mc)
     char *cols, *vars;         // digit operands of [A1 | W] and [US | US^2]
@@ -260,11 +265,14 @@ struct WaldWs {
     size_t bytes;
 };
 
-WaldWs carve_wald(void* base, int P, int Neff) {
+// Columns of the FP64 tile kernel that `bytes` hold; all of P in the shortest workspace that is taken.
+size_t tile_bytes(int P, int Neff) { return sizeof(double) * static_cast<size_t>(P) * (2 * static_cast<size_t>(Neff) + 1) + 512; }
+
+WaldWs carve_blocks(void* base, int pc, int mc, int Neff) {
     WaldWs w{};
-    w.pc = block_rows(kBlockP, kOzRowsA, Neff);
-    if (P < w.pc) w.pc = P > 0 ? P : 1;
-    w.mc = block_rows(kBlockM, kOzRowsB, Neff);
+    w.tensor = true;
+    w.pc = pc;
+    w.mc = mc;
     size_t off = 0;
     const uintptr_t b = reinterpret_cast<uintptr_t>(base);
     const uintptr_t b0 = (b + 1023) / 1024 * 1024;
@@ -284,7 +292,34 @@ WaldWs carve_wald(void* base, int P, int Neff) {
     return w;
 }
 
-size_t wald_ws(int P, int Neff) { return carve_wald(nullptr, P, Neff).bytes; }
+// The blocks of a scan of P columns x Mc variants in `bytes` of workspace.
+WaldWs carve_wald(void* base, int P, int Neff, int Mc, size_t bytes) {
+    int pc = block_rows(kBlockP, kOzRowsA, Neff), mc = block_rows(kBlockM, kOzRowsB, Neff);
+    if (P < pc) pc = P > 0 ? P : 1;
+    const int most = (Mc > 0 ? (Mc - 1) / kOzRowsB + 1 : 1) * kOzRowsB;
+    if (most < mc) mc = most;
+    for (; oz_worth(pc, Mc < mc ? Mc : mc, Neff);) {
+        const WaldWs w = carve_blocks(base, pc, mc, Neff);
+        if (w.bytes <= bytes) return w;
+        if (mc > 512 || (pc <= kOzRowsA && mc > kOzRowsB)) mc = (mc / 2 + kOzRowsB - 1) / kOzRowsB * kOzRowsB;
+        else if (pc > kOzRowsA) pc = (pc / 2 + kOzRowsA - 1) / kOzRowsA * kOzRowsA;
+        else break;
+    }
+    WaldWs w{};
+    w.mc = Mc;
+    w.A1 = static_cast<double*>(base);
+    const size_t column = sizeof(double) * (2 * static_cast<size_t>(Neff) + 1);
+    const size_t fit = bytes / column;
+    w.pc = fit < static_cast<size_t>(P) ? static_cast<int>(fit) : P;
+    w.W = w.A1 + static_cast<size_t>(w.pc) * Neff;
+    w.rWr = w.W + static_cast<size_t>(w.pc) * Neff;
+    w.bytes = tile_bytes(w.pc, Neff);
+    return w;
+}
+
+// What a scan of any number of variants can use (no more than kBlockM at a time), and what it can do with.
+size_t wald_ws(int P, int Neff) { return carve_wald(nullptr, P, Neff, kBlockM, SIZE_MAX).bytes; }
+size_t wald_least(int P, int Neff) { return std::min(wald_ws(P, Neff), tile_bytes(P, Neff)); }
 
 }  // namespace
 
@@ -325,8 +360,8 @@ __global__ void k_spectrum_pad(const double* __restrict__ s, int k, int n0, doub
 // (flmm_oz64.cu) where they are large enough, else in the fused FP64 tile kernel.
 int wald_impl(const double* s, int Neff, const double* UYt, int64_t ldu, const double* log_delta, int P, int n_real,
               const double* USt, int64_t ldus, int Mc, const int64_t* rows, double* f, double* beta, double* se,
-              double* sfve, int64_t ldo, double* max_F, double var_df, void* work, cudaStream_t st) {
-    const WaldWs w = carve_wald(work, P, Neff);
+              double* sfve, int64_t ldo, double* max_F, double var_df, void* work, size_t work_bytes, cudaStream_t st) {
+    const WaldWs w = carve_wald(work, P, Neff, Mc, work_bytes);
     int rc;
     for (int p0 = 0; p0 < P; p0 += w.pc) {
         const int pc = P - p0 < w.pc ? P - p0 : w.pc;
@@ -336,8 +371,7 @@ int wald_impl(const double* s, int Neff, const double* UYt, int64_t ldu, const d
                                                                                  log_delta + p0, pc, W, w.A1, w.rWr);
         if ((rc = check_launch("k_wald_prep"))) return rc;
         auto out = [&](double* x) { return x ? x + p0 : x; };
-        const bool tensor = oz_worth(pc, Mc < w.mc ? Mc : w.mc, Neff);
-        if (!tensor) {
+        if (!w.tensor || !oz_worth(pc, Mc < w.mc ? Mc : w.mc, Neff)) {
             const dim3 grid(ceil_div(Mc, TM), ceil_div(pc, TP));
             k_wald_f64<<<grid, NT, 0, st>>>(W, w.A1, w.rWr, Neff, var_df, pc, nr, USt, ldus, Mc, rows, out(f), out(beta),
                                             out(se), out(sfve), ldo, max_F + p0);
@@ -382,11 +416,11 @@ extern "C" int flmm_wald_f64(const double* s, int Neff, const double* UYt, int64
     FLMM_REQUIRE(n_real == 0 || Mc == 0 || (rows && f && beta && se && sfve && ldo >= n_real),
                  "flmm_wald_f64: real-column outputs missing");
     FLMM_REQUIRE(Mc == 0 || USt, "flmm_wald_f64: USt is NULL");
-    if (work_bytes < wald_ws(P, Neff))
-        return fail(FLMM_ERR_WORKSPACE, "flmm_wald_f64: need %zu bytes, got %zu", wald_ws(P, Neff), work_bytes);
+    if (work_bytes < wald_least(P, Neff))
+        return fail(FLMM_ERR_WORKSPACE, "flmm_wald_f64: need %zu bytes, got %zu", wald_least(P, Neff), work_bytes);
     if (P == 0 || Mc == 0) return FLMM_OK;
     return wald_impl(s, Neff, UYt, ldu, log_delta, P, n_real, USt, ldus, Mc, rows, f, beta, se, sfve, ldo, max_F,
-                     static_cast<double>(Neff - 1), work, as_stream(stream));
+                     static_cast<double>(Neff - 1), work, work_bytes, as_stream(stream));
 }
 
 extern "C" int flmm_wald_lowrank_f64_workspace_bytes(int k, int N, int P, int Mc, size_t* bytes) {
@@ -406,8 +440,7 @@ extern "C" int flmm_wald_lowrank_f64(const double* s, int k, const double* UYt, 
     FLMM_REQUIRE(n_real == 0 || Mc == 0 || (rows && f && beta && se && sfve && ldo >= n_real),
                  "flmm_wald_lowrank_f64: real-column outputs missing");
     FLMM_REQUIRE(Mc == 0 || (USt && UUSt), "flmm_wald_lowrank_f64: variant operands missing");
-    size_t need = 0;
-    flmm_wald_lowrank_f64_workspace_bytes(k, N, P, Mc, &need);
+    const size_t cat = sizeof(double) * lowrank_cat_doubles(k, N, P, Mc), need = cat + 256 + wald_least(P, k + N);
     if (work_bytes < need)
         return fail(FLMM_ERR_WORKSPACE, "flmm_wald_lowrank_f64: need %zu bytes, got %zu", need, work_bytes);
     if (P == 0 || Mc == 0) return FLMM_OK;
@@ -419,7 +452,8 @@ extern "C" int flmm_wald_lowrank_f64(const double* s, int k, const double* UYt, 
     double* s_cat = static_cast<double*>(work);
     double* UY_cat = s_cat + kc;
     double* US_cat = UY_cat + static_cast<size_t>(P) * kc;
-    void* rest = reinterpret_cast<char*>(work) + ((sizeof(double) * lowrank_cat_doubles(k, N, P, Mc) + 255) / 256) * 256;
+    const size_t at = (cat + 255) / 256 * 256;
+    void* rest = reinterpret_cast<char*>(work) + at;
     k_spectrum_pad<<<ceil_div(kc, 256), 256, 0, st>>>(s, k, N, s_cat);
     int rc = check_launch("k_spectrum_pad");
     if (rc) return rc;
@@ -429,5 +463,5 @@ extern "C" int flmm_wald_lowrank_f64(const double* s, int k, const double* UYt, 
                                                                                  US_cat);
     if ((rc = check_launch("k_concat_rows"))) return rc;
     return wald_impl(s_cat, kc, UY_cat, kc, log_delta, P, n_real, US_cat, kc, Mc, rows, f, beta, se, sfve, ldo, max_F,
-                     static_cast<double>(Neff - 1), rest, st);
+                     static_cast<double>(Neff - 1), rest, work_bytes - at, st);
 }

@@ -102,10 +102,22 @@ class _Work:
     def get(self, dev: torch.device, nbytes: int) -> tuple[C.c_void_p, int]:
         b = self.buf.get(dev)
         if b is None or b.numel() < nbytes:
+            b = None
+            self.buf.pop(dev, None)  # (given back before the larger one is asked for)
             b = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=dev)
             self.buf[dev] = b
         b.record_stream(torch.cuda.current_stream(dev))  # freed only after every stream that used it is done
         return C.c_void_p(b.data_ptr()), b.numel()
+
+    def up_to(self, dev: torch.device, nbytes: int) -> tuple[C.c_void_p, int]:
+        """For calls that take less than they ask for: half as often as it takes to find the memory."""
+        while True:
+            try:
+                return self.get(dev, nbytes)
+            except torch.cuda.OutOfMemoryError:
+                if nbytes <= 1 << 20:
+                    raise
+                nbytes //= 2
 
 
 _work = _Work()
@@ -244,21 +256,49 @@ def eigh_batched(A: Tensor, mode: int = 1, slot: int = -1, evals: Tensor | None 
     return evals
 
 
-# Matrices decomposed side by side are held at once, up to this many bytes of them (at least one).
-EIGH_MANY_BYTES = 2 << 30
+# Matrices decomposed side by side are held at once, with the solver's workspaces (two matrices' worth for each of up to
+# EIGH_WORKERS at a time): up to this many bytes of them (at least one matrix).
+EIGH_MANY_BYTES = 4 << 30
+EIGH_WORKERS = 8
 
 
 def eigh_groups(sizes: list[int]) -> list[range]:
     """Consecutive index ranges of matrices of the given sizes, each within EIGH_MANY_BYTES."""
-    groups, a, held = [], 0, 0
+    groups, a, held, most = [], 0, 0, 0
     for i, n in enumerate(sizes):
-        if i > a and held + 8 * n * n > EIGH_MANY_BYTES:
-            groups.append(range(a, i))
-            a, held = i, 0
         held += 8 * n * n
+        most = max(most, 16 * n * n)
+        if i > a and held + min(i + 1 - a, EIGH_WORKERS) * most > EIGH_MANY_BYTES:
+            groups.append(range(a, i))
+            a, held, most = i, 8 * n * n, 16 * n * n
     if sizes:
         groups.append(range(a, len(sizes)))
     return groups
+
+
+def eigh_each(sizes: list[int], form):
+    """(i, evals, eigenvector rows) of form(i), a contiguous square matrix of sizes[i] rows, for every i in order: as many
+    side by side as eigh_groups holds, one after another where there is no memory for that."""
+    for group in eigh_groups(sizes):
+        mats = []
+        try:
+            mats.extend(form(i) for i in group)
+            evals = eigh_many(mats)
+        except torch.cuda.OutOfMemoryError:
+            if len(group) == 1:
+                raise
+            mats.clear()
+            evals = None
+        if evals is None:
+            for i in group:
+                V = form(i)
+                yield i, eigh_many([V])[0], V
+                del V
+            continue
+        for k, i in enumerate(group):
+            V, mats[k] = mats[k], None
+            yield i, evals[k], V
+            del V
 
 
 def eigh_many(mats: list[Tensor]) -> list[Tensor]:
@@ -271,9 +311,10 @@ def eigh_many(mats: list[Tensor]) -> list[Tensor]:
     n = len(mats)
     evals = [torch.empty(m.shape[0], dtype=F64, device=dev) for m in mats]
     sizes = (C.c_int * n)(*(m.shape[0] for m in mats))
-    w, wb = _work.get(dev, _lib.query_bytes("flmm_eigh_many_workspace_bytes", ctx, sizes, n))
+    nbytes = _lib.query_bytes("flmm_eigh_many_workspace_bytes", ctx, sizes, n)
+    work = torch.empty(nbytes, dtype=torch.uint8, device=dev)  # (not the shared scratch, which would keep it)
     _lib.call("flmm_eigh_many", ctx, (C.c_void_p * n)(*(m.data_ptr() for m in mats)), sizes, n,
-              (C.c_void_p * n)(*(e.data_ptr() for e in evals)), w, wb, _stream(dev))
+              (C.c_void_p * n)(*(e.data_ptr() for e in evals)), _ptr(work), nbytes, _stream(dev))
     return evals
 
 
@@ -326,15 +367,21 @@ def rotate_variants(At: Tensor, Ut: Tensor, minus_from: Tensor | None = None) ->
     rounding noise of the loss, so another rounding of UY moves log delta by ~1e-7."""
     rows, N = At.shape
     Neff = Ut.shape[0]
-    if rows * Neff * N < TENSOR_MACS:
+    work = None
+    if rows * Neff * N >= TENSOR_MACS:
+        try:
+            work = _work.get(At.device, _lib.query_bytes("flmm_gemm_nt_f64_tc_workspace_bytes", rows, Neff, N))
+        except torch.cuda.OutOfMemoryError:
+            pass  # (the FP64 pipe's product needs none)
+    if work is None:
         out = rotate_rows(At, Ut)
         if minus_from is not None:
             res = minus_from.clone()
             _lib.call("flmm_axpy_f64", res.numel(), -1.0, _ptr(out), _ptr(res), _stream(At.device))
             return res
         return out
+    w, wb = work
     out = torch.empty((rows, Neff), dtype=F64, device=At.device)
-    w, wb = _work.get(At.device, _lib.query_bytes("flmm_gemm_nt_f64_tc_workspace_bytes", rows, Neff, N))
     _lib.call("flmm_gemm_nt_f64_tc", _ptr(At), At.stride(0), _ptr(Ut), Ut.stride(0), _ptr(minus_from),
               0 if minus_from is None else minus_from.stride(0), _ptr(out), Neff, rows, Neff, N, w, wb,
               _stream(At.device))
@@ -390,7 +437,7 @@ def wald_t(s: Tensor, UYt: Tensor, log_delta: Tensor, USt: Tensor, n_real: int, 
     Neff = s.shape[0]
     P = UYt.shape[0]
     Mc = USt.shape[0]
-    w, wb = _work.get(dev, _lib.query_bytes("flmm_wald_f64_workspace_bytes", P, Neff))
+    w, wb = _work.up_to(dev, _lib.query_bytes("flmm_wald_f64_workspace_bytes", P, Neff))
     _lib.call("flmm_wald_f64", _ptr(s), Neff, _ptr(UYt), UYt.stride(0), _ptr(log_delta), P, n_real, _ptr(USt),
               USt.stride(0), Mc, _ptr(rows), _ptr(out["f"]), _ptr(out["beta"]), _ptr(out["se"]), _ptr(out["sfve"]),
               n_real, _ptr(max_F), w, wb, _stream(dev))
@@ -507,27 +554,26 @@ def scan_t(Zt: Tensor, X: Tensor, Yt: Tensor, chrom: np.ndarray, *, n_real: int,
     D = X.shape[1]
     if N <= D:
         raise ValueError(f"need more samples than covariate columns (N={N}, D={D})")
-    for group in eigh_groups([N] * len(units)):
-        projected = []
-        for k_idx in group:
-            c = units[k_idx][0]
-            if c is None:
-                K = kinship_from_gram(Gtot, None, M_kin)
-            else:
-                K = kinship_from_gram(Gtot, grams.get(c), M_kin - int((kin_chrom == c).sum()))
-            projected.append(project_kinship(K, basis, K.new_empty(N, N)))
-        evals = eigh_many(projected)
-        for k_idx, Kp, ev in zip(group, projected, evals):
-            c, blk = units[k_idx]
-            s, Ut = compat_spectrum(ev, D), Kp[D:]
-            UYt = rotate_rows(Yrt, Ut)
-            ld, _ = fit_delta_t(s, UYt, n_grid=n_grid, log_delta_min=log_delta_min, log_delta_max=log_delta_max,
-                                refine=refine)
-            USt = rotate_variants(basis.regress_out(_take_rows(Zt, blk)), Ut)
-            wald_t(s, UYt, ld, USt, n_real, blk[0], out, max_F)
-            log_deltas[c if c is not None else 0] = ld
-            if on_chrom is not None:
-                on_chrom(k_idx + 1, len(units))
+
+    def projected(k_idx: int) -> Tensor:
+        c = units[k_idx][0]
+        if c is None:
+            K = kinship_from_gram(Gtot, None, M_kin)
+        else:
+            K = kinship_from_gram(Gtot, grams.get(c), M_kin - int((kin_chrom == c).sum()))
+        return project_kinship(K, basis, K.new_empty(N, N))
+
+    for k_idx, evals, Kp in eigh_each([N] * len(units), projected):
+        c, blk = units[k_idx]
+        s, Ut = compat_spectrum(evals, D), Kp[D:]
+        UYt = rotate_rows(Yrt, Ut)
+        ld, _ = fit_delta_t(s, UYt, n_grid=n_grid, log_delta_min=log_delta_min, log_delta_max=log_delta_max,
+                            refine=refine)
+        USt = rotate_variants(basis.regress_out(_take_rows(Zt, blk)), Ut)
+        wald_t(s, UYt, ld, USt, n_real, blk[0], out, max_F)
+        log_deltas[c if c is not None else 0] = ld
+        if on_chrom is not None:
+            on_chrom(k_idx + 1, len(units))
     return ScanResult(max_F=max_F, log_delta=log_deltas, **out)
 
 

@@ -20,8 +20,8 @@ from torch import Tensor
 
 from . import _lib
 from .core import (F64, ScanResult, _alloc_outputs, _chrom_blocks, _cuda_device, _f64, _ptr, _rows_major, _stream,
-                   _take_rows, _to_device, _work, eigh_groups, eigh_many, gram_t, kinship_from_gram, rotate_rows, rotate_variants,
-                   transpose)
+                   _take_rows, _to_device, _work, eigh_each, eigh_many, gram_t, kinship_from_gram, rotate_rows,
+                   rotate_variants, transpose)
 
 JITTER = 1e-6  # eigendecompose's diagonal jitter (fasterlmm/core.py:89)
 
@@ -54,23 +54,23 @@ def _spectrum_rows(spec: Spectrum, dev: torch.device) -> tuple[Tensor, Tensor, T
 
 # ---- eigendecomposition and rotation (fasterlmm/core.py:89-116) ------------------------------------------------
 
-def eigh_rows_many(Ks: list[Tensor], jitter: float = JITTER) -> list[tuple[Tensor, Tensor]]:
-    """eigh(K + jitter I) of each matrix, side by side, eigenvalues clamped at 0: [(s (N,), Ut (N, N) eigenvector
-    rows)]; the matrices are overwritten."""
-    for K in Ks:
-        N = K.shape[0]
-        _lib.call("flmm_shift_diagonal_f64", _ptr(K), N, N, float(jitter), _stream(K.device))
-    out = []
-    for K, evals in zip(Ks, eigh_many(Ks)):
-        s = torch.empty_like(evals)
-        _lib.call("flmm_clamp_nonneg_f64", _ptr(evals), K.shape[0], _ptr(s), _stream(K.device))
-        out.append((s, K))
-    return out
+def _jittered(K: Tensor, jitter: float) -> Tensor:
+    """K + jitter I, in place."""
+    N = K.shape[0]
+    _lib.call("flmm_shift_diagonal_f64", _ptr(K), N, N, float(jitter), _stream(K.device))
+    return K
+
+
+def _clamped(evals: Tensor) -> Tensor:
+    s = torch.empty_like(evals)
+    _lib.call("flmm_clamp_nonneg_f64", _ptr(evals), evals.shape[0], _ptr(s), _stream(evals.device))
+    return s
 
 
 def eigh_rows(K: Tensor, jitter: float = JITTER) -> tuple[Tensor, Tensor]:
     """eigh(K + jitter I) on device, eigenvalues clamped at 0: (s (N,), Ut (N, N) eigenvector rows)."""
-    return eigh_rows_many([K.clone()], jitter)[0]
+    A = _jittered(K.clone(), jitter)
+    return _clamped(eigh_many([A])[0]), A
 
 
 def eigendecompose(K: Tensor, jitter: float = JITTER) -> tuple[Tensor, Tensor]:
@@ -183,7 +183,7 @@ def wald_t(s: Tensor, Xrt: Tensor, Yrt: Tensor, log_delta: Tensor, Srt: Tensor, 
     C = Xrt.shape[0]
     P = Yrt.shape[0]
     Mc = Srt.shape[0]
-    w, wb = _work.get(dev, _lib.query_bytes("flmm_wald_gls_workspace_bytes", N, C, P))
+    w, wb = _work.up_to(dev, _lib.query_bytes("flmm_wald_gls_workspace_bytes", N, C, P))
     _lib.call("flmm_wald_gls_f64", _ptr(s), N, _ptr(Xrt), Xrt.stride(0), C, _ptr(Yrt), Yrt.stride(0), _ptr(log_delta),
               P, n_real, _ptr(Srt), Srt.stride(0), Mc, _ptr(rows), _ptr(out["f"]), _ptr(out["beta"]), _ptr(out["se"]),
               _ptr(out["sfve"]), n_real, _ptr(max_F), w, wb, _stream(dev))
@@ -238,23 +238,23 @@ def scan_t(Zt: Tensor, X: Tensor, Yt: Tensor, chrom: np.ndarray, *, n_real: int,
     M_kin = kin_Zt.shape[0]
     log_deltas = {}
     Xt = transpose(X)
-    for group in eigh_groups([N] * len(units)):
-        Ks = []
-        for k_idx in group:
-            c = units[k_idx][0]
-            if c is None:
-                Ks.append(kinship_from_gram(Gtot, None, M_kin))
-            else:
-                Ks.append(kinship_from_gram(Gtot, grams.get(c), M_kin - int((kin_chrom == c).sum())))
-        for k_idx, (s, Ut) in zip(group, eigh_rows_many(Ks)):
-            c, blk = units[k_idx]
-            Xrt, Yrt = rotate_rows(Xt, Ut), rotate_rows(Yt, Ut)
-            ld, _ = fit_delta_t(s, Xrt, Yrt)
-            Srt = rotate_variants(_take_rows(Zt, blk).contiguous(), Ut)
-            wald_t(s, Xrt, Yrt, ld, Srt, n_real, blk[0], out, max_F)
-            log_deltas[c if c is not None else 0] = ld
-            if on_chrom is not None:
-                on_chrom(k_idx + 1, len(units))
+
+    def kinship(k_idx: int) -> Tensor:
+        c = units[k_idx][0]
+        if c is None:
+            return _jittered(kinship_from_gram(Gtot, None, M_kin), JITTER)
+        return _jittered(kinship_from_gram(Gtot, grams.get(c), M_kin - int((kin_chrom == c).sum())), JITTER)
+
+    for k_idx, evals, Ut in eigh_each([N] * len(units), kinship):
+        c, blk = units[k_idx]
+        s = _clamped(evals)
+        Xrt, Yrt = rotate_rows(Xt, Ut), rotate_rows(Yt, Ut)
+        ld, _ = fit_delta_t(s, Xrt, Yrt)
+        Srt = rotate_variants(_take_rows(Zt, blk).contiguous(), Ut)
+        wald_t(s, Xrt, Yrt, ld, Srt, n_real, blk[0], out, max_F)
+        log_deltas[c if c is not None else 0] = ld
+        if on_chrom is not None:
+            on_chrom(k_idx + 1, len(units))
     return ScanResult(max_F=max_F, log_delta=log_deltas, **out)
 
 

@@ -20,7 +20,7 @@ from torch import Tensor
 
 from . import _lib
 from .core import (F64, CovariateBasis, ScanResult, _alloc_outputs, _BasisView, _cuda_device, _f64, _ptr,
-                   _rows_major, _stream, _to_device, _work, eigh_groups, eigh_many, gram_t, kinship_from_gram, rotate_rows,
+                   _rows_major, _stream, _to_device, _work, eigh_each, gram_t, kinship_from_gram, rotate_rows,
                    rotate_variants, transpose)
 
 
@@ -98,17 +98,16 @@ def loco_bases(Gt: Tensor, keeps: list[Tensor], basis: CovariateBasis, sv_floor:
     N = Gt.shape[1]
     Gr = basis.regress_out(Gt)
     gram = rotate_rows(Gr, Gr) if _one_gram_for_all(Gr.shape[0], [k.numel() for k in keeps if k.numel() < N]) else None
-    for group in eigh_groups([min(k.numel(), N) for k in keeps]):
-        mats = []
-        for i in group:
-            k = keeps[i]
-            if k.numel() < N and gram is not None:
-                mats.append(gram.index_select(0, k).index_select(1, k))
-                continue
-            rows = Gr.index_select(0, k)
-            mats.append(rotate_rows(rows, rows) if k.numel() < N else kinship_from_gram(gram_t(rows), None, k.numel()))
-        for i, V, evals in zip(group, mats, eigh_many(mats)):
-            yield _basis_of(evals, V, Gr.index_select(0, keeps[i]), sv_floor)
+
+    def matrix(i: int) -> Tensor:
+        k = keeps[i]
+        if k.numel() < N and gram is not None:
+            return gram.index_select(0, k).index_select(1, k)
+        rows = Gr.index_select(0, k)
+        return rotate_rows(rows, rows) if k.numel() < N else kinship_from_gram(gram_t(rows), None, k.numel())
+
+    for i, evals, V in eigh_each([min(k.numel(), N) for k in keeps], matrix):
+        yield _basis_of(evals, V, Gr.index_select(0, keeps[i]), sv_floor)
 
 
 def rotate_t(Yt: Tensor, Ut: Tensor, basis: CovariateBasis) -> tuple[Tensor, Tensor]:
@@ -203,7 +202,7 @@ def wald_t(s: Tensor, Ut: Tensor, UYt: Tensor, UUYt: Tensor, Neff: int, log_delt
     USt = rotate_variants(Sr, Ut)
     UUSt = rotate_variants(USt, transpose(Ut), minus_from=Sr)
     Mc = USt.shape[0]
-    w, wb = _work.get(dev, _lib.query_bytes("flmm_wald_lowrank_f64_workspace_bytes", k, N, P, Mc))
+    w, wb = _work.up_to(dev, _lib.query_bytes("flmm_wald_lowrank_f64_workspace_bytes", k, N, P, Mc))
     _lib.call("flmm_wald_lowrank_f64", _ptr(s), k, _ptr(UYt), UYt.stride(0), _ptr(UUYt), UUYt.stride(0), N, int(Neff),
               _ptr(log_delta), P, n_real, _ptr(USt), USt.stride(0), _ptr(UUSt), UUSt.stride(0), Mc, _ptr(rows),
               _ptr(out["f"]), _ptr(out["beta"]), _ptr(out["se"]), _ptr(out["sfve"]), n_real, _ptr(max_F), w, wb,

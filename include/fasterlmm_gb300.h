@@ -179,7 +179,9 @@ int flmm_fit_delta_f64(const double* s, int Neff, const double* UYt, int64_t ldu
 /* Plain FP64 form: for every column p < P and variant m < Mc: sWy = sum_n w UY US, sWs = sum_n w US^2 with
  * w = 1 / (s + exp(log_delta[p])), then beta, var_beta (df Neff - 1), F with the reference's clamps; max_F[p] is
  * raised to the column max (int64 atomic max on the FP64 bit pattern, F >= 0).  Real columns p < n_real write
- * f / beta / se / sfve at out[rows[m] * ldo + p].  Workspace holds w and w * UY (2 P Neff doubles). */
+ * f / beta / se / sfve at out[rows[m] * ldo + p].  Large scans form the sums on the tensor cores, in blocks whose
+ * operands are the workspace; a workspace shorter than the query's is taken from 2 P Neff + P doubles + 512 bytes on, with
+ * smaller blocks or the FP64 tile kernel. */
 int flmm_wald_f64_workspace_bytes(int P, int Neff, size_t* bytes);
 int flmm_wald_f64(const double* s, int Neff, const double* UYt, int64_t ldu, const double* log_delta, int P,
                   int n_real, const double* USt, int64_t ldus, int Mc, const int64_t* rows, double* f, double* beta,
@@ -483,7 +485,8 @@ int flmm_fit_delta_lowrank_f64(const double* s, int k, const double* UYt, int64_
                                int32_t* grid_idx, void* work, size_t work_bytes, void* stream);
 
 /* snp_wald_scan_lowrank (fasterlmm/lowrank.py:239-316): on-rank forms weighted by 1 / (s + delta), off-rank ones
- * by 1 / delta, df = Neff - 1; outputs as flmm_wald_f64. */
+ * by 1 / delta, df = Neff - 1; outputs and shorter workspaces (behind (k + N)(1 + P + Mc) doubles and 256 bytes) as
+ * flmm_wald_f64 with Neff = k + N. */
 int flmm_wald_lowrank_f64_workspace_bytes(int k, int N, int P, int Mc, size_t* bytes);
 int flmm_wald_lowrank_f64(const double* s, int k, const double* UYt, int64_t ldu, const double* UUYt, int64_t lduu,
                           int N, int Neff, const double* log_delta, int P, int n_real, const double* USt, int64_t ldus,
@@ -518,7 +521,8 @@ int flmm_fit_delta_gls_f64(const double* s, int N, const double* Xrt, int64_t ld
                            double* log_delta, int32_t* grid_idx, void* work, size_t work_bytes, void* stream);
 
 /* snp_wald_scan (fasterlmm/core.py:295-375): GLS Wald of every (variant, column) with the covariates in the model;
- * detail rows[m] * ldo + p for p < n_real, running max into max_F (P,) (initialise to -inf). */
+ * detail rows[m] * ldo + p for p < n_real, running max into max_F (P,) (initialise to -inf).  A workspace shorter than the
+ * query's is taken from min(P, 4096) ((C + 2) N + C^2 + 1) doubles + 1024 bytes on, as in flmm_wald_f64. */
 int flmm_wald_gls_workspace_bytes(int N, int C, int P, size_t* bytes);
 int flmm_wald_gls_f64(const double* s, int N, const double* Xrt, int64_t ldx, int C, const double* Yrt, int64_t ldy,
                       const double* log_delta, int P, int n_real, const double* Srt, int64_t lds, int M,

@@ -301,3 +301,57 @@ def test_without_the_tensor_cores():
     r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, FLMM_TC_PAIR="0"), capture_output=True, text=True,
                        timeout=300)
     assert r.returncode == 0 and "formed on the FP64 pipe" in r.stdout, r.stderr[-2000:]
+
+
+def _wald_call(kind, P, Mc, K, C):
+    """(call(work_bytes) -> outputs, full, least): flmm_wald_f64, flmm_wald_gls_f64 or flmm_wald_lowrank_f64 on one problem,
+    the workspace that it asks for and the shortest that it takes."""
+    from fasterlmm_gb300 import _lib, build, core
+    from fasterlmm_gb300.core import _ptr, _stream
+    build()
+    g = torch.Generator(device="cuda").manual_seed(P + K)
+    dev = torch.device("cuda", torch.cuda.current_device())
+    rn = lambda *s: torch.randn(*s, generator=g, device=dev, dtype=torch.float64)
+    k = K // 4  # on-rank directions of the low-rank form
+    s, X, Y, S, ld = rn(K).abs() + 0.05, rn(C, K), rn(P, K), rn(Mc, K), rn(P)
+    Yk, Yn, Sk, Sn = (t.contiguous() for t in (Y[:, :k], Y[:, k:], S[:, :k], S[:, k:]))
+    rows = torch.arange(Mc, device=dev)
+    cat = 8 * K * (1 + P + Mc) + 256
+    query, least = {
+        "compat": (("flmm_wald_f64_workspace_bytes", P, K), 8 * (2 * P * K + P) + 512),
+        "gls": (("flmm_wald_gls_workspace_bytes", K, C, P), 8 * P * ((C + 2) * K + C * C + 1) + 1024),
+        "lowrank": (("flmm_wald_lowrank_f64_workspace_bytes", k, K - k, P, Mc), cat + 8 * (2 * P * K + P) + 512)}[kind]
+
+    def call(nbytes):
+        out, max_F = core._alloc_outputs(Mc, P, P, dev)
+        work = torch.empty(nbytes + 4096, dtype=torch.uint8, device=dev)
+        work[nbytes:] = 171
+        o = [_ptr(out[x]) for x in ("f", "beta", "se", "sfve")]
+        end = (*o, P, _ptr(max_F), _ptr(work), nbytes, _stream(dev))
+        if kind == "compat":
+            _lib.call("flmm_wald_f64", _ptr(s), K, _ptr(Y), K, _ptr(ld), P, P, _ptr(S), K, Mc, _ptr(rows), *end)
+        elif kind == "gls":
+            _lib.call("flmm_wald_gls_f64", _ptr(s), K, _ptr(X), K, C, _ptr(Y), K, _ptr(ld), P, P, _ptr(S), K, Mc, _ptr(rows),
+                      *end)
+        else:
+            _lib.call("flmm_wald_lowrank_f64", _ptr(s), k, _ptr(Yk), k, _ptr(Yn), K - k, K - k, K, _ptr(ld), P, P, _ptr(Sk),
+                      k, _ptr(Sn), K - k, Mc, _ptr(rows), *end)
+        assert bool((work[nbytes:] == 171).all())  # nothing behind it was written
+        return [out[x] for x in ("f", "beta", "se", "sfve")] + [max_F]
+
+    return call, _lib.query_bytes(*query), least
+
+
+@pytest.mark.parametrize("kind", ["compat", "gls", "lowrank"])
+@pytest.mark.parametrize("P,Mc,K,C", [(300, 1500, 400, 5), (129, 4160, 130, 2), (7, 90, 64, 3)])
+def test_shorter_workspaces(kind, P, Mc, K, C):
+    """Whatever the workspace between the shortest and the one asked for, the same results to the rounding of the sums."""
+    from fasterlmm_gb300 import _lib
+    call, full, least = _wald_call(kind, P, Mc, K, C)
+    want = call(max(full, least))
+    for share in (0.0, 0.01, 0.03, 0.1, 0.2, 0.4, 0.7, 1.0):
+        for got, ref in zip(call(least + int(share * max(0, full - least))), want):
+            torch.testing.assert_close(got, ref, rtol=1e-9, atol=1e-12)
+    with pytest.raises(_lib.FlmmError) as e:
+        call(min(full, least) - 8)
+    assert e.value.status == 4
