@@ -162,7 +162,8 @@ __device__ __forceinline__ double warp_max(double v) {
 // fraction and one logarithm, sum u^2 / x = num / den and sum log x = log den, ~7 operations of the FP64 pipe an eigenvalue
 // for the ~60 of a division and a logarithm each, and the point that a step shares with the one before is not evaluated
 // again.  A step is certain when the two losses differ by more than twice what rounding can make of them here and in
-// k_golden together.  With u = 2^-53 and n eigenvalues, to first order and both sides: sum u^2 / x is a sum of positive
+// k_golden together.  exp and log are taken to be within one unit in the last place (CUDA's documented bounds; the same
+// delta goes into both sides).  With u = 2^-53 and n eigenvalues, to first order and both sides: sum u^2 / x is a sum of positive
 // terms, relative error below (n / 30 + 58) u; sum log x is off by at most (n / 30 + 20) u sum |log x| + n u; a shared
 // point whose position differs in its last bits moves the loss by at most (neff + n + |n_logd|) times that.  The first step
 // that is not certain ends the list, as does anything out of the range of these bounds.
@@ -360,9 +361,13 @@ int fit_delta_impl(const double* s, int Neff, const double* UYt, int64_t ldu, in
         k_grid_argmin<1><<<ceil_div(P, 16), NT, 0, st>>>(Wg, sum_log, grid, UYt, ldu, Neff, P, n_grid, off, grid_idx);
     if ((rc = check_launch("k_grid_argmin"))) return rc;
     if (refine) {
-        k_golden_certain<<<ceil_div(P, kCertainWarps), 32 * kCertainWarps, 0, st>>>(s, Neff, UYt, ldu, P, grid, n_grid, grid_idx,
-                                                                                   off, log_delta);
-        if ((rc = check_launch("k_golden_certain"))) return rc;
+        if (refine == FLMM_REFINE_EVERY_STEP) {
+            FLMM_CUDA(cudaMemsetAsync(log_delta, 0, sizeof(double) * P, st));  // empty lists
+        } else {
+            k_golden_certain<<<ceil_div(P, kCertainWarps), 32 * kCertainWarps, 0, st>>>(s, Neff, UYt, ldu, P, grid, n_grid,
+                                                                                       grid_idx, off, log_delta);
+            if ((rc = check_launch("k_golden_certain"))) return rc;
+        }
         k_golden<<<P, kBlockThreads, 0, st>>>(s, Neff, UYt, ldu, grid, n_grid, grid_idx, lo, hi, off, log_delta);
         return check_launch("k_golden");
     }

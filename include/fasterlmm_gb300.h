@@ -167,8 +167,10 @@ int flmm_gemm_nt_f64_tc(const double* A, int64_t lda, const double* B, int64_t l
 int flmm_delta_grid_nodes(double lo, double hi, int n_grid, double* grid, void* stream);
 
 /* Plain FP64 form: (G, P) grid loss, first argmin, then the reference's 50-step golden-section search on
- * [grid[i-1], grid[i+1]] with its update order, result clamped to [lo, hi]; refine = 0 returns the grid node.
+ * [grid[i-1], grid[i+1]] with its update order, result clamped to [lo, hi]; refine = 0 returns the grid node.  Steps
+ * whose outcome is certain are taken from bounded sums; refine = FLMM_REFINE_EVERY_STEP evaluates every loss (the same bits).
  * Outputs log_delta (P,) and grid_idx (P,).  Workspace holds the (G, Neff) weights. */
+#define FLMM_REFINE_EVERY_STEP 2
 int flmm_fit_delta_f64_workspace_bytes(int Neff, int n_grid, size_t* bytes);
 int flmm_fit_delta_f64(const double* s, int Neff, const double* UYt, int64_t ldu, int P, int n_grid, double lo,
                        double hi, int refine, double* log_delta, int32_t* grid_idx, void* work, size_t work_bytes,

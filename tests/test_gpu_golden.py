@@ -112,3 +112,70 @@ def test_steps_taken_from_grouped_sums(n, P, scale, off):
         left = fc < fd
         b, a = torch.where(sure & left, d, b), torch.where(sure & ~left, c, a)
     assert ((ld >= a - 1e-12) & (ld <= b + 1e-12)).all()
+
+
+SPECTRA = {
+    "half-normal": lambda g, n: torch.randn(n, generator=g, device="cuda", dtype=torch.float64).abs() * 2,
+    "falling": lambda g, n: torch.logspace(2, -9, n, device="cuda", dtype=torch.float64),
+    "with zeros": lambda g, n: torch.rand(n, generator=g, device="cuda", dtype=torch.float64).round(decimals=1),
+    "one value": lambda g, n: torch.full((n,), 0.75, device="cuda", dtype=torch.float64),
+    "tiny": lambda g, n: torch.rand(n, generator=g, device="cuda", dtype=torch.float64) * 1e-9,
+    "large": lambda g, n: torch.rand(n, generator=g, device="cuda", dtype=torch.float64) * 1e5,
+}
+
+
+@pytest.mark.parametrize("spectrum", list(SPECTRA))
+@pytest.mark.parametrize("n", [1, 2, 33, 300, 512, 995, 2049])
+@pytest.mark.parametrize("off", [0, 7])
+def test_certain_steps_leave_every_bit(spectrum, n, off):
+    """The search from the list of certain steps ends where the one that evaluates every loss ends, to the bit."""
+    from fasterlmm_gb300 import _lib, build
+    from fasterlmm_gb300.core import _ptr, _stream
+    build()
+    g = torch.Generator(device="cuda").manual_seed(n)
+    dev = torch.device("cuda", torch.cuda.current_device())
+    rn = lambda *x: torch.randn(*x, generator=g, device=dev, dtype=torch.float64)
+    s, P = SPECTRA[spectrum](g, n), 240
+    h2 = torch.rand(P, generator=g, device=dev, dtype=torch.float64)[:, None]
+    UY = rn(P, n) * (h2 * s[None, :] / s.mean() + (1 - h2)).sqrt() * torch.logspace(-4, 4, P, device=dev, dtype=torch.float64)[:, None]
+    UY[3] = 0.0
+    yy = UY.square().sum(1) * rn(P).square() * 0.1 if off else None
+    if off:
+        yy[5] = 0.0
+    got = []
+    for refine in (1, 2):
+        for lo, hi in ((-10.0, 10.0), (-3.0, 2.5)):
+            ld, idx = torch.empty(P, dtype=torch.float64, device=dev), torch.empty(P, dtype=torch.int32, device=dev)
+            nbytes = _lib.query_bytes("flmm_fit_delta_f64_workspace_bytes", n, G)
+            work = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+            end = (P, G, lo, hi, refine, _ptr(ld), _ptr(idx), _ptr(work), nbytes, _stream(dev))
+            if off:
+                _lib.call("flmm_fit_delta_lowrank_f64", _ptr(s), n, _ptr(UY), n, _ptr(yy), n + off, *end)
+            else:
+                _lib.call("flmm_fit_delta_f64", _ptr(s), n, _ptr(UY), n, *end)
+            got.append(ld)
+    same = lambda x, y: bool(((x == y) | (torch.isnan(x) & torch.isnan(y))).all())
+    assert same(got[0], got[2]) and same(got[1], got[3])
+
+
+@pytest.mark.parametrize("C", [1, 4])
+def test_gls_fit_by_warps(C):
+    """Beyond ~12,000 samples a warp per column searches instead of two blocks."""
+    from fasterlmm_gb300 import build, gls
+    build()
+    n, P = 12_900, 3
+    s, Y, rn = _inputs(n, P, C)
+    X = rn(C, n)
+    ld, idx = gls.fit_delta_t(s, X, Y)
+
+    def loss(x):
+        sd = s[None, :] + x.exp()[:, None]
+        w = 1.0 / sd
+        L = torch.linalg.cholesky(torch.einsum("pn,cn,dn->pcd", w, X, X))
+        z = torch.linalg.solve_triangular(L, torch.einsum("pn,cn,pn->pc", w, X, Y)[:, :, None], upper=False)[:, :, 0]
+        rwr = (w * Y * Y).sum(1) - (z * z).sum(1)
+        return n * (math.log(2 * math.pi) + torch.log(rwr / n) + 1.0) + torch.log(sd).sum(1)
+
+    want, i = _golden(loss, P, s.device)
+    assert torch.equal(idx.long(), i)
+    torch.testing.assert_close(loss(ld), loss(want), rtol=4 * n * 2.0 ** -53, atol=1e-10)
