@@ -954,9 +954,10 @@ int cluster_ctas(int dev, int N, int batch, int* out) {
     static bool known[64];
     std::lock_guard<std::mutex> lock(mu);
     if (dev < 0 || dev >= 64) return fail(FLMM_ERR_ARG, "eigh: device %d", dev);
+    // (per device context, so set on every call; the calls are cheap)
+    FLMM_CUDA(cudaFuncSetAttribute(k_sytrd_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
+    FLMM_CUDA(cudaFuncSetAttribute(k_sytrd_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     if (!known[dev]) {
-        FLMM_CUDA(cudaFuncSetAttribute(k_sytrd_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
-        FLMM_CUDA(cudaFuncSetAttribute(k_sytrd_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         for (int c = 2; c <= kMaxClusterCtas; ++c) {
             cudaLaunchConfig_t cfg = {};
             cudaLaunchAttribute attr[1];

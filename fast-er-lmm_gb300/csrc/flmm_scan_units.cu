@@ -19,6 +19,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <new>
 #include <vector>
 
 #include "flmm_common.cuh"
@@ -185,10 +186,14 @@ extern "C" int flmm_loco_kinships_f32(flmm_context* ctx, const double* Zt, int N
     }
     k_sum_grams<<<ceil_div(nn, 256), 256, 0, st>>>(grams, nn, n_blocks, Gtot);
     if ((rc = check_launch("k_sum_grams"))) return rc;
-    std::vector<UnitGram> host(n_units);
-    for (int u = 0; u < n_units; ++u)
-        host[u] = UnitGram{unit_block[u], static_cast<double>(M - (unit_block[u] >= 0 ? counts[unit_block[u]] : 0))};
-    if ((rc = put(host.data(), n_units, units, st))) return rc;
+    try {
+        std::vector<UnitGram> host(n_units);
+        for (int u = 0; u < n_units; ++u)
+            host[u] = UnitGram{unit_block[u], static_cast<double>(M - (unit_block[u] >= 0 ? counts[unit_block[u]] : 0))};
+        if ((rc = put(host.data(), n_units, units, st))) return rc;
+    } catch (const std::bad_alloc&) {
+        return fail(FLMM_ERR_ARG, "flmm_loco_kinships_f32: out of host memory");
+    }
     k_unit_kinships<<<dim3(ceil_div(nn, 256), n_units), 256, 0, st>>>(Gtot, grams, nn, units, Kp);
     if ((rc = check_launch("k_unit_kinships"))) return rc;
     return project_kinships(Kp, Qx, N, D, n_units, proj, st);
@@ -523,7 +528,11 @@ extern "C" int flmm_scan_units(flmm_context* ctx, const flmm_units* q, void* wor
     if ((rc = flmm_split_rows_f16(b.W, 1, Neff, U * b.R, Neff, b.Ws.hi, b.Ws.lo, b.ldk, b.Ws.scale, main))) return rc;
     const bool pipe = side != main;
     if (b.grouped) {
-        rc = run_grouped(ctx, q, b, main, side, ev);
+        try {
+            rc = run_grouped(ctx, q, b, main, side, ev);
+        } catch (const std::bad_alloc&) {  // (its tables; before anything is launched)
+            rc = fail(FLMM_ERR_ARG, "flmm_scan_units: out of host memory");
+        }
         if (rc && pipe && cudaEventRecord(ev.e[0], side) == cudaSuccess) cudaStreamWaitEvent(main, ev.e[0], 0);
         return rc;
     }

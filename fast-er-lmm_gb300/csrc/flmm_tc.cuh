@@ -335,8 +335,8 @@ __device__ __forceinline__ void mma_commit_pair(uint64_t* bar, uint16_t cta_mask
 // {BK, box_rows}, BK 32 (64-byte swizzle) or 64 (128-byte swizzle); rows and columns outside the matrix read as zero.
 int make_map_f16(CUtensorMap* map, const void* base, int rows, int K, int64_t ld, int BK, int box_rows);
 
-// CTA pairs of a kernel (one CTA per SM) that the current device runs at once, 0 if none fits.  `cache` is the kernel's
-// own, by device.
+// CTA pairs of a kernel (one CTA per SM) that the current device runs at once, 0 if none fits; sets its shared-memory
+// limit.  `cache` is the kernel's own, by device.
 struct PairCache {
     std::mutex mu;
     int pairs[64] = {};
@@ -349,8 +349,9 @@ int pair_count(Kernel* kernel, int threads, int smem_bytes, PairCache& cache, in
     FLMM_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64) return fail(FLMM_ERR_ARG, "pair_count: device %d", dev);
     std::lock_guard<std::mutex> lock(cache.mu);
+    // (per device context, so set on every call; the call is cheap)
+    FLMM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
     if (!cache.known[dev]) {
-        FLMM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
         FLMM_CUDA(cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev));
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr[1];
