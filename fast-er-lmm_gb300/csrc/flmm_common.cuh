@@ -119,6 +119,14 @@ int wald_refine_units(flmm_context* ctx, const int32_t* flags, const int32_t* fl
 int fill_nullh2_units(const double* log_delta, int P, int n_real, const int64_t* rows, const int* start, int n_units,
                       int most, double* out, int64_t ldo, cudaStream_t st);
 
+// SMs of the current device
+inline int sm_count(int* out) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(out, cudaDevAttrMultiProcessorCount, dev);
+    return e == cudaSuccess ? FLMM_OK : fail(FLMM_ERR_CUDA, "sm_count: %s", cudaGetErrorString(e));
+}
+
 inline unsigned ceil_div(int64_t a, int64_t b) { return static_cast<unsigned>((a + b - 1) / b); }
 
 #define FLMM_REQUIRE(cond, ...)                                                       \

@@ -355,7 +355,9 @@ int fit_delta_impl(const double* s, int Neff, const double* UYt, int64_t ldu, in
     if (rc) return rc;
     k_grid_weights<<<n_grid, 256, 0, st>>>(s, Neff, grid, Wg, sum_log);
     if ((rc = check_launch("k_grid_weights"))) return rc;
-    if (P >= 64 * 152)
+    int sms = 0;
+    if ((rc = sm_count(&sms))) return rc;
+    if (P >= 64 * sms)
         k_grid_argmin<4><<<ceil_div(P, 64), NT, 0, st>>>(Wg, sum_log, grid, UYt, ldu, Neff, P, n_grid, off, grid_idx);
     else
         k_grid_argmin<1><<<ceil_div(P, 16), NT, 0, st>>>(Wg, sum_log, grid, UYt, ldu, Neff, P, n_grid, off, grid_idx);

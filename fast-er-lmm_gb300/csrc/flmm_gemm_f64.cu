@@ -100,9 +100,9 @@ k_gemm_f64(const double* __restrict__ A, int64_t lda, const double* __restrict__
 template <bool AK, bool BKC, bool SYM>
 int launch_gemm(const double* A, int64_t lda, const double* B, int64_t ldb, double* C, int64_t ldc, int Mr, int Nr, int K,
                 double alpha, double beta, cudaStream_t st, const char* what) {
-    int dev = 0, sm = 0;
-    FLMM_CUDA(cudaGetDevice(&dev));
-    FLMM_CUDA(cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev));
+    int sm = 0;
+    const int rc = sm_count(&sm);
+    if (rc) return rc;
     auto tiles = [&](int r) {
         const int64_t ti = ceil_div(Mr, 16 * r), tj = ceil_div(Nr, 16 * r);
         return SYM ? ti * (ti + 1) / 2 : ti * tj;

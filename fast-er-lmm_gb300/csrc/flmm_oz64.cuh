@@ -79,9 +79,9 @@ int oz_gemm(const OzOperand& A, const OzOperand& B, const OzProduct& p, cudaStre
 // Gy, sWs in its row of Gs, and in the GLS form the nq terms whose squares add to B^T A^-1 B in nq rows of Gq (nq = 0 in
 // the compat form).  F, beta, SE, SFVE of the first n_real columns into rows `rows` of the outputs, column maxima into
 // max_F.
-int wald_finish(const double* Gy, const double* Gs, const double* Gq, int nq, int64_t ldg, const double* rWr, double var_df, int P,
-                int n_real, int Mc, const int64_t* rows, double* f, double* beta, double* se, double* sfve, int64_t ldo,
-                double* max_F, cudaStream_t st);
+int wald_finish(const double* Gy, const double* Gs, const double* Gq, int nq, int64_t ldg, const double* rWr,
+                double var_df, int P, int n_real, int Mc, const int64_t* rows, double* f, double* beta, double* se,
+                double* sfve, int64_t ldo, double* max_F, cudaStream_t st);
 
 // Products below this many multiply-adds stay on the FP64 pipe.
 bool oz_worth(int64_t Mr, int64_t Nr, int64_t K);

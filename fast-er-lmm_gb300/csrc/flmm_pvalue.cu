@@ -72,7 +72,8 @@ k_tail(const double* __restrict__ F, int64_t n, FTail tail, double* __restrict__
             at_s = __shfl_sync(0xffffffffu, at_s, 0);
             at_f = __shfl_sync(0xffffffffu, at_f, 0);
             const unsigned below = (1u << lane) - 1u;
-            if (in) list[frac ? m - 1 - (at_f + __popc(fr & below)) : at_s + __popc(all & ~fr & below)] = static_cast<uint16_t>(k);
+            const int place = frac ? m - 1 - (at_f + __popc(fr & below)) : at_s + __popc(all & ~fr & below);
+            if (in) list[place] = static_cast<uint16_t>(k);
         }
         __syncthreads();
         // the lists start on warp boundaries of their own, so no warp holds both
@@ -88,8 +89,11 @@ k_tail(const double* __restrict__ F, int64_t n, FTail tail, double* __restrict__
 
 template <Tail WHAT>
 int launch_tail(const double* F, int64_t n, int df2, double* out, cudaStream_t st) {
-    const int64_t chunks = (n + kTailChunk - 1) / kTailChunk;
-    k_tail<WHAT><<<static_cast<unsigned>(chunks < 152 * 8 ? chunks : 152 * 8), kTailThreads, 0, st>>>(F, n, tail_of(df2), out);
+    int sms = 0;
+    const int rc = sm_count(&sms);
+    if (rc) return rc;
+    const int64_t chunks = (n + kTailChunk - 1) / kTailChunk, most = 8 * static_cast<int64_t>(sms);
+    k_tail<WHAT><<<static_cast<unsigned>(chunks < most ? chunks : most), kTailThreads, 0, st>>>(F, n, tail_of(df2), out);
     return check_launch("k_tail");
 }
 

@@ -10,9 +10,8 @@
 // 150 samples x 1,500 variants on 16 chromosomes took 10.2 ms in 505 launches, 4.35 unit by unit and 3.00 grouped.  What
 // depends on the spectra alone (mean, FP32 copies, sWs node weights and their split) and the projections run for all units
 // in one launch each.  Where every unit's operands fit kGroupBytes together, so does the rest (run_grouped): the launches
-// then take all
-// units' rows, the split products with the units' tiles one after another.  The arithmetic is in every form that of the
-// C entry points called one by one.
+// then take all units' rows, the split products with the units' tiles one after another.  The arithmetic is in every form
+// that of the C entry points called one by one.
 #include <cuda_fp16.h>
 #include <limits.h>
 #include <math.h>
@@ -205,7 +204,8 @@ namespace {
 
 // Grouped launches when every unit's column operands (eigenvectors, rotated phenotypes and their weighted rows) take at
 // most this much together, and the variants' (rotations and their halves) too: 150 x 1,500 on 16 chromosomes 4.35 -> 3.00
-// ms, 563 x 20,011 on 22 15.1 -> 12.5, 1,600 x 6,000 on 8 169 -> 162.  With more columns a unit's launches fill the device for many waves, and the second stream hides the rest.
+// ms, 563 x 20,011 on 22 15.1 -> 12.5, 1,600 x 6,000 on 8 169 -> 162.  With more columns a unit's launches fill the device
+// for many waves, and the second stream hides the rest.
 constexpr size_t kGroupBytes = size_t{1} << 30;
 
 struct UnitBufs {

@@ -3,7 +3,7 @@
 // The products are FP64 sums of Neff terms per test and bound by the FP64 pipe (1.08 TFLOP/s measured of ~1.25), so
 // where they are large they run on the tensor cores from exact digit planes (flmm_oz64.cu) in blocks of columns and
 // variants whose sums an epilogue kernel reads back (16 bytes per test); 1,100 columns x 4,096 variants x 995 with its
-// rotation: 23.9 -> 1.83 ms.  Small products stay in the fused FP64 tile kernel, which needs one launch.
+// rotation: 23.9 -> 1.32 ms.  Small products stay in the fused FP64 tile kernel, which needs one launch.
 #include <math.h>
 #include <stdint.h>
 
@@ -154,7 +154,8 @@ __device__ __forceinline__ Test wald_test(double swy, double sws, double rwr, do
 // Epilogue over the sums of a block of columns and variants (layout: flmm_oz64.cuh): a thread block takes 32 columns x
 // kFinTile variants, transposed through shared memory so that the reads run along the variants and the detail stores along
 // the columns.  Real columns get the full epilogue; with 256 variants a block, those few blocks' FP64 pipes set the time
-// (1,100 columns, 100 of them real, x 4,096: 265 -> 161 us with one F a block; 660 with covariates, 60 real, x 4,000: 277 -> 138).  A permutation column needs its
+// (1,100 columns, 100 of them real, x 4,096: 265 -> 161 us with one F a block; 660 with covariates, 60 real, x 4,000:
+// 277 -> 138).  A permutation column needs its
 // largest F only, and F grows with q / denom, so its tests are ranked by cross-multiplication (three FP64 operations
 // instead of four divisions; GB300's FP64 pipe is the bound here) and one F is formed per block; sums outside
 // 1e-100 .. 1e100, and NaN, take the full formula.
@@ -164,8 +165,8 @@ template <bool GLS>
 __global__ void __launch_bounds__(256)
 k_wald_finish(const double* __restrict__ Gy, const double* __restrict__ Gs, const double* __restrict__ Gq, int nq,
               int64_t ldg, const double* __restrict__ rWr, double var_df, int P, int n_real, int Mc,
-              const int64_t* __restrict__ rows, double* __restrict__ f, double* __restrict__ beta, double* __restrict__ se, double* __restrict__ sfve, int64_t ldo,
-              double* __restrict__ max_F) {
+              const int64_t* __restrict__ rows, double* __restrict__ f, double* __restrict__ beta,
+              double* __restrict__ se, double* __restrict__ sfve, int64_t ldo, double* __restrict__ max_F) {
     __shared__ double sy[kFinP][kFinTile + 1];
     __shared__ double ss[kFinP][kFinTile + 1];
     __shared__ double red[8][kFinP], red_q[8][kFinP], red_den[8][kFinP], red_sy[8][kFinP];

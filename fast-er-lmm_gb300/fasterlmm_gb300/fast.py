@@ -410,8 +410,8 @@ def _scan_units(ctx, units: list, Ys: SplitRows, Zs: SplitRows, row_map: Tensor,
     lds = torch.empty((n, P), dtype=F64, device=dev)
     at = lambda t: t.data_ptr() or None
     q = _lib.Units(
-        N=N, D=D, P=P, n_real=n_real, n_units=n, refine_cap=min(REFINE_CAP, 2**31 - 1), Yh=at(Ys.hi), Yl=at(Ys.lo), Yscale=at(Ys.scale),
-        ldY=Ys.ld, Zh=at(Zs.hi), Zl=at(Zs.lo), Zscale=at(Zs.scale), ldZ=Zs.ld,
+        N=N, D=D, P=P, n_real=n_real, n_units=n, refine_cap=min(REFINE_CAP, 2**31 - 1), Yh=at(Ys.hi),
+        Yl=at(Ys.lo), Yscale=at(Ys.scale), ldY=Ys.ld, Zh=at(Zs.hi), Zl=at(Zs.lo), Zscale=at(Zs.scale), ldZ=Zs.ld,
         unit_start=(C.c_int64 * n)(*(a for _, a, _ in units)), unit_count=(C.c_int * n)(*(m for _, _, m in units)),
         rows=at(row_map), U=at(U), evals=at(evals),
         opts=_lib.ScanOpts(n_grid=n_grid, log_delta_min=log_delta_min, log_delta_max=log_delta_max,

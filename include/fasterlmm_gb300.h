@@ -607,10 +607,10 @@ int flmm_host_free_mapped(void* host_ptr);
  * grouped into n_blocks chromosomes of counts[c] variants (host); unit u leaves out block unit_block[u] (-1: none).
  * The steps of flmm_gemm_split_f16 Grams, flmm_loco_kinship_f32 and flmm_project_kinship, for all units.
  *
- * flmm_scan_units: every unit of a fast-form scan.  Units whose column and variant operands fit 1 GiB each together, and whose
- * variants follow one another, run in one launch each, the columns' side (UY, delta fit) on `side_stream` beside the variants' on `stream`;
- * others one by one, the column side one unit ahead.  The bits are the same.  The same stream twice: one after another.  All
- * pointers are device memory but unit_start and unit_count. */
+ * flmm_scan_units: every unit of a fast-form scan.  Units whose column and variant operands fit 1 GiB each together, and
+ * whose variants follow one another, run in one launch each, the columns' side (UY, delta fit) on `side_stream` beside the
+ * variants' on `stream`; others one by one, the column side one unit ahead.  The bits are the same.  The same stream twice:
+ * one after another.  All pointers are device memory but unit_start and unit_count. */
 int flmm_loco_kinships_f32_workspace_bytes(int N, int D, int n_blocks, const int* counts, int n_units, size_t* bytes);
 int flmm_loco_kinships_f32(flmm_context* ctx, const double* Zt, int N, const int* counts, int n_blocks,
                            const int* unit_block, int n_units, const double* Qx, int D, double* Kp, void* work,

@@ -137,7 +137,8 @@ def test_certain_steps_leave_every_bit(spectrum, n, off):
     rn = lambda *x: torch.randn(*x, generator=g, device=dev, dtype=torch.float64)
     s, P = SPECTRA[spectrum](g, n), 240
     h2 = torch.rand(P, generator=g, device=dev, dtype=torch.float64)[:, None]
-    UY = rn(P, n) * (h2 * s[None, :] / s.mean() + (1 - h2)).sqrt() * torch.logspace(-4, 4, P, device=dev, dtype=torch.float64)[:, None]
+    UY = rn(P, n) * (h2 * s[None, :] / s.mean() + (1 - h2)).sqrt()
+    UY *= torch.logspace(-4, 4, P, device=dev, dtype=torch.float64)[:, None]
     UY[3] = 0.0
     yy = UY.square().sum(1) * rn(P).square() * 0.1 if off else None
     if off:
