@@ -68,17 +68,19 @@ static_assert(kTmemCols == 512 && kSmemBytes <= 227 * 1024 && kEpiCols == 16, "b
 //   sqrt(K).  Measured on a scan's operands at K = 1,000, relative to the row norms: ratios 10 x 5 leave 1.1e-17 where the
 //   FP64 sum leaves 3.9e-17, so the two meet near a product of 150.
 //   kBalanced (max/mean, which unlike max/rms keeps growing when one entry dominates a row: balancing can put a row's
-//   largest entry where the other row is small, and max/rms of such a row is sqrt(K) at most): normal rows have 1.6 times the
-//   ratio, hence 6 sqrt(K).  With one entry of A 16 times and that of B a sixteenth of the others (K = 400, product 2.8
-//   sqrt(K)) the digits lose 2.1 times what the FP64 sum does, and 4 times at 5.3 sqrt(K) (K = 100).  A sum of
-//   non-negative terms is off by 2^-53 K^1.5 / 6 of the product of means: the two meet near 0.7 K.
+//   largest entry where the other row is small, and max/rms of such a row is sqrt(K) at most).  A scan's tiles have products
+//   of up to 7 sqrt(K) at K = 100 and 4 sqrt(K) at K = 1,000, and are 0.9 and 0.35 of the FP64 sum off; a row with one
+//   dominating entry has 4 K.  At the line the digits lose 2 to 3 times what the FP64 sum does where one entry is large, and
+//   8 times at worst, where the other row's entry is as small as that one is large (both of 5e-17 of the norms).  A sum of
+//   non-negative terms is off by 2^-53 K^1.5 / 6 of the product of means: a scan's tiles have products of up to 0.9 K (K =
+//   100) and 0.15 K (K = 1,000), and the two meet near 0.7 K.
 //   kTerms: with A over sqrt(mean w) the loss of a term is 2^-56 of the product against sqrt(sum w b^2), twice that of the
 //   term's square against sum w b^2, whose own FP64 sum is off by 2^-53 sqrt(K) / 6.
 __host__ inline float quality_limit(OzGate gate, bool square, int K) {
     const float k = static_cast<float>(K), root = sqrtf(k);
     if (gate == OzGate::kPlain) return 4.0f * root;
     if (gate == OzGate::kTerms) return 0.7f * root;
-    return square ? 0.75f * k : 6.0f * root;
+    return square ? k : 8.0f * root;
 }
 
 struct OzMaps {
@@ -234,7 +236,7 @@ k_digits64(const double* __restrict__ X, int64_t ldx, int rows, int K, const int
 __global__ void k_zero_f32(float* __restrict__ x, int n, int* __restrict__ flag) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) x[i] = 0.0f;
-    if (i == 0 && flag) *flag = 0;
+    if (i < 2 && flag) flag[i] = 0;
 }
 
 // ---- the product ------------------------------------------------------------------------------------------------
@@ -416,6 +418,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz64(const __grid_constant__ Oz
         bool ok = true;
         for (int t = cl; t < n_tiles && ok; t += n_cl) {
             const Tile tl = tile_at(t, args.pairs_i, args.tiles_m);
+            const Tile half{tl.b, 2 * tl.ti + static_cast<int>(rank), tl.tm};
+            const bool good = tile_good(args, half);
+            if (warp == 2 && lane == 0 && !good && half.ti < args.tiles_i) args.err[1] = 1;  // k_marked_f64 has work
             if (!pair_good(args, tl)) continue;
             long long hi[kEpiCols], lo[kEpiCols];
 #pragma unroll
@@ -445,8 +450,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz64(const __grid_constant__ Oz
                 tphase ^= 1u;
             }
             if (!ok) break;
-            const Tile half{tl.b, 2 * tl.ti + static_cast<int>(rank), tl.tm};
-            if (!tile_good(args, half)) continue;
+            if (!good) continue;
             // the outputs leave through shared memory, so that lanes go along the rows of C (and D)
             const int i0 = half.ti * kOzRowsA + q * 32;
             const int ea = i0 + lane < args.Ma ? args.ea[tl.b * args.Ma + i0 + lane] : 0;
@@ -488,61 +492,67 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz64(const __grid_constant__ Oz
 
 // ---- tiles left to the FP64 pipe ----------------------------------------------------------------------------------
 
-constexpr int kST = 64, kSK = 16, kSThreads = 256;
+constexpr int kST = 16, kSK = 16, kSThreads = 256;
+constexpr int kSubs = (kOzRowsA / kST) * (kOzRowsB / kST);  // 16 x 16 outputs of a digit tile
 constexpr int kNoPairs = 0x01010101;  // error word of a product that k_oz64 was not launched for
 
-// The 64 x 64 tiles of C whose digit tiles are not good, or all after an error, in FP64 (one block per tile; the others
-// leave at once).  Where D is C and k_oz64 gave up, some of D is gone: all NaN.
+// The tiles of C whose digits are not good, or all after an error, in FP64: every block lists them in the same order and takes
+// its share of their 16 x 16 parts, an output a thread.  One tile as two blocks of 64 x 64 outputs held up a launch for K
+// 64^2 / 2 cycles of an SM's FP64 pipe (2,338 columns x 445 variants x 281 with one such tile: 0.22 of 0.62 ms).  Where D is C
+// and k_oz64 gave up, some of D is gone: all NaN.
 __global__ void __launch_bounds__(kSThreads)
 k_marked_f64(const OzArgs args, const double* __restrict__ Xa, int64_t lda, int64_t xa_stride,
              const double* __restrict__ Xb, int64_t ldb, int square0, int square1) {
-    const int b = blockIdx.z;
-    const int i0 = blockIdx.y * kST, j0 = blockIdx.x * kST;
-    const int err = *args.err;
-    if (err == 0 && tile_good(args, Tile{b, i0 / kOzRowsA, j0 / kOzRowsB})) return;
-    const bool lost = args.D == args.C && err != 0 && err != kNoPairs;
     __shared__ double As[kSK][kST + 1];
     __shared__ double Bs[kSK][kST + 1];
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const bool sq = (b == 0 ? square0 : square1) != 0;
-    const double* A = Xa + b * xa_stride;
-    double acc[4][4] = {};
-    for (int k0 = 0; k0 < args.K; k0 += kSK) {
-#pragma unroll
-        for (int l = 0; l < (kST * kSK) / kSThreads; ++l) {
-            const int t = tid + l * kSThreads, r = t / kSK, k = t % kSK;
-            const bool kin = k0 + k < args.K;
-            As[k][r] = (kin && i0 + r < args.Ma) ? A[static_cast<int64_t>(i0 + r) * lda + k0 + k] : 0.0;
-            const double v = (kin && j0 + r < args.Nb) ? Xb[static_cast<int64_t>(j0 + r) * ldb + k0 + k] : 0.0;
-            Bs[k][r] = sq ? mul_rn(v, v) : v;
+    __shared__ int list[kSThreads], before[kSThreads / 32 + 1];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tx = tid & 15, ty = tid >> 4;
+    const int err = args.err[0];
+    if (err == 0 && args.err[1] == 0) return;
+    const bool lost = args.D == args.C && err != 0 && err != kNoPairs;
+    const int per = args.tiles_i * args.tiles_m, total = args.batches * per;
+    int64_t part = blockIdx.x;  // the block's next part, from the first of the tiles listed on
+    for (int t0 = 0; t0 < total; t0 += kSThreads) {
+        const int t = t0 + tid, in = t % per;
+        const bool bad = t < total && (err != 0 || !tile_good(args, Tile{t / per, in / args.tiles_m, in % args.tiles_m}));
+        const unsigned mask = __ballot_sync(0xffffffffu, bad);
+        if (lane == 0) before[warp + 1] = __popc(mask);
+        __syncthreads();
+        if (tid == 0) {
+            before[0] = 0;
+            for (int w = 1; w <= kSThreads / 32; ++w) before[w] += before[w - 1];
         }
         __syncthreads();
-#pragma unroll
-        for (int k = 0; k < kSK; ++k) {
-            double a[4], v[4];
-#pragma unroll
-            for (int r = 0; r < 4; ++r) a[r] = As[k][ty + 16 * r];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) v[c] = Bs[k][tx + 16 * c];
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-#pragma unroll
-                for (int c = 0; c < 4; ++c) acc[r][c] = fma(a[r], v[c], acc[r][c]);
-        }
+        if (bad) list[before[warp] + __popc(mask & ((1u << lane) - 1u))] = t;
+        const int parts = before[kSThreads / 32] * kSubs;
         __syncthreads();
-    }
+        for (; part < parts; part += gridDim.x) {
+            const int tile = list[part / kSubs], sub = static_cast<int>(part % kSubs), rem = tile % per, b = tile / per;
+            const int i0 = rem / args.tiles_m * kOzRowsA + sub / (kOzRowsB / kST) * kST;
+            const int j0 = rem % args.tiles_m * kOzRowsB + sub % (kOzRowsB / kST) * kST;
+            if (i0 >= args.Ma || j0 >= args.Nb) continue;
+            const bool sq = (b == 0 ? square0 : square1) != 0;
+            const double* a = Xa + b * xa_stride + static_cast<int64_t>(i0 + ty) * lda;
+            const double* x = Xb + static_cast<int64_t>(j0 + ty) * ldb;
+            double acc = 0.0;
+            for (int k0 = 0; k0 < args.K; k0 += kSK) {
+                const bool kin = k0 + tx < args.K;
+                As[tx][ty] = (kin && i0 + ty < args.Ma) ? a[k0 + tx] : 0.0;
+                const double v = (kin && j0 + ty < args.Nb) ? x[k0 + tx] : 0.0;
+                Bs[tx][ty] = sq ? mul_rn(v, v) : v;
+                __syncthreads();
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const int i = i0 + ty + 16 * r;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const int j = j0 + tx + 16 * c;
+                for (int k = 0; k < kSK; ++k) acc = fma(As[k][ty], Bs[k][tx], acc);
+                __syncthreads();
+            }
+            const int i = i0 + ty, j = j0 + tx;
             if (i < args.Ma && j < args.Nb) {
-                double* o = args.C + b * args.c_stride + static_cast<int64_t>(i) * args.ldc + j;
-                const double v = args.D ? args.D[static_cast<int64_t>(i) * args.ldd + j] - acc[r][c] : acc[r][c];
-                *o = lost ? NAN : v;
+                const double v = args.D ? args.D[static_cast<int64_t>(i) * args.ldd + j] - acc : acc;
+                args.C[b * args.c_stride + static_cast<int64_t>(i) * args.ldc + j] = lost ? NAN : v;
             }
         }
+        part -= parts;
+        __syncthreads();  // the list is read
     }
 }
 
@@ -556,7 +566,7 @@ size_t oz_operand_bytes(int rows, int K, int batches, int tile_rows) {
     const size_t ldp = (static_cast<size_t>(K) + kBK - 1) / kBK * kRowElems, n = static_cast<size_t>(rows) * batches;
     const size_t tiles = static_cast<size_t>((rows + tile_rows - 1) / tile_rows) * batches;
     return align_up(sizeof(__half) * n * ldp) + align_up(sizeof(int) * n) + align_up(sizeof(float) * n) +
-           align_up(sizeof(float) * (tiles + 1));
+           align_up(sizeof(float) * (tiles + 2));
 }
 
 OzOperand oz_carve(void* base, int rows, int K, int batches, int tile_rows) {
@@ -647,7 +657,11 @@ int oz_gemm(const OzOperand& A, const OzOperand& B, const OzProduct& p, cudaStre
     } else {
         FLMM_CUDA(cudaMemsetAsync(a.err, kNoPairs & 0xff, sizeof(int), st));
     }
-    const dim3 grid(ceil_div(B.rows, kST), ceil_div(A.rows, kST), a.batches);
+    int sms = 0;
+    if ((rc = sm_count(&sms))) return rc;
+    // (two blocks an SM: eight take 3 us longer to find that there is nothing to do)
+    const int64_t parts = static_cast<int64_t>(a.batches) * a.tiles_i * a.tiles_m * kSubs;
+    const int grid = static_cast<int>(std::min<int64_t>(int64_t{2} * sms, parts));
     k_marked_f64<<<grid, kSThreads, 0, st>>>(a, p.Xa, p.lda, p.xa_stride, p.Xb, p.ldb, p.square[0], p.square[1]);
     return check_launch("k_marked_f64");
 }

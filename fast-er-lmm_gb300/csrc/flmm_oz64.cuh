@@ -20,7 +20,8 @@ struct OzOperand {
     int* expo;        // [batch][row]
     float* mean;      // [batch][row]: mean |x| over 2^expo
     float* qual;      // [batch][tile]: largest quality of a tile's rows (oz_digits), infinity where digits cannot hold a row
-    int* err;         // of an operand A: set once a product with it gave up a wait; zeroed with its batch 0's digits
+    int* err;         // of an operand A: [0] set once a product with it gave up a wait, [1] once one had tiles that digits
+                      // do not hold; zeroed with its batch 0's digits
     int64_t ldp;
     int rows, K, batches, tile_rows;
     int tiles() const { return (rows + tile_rows - 1) / tile_rows; }
