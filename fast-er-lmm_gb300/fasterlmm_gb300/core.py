@@ -132,10 +132,15 @@ def transpose(A: Tensor) -> Tensor:
     return out
 
 
+def _pitched(rows: Tensor) -> Tensor:
+    """Contiguous rows with a pitch that the library takes: of a single row torch allows any."""
+    return rows if rows.shape[0] != 1 else rows.as_strided(rows.shape, (rows.shape[1], 1))
+
+
 def _rows_major(Z: Tensor) -> Tensor:
     """(N, M) matrix -> (M, N) contiguous variant-major copy (free when Z is already a transposed view)."""
     if Z.T.is_contiguous():
-        return Z.T
+        return _pitched(Z.T)
     return transpose(Z)
 
 

@@ -19,7 +19,7 @@ import torch
 from torch import Tensor
 
 from . import _lib
-from .core import (F64, ScanResult, _alloc_outputs, _chrom_blocks, _cuda_device, _f64, _ptr, _rows_major, _stream,
+from .core import (F64, ScanResult, _alloc_outputs, _chrom_blocks, _cuda_device, _f64, _pitched, _ptr, _rows_major, _stream,
                    _take_rows, _to_device, _work, eigh_each, eigh_many, gram_t, kinship_from_gram, rotate_rows,
                    rotate_variants, transpose)
 
@@ -44,7 +44,9 @@ class Spectrum:
 
 def _rows(view: Tensor, rows: Tensor | None, dev: torch.device) -> Tensor:
     """Row-major transpose of an (N, k) view: the stored rows when given, else a transposed copy."""
-    return rows if rows is not None else transpose(_f64(view, dev, contiguous=False))
+    if rows is None:
+        return transpose(_f64(view, dev, contiguous=False))
+    return _pitched(rows) if rows.is_contiguous() else rows
 
 
 def _spectrum_rows(spec: Spectrum, dev: torch.device) -> tuple[Tensor, Tensor, Tensor]:

@@ -103,3 +103,28 @@ def test_gls_rejects_too_many_covariates():
     spec = gls.rotate(_t((Z @ Z.T).numpy() / 40), _t(X.numpy()), _t(torch.randn(N, 2, generator=g, dtype=torch.float64).numpy()))
     with pytest.raises(_lib.FlmmError):
         gls.fit_delta_grid(spec)
+
+
+@pytest.mark.parametrize("C,P,M", [(1, 3, 5), (2, 1, 5), (2, 3, 1), (1, 1, 1)])
+def test_single_columns_of_any_stride(C, P, M):
+    """One covariate, phenotype or variant: a single row is contiguous to torch whatever its stride says."""
+    from fasterlmm_gb300 import core, gls
+    rng = np.random.default_rng(C * 10 + P)
+    N = 40
+    s, X, Y, S, ld = (rng.standard_normal(n) for n in ((N,), (N, C), (N, P), (N, M), (P,)))
+    s, row = np.abs(s) + 0.1, lambda a: _t(a).T.contiguous()
+    spec = gls.Spectrum(s=_t(s), U=None, X_rot=_t(X), Y_rot=_t(Y), Xrt=row(X), Yrt=row(Y))
+    res = _np(gls.snp_wald_scan(spec, _t(ld), _t(S)))
+    w = 1 / (s[:, None] + np.exp(ld))
+    for p in range(P):
+        A = (X * w[:, p:p + 1]).T @ X
+        r = Y[:, p] - X @ np.linalg.solve(A, X.T @ (w[:, p] * Y[:, p]))
+        B = (X * w[:, p:p + 1]).T @ S
+        den = w[:, p] @ (S * S) - (B * np.linalg.solve(A, B)).sum(0)
+        np.testing.assert_allclose(res["beta"][:, p], (w[:, p] * r) @ S / den, rtol=1e-9)
+    Q = np.linalg.qr(rng.standard_normal((N, N)))[0]
+    K = (Q * np.linspace(0.1, 2, N)) @ Q.T
+    Xc = np.c_[np.ones(N), X[:, 1:]]
+    cs = core.fastlmm_compat_rotate(_t(K), _t(Xc), _t(Y))
+    one, wide = core.snp_wald_scan_compat(cs, _t(ld), _t(S)), core.snp_wald_scan_compat(cs, _t(ld), _t(np.c_[S, S]))
+    np.testing.assert_array_equal(_np(one)["f"], _np(wide)["f"][:M])
