@@ -719,6 +719,7 @@ __global__ void k_clamp_nonneg(const double* __restrict__ x, int64_t n, double* 
     if (i < n) y[i] = fmax(x[i], 0.0);
 }
 
+// (the kernels' limit is that of kMaxGlsC whatever the call's C: another host thread's call must not lower it)
 size_t eval_smem_bytes(int C) {
     return sizeof(double) * kEvalWarps *
            (static_cast<size_t>(C + 1) * (C + 1) + static_cast<size_t>(C) * C + (C + 1));
@@ -749,8 +750,8 @@ extern "C" int flmm_gls_loss_f64(const double* s, int N, const double* Xrt, int6
     const size_t smem = eval_smem_bytes(C);
     if (per_column) {
         FLMM_REQUIRE(n_ld == P, "flmm_gls_loss_f64: per-column mode needs one log delta per column");
-        if (smem > 48 * 1024)
-            FLMM_CUDA(cudaFuncSetAttribute(k_gls_pheno_loss, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        FLMM_CUDA(cudaFuncSetAttribute(k_gls_pheno_loss, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)eval_smem_bytes(kMaxGlsC)));
         k_gls_pheno_loss<<<ceil_div(P, kEvalWarps), 32 * kEvalWarps, smem, st>>>(s, N, Xrt, ldx, C, Yrt, ldy, P,
                                                                                   log_delta, reml, loss);
         return check_launch("k_gls_pheno_loss");
@@ -805,8 +806,8 @@ extern "C" int flmm_fit_delta_gls_f64(const double* s, int N, const double* Xrt,
         return check_launch("k_gls_golden_block");
     }
     const size_t smem = eval_smem_bytes(C);
-    if (smem > 48 * 1024)
-        FLMM_CUDA(cudaFuncSetAttribute(k_gls_golden, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    FLMM_CUDA(cudaFuncSetAttribute(k_gls_golden, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)eval_smem_bytes(kMaxGlsC)));
     k_gls_golden<<<ceil_div(P, kEvalWarps), 32 * kEvalWarps, smem, st>>>(s, N, Xrt, ldx, C, Yrt, ldy, P, ws.grid,
                                                                           n_grid, grid_idx, refine, reml, lo, hi,
                                                                           log_delta);

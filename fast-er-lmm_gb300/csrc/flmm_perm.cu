@@ -211,9 +211,9 @@ extern "C" int flmm_perm_orders(const int64_t* seed_cols, int B, uint64_t seed, 
                                                                                 orders);
         return check_launch("k_perm_orders_packed");
     }
-    const size_t smem = static_cast<size_t>(npow2) * (sizeof(uint64_t) + sizeof(int32_t));
-    if (smem > 48 * 1024)
-        FLMM_CUDA(cudaFuncSetAttribute(k_perm_orders, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    const size_t entry = sizeof(uint64_t) + sizeof(int32_t), smem = static_cast<size_t>(npow2) * entry;
+    // (one bound whatever N: another host thread's call must not lower it under this launch)
+    FLMM_CUDA(cudaFuncSetAttribute(k_perm_orders, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(16384 * entry)));
     k_perm_orders<<<B * n_perm, kThreads, smem, as_stream(stream)>>>(seed_cols, seed, n_perm, N, npow2, orders);
     return check_launch("k_perm_orders");
 }

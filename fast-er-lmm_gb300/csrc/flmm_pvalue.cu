@@ -149,8 +149,8 @@ extern "C" int flmm_perm_threshold_p(const double* perm_max_F, int B, int n_perm
     int npow2 = 1;
     while (npow2 < n_perm) npow2 <<= 1;
     const size_t smem = sizeof(double) * npow2;
-    if (smem > 48 * 1024)
-        FLMM_CUDA(cudaFuncSetAttribute(k_perm_threshold, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    // (one bound whatever n_perm: another host thread's call must not lower it under this launch)
+    FLMM_CUDA(cudaFuncSetAttribute(k_perm_threshold, cudaFuncAttributeMaxDynamicSharedMemorySize, 16384 * sizeof(double)));
     k_perm_threshold<<<B, 256, smem, as_stream(stream)>>>(perm_max_F, B, n_perm, npow2, tail_of(df2), q, thresh);
     return check_launch("k_perm_threshold");
 }

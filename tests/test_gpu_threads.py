@@ -52,8 +52,24 @@ def _gls_fit(N, ctx, dev):
                              _ptr(idx), _ptr(work), nbytes, _stream(dev)), (s, X, Y, ld, idx, work)
 
 
+def _perm_orders(N, ctx, dev):
+    from fasterlmm_gb300 import _lib
+    from fasterlmm_gb300.core import _ptr, _stream
+    cols, out = torch.zeros(1, dtype=torch.int64, device=dev), torch.empty(N, dtype=torch.int32, device=dev)
+    return lambda: _lib.call("flmm_perm_orders", _ptr(cols), 1, 1, 1, N, _ptr(out), _stream(dev)), (cols, out)
+
+
+def _perm_threshold(n, ctx, dev):
+    from fasterlmm_gb300 import _lib
+    from fasterlmm_gb300.core import _ptr, _stream
+    F, out = torch.rand(n, dtype=torch.float64, device=dev), torch.empty(1, dtype=torch.float64, device=dev)
+    return lambda: _lib.call("flmm_perm_threshold_p", _ptr(F), 1, n, 100, 0.05, _ptr(out), _stream(dev)), (F, out)
+
+
 @pytest.mark.parametrize("make,sizes,calls", [(_eigh, (64, 1000), 400), (_eigh, (1320, 1600), 60),
-                                              (_prep_variants, (11_000, 50_000), 2000), (_gls_fit, (3200, 9000), 1000)])
+                                              (_prep_variants, (11_000, 50_000), 2000), (_gls_fit, (3200, 9000), 1000),
+                                              (_perm_orders, (5000, 16_384), 1000),
+                                              (_perm_threshold, (7000, 16_384), 1000)])
 def test_two_sizes_at_once(make, sizes, calls):
     from fasterlmm_gb300 import _lib, build
     build()
